@@ -1048,8 +1048,9 @@ int32_t fvg_kernels_per_step(const fvg_handle* h) {
   n += 1 + 1 + 1 + 1 + 2 + 1;                              // adjust2, vertvl x2, w/viscofh, grad3+adv_uv, vdif_uv
   n += 7;                                                  // grad_q, adv_q (2 phases), vdif_q (4 passes)
   if (h->P.closure) n += 3;                                // learned closure (compaction x2, network)
-  if (p.temperature_active || p.salinity_active)           // grad_ts, adv_ts (2 phases), vdif_ts,
-    n += 5 + (h->P.iobcn > 0 ? 1 : 0);                     // bcond_ts (rivers, open boundary)
+  if (p.temperature_active || p.salinity_active)           // grad_ts, adv_ts (2 phases and the open
+    n += 4 + (h->P.iobcn > 0 ? 2 : 0) + (h->P.numqbc > 0 ? 1 : 0);  // boundary), vdif_ts, bcond_ts (rivers,
+                                                           // open boundary)
   n += 1;                                                  // final
   return n;
 }

@@ -452,6 +452,18 @@ __device__ inline double obc_xflux_adv(const Dev& P, int i, int k, int t) {
   return (double)xa;
 }
 
+// XFLUX_OBC of every open-boundary node, layer and tracer (adv_t.F:572-579), one thread
+// each (blockIdx.y: the layer, blockIdx.z: the tracer).  The recomputation is a long chain
+// for few nodes: inside the node gather it held every block with an open-boundary node
+// back and cost all of them its registers (102 against 64-78).
+template <typename R>
+__global__ void __launch_bounds__(64) k_obc_xflux(const Dev P, int parts) {
+  const int ob = blockIdx.x * blockDim.x + threadIdx.x + 1, k = blockIdx.y + 1, t = blockIdx.z;
+  if (ob > P.iobcn || !(parts & (t == 0 ? AD_T : AD_S))) return;
+  (t == 0 ? P.xflux_obc_t : P.xflux_obc_s)[(size_t)(k - 1) * (P.iobcn + 1) + ob] =
+      obc_xflux_adv<R>(P, P.i_obc_n[ob], k, t);
+}
+
 // Signed sum of a node's half-edge fluxes on layer k, both tracers, in ascending
 // half-edge order (the order of the reference's scatter into XFLUX).
 // The loads are issued four entries at a time (codes, then fluxes) and added in order.
@@ -880,7 +892,6 @@ __global__ void __launch_bounds__(256) k_gather_ts(const Dev P, int parts) {
   int kb, ke;
   col_range(P, 1, P.KBM1, kb, ke);
   const bool wet = P.iswetn[i] * P.iswetnt[i] == 1;
-  const int ob = P.node_obc[i];
   const int nhe = P.node_he_ptr[i + 1] - P.node_he_ptr[i];
   for (int k = kb; k <= ke; ++k) {
   const double2 xs = gather_he<R>(P, i, nhe, k);
@@ -889,7 +900,6 @@ __global__ void __launch_bounds__(256) k_gather_ts(const Dev P, int parts) {
     const double* F1 = (t == 0 ? P.t1 : P.s1);
     double* FF1 = (t == 0 ? P.tf1 : P.sf1);
     double x = t == 0 ? xs.x : xs.y;
-    if (ob > 0) (t == 0 ? P.xflux_obc_t : P.xflux_obc_s)[(size_t)(k - 1) * (P.iobcn + 1) + ob] = obc_xflux_adv<R>(P, i, k, t);
     size_t q = N3(P, i, k);
     double ff;
     if (wet) {
@@ -1065,85 +1075,90 @@ __global__ void __launch_bounds__(128) k_vdif_ts(const Dev P, int parts) {
 // -------------------------------------------------------------------------------------
 // BCOND_TS(1) and BCOND_TS(2) (bcond_ts.F:60-262): river nodes take the river T/S; open
 // boundary nodes take the outflow estimate with the radiation perturbation of
-// OBC_TS_TYPE and the neighbour clamp, or keep T1/S1 on inflow.  One block.
+// OBC_TS_TYPE and the neighbour clamp, or keep T1/S1 on inflow.
 // -------------------------------------------------------------------------------------
+// One block per layer, its threads over the rivers.
 __global__ void k_bcond_ts_riv(const Dev P) {
-  const int KBM1 = P.KBM1;
+  const int k = blockIdx.x + 1;
   for (int r = threadIdx.x + 1; r <= P.numqbc; r += blockDim.x) {
     int n1 = P.river_location == 0 ? P.inodeq[r] : P.n_icellq[r];
     int n2 = P.river_location == 0 ? 0 : P.n_icellq[(size_t)(P.numqbc + 1) + r];
-    for (int k = 1; k <= KBM1; ++k) {
-      P.tf1[N3(P, n1, k)] = P.tdis[r];
-      P.sf1[N3(P, n1, k)] = P.sdis[r];
-      if (n2 > 0) {
-        P.tf1[N3(P, n2, k)] = P.tdis[r];
-        P.sf1[N3(P, n2, k)] = P.sdis[r];
-      }
+    P.tf1[N3(P, n1, k)] = P.tdis[r];
+    P.sf1[N3(P, n1, k)] = P.sdis[r];
+    if (n2 > 0) {
+      P.tf1[N3(P, n2, k)] = P.tdis[r];
+      P.sf1[N3(P, n2, k)] = P.sdis[r];
     }
   }
 }
 
-// Open-boundary part: one thread per (open-boundary node, tracer).  The nodes are
-// independent: each reads the old field, its own XFLUX_OBC and TF1/SF1 of its interior
-// neighbour NEXT_OBC, which is not an open-boundary node.
-__global__ void k_bcond_ts_obc(const Dev P, int parts) {
+// Open-boundary part: one block per (open-boundary node, tracer), one thread per layer.
+// The nodes are independent: each reads the old field, its own XFLUX_OBC and TF1/SF1 of
+// its interior neighbour NEXT_OBC, which is not an open-boundary node.  Only the three
+// depth sums are sequential: the layers' terms go through shared memory and three threads
+// add them in layer order, one sum each.
+__global__ void __launch_bounds__(64) k_bcond_ts_obc(const Dev P, int parts) {
+  __shared__ double term[3][64];
+  __shared__ double sum[3];
   const int KBM1 = P.KBM1;
-  const int id = blockIdx.x * blockDim.x + threadIdx.x;
-  const int ob = id / 2 + 1, t = id % 2;
-  if (ob > P.iobcn) return;
-  {
-    int j = P.i_obc_n[ob], j1 = P.next_obc[ob];
-    {
-      if (!(parts & (t == 0 ? AD_T : AD_S))) return;
-      const double* F1 = t == 0 ? P.t1 : P.s1;
-      double* FF1 = t == 0 ? P.tf1 : P.sf1;
-      const double* XO = t == 0 ? P.xflux_obc_t : P.xflux_obc_s;
-      double t2d = 0.0, t2dn = 0.0, xf2d = 0.0;
-      for (int k = 1; k <= KBM1; ++k) {
-        t2d = t2d + F1[N3(P, j, k)] * P.dz[N3(P, j, k)];
-        t2dn = t2dn + FF1[N3(P, j1, k)] * P.dz[N3(P, j1, k)];
-        xf2d = xf2d + XO[(size_t)(k - 1) * (P.iobcn + 1) + ob];
-      }
-      if (P.uard_obcn[ob] > 0.0) {
-        double tmp = xf2d + t2d * P.uard_obcn[ob];
-        double t2d_obc = (t2d * P.dt[j] - tmp * P.dti / P.art1[j]) / P.d[j];
-        double cc = 0.0, cp = 1.0;
-        if (P.obc_ts_type != 1) {
-          cc = sqrt(P.grav_n[j] * P.h[j]) * P.dti / P.dltn_obc[ob];
-          cp = cc + 1.0;
-        }
-        for (int k = 1; k <= KBM1; ++k) {
-          double ttmp;
-          double pert_next = FF1[N3(P, j1, k)] - t2dn;
-          if (P.obc_ts_type == 1) {
-            ttmp = pert_next;
-          } else if (P.obc_ts_type == 2) {
-            double pert = F1[N3(P, j, k)] - t2d;
-            ttmp = (cc * pert_next + pert) / cp;
-          } else {
-            double pert = F1[N3(P, j, k)] - t2d;
-            ttmp = (cc * pert_next + pert * (1.0 - P.dti / 10800.0)) / cp;
-          }
-          FF1[N3(P, j, k)] = t2d_obc + ttmp;
-        }
-        for (int k = 1; k <= KBM1; ++k) {
-          double fmx = F1[N3(P, NBSN(P, j, 1), k)], fmn = fmx;
-          for (int jj = 2; jj <= P.ntsn[j]; ++jj) {
-            double v = F1[N3(P, NBSN(P, j, jj), k)];
-            fmx = fmax(fmx, v);
-            fmn = fmin(fmn, v);
-          }
-          fct_layer_bounds(P, j, k, F1, fmx, fmn);
-          double ff = FF1[N3(P, j, k)];
-          if (fmn - ff > 0.0) ff = fmn;
-          if (ff - fmx > 0.0) ff = fmx;
-          FF1[N3(P, j, k)] = ff;
-        }
-      } else {
-        for (int k = 1; k <= KBM1; ++k) FF1[N3(P, j, k)] = F1[N3(P, j, k)];
-      }
-    }
+  const int ob = blockIdx.x + 1, t = blockIdx.y, k = threadIdx.x + 1;
+  if (!(parts & (t == 0 ? AD_T : AD_S))) return;
+  const int j = P.i_obc_n[ob], j1 = P.next_obc[ob];
+  const double* F1 = t == 0 ? P.t1 : P.s1;
+  double* FF1 = t == 0 ? P.tf1 : P.sf1;
+  const double* XO = t == 0 ? P.xflux_obc_t : P.xflux_obc_s;
+  const bool live = k <= KBM1;
+  const size_t q = N3(P, j, k), q1 = N3(P, j1, k);
+  if (!(P.uard_obcn[ob] > 0.0)) {
+    if (live) FF1[q] = F1[q];
+    return;
   }
+  double f1 = 0.0, fnext = 0.0;
+  if (live) {
+    f1 = F1[q];
+    fnext = FF1[q1];
+    term[0][k - 1] = f1 * P.dz[q];
+    term[1][k - 1] = fnext * P.dz[q1];
+    term[2][k - 1] = XO[(size_t)(k - 1) * (P.iobcn + 1) + ob];
+  }
+  __syncthreads();
+  if (threadIdx.x < 3) {
+    double s = 0.0;
+    for (int l = 0; l < KBM1; ++l) s = s + term[threadIdx.x][l];
+    sum[threadIdx.x] = s;
+  }
+  __syncthreads();
+  if (!live) return;
+  const double t2d = sum[0], t2dn = sum[1], xf2d = sum[2];
+  const double tmp = xf2d + t2d * P.uard_obcn[ob];
+  const double t2d_obc = (t2d * P.dt[j] - tmp * P.dti / P.art1[j]) / P.d[j];
+  double cc = 0.0, cp = 1.0;
+  if (P.obc_ts_type != 1) {
+    cc = sqrt(P.grav_n[j] * P.h[j]) * P.dti / P.dltn_obc[ob];
+    cp = cc + 1.0;
+  }
+  double ttmp;
+  const double pert_next = fnext - t2dn;
+  if (P.obc_ts_type == 1) {
+    ttmp = pert_next;
+  } else if (P.obc_ts_type == 2) {
+    const double pert = f1 - t2d;
+    ttmp = (cc * pert_next + pert) / cp;
+  } else {
+    const double pert = f1 - t2d;
+    ttmp = (cc * pert_next + pert * (1.0 - P.dti / 10800.0)) / cp;
+  }
+  double ff = t2d_obc + ttmp;
+  double fmx = F1[N3(P, NBSN(P, j, 1), k)], fmn = fmx;
+  for (int jj = 2; jj <= P.ntsn[j]; ++jj) {
+    const double v = F1[N3(P, NBSN(P, j, jj), k)];
+    fmx = fmax(fmx, v);
+    fmn = fmin(fmn, v);
+  }
+  fct_layer_bounds(P, j, k, F1, fmx, fmn);
+  if (fmn - ff > 0.0) ff = fmn;
+  if (ff - fmx > 0.0) ff = fmx;
+  FF1[q] = ff;
 }
 
 // DENS2_2D (eqs_of_state.F:290-319), same operation order.
@@ -1268,6 +1283,7 @@ void launch_turb_update(const Dev& P, cudaStream_t s) {
 void launch_adv_ts(const Dev& P, cudaStream_t s, int parts) {
   FVG_F32_FORWARD(launch_adv_ts(P, s, parts));
   k_he_adv<RF, 1><<<col_grid(P, P.N, P.KBM1), P.col_bc, 0, s>>>(P, parts);
+  if (P.iobcn > 0) k_obc_xflux<RF><<<dim3(nblk(P.iobcn, 64), P.KBM1, 2), 64, 0, s>>>(P, parts);
   k_gather_ts<RF><<<col_grid(P, P.M, P.KBM1), P.col_bc, 0, s>>>(P, parts);
 }
 void launch_fct_ts(const Dev& P, cudaStream_t s, int parts) {
@@ -1281,8 +1297,8 @@ void launch_vdif_ts(const Dev& P, cudaStream_t s, int parts) {
     k_vdif_ts<false><<<dim3(nblk(P.M, 128), 2), 128, 0, s>>>(P, parts);
 }
 void launch_bcond_ts(const Dev& P, cudaStream_t s, int parts) {
-  k_bcond_ts_riv<<<1, 128, 0, s>>>(P);
-  if (P.iobcn > 0) k_bcond_ts_obc<<<nblk(2 * P.iobcn, 64), 64, 0, s>>>(P, parts);
+  if (P.numqbc > 0) k_bcond_ts_riv<<<P.KBM1, 128, 0, s>>>(P);
+  if (P.iobcn > 0) k_bcond_ts_obc<<<dim3(P.iobcn, 2), 64, 0, s>>>(P, parts);
 }
 void launch_final(const Dev& P, cudaStream_t s, int parts) {
   int n = (P.M > P.N ? P.M : P.N) + 1;
