@@ -304,6 +304,8 @@ int fvg_closure_status(fvg_handle* h, int32_t* columns_on_network, int32_t* wait
 /* Launch shape of the 3-D gather kernels (results do not depend on it):
    "col_threads" = entities (threads) per block, 32..256 in steps of 32 (default 128);
    "col_layers"  = consecutive layers each thread walks, 1..KB (default 8);
+                   until one of the two is set, a launch that would not fill the chip
+                   takes fewer layers per thread, then fewer threads per block;
    "compact"     = 1 (default) lets the precision form's Runge-Kutta stages use the
                    compact cell kernel where fvg_set_precision found the mesh's edge metrics
                    to be the ones its coordinates define; 0 keeps the general kernel.

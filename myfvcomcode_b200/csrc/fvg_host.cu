@@ -399,6 +399,7 @@ int fvg_create(const fvg_mesh* m, const fvg_params* prm, const fvg_forcing* f, f
       P.nsm = 148;
   }
   P.col_lc = 8;
+  P.col_auto = 1;
   P.prec = FVG_PREC_FP64;
   P.nbsn_cols = m->nbsn_cols; P.nbve_cols = m->nbve_cols; P.trie_cols = m->trie_cols;
   P.iobcn = m->iobcn; P.numqbc = m->numqbc;
@@ -1287,9 +1288,11 @@ int fvg_set_tuning(fvg_handle* h, const char* key, int32_t value) {
   if (k == "col_threads") {
     if (value < 32 || value > 256 || value % 32 != 0) { h->err = "col_threads must be 32..256, a multiple of 32"; return FVG_ERR_ARG; }
     h->P.col_bc = value;
+    h->P.col_auto = 0;
   } else if (k == "col_layers") {
     if (value < 1 || value > h->P.KB) { h->err = "col_layers must be 1..KB"; return FVG_ERR_ARG; }
     h->P.col_lc = value;
+    h->P.col_auto = 0;
   } else if (k == "staged") {
     if (value < 0 || value > 2) { h->err = "staged must be 0, 1 or 2"; return FVG_ERR_ARG; }
     h->P.staged = value;

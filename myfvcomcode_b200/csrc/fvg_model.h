@@ -253,7 +253,9 @@ struct Dev {
   // Column tiling of the 3-D gather kernels: col_bc threads (entities) per block, each
   // walking col_lc consecutive layers, so the entity's index chain (cell -> edge ->
   // neighbour) is resolved from cache after the first layer.  Results do not depend on it.
-  int col_bc, col_lc;
+  // col_auto: the shape is the default one, which launches shrink where the mesh is small
+  // (col_shape); 0 once a tuning key has set it.
+  int col_bc, col_lc, col_auto;
   // 1: the external loop's stage kernels load what a stage reads once evict-first (ld1),
   // so that the arrays gathered from neighbours stay in L2 between stages (tuning key
   // "stream_hints"); results do not depend on it.
@@ -264,7 +266,30 @@ struct Dev {
   int ext_grid, nsm;
 };
 
-// Grid of a column-tiled kernel over n entities and nl layers.
+// Threads per block of a kernel with one thread per entity: `most`, or fewer (down to one
+// warp) where blocks of `most` would leave SMs without a block.  A small mesh's kernel is
+// a chain of dependent loads, and warps alone on their SMs run it fastest.
+inline int col_threads(const Dev& P, long n, int most) {
+  int b = most;
+  while (b > 32 && (n + b - 1) / b < P.nsm) b >>= 1;
+  return b;
+}
+// The launch shape of a column-tiled kernel over n entities and nl layers: the default
+// shape (col_bc threads, each walking col_lc layers) amortises the entity's index chain
+// over its layers, but a thread then runs that many layers one after the other, which is
+// the whole time of a kernel that does not fill the chip.  Below about four blocks per SM
+// the chunk is halved until there are, then the block.
+inline Dev col_shape(const Dev& P, int n, int nl) {
+  Dev Q = P;
+  if (!P.col_auto) return Q;
+  const long want = 4L * P.nsm;
+  while (Q.col_lc > 1 && (long)((n + Q.col_bc - 1) / Q.col_bc) * ((nl + Q.col_lc - 1) / Q.col_lc) < want)
+    Q.col_lc = (Q.col_lc + 1) / 2;
+  while (Q.col_bc > 32 && (long)((n + Q.col_bc - 1) / Q.col_bc) * ((nl + Q.col_lc - 1) / Q.col_lc) < P.nsm)
+    Q.col_bc >>= 1;
+  return Q;
+}
+// Grid of a column-tiled kernel over n entities and nl layers (P as col_shape returned it).
 inline dim3 col_grid(const Dev& P, int n, int nl) {
   return dim3((unsigned)((n + P.col_bc - 1) / P.col_bc), (unsigned)((nl + P.col_lc - 1) / P.col_lc));
 }

@@ -867,7 +867,8 @@ static inline int nblk(int n, int b) { return (n + b - 1) / b; }
 
 void launch_ext_node(const Dev& P, cudaStream_t s, int iext, int K, int parts, int pdl) {
   const int n = (parts & EN_GRAD) ? P.M + P.N : P.M;
-  launch_maybe_pdl(pdl, P.ldcs ? k_ext_node<true> : k_ext_node<false>, dim3(nblk(n, 256)), dim3(256), s, P, iext, K,
+  const int b = col_threads(P, n, 256);
+  launch_maybe_pdl(pdl, P.ldcs ? k_ext_node<true> : k_ext_node<false>, dim3(nblk(n, b)), dim3(b), s, P, iext, K,
                    parts);
 }
 void launch_ext_prep(const Dev& P, cudaStream_t s) { k_ext_prep<<<nblk(P.N, 256), 256, 0, s>>>(P); }
@@ -988,26 +989,28 @@ void launch_wet_judge(const Dev& P, cudaStream_t s) {
   k_wet_nodes<<<nblk(P.M, 256), 256, 0, s>>>(P);
 }
 void launch_wet_cells(const Dev& P, cudaStream_t s, int pdl) {
-  launch_maybe_pdl(pdl, P.ldcs ? k_wet_cells<true> : k_wet_cells<false>, dim3(nblk(P.N, 256)), dim3(256), s, P);
+  const int b = col_threads(P, P.N, 256);
+  launch_maybe_pdl(pdl, P.ldcs ? k_wet_cells<true> : k_wet_cells<false>, dim3(nblk(P.N, b)), dim3(b), s, P);
 }
 void launch_ext_cell(const Dev& P, cudaStream_t s, int iext, int K, int parts, int pdl) {
   FVG_F32_FORWARD(launch_ext_cell(P, s, iext, K, parts, pdl));
   void (*k)(const Dev, int, int, int);
 #ifdef FVG_F32_TU
   if ((parts & EC_COMPACT) && P.f.compact && !P.limiter && !P.gcy) {
-    const int nb = nblk(P.N, 128);
+    const int b = col_threads(P, P.N, 128), nb = nblk(P.N, b);
     if (P.ext_grid > 0 && nb > P.ext_grid * P.nsm) {
       launch_maybe_pdl(pdl, P.ldcs ? k_ext_cell_c<true, true> : k_ext_cell_c<false, true>, dim3(P.ext_grid * P.nsm),
                        dim3(128), s, P, iext, K, parts);
     } else {
-      launch_maybe_pdl(pdl, P.ldcs ? k_ext_cell_c<true, false> : k_ext_cell_c<false, false>, dim3(nb), dim3(128), s,
+      launch_maybe_pdl(pdl, P.ldcs ? k_ext_cell_c<true, false> : k_ext_cell_c<false, false>, dim3(nb), dim3(b), s,
                        P, iext, K, parts);
     }
     return;
   }
 #endif
   k = P.limiter ? k_ext_cell<RF, true> : k_ext_cell<RF, false>;
-  launch_maybe_pdl(pdl, k, dim3(nblk(P.N, 128)), dim3(128), s, P, iext, K, parts);
+  const int b = col_threads(P, P.N, 128);
+  launch_maybe_pdl(pdl, k, dim3(nblk(P.N, b)), dim3(b), s, P, iext, K, parts);
 }
 void launch_ext_update(const Dev& P, cudaStream_t s, int K) {
   int n = P.M > P.N ? P.M : P.N;

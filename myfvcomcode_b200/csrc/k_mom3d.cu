@@ -1029,8 +1029,9 @@ constexpr int kStagedSmemMax = 200 * 1024;
 template <typename R, bool UV>
 static void launch_mom3d_staged(const Dev& P, cudaStream_t s) {
   const size_t smem = staged_smem_bytes<R, UV>(P.tl.cap_cells, P.tl.cap_edges);
-  const dim3 grid((unsigned)P.tl.n, (unsigned)((P.KBM1 + P.col_lc - 1) / P.col_lc));
-  k_mom3d_staged<R, UV><<<grid, kTileCells, smem, s>>>(P);
+  const Dev Q = col_shape(P, P.N, P.KBM1);
+  const dim3 grid((unsigned)P.tl.n, (unsigned)((P.KBM1 + Q.col_lc - 1) / Q.col_lc));
+  k_mom3d_staged<R, UV><<<grid, kTileCells, smem, s>>>(Q);
 }
 // Whether the staged kernel of ADVECTION (UV false) or ADV_UV (UV true) runs: LIMITED_NO,
 // GCN, a tile table whose shared memory fits one CTA, and P.staged = 2 (every staged
@@ -1197,14 +1198,17 @@ __global__ void __launch_bounds__(128) k_vdif_uv(const Dev P, int parts) {
 }
 
 void launch_cell_pre(const Dev& P, cudaStream_t s, int parts) {
-  k_cell_pre<<<nblk(P.N, 128), 128, 0, s>>>(P, parts);
+  const int b = col_threads(P, P.N, 128);
+  k_cell_pre<<<nblk(P.N, b), b, 0, s>>>(P, parts);
 }
 void launch_grad3(const Dev& P, cudaStream_t s) {
   FVG_F32_FORWARD(launch_grad3(P, s));
-  k_grad3<RF><<<col_grid(P, P.N, P.KBM1), P.col_bc, 0, s>>>(P);
+  const Dev Q = col_shape(P, P.N, P.KBM1);
+  k_grad3<RF><<<col_grid(Q, P.N, P.KBM1), Q.col_bc, 0, s>>>(Q);
 }
 static void launch_alfa3(const Dev& P, cudaStream_t s) {
-  k_alfa3<RF><<<col_grid(P, P.N, P.KBM1), P.col_bc, 0, s>>>(P);
+  const Dev Q = col_shape(P, P.N, P.KBM1);
+  k_alfa3<RF><<<col_grid(Q, P.N, P.KBM1), Q.col_bc, 0, s>>>(Q);
 }
 void launch_advection3d(const Dev& P, cudaStream_t s) {
   FVG_F32_FORWARD(launch_advection3d(P, s));
@@ -1213,7 +1217,8 @@ void launch_advection3d(const Dev& P, cudaStream_t s) {
     return;
   }
   if (P.limiter) launch_alfa3(P, s);
-  (P.limiter ? k_advection3d<RF, true> : k_advection3d<RF, false>)<<<col_grid(P, P.N, P.KBM1), P.col_bc, 0, s>>>(P);
+  const Dev Q = col_shape(P, P.N, P.KBM1);
+  (P.limiter ? k_advection3d<RF, true> : k_advection3d<RF, false>)<<<col_grid(Q, P.N, P.KBM1), Q.col_bc, 0, s>>>(Q);
 }
 // -------------------------------------------------------------------------------------
 // PHY_BAROPG (phy_baropg.F:37-151), BAROCLINIC_PRESSURE_GRADIENT = 'z coordinates'.
@@ -1345,27 +1350,34 @@ __global__ void __launch_bounds__(128) k_phy_baropg(const Dev P) {
 }
 
 void launch_phy_baropg(const Dev& P, cudaStream_t s) {
-  k_phy_rhoz<<<nblk(P.M, 128), 128, 0, s>>>(P);
-  k_phy_baropg<<<nblk(P.N, 128), 128, 0, s>>>(P);
+  const int bm = col_threads(P, P.M, 128), bn = col_threads(P, P.N, 128);
+  k_phy_rhoz<<<nblk(P.M, bm), bm, 0, s>>>(P);
+  k_phy_baropg<<<nblk(P.N, bn), bn, 0, s>>>(P);
 }
 
 void launch_baropg(const Dev& P, cudaStream_t s, int do_baropg, int do_sums) {
-  k_baropg<<<nblk(P.N, 128), 128, 0, s>>>(P, do_baropg, do_sums);
+  const int b = col_threads(P, P.N, 128);
+  k_baropg<<<nblk(P.N, b), b, 0, s>>>(P, do_baropg, do_sums);
 }
 void launch_int_reset(const Dev& P, cudaStream_t s) {
   int n = (P.M > P.N ? P.M : P.N) + 1;
   k_int_reset<<<nblk(n, 256), 256, 0, s>>>(P);
 }
-void launch_adjust2(const Dev& P, cudaStream_t s, int parts) { k_adjust2<<<nblk(P.N + 1, 128), 128, 0, s>>>(P, parts); }
+void launch_adjust2(const Dev& P, cudaStream_t s, int parts) {
+  const int b = col_threads(P, P.N + 1, 128);
+  k_adjust2<<<nblk(P.N + 1, b), b, 0, s>>>(P, parts);
+}
 void launch_vertvl_flux(const Dev& P, cudaStream_t s) {
   k_vertvl_flux<<<dim3(nblk(P.M, 32), nblk(P.KBM1, 8)), dim3(32, 8), 0, s>>>(P);
 }
 void launch_vertvl_col(const Dev& P, cudaStream_t s, int parts) {
-  k_vertvl_col<<<nblk(P.M, 128), 128, 0, s>>>(P, parts);
+  const int b = col_threads(P, P.M, 128);
+  k_vertvl_col<<<nblk(P.M, b), b, 0, s>>>(P, parts);
 }
 void launch_w_viscofh(const Dev& P, cudaStream_t s, int do_w, int do_visc) {
   int n = P.M > P.N ? P.M : P.N;
-  k_w_viscofh<<<col_grid(P, n, P.KB), P.col_bc, 0, s>>>(P, do_w, do_visc);
+  const Dev Q = col_shape(P, n, P.KB);
+  k_w_viscofh<<<col_grid(Q, n, P.KB), Q.col_bc, 0, s>>>(Q, do_w, do_visc);
 }
 void launch_adv_uv(const Dev& P, cudaStream_t s) {
   FVG_F32_FORWARD(launch_adv_uv(P, s));
@@ -1374,10 +1386,12 @@ void launch_adv_uv(const Dev& P, cudaStream_t s) {
     return;
   }
   if (P.limiter) launch_alfa3(P, s);
-  (P.limiter ? k_adv_uv<RF, true> : k_adv_uv<RF, false>)<<<col_grid(P, P.N, P.KBM1), P.col_bc, 0, s>>>(P);
+  const Dev Q = col_shape(P, P.N, P.KBM1);
+  (P.limiter ? k_adv_uv<RF, true> : k_adv_uv<RF, false>)<<<col_grid(Q, P.N, P.KBM1), Q.col_bc, 0, s>>>(Q);
 }
 void launch_vdif_uv(const Dev& P, cudaStream_t s, int parts) {
-  k_vdif_uv<<<nblk(P.N, 128), 128, 0, s>>>(P, parts);
+  const int b = col_threads(P, P.N, 128);
+  k_vdif_uv<<<nblk(P.N, b), b, 0, s>>>(P, parts);
 }
 
 }  // namespace fvg / fvg_f32

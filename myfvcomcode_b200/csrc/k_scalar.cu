@@ -1252,13 +1252,16 @@ __global__ void k_budget_final(const double* part, int nb, double* out) {
 
 void launch_grad(const Dev& P, cudaStream_t s, int which) {
   FVG_F32_FORWARD(launch_grad(P, s, which));
-  const dim3 g = col_grid(P, P.M, which == 0 ? P.KBM1 - 1 : P.KBM1);
-  k_grad<RF><<<g, P.col_bc, 0, s>>>(P, which);
+  const int nl = which == 0 ? P.KBM1 - 1 : P.KBM1;
+  const Dev Q = col_shape(P, P.M, nl);
+  k_grad<RF><<<col_grid(Q, P.M, nl), Q.col_bc, 0, s>>>(Q, which);
 }
 void launch_adv_q(const Dev& P, cudaStream_t s, int parts) {
   FVG_F32_FORWARD(launch_adv_q(P, s, parts));
-  k_he_adv<RF, 0><<<col_grid(P, P.N, P.KBM1 - 1), P.col_bc, 0, s>>>(P, parts);
-  k_gather_q<RF><<<col_grid(P, P.M, P.KBM1 - 1), P.col_bc, 0, s>>>(P, parts);
+  const int nl = P.KBM1 - 1;
+  const Dev Q = col_shape(P, P.N, nl), G = col_shape(P, P.M, nl);
+  k_he_adv<RF, 0><<<col_grid(Q, P.N, nl), Q.col_bc, 0, s>>>(Q, parts);
+  k_gather_q<RF><<<col_grid(G, P.M, nl), G.col_bc, 0, s>>>(G, parts);
 }
 void launch_fct_q(const Dev& P, cudaStream_t s, int parts) {
   dim3 b(32, 8), g(nblk(P.M, 32), nblk(P.KBM1 - 1, 8));
@@ -1270,9 +1273,11 @@ void launch_vdif_q(const Dev& P, cudaStream_t s, int copy_back) {
                         : aux == 2 ? k_vdif_q_levels<2> : k_vdif_q_levels<3>;
   void (*cf)(const Dev, int) = aux == 0 ? k_vdif_q_coef<0> : aux == 1 ? k_vdif_q_coef<1>
                              : aux == 2 ? k_vdif_q_coef<2> : k_vdif_q_coef<3>;
-  lv<<<col_grid(P, P.M, P.KB), P.col_bc, 0, s>>>(P);
-  k_vdif_q_sweep<<<dim3(nblk(P.M, 128), 2), 128, 0, s>>>(P);
-  cf<<<col_grid(P, P.M, P.KB), P.col_bc, 0, s>>>(P, copy_back);
+  const Dev Q = col_shape(P, P.M, P.KB);  // one shape: the sweep reads the level kernel's chunk flags
+  const int b = col_threads(P, P.M, 128);
+  lv<<<col_grid(Q, P.M, P.KB), Q.col_bc, 0, s>>>(Q);
+  k_vdif_q_sweep<<<dim3(nblk(P.M, b), 2), b, 0, s>>>(Q);
+  cf<<<col_grid(Q, P.M, P.KB), Q.col_bc, 0, s>>>(Q, copy_back);
   if (!P.closure) launch_vdif_q_shallow(P, s);
 }
 void launch_turb_update(const Dev& P, cudaStream_t s) {
@@ -1282,19 +1287,21 @@ void launch_turb_update(const Dev& P, cudaStream_t s) {
 }
 void launch_adv_ts(const Dev& P, cudaStream_t s, int parts) {
   FVG_F32_FORWARD(launch_adv_ts(P, s, parts));
-  k_he_adv<RF, 1><<<col_grid(P, P.N, P.KBM1), P.col_bc, 0, s>>>(P, parts);
+  const Dev Q = col_shape(P, P.N, P.KBM1), G = col_shape(P, P.M, P.KBM1);
+  k_he_adv<RF, 1><<<col_grid(Q, P.N, P.KBM1), Q.col_bc, 0, s>>>(Q, parts);
   if (P.iobcn > 0) k_obc_xflux<RF><<<dim3(nblk(P.iobcn, 64), P.KBM1, 2), 64, 0, s>>>(P, parts);
-  k_gather_ts<RF><<<col_grid(P, P.M, P.KBM1), P.col_bc, 0, s>>>(P, parts);
+  k_gather_ts<RF><<<col_grid(G, P.M, P.KBM1), G.col_bc, 0, s>>>(G, parts);
 }
 void launch_fct_ts(const Dev& P, cudaStream_t s, int parts) {
   dim3 b(32, 8), g(nblk(P.M, 32), nblk(P.KBM1, 8));
   k_fct_ts<<<g, b, 0, s>>>(P, parts);
 }
 void launch_vdif_ts(const Dev& P, cudaStream_t s, int parts) {
+  const int b = col_threads(P, P.M, 128);
   if (P.heating_on)
-    k_vdif_ts<true><<<dim3(nblk(P.M, 128), 2), 128, 0, s>>>(P, parts);
+    k_vdif_ts<true><<<dim3(nblk(P.M, b), 2), b, 0, s>>>(P, parts);
   else
-    k_vdif_ts<false><<<dim3(nblk(P.M, 128), 2), 128, 0, s>>>(P, parts);
+    k_vdif_ts<false><<<dim3(nblk(P.M, b), 2), b, 0, s>>>(P, parts);
 }
 void launch_bcond_ts(const Dev& P, cudaStream_t s, int parts) {
   if (P.numqbc > 0) k_bcond_ts_riv<<<P.KBM1, 128, 0, s>>>(P);
