@@ -57,6 +57,10 @@ struct fvg_handle {
   // possible (the mesh check of fvg_set_precision passed)
   int compact_allowed = 1;
   int compact_ok = 0;
+  // resident external loop: allowed (tuning key "ext_loop"), possible (the device launches
+  // cooperatively, every cell's three edges are its three sides)
+  int ext_loop = 1;
+  int loop_ok = 0;
 };
 
 #define CK(call)                                                                      \
@@ -258,8 +262,20 @@ struct Marker {
   }
 };
 
+// Whether the external loop runs as one resident kernel (k_ext_loop).
+bool use_ext_loop(const fvg_handle* h) {
+  const Dev& P = h->P;
+  if (!h->ext_loop || !h->loop_ok || P.limiter) return false;
+  if (P.prec && !P.f.compact) return false;
+  return (long)std::max(P.M, P.N) <= (long)kLoopThreads * P.nsm;
+}
+
 // One INTERNAL_STEP as a kernel sequence (internal_step.F:115-1590).
-void enqueue_internal_step(fvg_handle* h, cudaStream_t s, Marker mk = Marker()) {
+// after: in a group, the event of the model before (its resident external loop is done, if
+// it has one), which this model's loop waits for, so that no two cooperative grids of one
+// graph compete for the SMs; done receives this model's.
+void enqueue_internal_step(fvg_handle* h, cudaStream_t s, Marker mk = Marker(), cudaEvent_t after = nullptr,
+                           cudaEvent_t done = nullptr) {
   const Dev& P = h->P;
   const fvg_params& p = h->prm;
   const int spc = p.scalar_positivity_control ? AD_FCT : 0;
@@ -291,7 +307,14 @@ void enqueue_internal_step(fvg_handle* h, cudaStream_t s, Marker mk = Marker()) 
   // clamp) moves the same way to the head of the next node kernel; FLUX_OBN, the one
   // reader of ELF in between, applies the clamp itself.
   int stage = 0;
-  for (int iext = 1; iext <= p.isplit; ++iext) {
+  const bool loop = use_ext_loop(h);
+  if (loop) {
+    if (after) cudaStreamWaitEvent(s, after, 0);
+    launch_ext_loop(P, s);
+    if (done) cudaEventRecord(done, s);
+    mk.mark(s, G_EXT_CELL);
+  }
+  for (int iext = 1; iext <= p.isplit && !loop; ++iext) {
     for (int K = 1; K <= 4; ++K, ++stage) {
       Dev Q = P;
       if (stage & 1) {
@@ -303,7 +326,7 @@ void enqueue_internal_step(fvg_handle* h, cudaStream_t s, Marker mk = Marker()) 
           stage > 0 ? (EN_FINISH_PREV | (p.wetting_drying_on ? EN_WET_PREV : 0) | ((K == 1 ? 4 : K - 1) << 8)) : 0;
       // stage > 0: each kernel of the loop overlaps its launch with the previous one's tail
       const int pdl = stage > 0 ? 1 : 0;
-      launch_ext_node(Q, s, iext, K, EN_EXTEL | EN_BC | EN_GRAD | (K == 1 ? EN_COPY_ELRK : 0) | prev, pdl);
+      launch_ext_node(Q, s, iext, K, EN_EXTEL | EN_BC | EN_GRAD | EN_TABLE | (K == 1 ? EN_COPY_ELRK : 0) | prev, pdl);
       mk.mark(s, G_EXT_NODE);
       if (p.wetting_drying_on) {
         launch_wet_cells(Q, s, 1);  // its node part opens the next stage's node kernel
@@ -395,6 +418,7 @@ int fvg_create(const fvg_mesh* m, const fvg_params* prm, const fvg_forcing* f, f
   P.nsm = 148;
   {
     int dev = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&h->loop_ok, cudaDevAttrCooperativeLaunch, dev);
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&P.nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
       P.nsm = 148;
   }
@@ -581,6 +605,54 @@ int fvg_create(const fvg_mesh* m, const fvg_params* prm, const fvg_forcing* f, f
       UPI(ce_j1, cj1.data(), S3); UPI(ce_j2, cj2.data(), S3);
       UPD(ce_xoa, xa.data(), S3); UPD(ce_yoa, ya.data(), S3); UPD(ce_xob, xb.data(), S3);
       UPD(ce_yob, yb.data(), S3); UPD(ce_dx, dx.data(), S3); UPD(ce_dy, dy.data(), S3);
+    }
+    // the resident external loop: the neighbours' nodes off the edges, the cells' least H
+    {
+      std::vector<int> far(3 * n1, 0), lx(4 * n1, 0), lo(4 * n1, 0);
+      std::vector<double> hm(n1, 0.0);
+      for (size_t i = 1; i < n1; ++i) {
+        // the node common to two slots' edges
+        auto common = [&](int sa, int sb) {
+          const int ea = cl[i][sa] >> 1, eb = cl[i][sb] >> 1;
+          const int a1 = m->ienode[ea], a2 = m->ienode[e1 + ea], b1 = m->ienode[eb], b2 = m->ienode[e1 + eb];
+          return (a1 == b1 || a1 == b2) ? a1 : ((a2 == b1 || a2 == b2) ? a2 : 0);
+        };
+        const int x[3] = {common(2, 0), common(0, 1), common(1, 2)};
+        int bits = 0, seen = 0;
+        for (int j = 0; j < 3; ++j)
+          for (int sl = 0; sl < 3; ++sl)
+            if (m->nv[j * n1 + i] == x[sl]) {
+              seen |= 1 << sl;
+              if (j == 2) bits |= sl << 6;
+            }
+        if (seen != 7) h->loop_ok = 0;
+        for (int sl = 0; sl < 3; ++sl) {
+          const int e = cl[i][sl] >> 1, side = cl[i][sl] & 1;
+          bits |= side << sl | (m->isbc[e] != 0 ? 1 : 0) << (3 + sl);
+          lo[4 * i + sl] = side == 0 ? m->iec[e1 + e] : m->iec[e];
+          lx[4 * i + sl] = x[sl] > 0 ? x[sl] : 1;
+        }
+        lx[4 * i + 3] = bits;
+        hm[i] = std::fmin(std::fmin(m->h[m->nv[i]], m->h[m->nv[n1 + i]]), m->h[m->nv[2 * n1 + i]]);
+        for (int sl = 0; sl < 3; ++sl) {
+          const int code = cl[i][sl], e = code >> 1;
+          const int o = (code & 1) == 0 ? m->iec[e1 + e] : m->iec[e];
+          for (int j = 0; o > 0 && j < 3; ++j) {
+            const int nd = m->nv[j * n1 + o];
+            if (nd != m->ienode[e] && nd != m->ienode[e1 + e]) far[sl * n1 + i] = nd;
+          }
+        }
+      }
+      UPI(wfar, far.data(), far.size());
+      UPI(loopx, lx.data(), lx.size());
+      UPI(loopo, lo.data(), lo.size());
+      if ((rc = dalloc(h, (double**)&P.xuv, 4 * n1))) return fail(rc);
+      if ((rc = dalloc(h, (double**)&P.xnd, 2 * m1))) return fail(rc);
+      if ((rc = dalloc(h, &P.xg, 4 * n1))) return fail(rc);
+      if ((rc = dalloc(h, &P.xvc, n1))) return fail(rc);
+      if ((rc = dalloc(h, &P.xw, 2 * n1))) return fail(rc);
+      if ((rc = dalloc(h, &P.obf, (size_t)4 * prm->isplit * (m->iobcn + 1)))) return fail(rc);
+      UPD(hmin, hm.data(), n1);
     }
     // cell tiles of the staged momentum flux kernels
     {
@@ -841,6 +913,9 @@ int fvg_create(const fvg_mesh* m, const fvg_params* prm, const fvg_forcing* f, f
     int* ctl;
     if ((rc = dalloc(h, &ctl, 4))) return fail(rc);
     P.ctl = ctl;
+    if ((rc = dalloc(h, &P.bar, 32))) return fail(rc);
+    P.bar_err = h->h_ctl + 1;  // pinned memory, written by the device only on an error
+    *P.bar_err = 0;
   }
   P.sched = h->d_sched;
   if (cudaDeviceSynchronize() != cudaSuccess) {
@@ -952,6 +1027,15 @@ static void finish_chunk(fvg_handle* h, int c) {
   h->ramp = h->prm.iramp != 0 ? std::tanh((double)h->iint / (double)h->prm.iramp) : 1.0;
 }
 
+// A grid barrier of the resident external loop whose bounded wait ran out, read once the
+// steps have run.
+static int loop_check(fvg_handle* h) {
+  if (!h->h_ctl || h->h_ctl[1] == 0) return FVG_OK;
+  h->h_ctl[1] = 0;
+  h->err = "external loop: a bounded wait of its grid barrier ran out";
+  return FVG_ERR_TIMEOUT;
+}
+
 // The learned closure's error word, read after the steps have run: a bounded wait of the
 // tensor-core kernel that ran out (its rows then took MY2.5's values) fails the call.
 static int closure_check(fvg_handle* h) {
@@ -1025,6 +1109,7 @@ static int run_steps(fvg_handle* h, int32_t nsteps, int mode, double* group_ms, 
     cudaEventDestroy(t0);
     cudaEventDestroy(t1);
   }
+  { int rc = loop_check(h); if (rc) return rc; }
   return closure_check(h);
 }
 
@@ -1043,7 +1128,7 @@ int32_t fvg_kernels_per_step(const fvg_handle* h) {
   if (!h) return -1;
   const fvg_params& p = h->prm;
   int n = 1 + 1 + 2 + 2 + 2;                                // begin, cell_pre, grad3+adv3d, baropg+prep, int advave+reset
-  n += p.isplit * 4 * (2 + (p.wetting_drying_on ? 1 : 0)) + 1; // RK stages, closing update
+  n += (use_ext_loop(h) ? 1 : p.isplit * 4 * (2 + (p.wetting_drying_on ? 1 : 0))) + 1; // RK stages, closing update
   if (p.limiter) n += p.isplit * 4 + 1 + 2;                  // slope limiters: stages, ADVAVE, 3-D
   if (p.baropg_z && !p.barotropic) n += 2;                   // PHY_BAROPG's two kernels
   n += 1 + 1 + 1 + 1 + 2 + 1;                              // adjust2, vertvl x2, w/viscofh, grad3+adv_uv, vdif_uv
@@ -1304,6 +1389,8 @@ int fvg_set_tuning(fvg_handle* h, const char* key, int32_t value) {
   } else if (k == "ext_grid") {
     if (value < 0 || value > 8) { h->err = "ext_grid must be 0..8 blocks per SM"; return FVG_ERR_ARG; }
     h->P.ext_grid = value;
+  } else if (k == "ext_loop") {
+    h->ext_loop = value != 0;
   } else {
     h->err = "unknown tuning key " + k;
     return FVG_ERR_ARG;
@@ -1324,6 +1411,7 @@ int fvg_get_tuning(const fvg_handle* h, const char* key, int32_t* value) {
   else if (k == "staged") *value = h->P.staged;
   else if (k == "stream_hints") *value = h->P.ldcs;
   else if (k == "ext_grid") *value = h->P.ext_grid;
+  else if (k == "ext_loop") *value = use_ext_loop(h);
   else return FVG_ERR_ARG;
   return FVG_OK;
 }
@@ -1479,7 +1567,7 @@ struct fvg_group {
   cudaStream_t stream = nullptr;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t gexec = nullptr;
-  std::vector<cudaEvent_t> ev;  // fork event + one join event per model
+  std::vector<cudaEvent_t> ev;  // fork event, one join event per model, one per resident loop
   std::string err;
 };
 
@@ -1505,10 +1593,13 @@ static void group_free(fvg_group* g) {
 static int group_capture(fvg_group* g) {
   GK(cudaStreamBeginCapture(g->stream, cudaStreamCaptureModeThreadLocal));
   GK(cudaEventRecord(g->ev[0], g->stream));
-  for (size_t q = 0; q < g->hs.size(); ++q) {
+  cudaEvent_t after = nullptr;
+  const size_t nh = g->hs.size();
+  for (size_t q = 0; q < nh; ++q) {
     fvg_handle* h = g->hs[q];
     GK(cudaStreamWaitEvent(h->stream, g->ev[0], 0));
-    enqueue_internal_step(h, h->stream);
+    enqueue_internal_step(h, h->stream, Marker(), after, g->ev[nh + 1 + q]);
+    if (use_ext_loop(h)) after = g->ev[nh + 1 + q];
     GK(cudaEventRecord(g->ev[q + 1], h->stream));
     GK(cudaStreamWaitEvent(g->stream, g->ev[q + 1], 0));
   }
@@ -1552,7 +1643,11 @@ static int group_steps(fvg_group* g, int32_t nsteps, double* ms) {
       total += f;
     }
     GK(cudaStreamSynchronize(g->stream));
-    for (fvg_handle* h : g->hs) finish_chunk(h, c);
+    for (fvg_handle* h : g->hs) {
+      int rc = loop_check(h);
+      if (rc) { g->err = h->err; return rc; }
+      finish_chunk(h, c);
+    }
     done += c;
   }
   if (ms) {
@@ -1576,7 +1671,7 @@ int fvg_group_create(fvg_handle* const* hs, int32_t n, fvg_group** out) {
   fvg_group* g = new fvg_group();
   g->hs.assign(hs, hs + n);
   if (cudaStreamCreateWithFlags(&g->stream, cudaStreamNonBlocking) != cudaSuccess) { group_free(g); return FVG_ERR_CUDA; }
-  g->ev.resize((size_t)n + 1, nullptr);
+  g->ev.resize(2 * (size_t)n + 1, nullptr);
   for (auto& e : g->ev)
     if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) { group_free(g); return FVG_ERR_CUDA; }
   *out = g;

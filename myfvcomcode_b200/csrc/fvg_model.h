@@ -97,6 +97,9 @@ struct ClosNorm {
 // counting from ptr[t]; own cell j's three edges in slot order are slots[ptr[t]+j], each
 // {local edge | side << 16 | ISBC << 17} (w unused).
 constexpr int kTileCells = 128;
+// Largest block of the resident external loop (one block per SM, a cell and a node per
+// thread).
+constexpr int kLoopThreads = 384;
 struct Tiles {
   int n, cap_cells, cap_edges;
   const int *ptr, *nc, *eptr, *cells;
@@ -196,6 +199,27 @@ struct Dev {
   double *km1, *viscofm;
   // wet/dry
   int *iswetn, *iswetnt, *iswetc, *iswetct, *iswetce;
+  // obf: the specified elevation of open-boundary node ob at stage st (0..4*ISPLIT-1) of
+  // the current internal step, at st*(IOBCN+1) + ob (k_ext_prep).
+  double* obf;
+  // The resident external loop (k_ext_loop).  loopx, per cell: its nodes X0, X1, X2 in the
+  // order in which slot s is the edge X(s), X(s+1 mod 3), and w: bit s the cell's side of
+  // slot s, bit 3+s its ISBC, bits 6-7 the place of NV(c,3) among X; loopo, per cell the
+  // other cell of slots 0, 1, 2; wfar, per slot and cell (s*(N+1) + c) the node of the other
+  // cell that is off the edge (0: none); hmin, per cell the smallest H of its nodes.
+  // Exchanged inside the loop: xuv {UA, VA} and xw (ISWETC), each in two buffers of N+1; xg
+  // the FP64 gradients (four per cell), xvc ART*|grad|*CC_HVC in the form's type, xnd
+  // {EL, D} per node.  bar: the grid barrier's counter; bar_err (pinned host memory), set
+  // when a wait ran out.  loop_cells, loop_nodes: cells and nodes per block.
+  const int4 *loopx, *loopo;
+  double2 *xuv, *xnd;
+  double *xg, *xvc;
+  int* xw;
+  int loop_cells, loop_nodes;
+  const int* wfar;
+  const double* hmin;
+  unsigned* bar;
+  int* bar_err;
   // open boundary
   double *xflux_obcn, *uard_obcn, *xflux_obc_t, *xflux_obc_s;
   // river discharge after the ramp
@@ -345,6 +369,21 @@ __device__ inline void ghost_uv(const Dev& P, const double* U, const double* V, 
   }
 }
 
+// The same from the cell's own velocity.
+__device__ inline void ghost_uv1(const Dev& P, double u, double v, int c, int j, double& uk, double& vk) {
+  if (P.isbce[c] != 2) {
+    const size_t q = (size_t)(j - 1) * (P.N + 1) + c;
+    const double ca = P.gh_cos[q], sa = P.gh_sin[q];
+    const double utmp = u * ca + v * sa;
+    const double vtmp = 0.0;
+    uk = utmp * ca - vtmp * sa;
+    vk = utmp * sa + vtmp * ca;
+  } else {
+    uk = u;
+    vk = v;
+  }
+}
+
 // RAMP of the current internal step, from its schedule row.
 __device__ inline double ramp_int(const Dev& P) { return P.sched[(size_t)P.ctl[0] * P.sl.len]; }
 
@@ -476,9 +515,11 @@ extern const double kAlphaRK[5];
 // ---------------- external mode (k_ext.cu) ----------------
 // EN_FINISH_PREV: first finish the node part of the previous stage's update (EL = ELF,
 // D, DTFA, the stage sums), that stage's K in bits 8-10 of parts.
+// EN_TABLE: the specified elevations come from obf (an internal step's external loop).
 // EN_WET_PREV: before that, the node part of the previous stage's WET_JUDGE (ISWETN and the
 // ELF clamp, mod_wd.F:222-284) from that stage's cell flags, then in ISWETCE.
-enum ExtNodeParts { EN_EXTEL = 1, EN_BC = 2, EN_COPY_ELRK = 4, EN_GRAD = 8, EN_FINISH_PREV = 16, EN_WET_PREV = 32 };
+enum ExtNodeParts { EN_EXTEL = 1, EN_BC = 2, EN_COPY_ELRK = 4, EN_GRAD = 8, EN_FINISH_PREV = 16, EN_WET_PREV = 32,
+                    EN_TABLE = 64 };
 // EC_FINISH: end with the cell part of the stage's update (EL1, D1, the stage sums, the
 // next stage's continuity fluxes from the new UAF, VAF), UA/VA being swapped with
 // UAF/VAF between stages instead of copied.
@@ -498,6 +539,7 @@ void launch_ext_cell(const Dev& P, cudaStream_t s, int iext, int K, int parts, i
 void launch_alfa2(const Dev& P, cudaStream_t s);
 void launch_ext_update(const Dev& P, cudaStream_t s, int K);
 void launch_begin_step(const Dev& P, cudaStream_t s);
+void launch_ext_loop(const Dev& P, cudaStream_t s);
 void launch_ext_prep(const Dev& P, cudaStream_t s);
 void launch_make_f32(const Dev& P, cudaStream_t s);
 // Fill the compact external stage's records and count (into *mismatch, device memory)
@@ -558,6 +600,7 @@ namespace fvg_f32 {
 using fvg::Dev;
 void launch_alfa2(const Dev& P, cudaStream_t s);
 void launch_ext_cell(const Dev& P, cudaStream_t s, int iext, int K, int parts, int pdl);
+void launch_ext_loop(const Dev& P, cudaStream_t s);
 void launch_grad3(const Dev& P, cudaStream_t s);
 void launch_advection3d(const Dev& P, cudaStream_t s);
 void launch_adv_uv(const Dev& P, cudaStream_t s);

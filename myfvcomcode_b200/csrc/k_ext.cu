@@ -59,6 +59,18 @@ struct Grad {
   R ux, uy, vx, vy;
 };
 
+// a*b and a*b + c in separate roundings, also where this file is compiled with
+// contraction: the node part of a stage is the same in the stage kernels (compiled
+// without) and in the precision form's resident loop (compiled with).
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double add_rn(double a, double b) { return __dadd_rn(a, b); }
+__device__ __forceinline__ float add_rn(float a, float b) { return __fadd_rn(a, b); }
+template <typename R>
+__device__ __forceinline__ R dot4(R a, R u, R b, R v, R c, R w, R d, R x) {
+  return add_rn(add_rn(add_rn(mul_rn(a, u), mul_rn(b, v)), mul_rn(c, w)), mul_rn(d, x));
+}
+
 template <typename R, bool CS = false>
 __device__ inline Grad<R> cell_grad(const Dev& P, int c, const double* U, const double* V) {
   typedef Mesh<R> Mh;
@@ -75,10 +87,10 @@ __device__ inline Grad<R> cell_grad(const Dev& P, int c, const double* U, const 
     if (k3 == 0) { ghost_uv(P, U, V, c, 3, gu, gv); u3 = (R)gu; v3 = (R)gv; }
   }
   Grad<R> g;
-  g.ux = a1 * u0 + a2 * u1 + a3 * u2 + a4 * u3;
-  g.uy = b1 * u0 + b2 * u1 + b3 * u2 + b4 * u3;
-  g.vx = a1 * v0 + a2 * v1 + a3 * v2 + a4 * v3;
-  g.vy = b1 * v0 + b2 * v1 + b3 * v2 + b4 * v3;
+  g.ux = dot4(a1, u0, a2, u1, a3, u2, a4, u3);
+  g.uy = dot4(b1, u0, b2, u1, b3, u2, b4, u3);
+  g.vx = dot4(a1, v0, a2, v1, a3, v2, a4, v3);
+  g.vy = dot4(b1, v0, b2, v1, b3, v2, b4, v3);
   return g;
 }
 // Least-squares gradient of UA, VA of cell c (advave_edge_gcn.F:634-637, 699-702), stored
@@ -276,18 +288,20 @@ __device__ __forceinline__ void ext_node_job(const Dev& P, const int i, int iext
   if ((parts & EN_BC) && ob > 0) {
     int kind = P.obc_kind[ob];
     if (kind == 1) {
-      if (P.obc_elev_on) {
+      if (P.obc_elev_on && (parts & EN_TABLE)) {
+        P.elf[i] = P.obf[(size_t)((iext - 1) * 4 + K - 1) * (P.iobcn + 1) + ob];
+      } else if (P.obc_elev_on) {
         const double* row = sched_row(P);
         double force = 0.0;
         for (int j = 0; j < P.ntide; ++j) {
           size_t q = (size_t)j * (P.iobcn + 1) + ob;
           double targ = row[P.sl.targ(iext, K, j)];
-          force = P.apt[q] * cos(targ - P.phai_rad[q]) + force;
+          force = add_rn(mul_rn(P.apt[q], cos(targ - P.phai_rad[q])), force);
         }
         force = force + P.emean[ob];
         P.elf[i] = force * row[P.sl.ramp_ext(iext)];
       }
-      P.elf[i] = P.elrk[i] + alpha * (P.elf[i] - P.elrk[i]);
+      P.elf[i] = add_rn(P.elrk[i], mul_rn(alpha, P.elf[i] - P.elrk[i]));
     } else if (kind == 2) {
       P.elf[i] = 0.0;
     }
@@ -817,6 +831,508 @@ __global__ void __launch_bounds__(128, 8) k_ext_cell_c(const Dev P, int iext, in
 #endif  // FVG_F32_TU
 
 // -------------------------------------------------------------------------------------
+// The external loop of one internal step (ISPLIT x 4 Runge-Kutta stages) as one resident
+// kernel, for meshes with at most one cell and one node per thread of a grid of one block
+// per SM, launched cooperatively so that all its blocks are resident.  There a stage kernel
+// is one wave of dependent loads behind a launch, and 80 to 120 of them were half of the
+// step.  A stage is two phases with a grid barrier behind each:
+//   node phase   the update of the previous stage, EXTEL_EDGE and the boundary elevation of
+//                the thread's node; the least-squares gradient of the thread's cell and its
+//                viscosity term ART*|grad|*CC_HVC, which its neighbours' edges share;
+//   cell phase   WET_JUDGE's cell part (a dry cell forms its neighbours' flags itself),
+//                ADVAVE, EXTUV, BCOND_GCN(2) and the update of the thread's cell.
+// What bounds a stage is the chain of loads behind a barrier, so a phase's addresses are
+// all known when it begins: the thread keeps its neighbours' and nodes' numbers, the river
+// and open-boundary entries are resolved before the loop, and what is exchanged between
+// threads goes through packed arrays read in L2 (xuv, xg, xvc, xnd, ELF, exf2d).  ISWETN is
+// left to the closing kernel: nothing inside the loop reads it.  In FP64 every value is
+// formed as the stage kernels form it, with the sums that commute taken in the cell's own
+// order: results are theirs bit for bit.
+// -------------------------------------------------------------------------------------
+// Barrier over the grid: every block adds one to the counter (zeroed by k_begin_step) and
+// waits until all have.  The wait is bounded; a block whose wait runs out reports it and
+// leaves, and so do the others in their turn.
+constexpr long kBarSpin = 1L << 22;
+__device__ __forceinline__ bool grid_barrier(const Dev& P, unsigned target) {
+  __syncthreads();
+  int ok = 1;
+  if (threadIdx.x == 0) {
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(P.bar) : "memory");
+    unsigned seen = 0;
+    long it = 0;
+    do {
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(P.bar) : "memory");
+    } while (seen < target && ++it < kBarSpin);
+    if (seen < target) {
+      ok = 0;
+      *P.bar_err = 1;
+    }
+  }
+  return __syncthreads_and(ok);
+}
+
+// The loop's exchange arrays by arithmetic type: the gradient record of a cell.
+template <typename R>
+__device__ __forceinline__ Grad<R> ld_xg(const Dev& P, int c) {
+  if constexpr (sizeof(R) == 4) {
+    const float4 a = __ldcg(P.f.g2d4 + c);
+    return Grad<R>{a.x, a.y, a.z, a.w};
+  } else {
+    const double2* g = reinterpret_cast<const double2*>(P.xg) + 2 * (size_t)c;
+    const double2 a = __ldcg(g), b = __ldcg(g + 1);
+    return Grad<R>{a.x, a.y, b.x, b.y};
+  }
+}
+template <typename R>
+__device__ __forceinline__ void st_xg(const Dev& P, int c, const Grad<R>& g) {
+  if constexpr (sizeof(R) == 4) {
+    P.f.g2d4[c] = make_float4(g.ux, g.uy, g.vx, g.vy);
+  } else {
+    double2* q = reinterpret_cast<double2*>(P.xg) + 2 * (size_t)c;
+    q[0] = make_double2(g.ux, g.uy);
+    q[1] = make_double2(g.vx, g.vy);
+  }
+}
+
+template <typename R, int T>
+__global__ void __launch_bounds__(T, 1) k_ext_loop(const __grid_constant__ Dev P) {
+  typedef Mesh<R> Mh;
+  const R half = (R)0.5, one = (R)1.0;
+  const int tid = threadIdx.x;
+  const int c = blockIdx.x * P.loop_cells + tid + 1, i = blockIdx.x * P.loop_nodes + tid + 1;
+  const bool hc = tid < P.loop_cells && c <= P.N, hn = tid < P.loop_nodes && i <= P.M;
+  const size_t n1 = P.N + 1, ns = P.ns, ms = P.ms;
+  R* const xvc = reinterpret_cast<R*>(P.xvc);
+  const bool wd = P.wetting_drying_on != 0;
+
+  // ---- the thread's cell: neighbours, nodes, flags ----
+  int4 xn = make_int4(0, 0, 0, 0), oo = xn, nb = xn;
+  int isbce = 0, bcriv = 0, nobc = 0, nriv = 0;
+  int ob_[2] = {0, 0}, obn[2] = {0, 0};
+  double obf[2] = {0.0, 0.0}, rvx[2] = {0.0, 0.0}, rvy[2] = {0.0, 0.0};
+  double u = 0.0, v = 0.0;
+  if (hc) {
+    xn = P.loopx[c];  // nodes X0, X1, X2: slot s is the edge X(s), X(s+1); bits, see loopx
+    oo = P.loopo[c];  // the other cell of slots 0, 1, 2
+    nb = P.nbe4[c];
+    isbce = P.isbce[c];
+    if (isbce == 1) bcriv = P.cell_bcriv[c];
+    const int q0 = P.cell_obc_ptr[c], q1 = P.cell_obc_ptr[c + 1];
+    nobc = q1 - q0;
+    if (nobc <= 2)
+      for (int q = 0; q < nobc; ++q) {
+        const int code = P.cell_obc[q0 + q];
+        ob_[q] = code >> 1;
+        obn[q] = P.i_obc_n[code >> 1];
+        obf[q] = P.fluxf_obc[(size_t)(code & 1) * (P.iobcn + 1) + (code >> 1)];
+      }
+    else
+      P.fluxobn[c] = 0.0;
+    if (nobc == 0) P.fluxobn[c] = 0.0;
+    const int r0 = P.cell_riv_ptr[c];
+    nriv = P.cell_riv_ptr[c + 1] - r0;
+    for (int q = 0; q < nriv && q < 2; ++q) {
+      const int k = P.cell_riv[r0 + q] >> 1;
+      const double vlctyq = P.qdis[k] / P.qarea[k];
+      if (P.river_location == 0) {
+        rvx[q] = 0.5 * P.qdis[k] * vlctyq * P.cos_angleq[k];
+        rvy[q] = 0.5 * P.qdis[k] * vlctyq * P.sin_angleq[k];
+      } else {
+        const double temp = P.qdis[k] * vlctyq;
+        rvx[q] = temp * P.cos_angleq[k];
+        rvy[q] = temp * P.sin_angleq[k];
+      }
+    }
+    u = P.ua[c];
+    v = P.va[c];
+    P.xuv[c] = make_double2(u, v);
+    P.xw[n1 + c] = P.iswetce[c];
+  }
+  if (blockIdx.x == 0 && tid == 0) {
+    // the ghost cell 0 of both buffers
+    P.xuv[0] = make_double2(P.ua[0], P.va[0]);
+    P.xuv[n1] = make_double2(P.uaf[0], P.vaf[0]);
+    P.xw[0] = P.iswetc[0];
+    P.xw[n1] = P.iswetce[0];
+    const Grad<R> g = load_grad<R>(P, 0);
+    st_xg<R>(P, 0, g);
+    xvc[0] = Mh::art(P, 0) * sqrt(g.ux * g.ux + g.vy * g.vy + half * ((g.uy + g.vx) * (g.uy + g.vx))) * Mh::cc_hvc(P, 0);
+  }
+  // ---- the thread's node ----
+  double elf = 0.0, el = 0.0, elrk = 0.0, dn = 0.0, egf = 0.0, hnode = 0.0, art1 = 1.0;
+  double nrv[2] = {0.0, 0.0};
+  int ob = 0, kind = 0, nhe = 0, nnriv = 0;
+  if (hn) {
+    elf = P.elf[i];
+    el = P.el[i];
+    dn = P.d[i];
+    egf = P.egf[i];
+    hnode = P.h[i];
+    art1 = P.art1[i];
+    ob = P.node_obc[i];
+    if (ob > 0) kind = P.obc_kind[ob];
+    nhe = P.node_he_ptr[i + 1] - P.node_he_ptr[i];
+    const int r0 = P.node_riv_ptr[i];
+    nnriv = P.node_riv_ptr[i + 1] - r0;
+    for (int q = 0; q < nnriv && q < 2; ++q) {
+      const int r = P.node_riv[r0 + q], j = r >> 1;
+      nrv[q] = P.river_location == 0 ? P.qdis[j] : P.qdis[j] * P.rdisq[(size_t)(r & 1) * (P.numqbc + 1) + j];
+    }
+  }
+  unsigned target = 0;
+  if (!grid_barrier(P, target += gridDim.x)) return;
+
+  const int nst = 4 * P.isplit;
+  for (int st = 0; st < nst; ++st) {
+    const int iext = st / 4 + 1, K = st % 4 + 1;
+    const double2* const uv = P.xuv + (st & 1) * n1;
+    double2* const uvn = P.xuv + ((st + 1) & 1) * n1;
+    int* const wn = P.xw + (st & 1) * n1;
+    const int* const wp = P.xw + ((st + 1) & 1) * n1;
+    // ================= node phase =================
+    double2 b1, b2, b3;
+    R A[4], B[4];
+    R gart = 0, gcc = 0;
+    if (hc) {
+      b1 = __ldcg(uv + nb.x);
+      b2 = __ldcg(uv + nb.y);
+      b3 = __ldcg(uv + nb.z);
+      int k1, k2, k3;
+      lsq_coef<R>(P, c, k1, k2, k3, A, B);
+      gart = Mh::art(P, c);
+      gcc = Mh::cc_hvc(P, c);
+    }
+    if (hn) {
+      double x = 0.0;
+      const int* L = P.node_vpos_ell + i;
+      int j = 0;
+      for (; j + 6 <= nhe; j += 6) {
+        int e[6];
+        double f[6];
+#pragma unroll
+        for (int q = 0; q < 6; ++q) e[q] = L[(j + q) * ms];
+#pragma unroll
+        for (int q = 0; q < 6; ++q) f[q] = __ldcg(P.exf2d + (e[q] >> 1));
+#pragma unroll
+        for (int q = 0; q < 6; ++q) x = (e[q] & 1) ? x + f[q] : x - f[q];
+      }
+      for (; j + 2 <= nhe; j += 2) {
+        const int e0 = L[j * ms], e1 = L[(j + 1) * ms];
+        const double f0 = __ldcg(P.exf2d + (e0 >> 1)), f1 = __ldcg(P.exf2d + (e1 >> 1));
+        x = (e0 & 1) ? x + f0 : x - f0;
+        x = (e1 & 1) ? x + f1 : x - f1;
+      }
+      if (j < nhe) {
+        const int e0 = L[j * ms];
+        const double f0 = __ldcg(P.exf2d + (e0 >> 1));
+        x = (e0 & 1) ? x + f0 : x - f0;
+      }
+      if (st > 0) {
+        // the previous stage's clamp (WET_JUDGE) and update (ext_update_node)
+        if (wd) elf = fmax(elf, -hnode + P.min_depth);
+        el = elf;
+        dn = hnode + elf;
+        if (K == 4) egf = egf + elf / (double)P.isplit;  // previous stage 3
+        if (K == 1 && ob > 0) {
+          const double tmp = -(elf - elrk) * art1 / P.dte - P.xflux_obcn[ob];
+          P.uard_obcn[ob] = P.uard_obcn[ob] + tmp / (double)(float)P.isplit;
+        }
+      }
+      if (K == 1) elrk = el;
+      if (ob > 0) {
+        P.xflux_obcn[ob] = x;
+        x = 0.0;
+      }
+      if (nnriv > 0) {
+        x = x - nrv[0];
+        if (nnriv > 1) x = x - nrv[1];
+        for (int q = P.node_riv_ptr[i] + 2; q < P.node_riv_ptr[i + 1]; ++q) {
+          const int r = P.node_riv[q], jr = r >> 1;
+          x = x - (P.river_location == 0 ? P.qdis[jr] : P.qdis[jr] * P.rdisq[(size_t)(r & 1) * (P.numqbc + 1) + jr]);
+        }
+      }
+      const double alpha = dAlphaRK[K], dtk = alpha * P.dte;
+      elf = elrk - dtk * x / art1;
+      if (ob > 0) {
+        if (kind == 1) {
+          if (P.obc_elev_on) elf = P.obf[(size_t)st * (P.iobcn + 1) + ob];
+          elf = add_rn(elrk, mul_rn(alpha, elf - elrk));
+        } else if (kind == 2) {
+          elf = 0.0;
+        }
+        P.elrk[i] = elrk;
+      }
+      P.elf[i] = elf;
+      P.xnd[i] = make_double2(el, dn);
+    }
+    Grad<R> gi = {0, 0, 0, 0};
+    R vci = 0;
+    if (hc) {
+      R u1 = (R)b1.x, u2 = (R)b2.x, u3 = (R)b3.x, v1 = (R)b1.y, v2 = (R)b2.y, v3 = (R)b3.y;
+      if (P.gcy && (nb.x == 0 || nb.y == 0 || nb.z == 0)) {
+        double gu, gv;
+        if (nb.x == 0) { ghost_uv1(P, u, v, c, 1, gu, gv); u1 = (R)gu; v1 = (R)gv; }
+        if (nb.y == 0) { ghost_uv1(P, u, v, c, 2, gu, gv); u2 = (R)gu; v2 = (R)gv; }
+        if (nb.z == 0) { ghost_uv1(P, u, v, c, 3, gu, gv); u3 = (R)gu; v3 = (R)gv; }
+      }
+      gi.ux = dot4(A[0], (R)u, A[1], u1, A[2], u2, A[3], u3);
+      gi.uy = dot4(B[0], (R)u, B[1], u1, B[2], u2, B[3], u3);
+      gi.vx = dot4(A[0], (R)v, A[1], v1, A[2], v2, A[3], v3);
+      gi.vy = dot4(B[0], (R)v, B[1], v1, B[2], v2, B[3], v3);
+      st_xg<R>(P, c, gi);
+      vci = gart * sqrt(gi.ux * gi.ux + gi.vy * gi.vy + half * ((gi.uy + gi.vx) * (gi.uy + gi.vx))) * gcc;
+      xvc[c] = vci;
+    }
+    if (!grid_barrier(P, target += gridDim.x)) return;
+    // ================= cell phase =================
+    if (hc) {
+      const int xs[3] = {xn.x, xn.y, xn.z}, os[3] = {oo.x, oo.y, oo.z};
+      const int bits = xn.w;
+      // everything the phase reads is loaded before its arithmetic and its stores
+      double2 nd[3], ou[3];
+      double en[3], hn3[3], edx[3], edy[3], hgx[3], hgy[3];
+      Grad<R> go[3];
+      R vo[3], xi[3], yi[3], xo[3], yo[3];
+#pragma unroll
+      for (int s = 0; s < 3; ++s) {
+        nd[s] = __ldcg(P.xnd + xs[s]);
+        en[s] = __ldcg(P.elf + xs[s]);
+        ou[s] = __ldcg(uv + os[s]);
+        go[s] = ld_xg<R>(P, os[s]);
+        vo[s] = __ldcg(xvc + os[s]);
+      }
+#pragma unroll
+      for (int s = 0; s < 3; ++s) {
+        const int side = (bits >> s) & 1;
+        const size_t q = (size_t)s * n1 + c, pos = (size_t)s * ns + c;
+        hn3[s] = P.h[xs[s]];
+        if constexpr (sizeof(R) == 4) {
+          const float4 G = P.f.ce_geo[q];  // XOA, YOA, XOB, YOB
+          xi[s] = side ? G.z : G.x;
+          yi[s] = side ? G.w : G.y;
+          xo[s] = side ? G.x : G.z;
+          yo[s] = side ? G.y : G.w;
+        } else {
+          xi[s] = (side ? P.ce_xob : P.ce_xoa)[q];
+          yi[s] = (side ? P.ce_yob : P.ce_yoa)[q];
+          xo[s] = (side ? P.ce_xoa : P.ce_xob)[q];
+          yo[s] = (side ? P.ce_yoa : P.ce_yob)[q];
+        }
+        edx[s] = P.ce_dx[q];
+        edy[s] = P.ce_dy[q];
+        hgx[s] = Mesh<double>::hg(P, 0, pos);
+        hgy[s] = Mesh<double>::hg(P, 1, pos);
+      }
+      const double d1i = P.d1[c], h1i = P.h1[c], grav = P.grav_e[c], hmin = P.hmin[c], sp = P.cc_sponge[c];
+      const double iu = P.iucp[c];
+      const R epor = (R)P.epor[c], iucp = (R)iu;
+      const double uark = K == 1 ? u : P.uark[c], vark = K == 1 ? v : P.vark[c];
+      const double elrk1 = (K == 1 ? P.el1 : P.elrk1)[c];
+      const int wce = wp[c], wci = wd ? 0 : P.iswetc[c];  // ISWETCE; ISWETC where it is fixed
+      const double uard = K == 3 ? P.uard[c] : 0.0, vard = K == 3 ? P.vard[c] : 0.0;
+      const double ramp = sched_row(P)[P.sl.ramp_ext(iext)];
+      // EXTUV's terms that stay fixed over the loop; in the FP32 form summed by the
+      // internal-step ADVAVE call (exc0, exc1)
+      double4 e0 = make_double4(0.0, 0.0, 0.0, 0.0), e1 = e0;
+      double adx = 0.0, ady = 0.0, drx = 0.0, dry = 0.0, wbx = 0.0, wby = 0.0, wsx = 0.0, wsy = 0.0, art, cor;
+      if constexpr (sizeof(R) == 4) {
+        e0 = P.f.exc0[c];
+        e1 = P.f.exc1[c];
+        art = e1.y;
+        cor = e1.x;
+      } else {
+        adx = P.adx2d[c];
+        ady = P.ady2d[c];
+        drx = P.drx2d[c];
+        dry = P.dry2d[c];
+        wbx = P.wubot[c];
+        wby = P.wvbot[c];
+        art = P.art[c];
+        cor = P.cor[c];
+        if (P.have_wind) {
+          wsx = P.wsx[c];
+          wsy = P.wsy[c];
+        }
+      }
+      const double ged1 = grav * d1i;
+      // WET_JUDGE's cell part, or N2E2D; the mean in NV order (its last node's place in bits)
+      const int k3 = (bits >> 6) & 3;
+      double cl[3] = {en[0], en[1], en[2]};
+      int wetc = wci;
+      if (wd) {
+        const double md = P.min_depth;
+        const double dtmp = fmax(fmax(en[0], en[1]), en[2]) + hmin;
+        wetc = ((dtmp - md) < 1.0e-5) ? 0 : 1;
+#pragma unroll
+        for (int s = 0; s < 3; ++s) cl[s] = fmax(en[s], -hn3[s] + md);
+      }
+      const double l3 = k3 == 0 ? cl[0] : (k3 == 1 ? cl[1] : cl[2]);
+      const double l12 = k3 == 0 ? cl[1] + cl[2] : (k3 == 1 ? cl[0] + cl[2] : cl[0] + cl[1]);
+      const double elf1 = ONE_THIRD * (l12 + l3);
+      const int weti = wce * wetc;
+      // FLUX_OBN
+      double fob = 0.0;
+      if (nobc > 0) {
+        if (nobc <= 2) {
+#pragma unroll
+          for (int q = 0; q < 2; ++q) {
+            if (q < nobc) {
+              const int j = obn[q];
+              const double ej0 = __ldcg(P.elf + j);
+              const double ej = wd ? fmax(ej0, -P.h[j] + P.min_depth) : ej0;
+              const double flux =
+                  -(ej - __ldcg(P.elrk + j)) * P.art1[j] / (dAlphaRK[K] * P.dte) - __ldcg(P.xflux_obcn + ob_[q]);
+              fob = fob + obf[q] * flux;
+            }
+          }
+        } else {
+          fob = fluxobn_cell(P, c, K);
+        }
+        P.fluxobn[c] = fob;
+      }
+      if (K == 1) {
+        P.elrk1[c] = elrk1;
+        P.uark[c] = u;
+        P.vark[c] = v;
+      }
+      R xr = 0, yr = 0;
+      double px = 0.0, py = 0.0;
+      const R ui = (R)u, vi = (R)v;
+#pragma unroll
+      for (int s = 0; s < 3; ++s) {
+        const int side = (bits >> s) & 1, isbc = (bits >> (3 + s)) & 1, o = os[s];
+        const size_t q = (size_t)s * n1 + c;
+        const double2 na = nd[s], nbb = nd[(s + 1) % 3];
+        const R dij = (R)(0.5 * (na.y + nbb.y));
+        const double elij = 0.5 * (na.x + nbb.x);
+        bool on = weti == 1;
+        if (!on) {
+          // a dry cell: the neighbour's flags of the stage before and of this one
+          int wo = wp[o];
+          if (wd && o != 0) {
+            const double e = fmax(fmax(en[s], en[(s + 1) % 3]), __ldcg(P.elf + P.wfar[q]));
+            wo = wo * (((e + P.hmin[o]) - P.min_depth) < 1.0e-5 ? 0 : 1);
+          } else {
+            wo = wo * (wd ? P.xw[(st & 1) * n1] : P.iswetc[o]);
+          }
+          on = wo == 1;
+        }
+        const R dx = (R)edx[s], dy = (R)edy[s];
+        if (on) {
+          const R uo = (R)ou[s].x, vv = (R)ou[s].y;
+          const R uown = ui + gi.ux * xi[s] + gi.uy * yi[s], vown = vi + gi.vx * xi[s] + gi.vy * yi[s];
+          const R uoth = uo + go[s].ux * xo[s] + go[s].uy * yo[s], voth = vv + go[s].vx * xo[s] + go[s].vy * yo[s];
+          const R uij = half * (uown + uoth), vij = half * (vown + voth);
+          const R un = -uij * dy + vij * dx;
+          R viscof = (R)P.fact * half * (vci + vo[s]);
+          viscof = viscof + (R)P.fm1 * half * (P.fm1 != 0.0 ? gcc + Mh::cc_hvc(P, o) : (R)0);
+          if (P.hprnu != 1.0) viscof = viscof / (R)P.hprnu;
+          const R vxa = side ? go[s].vx : gi.vx, vxb = side ? gi.vx : go[s].vx;
+          const R txx = (gi.ux + go[s].ux) * viscof;
+          const R tyy = (gi.vy + go[s].vy) * viscof;
+          const R txy = half * (gi.uy + go[s].uy + vxa + vxb) * viscof;
+          const R fxx = dij * (txx * dy - txy * dx);
+          const R fyy = dij * (txy * dy - tyy * dx);
+          const R sg = fsign1(un), sgo = side ? -sg : sg;
+          const R xadv = dij * un * ((one - sgo) * uoth + (one + sgo) * uown) * half;
+          const R yadv = dij * un * ((one - sgo) * voth + (one + sgo) * vown) * half;
+          const R nbd = one - (R)isbc;
+          const R ax = (xadv + fxx * epor) * nbd * iucp, ay = (yadv + fyy * epor) * nbd * iucp;
+          xr = side ? xr - ax : xr + ax;
+          yr = side ? yr - ay : yr + ay;
+        }
+        const double tx = ged1 * elij * edy[s], ty = ged1 * elij * edx[s];
+        px = side ? px + tx : px - tx;
+        py = side ? py - ty : py + ty;
+      }
+      const R w = (R)weti;
+      double xf = (double)(xr * w), yf = (double)(yr * w);
+      if (isbce == 2) {
+        if (P.gcy) {
+          xf = xf + fob * u * iu;
+          yf = yf + fob * v * iu;
+        } else {
+          xf = (xf + fob * u) * iu;
+          yf = (yf + fob * v) * iu;
+        }
+      }
+      if (nriv > 0) {
+        xf = xf - rvx[0];
+        yf = yf - rvy[0];
+        if (nriv > 1) {
+          xf = xf - rvx[1];
+          yf = yf - rvy[1];
+        }
+        for (int q = P.cell_riv_ptr[c] + 2; q < P.cell_riv_ptr[c + 1]; ++q) {
+          const int k = P.cell_riv[q] >> 1;
+          const double vl = P.qdis[k] / P.qarea[k];
+          const double t = P.river_location == 0 ? 0.5 * P.qdis[k] * vl : P.qdis[k] * vl;
+          xf = xf - t * P.cos_angleq[k];
+          yf = yf - t * P.sin_angleq[k];
+        }
+      }
+      if (st == nst - 1) {
+        P.advua[c] = xf;
+        P.advva[c] = yf;
+        P.pstx[c] = px;
+        P.psty[c] = py;
+      }
+      double uaf = 0.0, vaf = 0.0;
+      if (weti == 1) {
+        const double a = dAlphaRK[K];
+        double resx, resy;
+        if constexpr (sizeof(R) == 4) {
+          resx = e0.x + xf + px - cor * v * d1i - ramp * e0.z;
+          resy = e0.y + yf + py + cor * u * d1i - ramp * e0.w;
+        } else {
+          const double wus = P.have_wind ? wsx * ramp * 0.001 : 0.0;
+          const double wvs = P.have_wind ? wsy * ramp * 0.001 : 0.0;
+          resx = adx + xf + drx + px - cor * v * d1i * art - (wus + wbx) * art;
+          resy = ady + yf + dry + py + cor * u * d1i * art - (wvs + wby) * art;
+        }
+        uaf = (uark * (h1i + elrk1) - a * P.dte * resx / art) / (h1i + elf1);
+        vaf = (vark * (h1i + elrk1) - a * P.dte * resy / art) / (h1i + elf1);
+      }
+      if (sp != 0.0) {
+        uaf = uaf / (1.0 + sp * (uaf * uaf));
+        vaf = vaf / (1.0 + sp * (vaf * vaf));
+      }
+      if (isbce == 3 && !P.gcy) { uaf = 0.0; vaf = 0.0; }
+      if (isbce == 1 && (!P.gcy || bcriv > 0)) bc_solid(P, c, bcriv, uaf, vaf);
+      u = uaf;
+      v = vaf;
+      uvn[c] = make_double2(u, v);
+      if (wd) wn[c] = wetc;
+      else wn[c] = wce;
+      P.el1[c] = elf1;
+      const double dd1 = h1i + elf1;
+      P.d1[c] = dd1;
+      if (K == 3) {
+        P.uard[c] = uard + u * dd1;
+        P.vard[c] = vard + v * dd1;
+      }
+#pragma unroll
+      for (int s = 0; s < 3; ++s) P.exf2d[(size_t)s * ns + c] = dd1 * (-u * hgy[s] + v * hgx[s]);
+      if (st == nst - 1) {
+        // as the launched loop leaves its arrays before k_ext_finish
+        P.elf1[c] = elf1;
+        P.ua[c] = u;
+        P.va[c] = v;
+        if (wd) P.iswetce[c] = wetc;
+      }
+    }
+    if (st < nst - 1 && !grid_barrier(P, target += gridDim.x)) return;
+  }
+  if (hn) {
+    P.el[i] = el;
+    P.d[i] = dn;
+    P.dtfa[i] = dn;
+    P.egf[i] = egf;
+    P.elrk[i] = elrk;
+  }
+}
+
+// -------------------------------------------------------------------------------------
 // external_step.F:333-436: EL=ELF, EL1=N2E2D(EL), D, D1, UA=UAF, DTFA, the K==3 sums
 // for the 3-D correction, the K==4 open-boundary transport and WD_UPDATE(1).
 // -------------------------------------------------------------------------------------
@@ -846,8 +1362,27 @@ __global__ void k_ext_finish(const Dev P, int K, int wet_prev) {
     P.iswetc[i] = P.iswetce[i];
   }
 }
+// The specified elevation of every open-boundary node and stage of the external loop
+// (BCOND_ASL, mod_obcs.F:554-583), for the loop's node phase: inside it the cosines were the
+// longest chain of a stage, on a few threads.
+__device__ inline void tide_entry(const Dev& P, int st, int ob) {
+  if (P.obc_kind[ob] != 1) return;
+  const int iext = st / 4 + 1, K = st % 4 + 1;
+  const double* row = sched_row(P);
+  double force = 0.0;
+  for (int j = 0; j < P.ntide; ++j) {
+    const size_t q = (size_t)j * (P.iobcn + 1) + ob;
+    const double targ = row[P.sl.targ(iext, K, j)];
+    force = add_rn(mul_rn(P.apt[q], cos(targ - P.phai_rad[q])), force);
+  }
+  force = force + P.emean[ob];
+  P.obf[(size_t)st * (P.iobcn + 1) + ob] = force * row[P.sl.ramp_ext(iext)];
+}
 __global__ void k_ext_prep(const Dev P) {
   int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
+  if (P.obc_elev_on)
+    for (int q = i - 1; q < 4 * P.isplit * P.iobcn; q += gridDim.x * blockDim.x)
+      tide_entry(P, q / P.iobcn, q % P.iobcn + 1);
   if (i > P.N) return;
   store_grad<false>(P, i);
   store_exf(P, i);
@@ -859,6 +1394,7 @@ __global__ void k_begin_step(const Dev P, int advance) {
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
   int slot = P.ctl[0] + advance;
   P.ctl[0] = slot;
+  *P.bar = 0;
   double ramp = P.sched[(size_t)slot * P.sl.len];
   for (int j = 1; j <= P.numqbc; ++j) P.qdis[j] = P.qdis0[j] * ramp;
 }
@@ -1019,6 +1555,33 @@ void launch_ext_update(const Dev& P, cudaStream_t s, int K) {
 void launch_ext_finish(const Dev& P, cudaStream_t s, int K, int wet_prev) {
   int n = P.M > P.N ? P.M : P.N;
   k_ext_finish<<<nblk(n, 256), 256, 0, s>>>(P, K, wet_prev);
+}
+template <int T>
+static void loop_launch(const Dev& P, cudaStream_t s, int grid) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(T);
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeCooperative;
+  at[0].val.cooperative = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, k_ext_loop<RF, T>, P);
+}
+// One block per SM at most; the smallest block that then holds a cell and a node per thread,
+// so that the threads of a small mesh spread over the SMs.
+void launch_ext_loop(const Dev& P, cudaStream_t s) {
+  FVG_F32_FORWARD(launch_ext_loop(P, s));
+  const int need = nblk(P.N > P.M ? P.N : P.M, P.nsm);
+  const int t = need <= 128 ? 128 : need <= 288 ? 288 : kLoopThreads;
+  Dev Q = P;
+  const int grid = t > 128 ? P.nsm : nblk(P.N > P.M ? P.N : P.M, t);
+  Q.loop_cells = nblk(P.N, grid);
+  Q.loop_nodes = nblk(P.M, grid);
+  if (t == 128) loop_launch<128>(Q, s, grid);
+  else if (t == 288) loop_launch<288>(Q, s, grid);
+  else loop_launch<kLoopThreads>(Q, s, grid);
 }
 void launch_begin_step(const Dev& P, cudaStream_t s) { k_begin_step<<<1, 32, 0, s>>>(P, 1); }
 void launch_set_qdis(const Dev& P, cudaStream_t s) { k_begin_step<<<1, 32, 0, s>>>(P, 0); }
