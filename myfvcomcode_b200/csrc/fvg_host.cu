@@ -697,21 +697,35 @@ int fvg_create(const fvg_mesh* m, const fvg_params* prm, const fvg_forcing* f, f
     UPI(cell_he, chv.data(), chv.size());
     // Half-edge positions pos = slot*ns + cell; the node lists over positions, entry j of
     // node i at j*ms + i, code = pos*2 + side, ascending half-edge id; the metrics by position
-    std::vector<int> slot(v1, 0);
+    std::vector<int> slot(v1, 0), hex(4 * n1, 0);
     std::vector<double> hg(18 * ns, 0.0);
-    for (size_t i = 1; i < n1; ++i)
+    for (size_t i = 1; i < n1; ++i) {
+      // X(s): the node common to the half-edges of slots s-1 and s
+      auto common = [&](int sa, int sb) {
+        const int ha = chv[3 * i + sa], hb = chv[3 * i + sb];
+        const int a1 = m->niec[ha], a2 = m->niec[v1 + ha], b1 = m->niec[hb], b2 = m->niec[v1 + hb];
+        return (a1 == b1 || a1 == b2) ? a1 : a2;
+      };
+      const int x[3] = {common(2, 0), common(0, 1), common(1, 2)};
       for (int s2 = 0; s2 < 3; ++s2) {
-        const int he = chv[3 * i + s2];
+        const int he = chv[3 * i + s2], a = x[s2], b = x[(s2 + 1) % 3];
+        const bool straight = m->niec[he] == a && m->niec[v1 + he] == b;
+        const bool flip = m->niec[he] == b && m->niec[v1 + he] == a;
+        if (a == b || !(straight || flip)) { h->err = "half-edges of a cell that do not part its three nodes"; return fail(FVG_ERR_BOUNDS); }
+        hex[4 * i + s2] = a;
+        hex[4 * i + 3] |= (flip ? 1 : 0) << s2;
         slot[he] = s2;
-        const size_t pos = (size_t)s2 * ns + i, pl = 3 * ns;
+        const size_t pos = (size_t)s2 * ns + i, pl = 3 * ns, sa = flip ? vi1 : 0, sb = flip ? 0 : vi1;
         hg[pos] = m->dltxe[he];
         hg[pl + pos] = m->dltye[he];
-        hg[2 * pl + pos] = m->dltxncve[he];
-        hg[3 * pl + pos] = m->dltyncve[he];
-        hg[4 * pl + pos] = m->dltxncve[vi1 + he];
-        hg[5 * pl + pos] = m->dltyncve[vi1 + he];
+        hg[2 * pl + pos] = m->dltxncve[sa + he];
+        hg[3 * pl + pos] = m->dltyncve[sa + he];
+        hg[4 * pl + pos] = m->dltxncve[sb + he];
+        hg[5 * pl + pos] = m->dltyncve[sb + he];
       }
+    }
     UPD(hg, hg.data(), hg.size());
+    UPI(hex, hex.data(), hex.size());
     std::vector<std::vector<int>> vl(m1);
     for (int he = 1; he <= m->ncv; ++he) {
       const long pos = (long)slot[he] * (long)ns + m->ntrg[he];
@@ -865,6 +879,7 @@ int fvg_create(const fvg_mesh* m, const fvg_params* prm, const fvg_forcing* f, f
       if ((rc = dalloc(h, &P.gq[t][g], ms * KB))) return fail(rc);
       if ((rc = dalloc(h, &P.gt[t][g], ms * KB))) return fail(rc);
     }
+  if ((rc = dalloc(h, &P.gvn, ms * KB))) return fail(rc);
   if ((rc = dalloc(h, &P.budget, 3 + 3 * 148))) return fail(rc);
   for (double** pp : {&P.vq_prod, &P.vq_gh, &P.vq_dtef, &P.vq_dtefl})
     if ((rc = dalloc(h, pp, ms * KB))) return fail(rc);

@@ -156,8 +156,11 @@ struct Dev {
   // the threads of consecutive nodes read entry j in one coalesced load.
   const int* node_vpos_ell;
   // Metrics by position, plane j at j*ncvs: DLTXE, DLTYE, DLTXNCVE and DLTYNCVE of the
-  // NIEC(he,1) side, DLTXNCVE and DLTYNCVE of the NIEC(he,2) side.
+  // side of X(s), DLTXNCVE and DLTYNCVE of the side of X(s+1) (hex).
   const double* hg;
+  // Per cell its nodes X0, X1, X2 in the order in which the half-edge of slot s separates
+  // X(s) and X(s+1 mod 3); w: bit s where NIEC(he,1) is X(s+1).
+  const int4* hex;
   const int *cell_edge;               // cell -> its 3 edges (id*2 + side), ascending id
   // Slot table of the cell edge loops, slot s of cell i at s*(N+1) + i (edges in the order
   // of cell_edge): code = edge*4 + ISBC*2 + side, the two cells, the two nodes, the edge
@@ -228,6 +231,7 @@ struct Dev {
   double *scr_xflux;                         // VERTVL flux
   double *gq[2][6];  // ADV_Q of Q2 / Q2L: PQPX, PQPY, PQPXD, PQPYD, ring min, ring max
   double *gt[2][6];  // ADV_T / ADV_S: the same six per tracer
+  double* gvn;       // VISCOFH*NN_HVC of the half-edge fluxes, per node and layer or level (FP64 form)
   double* budget;                            // 3 doubles
   // VDIF_Q between its passes: PROD, GH, DTEF, the q2l DTEF (node 3-D) and UTAU2 (node)
   double *vq_prod, *vq_gh, *vq_dtef, *vq_dtefl, *vq_ut;

@@ -187,16 +187,16 @@ __global__ void __launch_bounds__(256) k_grad(const Dev P, int which) {
       w1 = w2;
     }
     const size_t q = N3(P, i, k);
-    // the node's mixing coefficient as the half-edge fluxes take it (FP32 records)
-    R vf = 0;
-    if (sizeof(R) == 4) {
-      if (which == 0) {
-        const size_t qm = N3(P, i, k - 1);
-        vf = (R)((P.viscofh[q] * P.dz[qm] + P.viscofh[qm] * P.dz[q]) / (P.dz[q] + P.dz[qm]));
-      } else {
-        vf = (R)P.viscofh[q];
-      }
+    // the node's mixing coefficient as the half-edge fluxes take it: VISCOFH on the layer or
+    // interpolated to the level, in the FP32 records, and times NN_HVC in the plane gvn in FP64
+    R vf;
+    if (which == 0) {
+      const size_t qm = N3(P, i, k - 1);
+      vf = (R)((P.viscofh[q] * P.dz[qm] + P.viscofh[qm] * P.dz[q]) / (P.dz[q] + P.dz[qm]));
+    } else {
+      vf = (R)P.viscofh[q];
     }
+    if (sizeof(R) == 8) P.gvn[q] = vf * P.nn_hvc[i];
     for (int t = 0; t < 2; ++t) {
       const R gx = px[t] / art2, gy = py[t] / art2, gxd = pxd[t] / art2, gyd = pyd[t] / art2;
       NodeRec<R>::store(P, which, t, q, qi[t], gx, gy, gxd, gyd, rmin[t], rmax[t], vf);
@@ -269,59 +269,35 @@ __device__ inline void fct_level_bounds(const Dev& P, int i, int k, const double
 // and applies the vertical flux, the update and the FCT clamp.
 // MODE 0: Q2 and Q2L on interfaces K=2..KBM1; MODE 1: T and S on layers K=1..KBM1.
 // -------------------------------------------------------------------------------------
+// A cell's half-edge in slot s separates two of its nodes; the cell's nodes are taken in the
+// order X0, X1, X2 (hex) in which slot s separates X(s) and X(s+1 mod 3), so that every node
+// record has a fixed place and no value is selected at run time (the selects between the
+// records were a third of the kernel's instructions, which bound it).  Bit s of the order's
+// fourth word tells that NIEC(he,1) is X(s+1): the two sides then swap roles, which the
+// upwind weights alone see.
 template <typename R>
 struct HeCell {
   R uq, vq, dtij;
-  int nd[3];
-  R vf[3], nn[3];
 };
 
-// The layer-independent part of a cell's half-edge data: its three nodes and their
-// NN_HVC, loaded once per thread for the layers it walks.
-template <typename R>
-__device__ inline void he_cell_static(const Dev& P, int c, HeCell<R>& hc) {
-  const size_t n1 = P.N + 1;
-  for (int j = 0; j < 3; ++j) {
-    const int n = P.nv[j * n1 + c];
-    hc.nd[j] = n;
-    hc.nn[j] = (R)P.nn_hvc[n];
-  }
-}
-// Cell data of the half-edge fluxes on layer k, formed in FP64 and rounded to R; with
-// STATIC false, hc already holds he_cell_static's part.
-template <typename R, int MODE, bool STATIC = true>
+// Cell data of the half-edge fluxes on layer k, formed in FP64 and rounded to R.
+template <typename R, int MODE>
 __device__ inline void he_cell_load(const Dev& P, int c, int k, HeCell<R>& hc) {
   size_t ck = C3(P, c, k);
   if (MODE == 0) {
     size_t ckm = C3(P, c, k - 1);
-    hc.uq = (R)((P.u[ck] * P.dz1[ckm] + P.u[ckm] * P.dz1[ck]) / (P.dz1[ck] + P.dz1[ckm]));
-    hc.vq = (R)((P.v[ck] * P.dz1[ckm] + P.v[ckm] * P.dz1[ck]) / (P.dz1[ck] + P.dz1[ckm]));
+    const double za = P.dz1[ckm], zb = P.dz1[ck], zs = zb + za;
+    hc.uq = (R)((P.u[ck] * za + P.u[ckm] * zb) / zs);
+    hc.vq = (R)((P.v[ck] * za + P.v[ckm] * zb) / zs);
     hc.dtij = (R)(P.dt1[c] * P.dzz1[ckm]);
   } else {
     hc.uq = (R)P.u[ck];
     hc.vq = (R)P.v[ck];
     hc.dtij = (R)(P.dt1[c] * P.dz1[ck]);
   }
-  if (STATIC) he_cell_static<R>(P, c, hc);
-  for (int j = 0; j < 3; ++j) {
-    if (sizeof(R) == 4) continue;  // FP32: VISCOFH travels in the node records
-    const int n = hc.nd[j];
-    size_t q = N3(P, n, k);
-    if (MODE == 0) {
-      size_t qm = N3(P, n, k - 1);
-      hc.vf[j] = (R)((P.viscofh[q] * P.dz[qm] + P.viscofh[qm] * P.dz[q]) / (P.dz[q] + P.dz[qm]));
-    } else {
-      hc.vf[j] = (R)P.viscofh[q];
-    }
-  }
 }
 
-// v[j] for a run-time slot j in 0..2, by selects, so v stays in registers.
-template <typename R>
-__device__ inline R sel3(const R* v, int j) { return j == 0 ? v[0] : (j == 1 ? v[1] : v[2]); }
-__device__ inline int sel3i(const int* v, int j) { return j == 0 ? v[0] : (j == 1 ? v[1] : v[2]); }
-
-// Metrics of one half-edge (DLTXE, DLTYE and the DLTXNCVE/DLTYNCVE of both sides), read
+// Metrics of one half-edge (DLTXE, DLTYE and the DLTXNCVE/DLTYNCVE of X(s) and X(s+1)), read
 // by position (coalesced over the threads of consecutive cells).
 template <typename R>
 struct HeGeo {
@@ -340,53 +316,54 @@ __device__ inline HeGeo<R> he_geo(const Dev& P, size_t pos) {
   }
 }
 
-// EXFLUX of a half-edge with metrics g for tracer t, in R; a and b are the positions of
-// NIEC(he,1) and NIEC(he,2) among the cell's nodes, ra and rb their data.  xadv receives
-// EXFLUX-FXX-FYY.
+// VISCOFH*NN_HVC of a node as the half-edge fluxes take it (in FP32 from its record).
+template <typename R>
+__device__ inline R he_vn(const Dev& P, int n, int k, R nn, R vf) {
+  if constexpr (sizeof(R) == 4)
+    return vf * nn;
+  else
+    return P.gvn[N3(P, n, k)];
+}
+// Horizontal viscosity of a half-edge from its nodes' VISCOFH*NN_HVC and NN_HVC.
 template <typename R, int MODE>
-__device__ inline R he_flux(const Dev& P, const HeCell<R>& hc, const HeGeo<R>& g, int a, int b, const TRec<R>& ra,
-                            const TRec<R>& rb, R* xadv) {
+__device__ inline R he_visc(const Dev& P, R vna, R vnb, R nna, R nnb) {
+  const R half = (R)0.5;
+  R viscof = (R)P.fact * half * (vna + vnb) + (R)P.fm1 * half * (nna + nnb);
+  if (MODE == 0 && P.hprnu != 1.0) viscof = viscof / (R)P.hprnu;
+  return viscof;
+}
+// The bounds of a node's face values: its ring and itself.
+template <typename R>
+__device__ inline void he_bounds(TRec<R>& r) {
+  r.rmin = fmin(r.rmin, r.q);
+  r.rmax = fmax(r.rmax, r.q);
+}
+
+// EXFLUX of a half-edge with metrics g for one tracer, in R; ra and rb are the records of
+// X(s) and X(s+1) with their bounds (he_bounds), flip the slot's bit of hex, viscof its
+// viscosity.  xadv receives EXFLUX-FXX-FYY.
+template <typename R>
+__device__ inline R he_flux(const HeCell<R>& hc, const HeGeo<R>& g, int flip, const TRec<R>& ra, const TRec<R>& rb,
+                            R viscof, R* xadv) {
   const R half = (R)0.5, one = (R)1.0;
   const R dltxe = g.dx, dltye = g.dy;
   R un = hc.vq * dltxe - hc.uq * dltye;
-  R fij1 = ra.q + g.xa * ra.px + g.ya * ra.py;
-  R fij2 = rb.q + g.xb * rb.px + g.yb * rb.py;
-  R q1min = fmin(ra.rmin, ra.q), q1max = fmax(ra.rmax, ra.q);
-  R q2min = fmin(rb.rmin, rb.q), q2max = fmax(rb.rmax, rb.q);
-  if (fij1 < q1min) fij1 = q1min;
-  if (fij1 > q1max) fij1 = q1max;
-  if (fij2 < q2min) fij2 = q2min;
-  if (fij2 > q2max) fij2 = q2max;
-  const R vfa = sizeof(R) == 4 ? ra.vf : sel3(hc.vf, a), vfb = sizeof(R) == 4 ? rb.vf : sel3(hc.vf, b);
-  const R nna = sel3(hc.nn, a), nnb = sel3(hc.nn, b);
-  R viscof = (R)P.fact * half * (vfa * nna + vfb * nnb) + (R)P.fm1 * half * (nna + nnb);
-  if (MODE == 0) viscof = viscof / (R)P.hprnu;
+  R fa = ra.q + g.xa * ra.px + g.ya * ra.py;
+  R fb = rb.q + g.xb * rb.px + g.yb * rb.py;
+  if (fa < ra.rmin) fa = ra.rmin;
+  if (fa > ra.rmax) fa = ra.rmax;
+  if (fb < rb.rmin) fb = rb.rmin;
+  if (fb > rb.rmax) fb = rb.rmax;
   R txx = half * (ra.pxd + rb.pxd) * viscof;
   R tyy = half * (ra.pyd + rb.pyd) * viscof;
   R fxx = -hc.dtij * txx * dltye;
   R fyy = hc.dtij * tyy * dltxe;
   R sg = fsign1(un);
-  R exflux = -un * hc.dtij * ((one + sg) * fij2 + (one - sg) * fij1) * half + fxx + fyy;
+  if (flip) sg = -sg;
+  R exflux = -un * hc.dtij * ((one + sg) * fb + (one - sg) * fa) * half + fxx + fyy;
   if (xadv) *xadv = exflux - fxx - fyy;
   return exflux;
 }
-
-template <typename R>
-__device__ inline TRec<R> sel_trec(const TRec<R>& a, const TRec<R>& b, const TRec<R>& c, int j) {
-  TRec<R> r;
-  r.q = j == 0 ? a.q : (j == 1 ? b.q : c.q);
-  r.px = j == 0 ? a.px : (j == 1 ? b.px : c.px);
-  r.py = j == 0 ? a.py : (j == 1 ? b.py : c.py);
-  r.pxd = j == 0 ? a.pxd : (j == 1 ? b.pxd : c.pxd);
-  r.pyd = j == 0 ? a.pyd : (j == 1 ? b.pyd : c.pyd);
-  r.rmin = j == 0 ? a.rmin : (j == 1 ? b.rmin : c.rmin);
-  r.rmax = j == 0 ? a.rmax : (j == 1 ? b.rmax : c.rmax);
-  r.vf = j == 0 ? a.vf : (j == 1 ? b.vf : c.vf);
-  return r;
-}
-
-template <typename R>
-__device__ inline int pos3(const HeCell<R>& hc, int n) { return n == hc.nd[0] ? 0 : (n == hc.nd[1] ? 1 : 2); }
 
 template <typename R, int MODE>
 __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 3 : 2) k_he_adv(const Dev P, int parts) {
@@ -395,36 +372,35 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 3 : 2) k_he_adv(const De
   if (c > P.N) return;
   int kb, ke;
   col_range(P, MODE == 0 ? 2 : 1, P.KBM1, kb, ke);
-  const size_t v1 = P.NCV + 1;
   const bool do0 = parts & (MODE == 0 ? AD_Q2 : AD_T), do1 = parts & (MODE == 0 ? AD_Q2L : AD_S);
-  int pa[3], pb[3];
-  {
-    int nd0 = P.nv[c], nd1 = P.nv[(size_t)(P.N + 1) + c];
-    for (int s = 0; s < 3; ++s) {
-      int he = P.cell_he[3 * c + s];
-      int na = P.niec[he], nb = P.niec[v1 + he];
-      pa[s] = na == nd0 ? 0 : (na == nd1 ? 1 : 2);
-      pb[s] = nb == nd0 ? 0 : (nb == nd1 ? 1 : 2);
-    }
-  }
-  // Each of the cell's three nodes ends two of its half-edges: its record is loaded once
-  // per tracer and layer and handed to both.  The metrics and the fluxes are by position
-  // s*ns + c.  For Q2/Q2L the cell's nodes are loaded once for the layers this thread
-  // walks (for T/S, which hold more live values, that spills: they are reloaded per layer).
+  const int4 hx = P.hex[c];
+  const R nn0 = (R)P.nn_hvc[hx.x], nn1 = (R)P.nn_hvc[hx.y], nn2 = (R)P.nn_hvc[hx.z];
+  // Each node's record is loaded once per tracer and layer and serves its two half-edges.
   HeCell<R> hc;
-  if (MODE == 0) he_cell_static<R>(P, c, hc);
   for (int k = kb; k <= ke; ++k) {
-    he_cell_load<R, MODE, MODE != 0>(P, c, k, hc);
+    he_cell_load<R, MODE>(P, c, k, hc);
     R2* EX = Mesh<R>::ex2(P) + (size_t)(k - 1) * P.ncvs + c;
     R e[2][3] = {{0, 0, 0}, {0, 0, 0}};
+    R vs0 = 0, vs1 = 0, vs2 = 0;
+#pragma unroll
     for (int t = 0; t < 2; ++t) {
       if (!(t == 0 ? do0 : do1)) continue;
-      const TRec<R> r0 = load_trec<R, MODE>(P, hc.nd[0], k, t);
-      const TRec<R> r1 = load_trec<R, MODE>(P, hc.nd[1], k, t);
-      const TRec<R> r2 = load_trec<R, MODE>(P, hc.nd[2], k, t);
-      for (int s = 0; s < 3; ++s)
-        e[t][s] = he_flux<R, MODE>(P, hc, he_geo<R>(P, (size_t)s * P.ns + c), pa[s], pb[s],
-                                   sel_trec(r0, r1, r2, pa[s]), sel_trec(r0, r1, r2, pb[s]), nullptr);
+      TRec<R> r0 = load_trec<R, MODE>(P, hx.x, k, t);
+      TRec<R> r1 = load_trec<R, MODE>(P, hx.y, k, t);
+      TRec<R> r2 = load_trec<R, MODE>(P, hx.z, k, t);
+      if (t == 0 || !do0) {  // the mixing is the same for both tracers
+        const R v0 = he_vn<R>(P, hx.x, k, nn0, r0.vf), v1 = he_vn<R>(P, hx.y, k, nn1, r1.vf),
+                v2 = he_vn<R>(P, hx.z, k, nn2, r2.vf);
+        vs0 = he_visc<R, MODE>(P, v0, v1, nn0, nn1);
+        vs1 = he_visc<R, MODE>(P, v1, v2, nn1, nn2);
+        vs2 = he_visc<R, MODE>(P, v2, v0, nn2, nn0);
+      }
+      he_bounds(r0);
+      he_bounds(r1);
+      he_bounds(r2);
+      e[t][0] = he_flux<R>(hc, he_geo<R>(P, c), hx.w & 1, r0, r1, vs0, nullptr);
+      e[t][1] = he_flux<R>(hc, he_geo<R>(P, (size_t)P.ns + c), hx.w & 2, r1, r2, vs1, nullptr);
+      e[t][2] = he_flux<R>(hc, he_geo<R>(P, (size_t)2 * P.ns + c), hx.w & 4, r2, r0, vs2, nullptr);
     }
     for (int s = 0; s < 3; ++s) EX[(size_t)s * P.ns] = mk2(e[0][s], e[1][s]);
   }
@@ -434,19 +410,23 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 3 : 2) k_he_adv(const De
 // its half-edge fluxes, recomputed with the same arithmetic as phase 1.
 template <typename R>
 __device__ inline double obc_xflux_adv(const Dev& P, int i, int k, int t) {
-  const size_t v1 = P.NCV + 1;
   R xa = 0;
   for (int q = P.node_he_ptr[i]; q < P.node_he_ptr[i + 1]; ++q) {
     int code = P.node_he[q];
     int he = code >> 1;
     int c = P.ntrg[he];
     const int sl = P.cell_he[3 * c] == he ? 0 : (P.cell_he[3 * c + 1] == he ? 1 : 2);
+    const int4 hx = P.hex[c];
+    const int na = sl == 0 ? hx.x : (sl == 1 ? hx.y : hx.z), nb = sl == 0 ? hx.y : (sl == 1 ? hx.z : hx.x);
     HeCell<R> hc;
     he_cell_load<R, 1>(P, c, k, hc);
-    const int na = P.niec[he], nb = P.niec[v1 + he];
+    TRec<R> ra = load_trec<R, 1>(P, na, k, t), rb = load_trec<R, 1>(P, nb, k, t);
+    const R nna = (R)P.nn_hvc[na], nnb = (R)P.nn_hvc[nb];
+    const R visc = he_visc<R, 1>(P, he_vn<R>(P, na, k, nna, ra.vf), he_vn<R>(P, nb, k, nnb, rb.vf), nna, nnb);
+    he_bounds(ra);
+    he_bounds(rb);
     R part;
-    he_flux<R, 1>(P, hc, he_geo<R>(P, (size_t)sl * P.ns + c), pos3(hc, na), pos3(hc, nb),
-                  load_trec<R, 1>(P, na, k, t), load_trec<R, 1>(P, nb, k, t), &part);
+    he_flux<R>(hc, he_geo<R>(P, (size_t)sl * P.ns + c), (hx.w >> sl) & 1, ra, rb, visc, &part);
     xa = (code & 1) ? xa - part : xa + part;
   }
   return (double)xa;
