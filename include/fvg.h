@@ -312,8 +312,8 @@ int fvg_closure_status(fvg_handle* h, int32_t* columns_on_network, int32_t* wait
                    fvg_get_tuning("compact") reports whether the compact kernel is in use;
    "staged"      = 2 runs ADVECTION_EDGE_GCN and ADV_UV_EDGE_GCN (LIMITED_NO, GCN) as the
                    tile-staged kernels (neighbour cells in shared memory, each edge
-                   evaluated once per tile); 1 (default) only the FP64 ADV_UV, where the
-                   staged kernel measured faster; 0 keeps one thread per cell everywhere.
+                   evaluated once per tile); 1 (default) and 0 one thread per cell, which
+                   measured faster in every form.
                    Results do not depend on it (bit for bit in FP64);
    "stream_hints" = 1 (default): the external loop's stage kernels load the arrays a
                    stage reads once (gather lists, slot records, EXTUV's fixed terms, the
@@ -323,7 +323,11 @@ int fvg_closure_status(fvg_handle* h, int32_t* columns_on_network, int32_t* wait
    "ext_grid"     = blocks per SM (1..8, default 8) of the external loop's compact cell
                    kernel, launched as one wave whose threads walk the cells so that no
                    partly filled last wave is left; 0 launches one thread per cell.
-                   Results do not depend on it. */
+                   Results do not depend on it;
+   "ext_loop"     = 1 (default): the external loop of a mesh of at most 384 cells per SM runs
+                   as one resident cooperative kernel (no limiter; the FP32-flux form with
+                   the compact kernel's records); 0 launches every stage.  FP64 results do
+                   not depend on it; fvg_get_tuning reports whether it is in use. */
 int fvg_set_tuning(fvg_handle* h, const char* key, int32_t value);
 int fvg_get_tuning(const fvg_handle* h, const char* key, int32_t* value);
 

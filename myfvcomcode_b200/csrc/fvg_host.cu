@@ -58,7 +58,7 @@ struct fvg_handle {
   int compact_allowed = 1;
   int compact_ok = 0;
   // resident external loop: allowed (tuning key "ext_loop"), possible (the device launches
-  // cooperatively, every cell's three edges are its three sides)
+  // cooperatively)
   int ext_loop = 1;
   int loop_ok = 0;
 };
@@ -625,12 +625,12 @@ int fvg_create(const fvg_mesh* m, const fvg_params* prm, const fvg_forcing* f, f
               seen |= 1 << sl;
               if (j == 2) bits |= sl << 6;
             }
-        if (seen != 7) h->loop_ok = 0;
+        if (seen != 7) { h->err = "cell whose three edges are not its sides"; return fail(FVG_ERR_BOUNDS); }
         for (int sl = 0; sl < 3; ++sl) {
           const int e = cl[i][sl] >> 1, side = cl[i][sl] & 1;
           bits |= side << sl | (m->isbc[e] != 0 ? 1 : 0) << (3 + sl);
           lo[4 * i + sl] = side == 0 ? m->iec[e1 + e] : m->iec[e];
-          lx[4 * i + sl] = x[sl] > 0 ? x[sl] : 1;
+          lx[4 * i + sl] = x[sl];
         }
         lx[4 * i + 3] = bits;
         hm[i] = std::fmin(std::fmin(m->h[m->nv[i]], m->h[m->nv[n1 + i]]), m->h[m->nv[2 * n1 + i]]);
@@ -913,6 +913,7 @@ int fvg_create(const fvg_mesh* m, const fvg_params* prm, const fvg_forcing* f, f
   if ((rc = dalloc(h, &P.exf2d, 3 * ns))) return fail(rc);
   for (int q = 0; q < 4; ++q)
     if ((rc = dalloc(h, &P.g3[q], ns * KB))) return fail(rc);
+  if ((rc = dalloc(h, &P.vc3, ns * KB))) return fail(rc);
   if ((rc = dalloc(h, (double**)&P.ex2, (size_t)P.ncvs * KB * 2))) return fail(rc);
   P.he_vflux = (double*)P.ex2;
 
@@ -1226,6 +1227,7 @@ int fvg_set_precision(fvg_handle* h, int32_t mode) {
     F32& f = P.f;
     auto fail = [&](int r) { return r; };
     if ((rc = dalloc(h, (float**)&f.g34, 4 * ns * KB))) return fail(rc);
+    if ((rc = dalloc(h, &f.vc3, ns * KB))) return fail(rc);
     if ((rc = dalloc(h, (float**)&f.g2d4, 4 * n1))) return fail(rc);
     if (P.limiter) {
       std::vector<float> ones(std::max(n1, ns * KB), 1.0f);

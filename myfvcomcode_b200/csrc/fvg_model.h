@@ -42,6 +42,7 @@ struct SchedLayout {
 // and rounded once: xo[e] = XIJC(e)-XC(IEC(e,1)), xo[NE+1+e] = XIJC(e)-XC(IEC(e,2)), the
 // same for y.
 struct F32 {
+  float* vc3;   // Dev::vc3 in FP32
   float4* g34;  // least-squares gradient of U, V per cell and layer {UX, UY, VX, VY} (ns x KB)
   float *alfa2[2], *alfa3[2];  // slope limiters UALFA, VALFA (see Dev)
   float* npk;  // node records of the ring gradients, 16 floats per (node, layer)
@@ -245,6 +246,7 @@ struct Dev {
   double *alfa2[2], *alfa3[2];
   double* exf2d;                             // EXTEL_EDGE flux of each half-edge position (ncvs)
   double* g3[4];                             // least-squares gradient of U, V per cell and layer (ns x KB)
+  double* vc3;  // ART*|grad U,V|*CC_HVC per cell and layer: the cell's part of its edges' viscosity
   int ncvs;                                  // layer stride of the half-edge arrays by position (3*ns)
   // Precision form (fvg_set_precision): 0 = FP64 everywhere; 1 = the edge fluxes and
   // advection (ADVAVE's edge loop, the 3-D momentum edge fluxes, ADV_Q/ADV_T/ADV_S with
@@ -275,8 +277,8 @@ struct Dev {
   int *clos_list, *clos_cnt;
   int* clos_err;
   Tiles tl;
-  // 1: ADVECTION_EDGE_GCN and ADV_UV_EDGE_GCN run as the tile-staged kernels (no limiter,
-  // GCN); 0: one thread per cell gathering its neighbours (tuning key "staged").
+  // 2: ADVECTION_EDGE_GCN and ADV_UV_EDGE_GCN run as the tile-staged kernels (no limiter,
+  // GCN); 0, 1: one thread per cell gathering its neighbours (tuning key "staged").
   int staged;
   // Column tiling of the 3-D gather kernels: col_bc threads (entities) per block, each
   // walking col_lc consecutive layers, so the entity's index chain (cell -> edge ->
@@ -437,6 +439,7 @@ template <> struct Mesh<double> {
   __device__ static double* alfa2(const Dev& P, int q) { return P.alfa2[q]; }
   __device__ static double* alfa3(const Dev& P, int q) { return P.alfa3[q]; }
   __device__ static double* g3(const Dev& P, int q) { return P.g3[q]; }
+  __device__ static double* vc3(const Dev& P) { return P.vc3; }
   __device__ static double2* ex2(const Dev& P) { return P.ex2; }
   __device__ static double hg(const Dev& P, int j, size_t pos) { return P.hg[(size_t)j * P.ncvs + pos]; }
 };
@@ -464,6 +467,7 @@ template <> struct Mesh<float> {
   __device__ static float* alfa2(const Dev& P, int q) { return P.f.alfa2[q]; }
   __device__ static float* alfa3(const Dev& P, int q) { return P.f.alfa3[q]; }
   __device__ static float2* ex2(const Dev& P) { return P.f.ex2; }
+  __device__ static float* vc3(const Dev& P) { return P.f.vc3; }
 };
 // The cell's NBE and its least-squares coefficients A1U(c,1..4), A2U(c,1..4) in the
 // form's type (FP32: one packed load each).

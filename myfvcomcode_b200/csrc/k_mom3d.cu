@@ -167,9 +167,14 @@ __global__ void __launch_bounds__(256) k_grad3(const Dev P) {
   if (i > P.N) return;
   int kb, ke;
   col_range(P, 1, P.KBM1, kb, ke);
+  const R art = Mesh<R>::art(P, i), cc = Mesh<R>::cc_hvc(P, i);
   for (int k = kb; k <= ke; ++k) {
     G3<R> g = grad3<R>(P, i, P.u + C3(P, 0, k), P.v + C3(P, 0, k));
     size_t q = C3(P, i, k);
+    // ART*|grad|*CC_HVC, the cell's part of its three edges' viscosity
+    const R half = (R)0.5;
+    Mesh<R>::vc3(P)[q] =
+        art * sqrt(g.ux * g.ux + g.vy * g.vy + half * ((g.uy + g.vx) * (g.uy + g.vx))) * cc;
     if constexpr (sizeof(R) == 4) {
       P.f.g34[q] = make_float4(g.ux, g.uy, g.vx, g.vy);
     } else {
@@ -212,19 +217,10 @@ __global__ void __launch_bounds__(256) k_alfa3(const Dev P) {
   }
 }
 
-// q: the edge's slot in the cell slot table (offsets and DLTXC/DLTYC of the edge).
-// The cell's own side of its edges on one layer, loaded once for its three edges.
+// Limited schemes.  q: the edge's slot in the cell slot table (offsets and DLTXC/DLTYC of the
+// edge).
 template <typename R>
-struct Own3 {
-  G3<R> g;
-  R u, v, art, cc;
-};
-
-// OWN (FP32 form, no limiter): `own` holds the values of the cell on the edge's `side`
-// (0: IA, 1: IB), so that only the other cell is gathered.
-template <typename R, bool LIM, bool OWN = false>
-__device__ inline EdgeFlux<R> edge_flux3(const Dev& P, size_t q, int ia, int ib, int k, R dij, bool exflux_form,
-                                         const Own3<R>& own = Own3<R>(), int side = 0) {
+__device__ inline EdgeFlux<R> edge_flux3(const Dev& P, size_t q, int ia, int ib, int k, R dij, bool exflux_form) {
   typedef Mesh<R> Mh;
   const R half = (R)0.5, one = (R)1.0;
   const double* U = P.u + C3(P, 0, k);
@@ -235,49 +231,17 @@ __device__ inline EdgeFlux<R> edge_flux3(const Dev& P, size_t q, int ia, int ib,
   G3<R> ga, gb;
   R uij1, vij1, uij2, vij2;
   R arta, artb, cca, ccb;
-  if constexpr (!LIM) {
-    if constexpr (OWN) {
-      const int o = side == 0 ? ib : ia;
-      const G3<R> go = load_g3<R>(P, o, k);
-      const R uo = (R)U[o], vo = (R)V[o];
-      ga = side == 0 ? own.g : go;
-      gb = side == 0 ? go : own.g;
-      const R ua = side == 0 ? own.u : uo, va = side == 0 ? own.v : vo;
-      const R ub = side == 0 ? uo : own.u, vb = side == 0 ? vo : own.v;
-      uij1 = ua + ga.ux * xija + ga.uy * yija;
-      vij1 = va + ga.vx * xija + ga.vy * yija;
-      uij2 = ub + gb.ux * xijb + gb.uy * yijb;
-      vij2 = vb + gb.vx * xijb + gb.vy * yijb;
-      const R arto = Mh::art(P, o), cco = Mh::cc_hvc(P, o);
-      arta = side == 0 ? own.art : arto;
-      artb = side == 0 ? arto : own.art;
-      cca = side == 0 ? own.cc : cco;
-      ccb = side == 0 ? cco : own.cc;
-    } else {
-      ga = load_g3<R>(P, ia, k);
-      uij1 = (R)U[ia] + ga.ux * xija + ga.uy * yija;
-      vij1 = (R)V[ia] + ga.vx * xija + ga.vy * yija;
-      gb = load_g3<R>(P, ib, k);
-      uij2 = (R)U[ib] + gb.ux * xijb + gb.uy * yijb;
-      vij2 = (R)V[ib] + gb.vx * xijb + gb.vy * yijb;
-      arta = Mh::art(P, ia);
-      artb = Mh::art(P, ib);
-      cca = Mh::cc_hvc(P, ia);
-      ccb = Mh::cc_hvc(P, ib);
-    }
-  } else {
-    arta = Mh::art(P, ia);
-    artb = Mh::art(P, ib);
-    cca = Mh::cc_hvc(P, ia);
-    ccb = Mh::cc_hvc(P, ib);
-    ga = load_g3<R>(P, ia, k);
-    gb = load_g3<R>(P, ib, k);
-    const size_t qa = C3(P, ia, k), qb = C3(P, ib, k);
-    lim_faces<R>(P.limiter, (R)U[ia], (R)U[ib], ga.ux * xija + ga.uy * yija, gb.ux * xijb + gb.uy * yijb,
-                 Mh::alfa3(P, 0)[qa], Mh::alfa3(P, 0)[qb], uij1, uij2);
-    lim_faces<R>(P.limiter, (R)V[ia], (R)V[ib], ga.vx * xija + ga.vy * yija, gb.vx * xijb + gb.vy * yijb,
-                 Mh::alfa3(P, 1)[qa], Mh::alfa3(P, 1)[qb], vij1, vij2);
-  }
+  arta = Mh::art(P, ia);
+  artb = Mh::art(P, ib);
+  cca = Mh::cc_hvc(P, ia);
+  ccb = Mh::cc_hvc(P, ib);
+  ga = load_g3<R>(P, ia, k);
+  gb = load_g3<R>(P, ib, k);
+  const size_t qa = C3(P, ia, k), qb = C3(P, ib, k);
+  lim_faces<R>(P.limiter, (R)U[ia], (R)U[ib], ga.ux * xija + ga.uy * yija, gb.ux * xijb + gb.uy * yijb,
+               Mh::alfa3(P, 0)[qa], Mh::alfa3(P, 0)[qb], uij1, uij2);
+  lim_faces<R>(P.limiter, (R)V[ia], (R)V[ib], ga.vx * xija + ga.vy * yija, gb.vx * xijb + gb.vy * yijb,
+               Mh::alfa3(P, 1)[qa], Mh::alfa3(P, 1)[qb], vij1, vij2);
   R uij = half * (uij1 + uij2);
   R vij = half * (vij1 + vij2);
   R viscof1 = arta * sqrt(ga.ux * ga.ux + ga.vy * ga.vy + half * ((ga.uy + ga.vx) * (ga.uy + ga.vx)));
@@ -345,8 +309,8 @@ __device__ inline void advection3d_tail(const Dev& P, int i, int k, R xr, R yr) 
 // ADVECTION_EDGE_GCN (advection_edge_gcn.F:397-708): per cell and layer, the cell's three
 // edges in ascending edge number.
 // -------------------------------------------------------------------------------------
-template <typename R, bool LIM>
-__global__ void __launch_bounds__(256, (sizeof(R) == 4 && !LIM) ? 4 : 1) k_advection3d(const Dev P) {
+template <typename R>
+__global__ void __launch_bounds__(256) k_advection3d(const Dev P) {
   int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
   if (i > P.N) return;
   int kb, ke;
@@ -355,16 +319,6 @@ __global__ void __launch_bounds__(256, (sizeof(R) == 4 && !LIM) ? 4 : 1) k_advec
   const size_t n1 = P.N + 1;
   const R epor = (R)P.epor[i], three = (R)3.0;
   R xr = 0, yr = 0;
-    // FP32 form without a limiter: the cell's own side of its three edges, once
-    constexpr bool OWN = !LIM && sizeof(R) == 4;
-    Own3<R> own;
-    if constexpr (OWN) {
-      own.g = load_g3<R>(P, i, k);
-      own.u = (R)P.u[C3(P, i, k)];
-      own.v = (R)P.v[C3(P, i, k)];
-      own.art = Mesh<R>::art(P, i);
-      own.cc = Mesh<R>::cc_hvc(P, i);
-    }
   for (int s = 0; s < 3; ++s) {
     const size_t q = (size_t)s * n1 + i;
     const int4 ci = P.ce_i4[q];  // {code, IA, IB, J1}
@@ -373,7 +327,7 @@ __global__ void __launch_bounds__(256, (sizeof(R) == 4 && !LIM) ? 4 : 1) k_advec
     if (!(P.iswetct[ia] * P.iswetc[ia] == 1 || P.iswetct[ib] * P.iswetc[ib] == 1)) continue;
     const int j1 = ci.w, j2 = P.ce_j2[q];
     R dij = (R)(0.5 * (P.dt[j1] * P.dz[N3(P, j1, k)] + P.dt[j2] * P.dz[N3(P, j2, k)]));
-    EdgeFlux<R> f = edge_flux3<R, LIM, OWN>(P, q, ia, ib, k, dij, false, own, side);
+    EdgeFlux<R> f = edge_flux3<R>(P, q, ia, ib, k, dij, false);
     R isb = (R)isbc;
     R tp = (R)((double)(float)(1 - isbc) * P.epor[i]);
     // viscous part: GCN (fxx + 3 fxx ISBC) EPOR; GCY (advection_edge_gcy.F) fxx TPA
@@ -781,8 +735,8 @@ __device__ inline void adv_uv_tail(const Dev& P, int i, int k, R xr, R yr, R vmr
 // internal barotropic pressure gradient from EGF, vertical advection, baroclinic
 // pressure gradient, Coriolis, river momentum and the explicit update to UF/VF.
 // -------------------------------------------------------------------------------------
-template <typename R, bool LIM>
-__global__ void __launch_bounds__(256, (sizeof(R) == 4 && !LIM) ? 4 : 1) k_adv_uv(const Dev P) {
+template <typename R>
+__global__ void __launch_bounds__(256) k_adv_uv(const Dev P) {
   int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
   if (i > P.N) return;
   int kb, ke;
@@ -794,16 +748,6 @@ __global__ void __launch_bounds__(256, (sizeof(R) == 4 && !LIM) ? 4 : 1) k_adv_u
   R xr = 0, yr = 0, vmr = 0;
   const double dz1i = P.dz1[C3(P, i, k)];
   const double gdd = P.grav_e[i] * P.dt1[i] * dz1i;
-    // FP32 form without a limiter: the cell's own side of its three edges, once
-    constexpr bool OWN = !LIM && sizeof(R) == 4;
-    Own3<R> own;
-    if constexpr (OWN) {
-      own.g = load_g3<R>(P, i, k);
-      own.u = (R)P.u[C3(P, i, k)];
-      own.v = (R)P.v[C3(P, i, k)];
-      own.art = Mesh<R>::art(P, i);
-      own.cc = Mesh<R>::cc_hvc(P, i);
-    }
   for (int s = 0; s < 3; ++s) {
     const size_t q = (size_t)s * n1 + i;
     const int4 ci = P.ce_i4[q];  // {code, IA, IB, J1}
@@ -813,7 +757,7 @@ __global__ void __launch_bounds__(256, (sizeof(R) == 4 && !LIM) ? 4 : 1) k_adv_u
     double elij = 0.5 * (P.egf[j1] + P.egf[j2]);
     R dij = (R)(0.5 * (P.dt[j1] * P.dz[N3(P, j1, k)] + P.dt[j2] * P.dz[N3(P, j2, k)]));
     if (P.iswetct[ia] * P.iswetc[ia] == 1 || P.iswetct[ib] * P.iswetc[ib] == 1) {
-      EdgeFlux<R> f = edge_flux3<R, LIM, OWN>(P, q, ia, ib, k, dij, true, own, side);
+      EdgeFlux<R> f = edge_flux3<R>(P, q, ia, ib, k, dij, true);
       vmr = vmr + f.viscof;
       R isb = (R)isbc;
       R tp = (R)((double)(float)(1 - isbc) * P.epor[i]);
@@ -837,6 +781,205 @@ __global__ void __launch_bounds__(256, (sizeof(R) == 4 && !LIM) ? 4 : 1) k_adv_u
     }
   }
   adv_uv_tail<R>(P, i, k, xr, yr, vmr, px, py, dz1i);
+  }
+}
+
+// -------------------------------------------------------------------------------------
+// ADVECTION_EDGE_GCN (UV = false) and ADV_UV_EDGE_GCN (UV = true) without a limiter, one
+// thread per cell walking a chunk of layers.  These kernels were bound by instructions (about
+// 1,000 per cell and layer at 40 % of the issue slots and 23 % occupancy), so:
+//   * an edge is evaluated as the cell sees it, its own values loaded once per layer; sums
+//     that commute need no sides, the others select one operand, and the upwind weights
+//     take the cell's side as a sign;
+//   * the viscosity's ART*|grad|*CC_HVC comes from the gradient kernel once per cell (vc3)
+//     instead of two square roots per edge;
+//   * the edges' cells, nodes, depths and wet flags are resolved once for the layers;
+//   * ADV_UV's vertical flux through a layer's lower interface is the next layer's upper one.
+// The terms and their order are the reference's: FP64 results are bit for bit those of the
+// per-edge evaluation.
+// -------------------------------------------------------------------------------------
+template <typename R, bool UV>
+__global__ void __launch_bounds__(128, sizeof(R) == 4 ? (UV ? 6 : 7) : 4) k_mom3d(const Dev P) {
+  typedef Mesh<R> Mh;
+  const R half = (R)0.5, one = (R)1.0, three = (R)3.0;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
+  if (i > P.N) return;
+  int kb, ke;
+  col_range(P, 1, P.KBM1, kb, ke);
+  const size_t n1 = P.N + 1;
+  const int4 xn = P.loopx[i], oo = P.loopo[i];  // nodes and other cells by slot (see loopx)
+  const int xs[3] = {xn.x, xn.y, xn.z}, os[3] = {oo.x, oo.y, oo.z};
+  const int bits = xn.w;
+  const int weti = P.iswetct[i] * P.iswetc[i];
+  double dts[3], els[3] = {0.0, 0.0, 0.0};
+  int on = 0;
+#pragma unroll
+  for (int s = 0; s < 3; ++s) {
+    dts[s] = P.dt[xs[s]];
+    if (UV) els[s] = P.egf[xs[s]];
+    if (weti == 1 || P.iswetct[os[s]] * P.iswetc[os[s]] == 1) on |= 1 << s;
+  }
+  const double epord = P.epor[i];
+  const R epor = (R)epord;
+  const bool wet = weti == 1, ob = P.isbce[i] == 2;
+  const double w = (double)weti;
+  const bool rivers = P.cell_riv_ptr[i + 1] > P.cell_riv_ptr[i];
+  double art = 0.0, dt1 = 0.0, d1 = 0.0, gd = 0.0;
+  // ADV_UV: U, V, DZ1 of the layer above and the flux through the upper interface
+  double um = 0.0, vm = 0.0, zm = 0.0, xtop = 0.0, ytop = 0.0;
+  double ui_d = P.u[C3(P, i, kb)], vi_d = P.v[C3(P, i, kb)], z = 0.0;
+  if (UV) {
+    art = P.art[i];
+    dt1 = P.dt1[i];
+    d1 = P.d1[i];
+    gd = P.grav_e[i] * dt1;
+    z = P.dz1[C3(P, i, kb)];
+    if (kb > 1) {
+      const size_t qm = C3(P, i, kb - 1);
+      um = P.u[qm];
+      vm = P.v[qm];
+      zm = P.dz1[qm];
+      const double wk = P.w[C3(P, i, kb)];
+      xtop = wk * (ui_d * zm + um * z) / (z + zm);
+      ytop = wk * (vi_d * zm + vm * z) / (z + zm);
+    }
+  }
+  for (int k = kb; k <= ke; ++k) {
+    const size_t base = C3(P, 0, k), nbase = N3(P, 0, k);
+    const double *U = P.u + base, *V = P.v + base, *DZ = P.dz + nbase;
+    const G3<R> gi = load_g3<R>(P, i, k);
+    const R* VC = Mh::vc3(P) + base;
+    const R vci = VC[i], ui = (R)ui_d, vi = (R)vi_d;
+    const double dd[3] = {dts[0] * DZ[xs[0]], dts[1] * DZ[xs[1]], dts[2] * DZ[xs[2]]};
+    const double gdd = gd * z;
+    R xr = 0, yr = 0, vmr = 0;
+    double px = 0.0, py = 0.0;
+#pragma unroll
+    for (int s = 0; s < 3; ++s) {
+      const int side = (bits >> s) & 1, isbc = (bits >> (3 + s)) & 1, o = os[s];
+      const size_t q = (size_t)s * n1 + i;
+      double edx, edy;
+      if (UV || sizeof(R) == 8) {
+        edx = P.ce_dx[q];
+        edy = P.ce_dy[q];
+      }
+      if (on >> s & 1) {
+        const R dij = (R)(0.5 * (dd[s] + dd[(s + 1) % 3]));
+        R xi, yi, xo, yo, dx, dy;
+        if constexpr (sizeof(R) == 4) {
+          const float4 G = P.f.ce_geo[q];  // XOA, YOA, XOB, YOB
+          const float2 D = P.f.ce_dd[q];
+          xi = side ? G.z : G.x;
+          yi = side ? G.w : G.y;
+          xo = side ? G.x : G.z;
+          yo = side ? G.y : G.w;
+          dx = D.x;
+          dy = D.y;
+        } else {
+          xi = (side ? P.ce_xob : P.ce_xoa)[q];
+          yi = (side ? P.ce_yob : P.ce_yoa)[q];
+          xo = (side ? P.ce_xoa : P.ce_xob)[q];
+          yo = (side ? P.ce_yoa : P.ce_yob)[q];
+          dx = edx;
+          dy = edy;
+        }
+        const G3<R> go = load_g3<R>(P, o, k);
+        const R uo = (R)U[o], vo = (R)V[o], vco = VC[o];
+        const R uown = ui + gi.ux * xi + gi.uy * yi, vown = vi + gi.vx * xi + gi.vy * yi;
+        const R uoth = uo + go.ux * xo + go.uy * yo, voth = vo + go.vx * xo + go.vy * yo;
+        const R uij = half * (uown + uoth), vij = half * (vown + voth);
+        R viscof = (R)P.fact * half * (vci + vco);
+        viscof = viscof + (R)P.fm1 * half * (P.fm1 != 0.0 ? Mh::cc_hvc(P, i) + Mh::cc_hvc(P, o) : (R)0);
+        if (P.hprnu != 1.0) viscof = viscof / (R)P.hprnu;
+        const R vxa = side ? go.vx : gi.vx, vxb = side ? gi.vx : go.vx;
+        const R txx = (gi.ux + go.ux) * viscof;
+        const R tyy = (gi.vy + go.vy) * viscof;
+        const R txy = half * (gi.uy + go.uy + vxa + vxb) * viscof;
+        const R fxx = dij * (txx * dy - txy * dx);
+        const R fyy = dij * (txy * dy - tyy * dx);
+        R xadv, yadv;
+        if (UV) {
+          // adv_uv_edge_gcn.F:730, 752-753
+          const R exflux = dij * (-uij * dy + vij * dx);
+          const R sg = fsign1(exflux), so = side ? -sg : sg;
+          xadv = exflux * ((one - so) * uoth + (one + so) * uown) * half;
+          yadv = exflux * ((one - so) * voth + (one + so) * vown) * half;
+          vmr = vmr + viscof;
+        } else {
+          // advection_edge_gcn.F:559, 576-577
+          const R un = vij * dx - uij * dy;
+          const R sg = fsign1(un), so = side ? -sg : sg;
+          xadv = dij * un * ((one - so) * uoth + (one + so) * uown) * half;
+          yadv = dij * un * ((one - so) * voth + (one + so) * vown) * half;
+        }
+        const R isb = (R)isbc;
+        const R tp = isbc ? (R)(0.0 * epord) : epor;
+        // viscous part: GCN (fxx + 3 fxx ISBC) EPOR; GCY (advection_edge_gcy.F) fxx TPA
+        const R vfx = P.gcy ? fxx * tp : (fxx + three * fxx * isb) * epor;
+        const R vfy = P.gcy ? fyy * tp : (fyy + three * fyy * isb) * epor;
+        const R ax = xadv * tp, ay = yadv * tp;
+        xr = side ? xr - ax - vfx : xr + ax + vfx;
+        yr = side ? yr - ay - vfy : yr + ay + vfy;
+      }
+      if (UV) {
+        const double elij = 0.5 * (els[s] + els[(s + 1) % 3]);
+        const double tx = gdd * elij * edy, ty = gdd * elij * edx;
+        px = side ? px + tx : px - tx;
+        py = side ? py - ty : py + ty;
+      }
+    }
+    const size_t q = base + i;
+    double x = (double)xr * w, y = (double)yr * w;
+    if (!UV) {
+      // the end of ADVECTION_EDGE_GCN (advection_edge_gcn.F:674-708)
+      if (ob) { x = 0.0; y = 0.0; }
+      if (rivers) river3(P, i, k, x, y);
+      P.advx[q] = x;
+      P.advy[q] = y;
+      if (k < ke) {
+        ui_d = P.u[q + P.ns];
+        vi_d = P.v[q + P.ns];
+      }
+      continue;
+    }
+    // the end of ADV_UV_EDGE_GCN (adv_uv_edge_gcn.F:884-1193), as adv_uv_tail
+    px = px * w;
+    py = py * w;
+    x = x + px;
+    y = y + py;
+    double up = 0.0, vp = 0.0, zp = 0.0, xbot = 0.0, ybot = 0.0;
+    if (k < P.KBM1) {
+      const size_t qp = q + P.ns;
+      up = P.u[qp];
+      vp = P.v[qp];
+      zp = P.dz1[qp];
+      const double wk = P.w[qp], zs = z + zp;
+      xbot = wk * (ui_d * zp + up * z) / zs;
+      ybot = wk * (vi_d * zp + vp * z) / zs;
+    }
+    if (wet) {
+      const double xfv = k == 1 ? -xbot : (k == P.KBM1 ? xtop : xtop - xbot);
+      const double yfv = k == 1 ? -ybot : (k == P.KBM1 ? ytop : ytop - ybot);
+      const double cor = P.cor[i];
+      x = x + xfv * art + P.drhox[q] - cor * vi_d * dt1 * z * art;
+      y = y + yfv * art + P.drhoy[q] + cor * ui_d * dt1 * z * art;
+    }
+    if (ob) { x = 0.0; y = 0.0; }
+    if (rivers) river3(P, i, k, x, y);
+    double uf = 0.0, vf = 0.0;
+    if (wet) {
+      const double dz1d = d1 * z;
+      uf = ui_d * dt1 / d1 - P.dti * x / art / dz1d;
+      vf = vi_d * dt1 / d1 - P.dti * y / art / dz1d;
+    }
+    P.uf[q] = uf;
+    P.vf[q] = vf;
+    P.viscofm[q] = (double)vmr / art;
+    ui_d = up;
+    vi_d = vp;
+    z = zp;
+    xtop = xbot;
+    ytop = ybot;
   }
 }
 
@@ -1033,15 +1176,11 @@ static void launch_mom3d_staged(const Dev& P, cudaStream_t s) {
   const dim3 grid((unsigned)P.tl.n, (unsigned)((P.KBM1 + Q.col_lc - 1) / Q.col_lc));
   k_mom3d_staged<R, UV><<<grid, kTileCells, smem, s>>>(Q);
 }
-// Whether the staged kernel of ADVECTION (UV false) or ADV_UV (UV true) runs: LIMITED_NO,
-// GCN, a tile table whose shared memory fits one CTA, and P.staged = 2 (every staged
-// kernel), or P.staged = 1 (the default: only where it measured faster than the per-cell
-// kernel on the 200k-node, 40-layer coastal mesh, which is FP64 ADV_UV: 2.13 against
-// 2.52 ms per step; FP64 ADVECTION 1.35 against 1.26, FP32 ADVECTION 1.00 against 0.76,
-// FP32 ADV_UV 1.90 against 1.30).
-static bool staged_ok(const Dev& P, bool uv) {
-  const bool want = P.staged == 2 || (P.staged == 1 && uv && sizeof(RF) == 8);
-  return want && !P.limiter && !P.gcy && P.tl.n > 0 &&
+// Whether the staged kernels run: asked for (P.staged = 2), LIMITED_NO, GCN, a tile table whose
+// shared memory fits one CTA.  k_mom3d is faster in every form (200k nodes x 30 layers FP64:
+// ADV_UV 1.10 against 1.96 ms per step), so the default never takes them.
+static bool staged_ok(const Dev& P) {
+  return P.staged == 2 && !P.limiter && !P.gcy && P.tl.n > 0 &&
          staged_smem_bytes<double, true>(P.tl.cap_cells, P.tl.cap_edges) <= (size_t)kStagedSmemMax;
 }
 // Allow the staged kernels of this translation unit's arithmetic type up to
@@ -1210,15 +1349,24 @@ static void launch_alfa3(const Dev& P, cudaStream_t s) {
   const Dev Q = col_shape(P, P.N, P.KBM1);
   k_alfa3<RF><<<col_grid(Q, P.N, P.KBM1), Q.col_bc, 0, s>>>(Q);
 }
+template <bool UV>
+static void launch_mom3d(const Dev& P, cudaStream_t s) {
+  Dev Q = col_shape(P, P.N, P.KBM1);
+  if (P.limiter) {
+    launch_alfa3(P, s);
+    (UV ? k_adv_uv<RF> : k_advection3d<RF>)<<<col_grid(Q, P.N, P.KBM1), Q.col_bc, 0, s>>>(Q);
+    return;
+  }
+  if (Q.col_bc > 128) Q.col_bc = 128;  // the kernel's largest block
+  k_mom3d<RF, UV><<<col_grid(Q, P.N, P.KBM1), Q.col_bc, 0, s>>>(Q);
+}
 void launch_advection3d(const Dev& P, cudaStream_t s) {
   FVG_F32_FORWARD(launch_advection3d(P, s));
-  if (staged_ok(P, false)) {
+  if (staged_ok(P)) {
     launch_mom3d_staged<RF, false>(P, s);
     return;
   }
-  if (P.limiter) launch_alfa3(P, s);
-  const Dev Q = col_shape(P, P.N, P.KBM1);
-  (P.limiter ? k_advection3d<RF, true> : k_advection3d<RF, false>)<<<col_grid(Q, P.N, P.KBM1), Q.col_bc, 0, s>>>(Q);
+  launch_mom3d<false>(P, s);
 }
 // -------------------------------------------------------------------------------------
 // PHY_BAROPG (phy_baropg.F:37-151), BAROCLINIC_PRESSURE_GRADIENT = 'z coordinates'.
@@ -1381,13 +1529,11 @@ void launch_w_viscofh(const Dev& P, cudaStream_t s, int do_w, int do_visc) {
 }
 void launch_adv_uv(const Dev& P, cudaStream_t s) {
   FVG_F32_FORWARD(launch_adv_uv(P, s));
-  if (staged_ok(P, true)) {
+  if (staged_ok(P)) {
     launch_mom3d_staged<RF, true>(P, s);
     return;
   }
-  if (P.limiter) launch_alfa3(P, s);
-  const Dev Q = col_shape(P, P.N, P.KBM1);
-  (P.limiter ? k_adv_uv<RF, true> : k_adv_uv<RF, false>)<<<col_grid(Q, P.N, P.KBM1), Q.col_bc, 0, s>>>(Q);
+  launch_mom3d<true>(P, s);
 }
 void launch_vdif_uv(const Dev& P, cudaStream_t s, int parts) {
   const int b = col_threads(P, P.N, 128);
