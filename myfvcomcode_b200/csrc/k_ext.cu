@@ -93,11 +93,16 @@ __device__ inline Grad<R> cell_grad(const Dev& P, int c, const double* U, const 
   g.vy = dot4(b1, v0, b2, v1, b3, v2, b4, v3);
   return g;
 }
-// Least-squares gradient of UA, VA of cell c (advave_edge_gcn.F:634-637, 699-702), stored
-// for the edge loop of the next ADVAVE call in the handle's precision.
+// Least-squares gradient of UA, VA of cell c (advave_edge_gcn.F:634-637, 699-702) and the
+// cell's part ART*|grad|*CC_HVC of its three edges' viscosity, stored for the edge loop of the
+// next ADVAVE call in the handle's precision.
 template <typename R, bool CS>
 __device__ inline void store_grad_t(const Dev& P, int c) {
+  typedef Mesh<R> Mh;
   Grad<R> g = cell_grad<R, CS>(P, c, P.ua, P.va);
+  const R half = (R)0.5;
+  reinterpret_cast<R*>(P.xvc)[c] = Mh::art(P, c) *
+      sqrt(g.ux * g.ux + g.vy * g.vy + half * ((g.uy + g.vx) * (g.uy + g.vx))) * Mh::cc_hvc(P, c);
   if constexpr (sizeof(R) == 4) {
     P.f.g2d4[c] = make_float4(g.ux, g.uy, g.vx, g.vy);
   } else {
@@ -263,12 +268,34 @@ __device__ __forceinline__ void ext_node_job(const Dev& P, const int i, int iext
       x = (e & 1) ? x + exflux : x - exflux;
     }
   }
-  // the previous stage's node judgement, its cell flags now in ISWETCE (roles swapped)
-  if (parts & EN_WET_PREV) wet_node<CS>(P, i, P.iswetce);
-  if (parts & EN_FINISH_PREV) ext_update_node<CS>(P, i, (parts >> 8) & 7);
-  if (parts & EN_COPY_ELRK) P.elrk[i] = P.el[i];
+  // the previous stage's ELF clamp (WET_JUDGE) and update (ext_update_node); ISWETN and DTFA,
+  // which nothing inside the loop reads, are left to k_ext_finish
+  double e = 0.0;
+  const int ob = ld1<CS>(P.node_obc + i);
+  if (parts & EN_FINISH_PREV) {
+    const double h = P.h[i];
+    const int Kp = (parts >> 8) & 7;
+    e = P.elf[i];
+    if (parts & EN_WET_PREV) e = fmax(e, -h + P.min_depth);
+    P.el[i] = e;
+    P.d[i] = h + e;
+    if (Kp == 3) P.egf[i] = ld1<CS>(P.egf + i) + e / (double)P.isplit;
+    if (Kp == 4 && ob > 0) {
+      const double tmp = -(e - P.elrk[i]) * P.art1[i] / P.dte - P.xflux_obcn[ob];
+      P.uard_obcn[ob] = P.uard_obcn[ob] + tmp / (double)(float)P.isplit;
+    }
+  } else if (parts & EN_COPY_ELRK) {
+    e = P.el[i];
+  }
+  double elrk;
+  if (parts & EN_COPY_ELRK) {
+    elrk = e;
+    P.elrk[i] = e;
+  } else {
+    elrk = ld1<CS>(P.elrk + i);
+  }
   const double alpha = dAlphaRK[K];
-  int ob = ld1<CS>(P.node_obc + i);
+  double elf = 0.0;
   if (parts & EN_EXTEL) {
     if (ob > 0) {
       P.xflux_obcn[ob] = x;
@@ -283,13 +310,15 @@ __device__ __forceinline__ void ext_node_job(const Dev& P, const int i, int iext
         x = x - P.qdis[j] * P.rdisq[(size_t)(r & 1) * (P.numqbc + 1) + j];
     }
     double dtk = alpha * P.dte;
-    P.elf[i] = ld1<CS>(P.elrk + i) - dtk * x / ld1<CS>(P.art1 + i);
+    elf = elrk - dtk * x / ld1<CS>(P.art1 + i);
+  } else {
+    elf = P.elf[i];
   }
   if ((parts & EN_BC) && ob > 0) {
     int kind = P.obc_kind[ob];
     if (kind == 1) {
       if (P.obc_elev_on && (parts & EN_TABLE)) {
-        P.elf[i] = P.obf[(size_t)((iext - 1) * 4 + K - 1) * (P.iobcn + 1) + ob];
+        elf = P.obf[(size_t)((iext - 1) * 4 + K - 1) * (P.iobcn + 1) + ob];
       } else if (P.obc_elev_on) {
         const double* row = sched_row(P);
         double force = 0.0;
@@ -299,13 +328,14 @@ __device__ __forceinline__ void ext_node_job(const Dev& P, const int i, int iext
           force = add_rn(mul_rn(P.apt[q], cos(targ - P.phai_rad[q])), force);
         }
         force = force + P.emean[ob];
-        P.elf[i] = force * row[P.sl.ramp_ext(iext)];
+        elf = force * row[P.sl.ramp_ext(iext)];
       }
-      P.elf[i] = add_rn(P.elrk[i], mul_rn(alpha, P.elf[i] - P.elrk[i]));
+      elf = add_rn(elrk, mul_rn(alpha, elf - elrk));
     } else if (kind == 2) {
-      P.elf[i] = 0.0;
+      elf = 0.0;
     }
   }
+  P.elf[i] = elf;
 }
 
 // One job per thread, 48 registers (five blocks of 256 per SM; at 40 registers it
@@ -360,105 +390,130 @@ __device__ inline void advave_cell(const Dev& P, int i, double& xfo, double& yfo
   px = 0.0; py = 0.0;
   const size_t n1 = P.N + 1;
   const R epor = (R)P.epor[i], iucp = (R)P.iucp[i];
-  // The cell's own side of its three edges is loaded once; per edge only the other
-  // cell's gradient, UA, VA, ART, CC_HVC and wet flags are gathered (FP32 form).
   const Grad<R> gi = load_grad<R>(P, i);
-  const R ui = (R)P.ua[i], vi = (R)P.va[i], arti = Mh::art(P, i), cci = Mh::cc_hvc(P, i);
+  const R ui = (R)P.ua[i], vi = (R)P.va[i];
   const int weti = P.iswetce[i] * P.iswetc[i];
   const double ged1 = P.grav_e[i] * P.d1[i];
-  for (int s = 0; s < 3; ++s) {
-    const size_t q = (size_t)s * n1 + i;
-    const int4 ci = P.ce_i4[q];  // {code, IA, IB, J1}
-    const int code = ci.x;
-    const int side = code & 1;
-    const int ia = ci.y, ib = ci.z;
-    const int j1 = ci.w, j2 = P.ce_j2[q];
-    R dij = (R)(0.5 * (P.d[j1] + P.d[j2]));
-    double elij = 0.5 * (P.el[j1] + P.el[j2]);
-    const int o = side == 0 ? ib : ia;  // the other cell of the edge
-    if (weti == 1 || P.iswetce[o] * P.iswetc[o] == 1) {
-      R uij1, vij1, uij2, vij2;
-      Grad<R> ga, gb;
-      R arta, artb, cca, ccb;
-      if constexpr (!LIM && sizeof(R) == 8) {
-        // FP64: per-edge loads of both sides keep the kernel at 108 registers
-        ga = load_grad<R>(P, ia);
-        R xij = Mh::s_xoa(P, q);
-        R yij = Mh::s_yoa(P, q);
-        uij1 = (R)P.ua[ia] + ga.ux * xij + ga.uy * yij;
-        vij1 = (R)P.va[ia] + ga.vx * xij + ga.vy * yij;
-        gb = load_grad<R>(P, ib);
-        xij = Mh::s_xob(P, q);
-        yij = Mh::s_yob(P, q);
-        uij2 = (R)P.ua[ib] + gb.ux * xij + gb.uy * yij;
-        vij2 = (R)P.va[ib] + gb.vx * xij + gb.vy * yij;
-        arta = Mh::art(P, ia);
-        artb = Mh::art(P, ib);
-        cca = Mh::cc_hvc(P, ia);
-        ccb = Mh::cc_hvc(P, ib);
-      } else if constexpr (!LIM) {
+  if constexpr (!LIM) {
+    // Each edge as the cell sees it: its own side from the values above, sums that commute
+    // without regard to the sides, the upwind weights with the side as a sign, and both
+    // cells' ART*|grad|*CC_HVC from the gradient job (xvc), so that the values and their
+    // order are the reference's and the square roots are one per cell instead of six.
+    const R* VC = reinterpret_cast<const R*>(P.xvc);
+    const R vci = VC[i];
+    const int4 xn = P.loopx[i], oo = P.loopo[i];
+    const int xs[3] = {xn.x, xn.y, xn.z}, os[3] = {oo.x, oo.y, oo.z};
+    const int bits = xn.w;
+    const double dn[3] = {P.d[xs[0]], P.d[xs[1]], P.d[xs[2]]};
+    const double en[3] = {P.el[xs[0]], P.el[xs[1]], P.el[xs[2]]};
+#pragma unroll
+    for (int s = 0; s < 3; ++s) {
+      const int side = (bits >> s) & 1, o = os[s];
+      const size_t q = (size_t)s * n1 + i;
+      const double edx = P.ce_dx[q], edy = P.ce_dy[q];
+      if (weti == 1 || P.iswetce[o] * P.iswetc[o] == 1) {
+        const R dij = (R)(0.5 * (dn[s] + dn[(s + 1) % 3]));
+        R xi, yi, xo, yo, dx, dy;
+        if constexpr (sizeof(R) == 4) {
+          const float4 G = P.f.ce_geo[q];  // XOA, YOA, XOB, YOB
+          const float2 D = P.f.ce_dd[q];
+          xi = side ? G.z : G.x;
+          yi = side ? G.w : G.y;
+          xo = side ? G.x : G.z;
+          yo = side ? G.y : G.w;
+          dx = D.x;
+          dy = D.y;
+        } else {
+          xi = (side ? P.ce_xob : P.ce_xoa)[q];
+          yi = (side ? P.ce_yob : P.ce_yoa)[q];
+          xo = (side ? P.ce_xoa : P.ce_xob)[q];
+          yo = (side ? P.ce_yoa : P.ce_yob)[q];
+          dx = edx;
+          dy = edy;
+        }
         const Grad<R> go = load_grad<R>(P, o);
-        const R uo = (R)P.ua[o], vo = (R)P.va[o];
-        ga = side == 0 ? gi : go;
-        gb = side == 0 ? go : gi;
-        const R uia = side == 0 ? ui : uo, via = side == 0 ? vi : vo;
-        const R uib = side == 0 ? uo : ui, vib = side == 0 ? vo : vi;
-        const auto G = Mh::s_geo(P, q);  // XOA, YOA, XOB, YOB
-        uij1 = uia + ga.ux * G.x + ga.uy * G.y;
-        vij1 = via + ga.vx * G.x + ga.vy * G.y;
-        uij2 = uib + gb.ux * G.z + gb.uy * G.w;
-        vij2 = vib + gb.vx * G.z + gb.vy * G.w;
-        const R arto = Mh::art(P, o), cco = Mh::cc_hvc(P, o);
-        arta = side == 0 ? arti : arto;
-        artb = side == 0 ? arto : arti;
-        cca = side == 0 ? cci : cco;
-        ccb = side == 0 ? cco : cci;
-      } else {
-        arta = Mh::art(P, ia);
-        artb = Mh::art(P, ib);
-        cca = Mh::cc_hvc(P, ia);
-        ccb = Mh::cc_hvc(P, ib);
-        ga = load_grad<R>(P, ia);
-        gb = load_grad<R>(P, ib);
+        const R uo = (R)P.ua[o], vo = (R)P.va[o], vco = VC[o];
+        const R uown = ui + gi.ux * xi + gi.uy * yi, vown = vi + gi.vx * xi + gi.vy * yi;
+        const R uoth = uo + go.ux * xo + go.uy * yo, voth = vo + go.vx * xo + go.vy * yo;
+        const R uij = half * (uown + uoth), vij = half * (vown + voth);
+        const R un = -uij * dy + vij * dx;
+        R viscof = (R)P.fact * half * (vci + vco);
+        viscof = viscof + (R)P.fm1 * half * (P.fm1 != 0.0 ? Mh::cc_hvc(P, i) + Mh::cc_hvc(P, o) : (R)0);
+        if (P.hprnu != 1.0) viscof = viscof / (R)P.hprnu;
+        const R vxa = side ? go.vx : gi.vx, vxb = side ? gi.vx : go.vx;
+        const R txx = (gi.ux + go.ux) * viscof;
+        const R tyy = (gi.vy + go.vy) * viscof;
+        const R txy = half * (gi.uy + go.uy + vxa + vxb) * viscof;
+        const R fxx = dij * (txx * dy - txy * dx);
+        const R fyy = dij * (txy * dy - tyy * dx);
+        const R sg = fsign1(un), so = side ? -sg : sg;
+        const R xadv = dij * un * ((one - so) * uoth + (one + so) * uown) * half;
+        const R yadv = dij * un * ((one - so) * voth + (one + so) * vown) * half;
+        const R nb = one - (R)((bits >> (3 + s)) & 1);
+        const R ax = (xadv + fxx * epor) * nb * iucp, ay = (yadv + fyy * epor) * nb * iucp;
+        xf = side ? xf - ax : xf + ax;
+        yf = side ? yf - ay : yf + ay;
+      }
+      const double elij = 0.5 * (en[s] + en[(s + 1) % 3]);
+      const double tx = ged1 * elij * edy, ty = ged1 * elij * edx;
+      px = side ? px + tx : px - tx;
+      py = side ? py - ty : py + ty;
+    }
+  } else {
+    for (int s = 0; s < 3; ++s) {
+      const size_t q = (size_t)s * n1 + i;
+      const int4 ci = P.ce_i4[q];  // {code, IA, IB, J1}
+      const int code = ci.x;
+      const int side = code & 1;
+      const int ia = ci.y, ib = ci.z;
+      const int j1 = ci.w, j2 = P.ce_j2[q];
+      R dij = (R)(0.5 * (P.d[j1] + P.d[j2]));
+      double elij = 0.5 * (P.el[j1] + P.el[j2]);
+      const int o = side == 0 ? ib : ia;  // the other cell of the edge
+      if (weti == 1 || P.iswetce[o] * P.iswetc[o] == 1) {
+        R uij1, vij1, uij2, vij2;
+        const R arta = Mh::art(P, ia), artb = Mh::art(P, ib);
+        const R cca = Mh::cc_hvc(P, ia), ccb = Mh::cc_hvc(P, ib);
+        const Grad<R> ga = load_grad<R>(P, ia), gb = load_grad<R>(P, ib);
         const R xija = Mh::s_xoa(P, q), yija = Mh::s_yoa(P, q);
         const R xijb = Mh::s_xob(P, q), yijb = Mh::s_yob(P, q);
         lim_faces<R>(P.limiter, (R)P.ua[ia], (R)P.ua[ib], ga.ux * xija + ga.uy * yija, gb.ux * xijb + gb.uy * yijb,
                      Mh::alfa2(P, 0)[ia], Mh::alfa2(P, 0)[ib], uij1, uij2);
         lim_faces<R>(P.limiter, (R)P.va[ia], (R)P.va[ib], ga.vx * xija + ga.vy * yija, gb.vx * xijb + gb.vy * yijb,
                      Mh::alfa2(P, 1)[ia], Mh::alfa2(P, 1)[ib], vij1, vij2);
+        R uij = half * (uij1 + uij2);
+        R vij = half * (vij1 + vij2);
+        const auto DD = Mh::s_dd(P, q);
+        const R dltxc = DD.x, dltyc = DD.y;
+        R un = -uij * dltyc + vij * dltxc;
+        R viscof1 = arta * sqrt(ga.ux * ga.ux + ga.vy * ga.vy + half * ((ga.uy + ga.vx) * (ga.uy + ga.vx)));
+        R viscof2 = artb * sqrt(gb.ux * gb.ux + gb.vy * gb.vy + half * ((gb.uy + gb.vx) * (gb.uy + gb.vx)));
+        R viscof = ((R)P.fact * half * (viscof1 * cca + viscof2 * ccb) + (R)P.fm1 * half * (cca + ccb)) / (R)P.hprnu;
+        R txx = (ga.ux + gb.ux) * viscof;
+        R tyy = (ga.vy + gb.vy) * viscof;
+        R txy = half * (ga.uy + gb.uy + ga.vx + gb.vx) * viscof;
+        R fxx = dij * (txx * dltyc - txy * dltxc);
+        R fyy = dij * (txy * dltyc - tyy * dltxc);
+        R sg = fsign1(un);
+        R xadv = dij * un * ((one - sg) * uij2 + (one + sg) * uij1) * half;
+        R yadv = dij * un * ((one - sg) * vij2 + (one + sg) * vij1) * half;
+        R nb = one - (R)((code >> 1) & 1);
+        if (side == 0) {
+          xf = xf + (xadv + fxx * epor) * nb * iucp;
+          yf = yf + (yadv + fyy * epor) * nb * iucp;
+        } else {
+          xf = xf - (xadv + fxx * epor) * nb * iucp;
+          yf = yf - (yadv + fyy * epor) * nb * iucp;
+        }
       }
-      R uij = half * (uij1 + uij2);
-      R vij = half * (vij1 + vij2);
-      const auto DD = Mh::s_dd(P, q);
-      const R dltxc = DD.x, dltyc = DD.y;
-      R un = -uij * dltyc + vij * dltxc;
-      R viscof1 = arta * sqrt(ga.ux * ga.ux + ga.vy * ga.vy + half * ((ga.uy + ga.vx) * (ga.uy + ga.vx)));
-      R viscof2 = artb * sqrt(gb.ux * gb.ux + gb.vy * gb.vy + half * ((gb.uy + gb.vx) * (gb.uy + gb.vx)));
-      R viscof = ((R)P.fact * half * (viscof1 * cca + viscof2 * ccb) + (R)P.fm1 * half * (cca + ccb)) / (R)P.hprnu;
-      R txx = (ga.ux + gb.ux) * viscof;
-      R tyy = (ga.vy + gb.vy) * viscof;
-      R txy = half * (ga.uy + gb.uy + ga.vx + gb.vx) * viscof;
-      R fxx = dij * (txx * dltyc - txy * dltxc);
-      R fyy = dij * (txy * dltyc - tyy * dltxc);
-      R sg = fsign1(un);
-      R xadv = dij * un * ((one - sg) * uij2 + (one + sg) * uij1) * half;
-      R yadv = dij * un * ((one - sg) * vij2 + (one + sg) * vij1) * half;
-      R nb = one - (R)((code >> 1) & 1);
+      const double edx = P.ce_dx[q], edy = P.ce_dy[q];
       if (side == 0) {
-        xf = xf + (xadv + fxx * epor) * nb * iucp;
-        yf = yf + (yadv + fyy * epor) * nb * iucp;
+        px = px - ged1 * elij * edy;
+        py = py + ged1 * elij * edx;
       } else {
-        xf = xf - (xadv + fxx * epor) * nb * iucp;
-        yf = yf - (yadv + fyy * epor) * nb * iucp;
+        px = px + ged1 * elij * edy;
+        py = py - ged1 * elij * edx;
       }
-    }
-    const double edx = P.ce_dx[q], edy = P.ce_dy[q];
-    if (side == 0) {
-      px = px - ged1 * elij * edy;
-      py = py + ged1 * elij * edx;
-    } else {
-      px = px + ged1 * elij * edy;
-      py = py - ged1 * elij * edx;
     }
   }
   R w = (R)weti;
@@ -505,7 +560,7 @@ __device__ inline void bc_solid(const Dev& P, int i, int rj, double& uu, double&
 // followed by ADX2D -= ADVUA (internal_step.F:387-392).
 // -------------------------------------------------------------------------------------
 template <typename R, bool LIM>
-__global__ void __launch_bounds__(128, sizeof(R) == 4 ? 8 : 1) k_ext_cell(const Dev P, int iext, int K, int parts) {
+__global__ void __launch_bounds__(128, sizeof(R) == 4 ? 8 : (LIM ? 1 : 5)) k_ext_cell(const Dev P, int iext, int K, int parts) {
   pdl_enter();
   int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
   if (i > P.N) return;
@@ -581,8 +636,11 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 8 : 1) k_ext_cell(const 
         uaf = 0.0;
         vaf = 0.0;
       }
-      uaf = uaf / (1.0 + P.cc_sponge[i] * (uaf * uaf));
-      vaf = vaf / (1.0 + P.cc_sponge[i] * (vaf * vaf));
+      const double sp = P.cc_sponge[i];
+      if (sp != 0.0) {
+        uaf = uaf / (1.0 + sp * (uaf * uaf));
+        vaf = vaf / (1.0 + sp * (vaf * vaf));
+      }
     } else {
       uaf = P.uaf[i];
       vaf = P.vaf[i];
@@ -656,7 +714,8 @@ __device__ __forceinline__ void ext_cell_c(const Dev& P, const int i, int iext, 
     const float half = 0.5f, one = 1.0f;
     const double ged1 = e1.w * d1i;
     const float4 gi4 = P.f.g2d4[i];
-    const float2 aci = P.f.artcc[i];
+    const float* VC = reinterpret_cast<const float*>(P.xvc);
+    const float vci = VC[i];
     const double2 xyi = P.f.xyc[i];
     const float ui = (float)ua_i, vi = (float)va_i;
     const float epor = (fl & 8) ? 1.0f : 0.0f, iucp = (fl & 4) ? 1.0f : 0.0f;
@@ -672,7 +731,7 @@ __device__ __forceinline__ void ext_cell_c(const Dev& P, const int i, int iext, 
       const double elij = 0.5 * (P.el[j1] + P.el[j2]);
       if (weti == 1 || P.iswetce[o] * P.iswetc[o] == 1) {
         const float4 go4 = P.f.g2d4[o];
-        const float2 aco = P.f.artcc[o];
+        const float vco = VC[o];
         const double2 xyo = P.f.xyc[o];
         const float uo = (float)P.ua[o], vo = (float)P.va[o];
         const float xoi = (float)(xijc - xyi.x), yoi = (float)(yijc - xyi.y);
@@ -683,8 +742,6 @@ __device__ __forceinline__ void ext_cell_c(const Dev& P, const int i, int iext, 
         const float uib = side == 0 ? uo : ui, vib = side == 0 ? vo : vi;
         const float xa = side == 0 ? xoi : xoo, ya = side == 0 ? yoi : yoo;
         const float xb = side == 0 ? xoo : xoi, yb = side == 0 ? yoo : yoi;
-        const float arta = side == 0 ? aci.x : aco.x, artb = side == 0 ? aco.x : aci.x;
-        const float cca = side == 0 ? aci.y : aco.y, ccb = side == 0 ? aco.y : aci.y;
         // ga = {UX, UY, VX, VY} of IA, gb of IB
         const float uij1 = uia + ga.x * xa + ga.y * ya;
         const float vij1 = via + ga.z * xa + ga.w * ya;
@@ -694,10 +751,9 @@ __device__ __forceinline__ void ext_cell_c(const Dev& P, const int i, int iext, 
         const float vij = half * (vij1 + vij2);
         const float dx = (float)dltxc, dy = (float)dltyc;
         const float un = -uij * dy + vij * dx;
-        const float viscof1 = arta * sqrtf(ga.x * ga.x + ga.w * ga.w + half * ((ga.y + ga.z) * (ga.y + ga.z)));
-        const float viscof2 = artb * sqrtf(gb.x * gb.x + gb.w * gb.w + half * ((gb.y + gb.z) * (gb.y + gb.z)));
-        const float viscof =
-            ((float)P.fact * half * (viscof1 * cca + viscof2 * ccb) + (float)P.fm1 * half * (cca + ccb)) / (float)P.hprnu;
+        float viscof = (float)P.fact * half * (vci + vco);
+        if (P.fm1 != 0.0) viscof += (float)P.fm1 * half * (P.f.artcc[i].y + P.f.artcc[o].y);
+        if (P.hprnu != 1.0) viscof = viscof / (float)P.hprnu;
         const float txx = (ga.x + gb.x) * viscof;
         const float tyy = (ga.w + gb.w) * viscof;
         const float txy = half * (ga.y + gb.y + ga.z + gb.z) * viscof;
