@@ -328,14 +328,14 @@ void enqueue_internal_step(fvg_handle* h, cudaStream_t s, Marker mk = Marker(), 
       const int pdl = stage > 0 ? 1 : 0;
       launch_ext_node(Q, s, iext, K, EN_EXTEL | EN_BC | EN_GRAD | EN_TABLE | (K == 1 ? EN_COPY_ELRK : 0) | prev, pdl);
       mk.mark(s, G_EXT_NODE);
-      if (p.wetting_drying_on) {
+      if (p.wetting_drying_on && P.limiter) {
         launch_wet_cells(Q, s, 1);  // its node part opens the next stage's node kernel
         mk.mark(s, G_WET);
       }
       if (P.limiter) launch_alfa2(Q, s);
       launch_ext_cell(Q, s, iext, K,
-                      (p.wetting_drying_on ? 0 : EC_N2E) | EC_FLUXOBN | EC_ADVAVE | EC_EXTUV | EC_BC2 |
-                          (K == 1 ? EC_COPY_RK : 0) | EC_FINISH | EC_COMPACT |
+                      (!p.wetting_drying_on ? EC_N2E : P.limiter ? 0 : EC_WET) | EC_FLUXOBN | EC_ADVAVE | EC_EXTUV |
+                          EC_BC2 | (K == 1 ? EC_COPY_RK : 0) | EC_FINISH | EC_COMPACT |
                           (iext == p.isplit && K == 4 ? EC_LAST : 0),
                       P.limiter ? 0 : 1);
       mk.mark(s, G_EXT_CELL);
@@ -1144,7 +1144,7 @@ int32_t fvg_kernels_per_step(const fvg_handle* h) {
   if (!h) return -1;
   const fvg_params& p = h->prm;
   int n = 1 + 1 + 2 + 2 + 2;                                // begin, cell_pre, grad3+adv3d, baropg+prep, int advave+reset
-  n += (use_ext_loop(h) ? 1 : p.isplit * 4 * (2 + (p.wetting_drying_on ? 1 : 0))) + 1; // RK stages, closing update
+  n += (use_ext_loop(h) ? 1 : p.isplit * 4 * (2 + (p.wetting_drying_on && p.limiter ? 1 : 0))) + 1; // RK stages, closing update
   if (p.limiter) n += p.isplit * 4 + 1 + 2;                  // slope limiters: stages, ADVAVE, 3-D
   if (p.baropg_z && !p.barotropic) n += 2;                   // PHY_BAROPG's two kernels
   n += 1 + 1 + 1 + 1 + 2 + 1;                              // adjust2, vertvl x2, w/viscofh, grad3+adv_uv, vdif_uv

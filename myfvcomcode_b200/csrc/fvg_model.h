@@ -534,8 +534,9 @@ enum ExtNodeParts { EN_EXTEL = 1, EN_BC = 2, EN_COPY_ELRK = 4, EN_GRAD = 8, EN_F
 // EC_COMPACT: the stage loop of an internal step may use the compact FP32 kernel (when
 // F32::compact is set); EC_LAST: the last stage of that loop (the compact kernel writes
 // ADVUA, ADVVA, PSTX, PSTY only there and in the internal-step ADVAVE call).
+// EC_WET: WET_JUDGE's cell part first (no limiter, whose alfa kernel needs the flags before).
 enum ExtCellParts { EC_N2E = 1, EC_FLUXOBN = 2, EC_ADVAVE = 4, EC_EXTUV = 8, EC_BC2 = 16, EC_COPY_RK = 32,
-                    EC_INT_ADVAVE = 64, EC_FINISH = 128, EC_COMPACT = 256, EC_LAST = 512 };
+                    EC_INT_ADVAVE = 64, EC_FINISH = 128, EC_COMPACT = 256, EC_LAST = 512, EC_WET = 1024 };
 void launch_ext_finish(const Dev& P, cudaStream_t s, int K, int wet_prev);
 // pdl: launched as a programmatic dependent of the previous kernel in the stream (the
 // fused external loop); the kernel waits for that kernel's completion before it touches

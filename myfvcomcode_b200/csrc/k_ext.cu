@@ -192,8 +192,7 @@ __device__ inline void ext_update_node(const Dev& P, int i, int K) {
 
 // Cell part of the update after stage K with the new UA, VA: EL1, D1, the K == 3 sums and
 // the half-edge continuity fluxes of the next stage.
-__device__ inline void ext_update_cell(const Dev& P, int i, int K, double u, double v) {
-  double e1 = P.elf1[i];
+__device__ inline void ext_update_cell(const Dev& P, int i, int K, double e1, double u, double v) {
   P.el1[i] = e1;
   double dd1 = P.h1[i] + e1;
   P.d1[i] = dd1;
@@ -356,21 +355,25 @@ __global__ void __launch_bounds__(256, 5) k_ext_node(const Dev P, int iext, int 
 // forms itself from h and ELF.  Then nodes: the node flag and the clamp of ELF.
 // -------------------------------------------------------------------------------------
 template <bool CS>
-__device__ __forceinline__ void wet_cell(const Dev& P, const int i) {
+__device__ __forceinline__ int wet_cell(const Dev& P, const int i, double& elf1) {
   int n1 = ld1<CS>(P.nv + i), n2 = ld1<CS>(P.nv + (size_t)(P.N + 1) + i), n3 = ld1<CS>(P.nv + (size_t)2 * (P.N + 1) + i);
   double e1 = P.elf[n1], e2 = P.elf[n2], e3 = P.elf[n3];
   double dtmp = fmax(fmax(e1, e2), e3) + fmin(fmin(P.h[n1], P.h[n2]), P.h[n3]);
-  P.iswetc[i] = ((dtmp - P.min_depth) < 1.0e-5) ? 0 : 1;
+  const int wet = ((dtmp - P.min_depth) < 1.0e-5) ? 0 : 1;
+  P.iswetc[i] = wet;
   double c1 = fmax(e1, -P.h[n1] + P.min_depth);
   double c2 = fmax(e2, -P.h[n2] + P.min_depth);
   double c3 = fmax(e3, -P.h[n3] + P.min_depth);
-  P.elf1[i] = ONE_THIRD * (c1 + c2 + c3);
+  elf1 = ONE_THIRD * (c1 + c2 + c3);
+  P.elf1[i] = elf1;
+  return wet;
 }
 template <bool CS>
 __global__ void k_wet_cells(const Dev P) {
   pdl_enter();
   const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
-  if (i <= P.N) wet_cell<CS>(P, i);
+  double elf1;
+  if (i <= P.N) wet_cell<CS>(P, i, elf1);
 }
 
 __global__ void k_wet_nodes(const Dev P) {
@@ -379,11 +382,25 @@ __global__ void k_wet_nodes(const Dev P) {
   wet_node(P, i, P.iswetc);
 }
 
+// Whether cell o on the other side of slot s (nodes j1, j2) of cell i counts as wet,
+// ISWETCE*ISWETC.  judge: WET_JUDGE's cell part runs in the same kernel (EC_WET), so the flag
+// of this stage is formed from the neighbour's three nodes, its node off the edge in wfar, as
+// wet_cell forms it.  A cell that is wet itself needs no neighbour's flag, so that only dry
+// cells pay for this.
+__device__ inline bool wet_other(const Dev& P, bool judge, int i, int s, int o, int j1, int j2) {
+  if (judge && o != 0) {
+    const double e = fmax(fmax(P.elf[j1], P.elf[j2]), P.elf[P.wfar[(size_t)s * (P.N + 1) + i]]);
+    return (((e + P.hmin[o]) - P.min_depth) < 1.0e-5 ? 0 : 1) * P.iswetce[o] == 1;
+  }
+  return P.iswetce[o] * P.iswetc[o] == 1;
+}
+
 // ADVAVE_EDGE_GCN for one cell (advave_edge_gcn.F:115-1003, LIMITED_NO branch), over the
 // cell's slot table.  The edge fluxes are evaluated in R; the surface-slope pressure
 // gradient PSTX/PSTY stays FP64.
 template <typename R, bool LIM>
-__device__ inline void advave_cell(const Dev& P, int i, double& xfo, double& yfo, double& px, double& py) {
+__device__ inline void advave_cell(const Dev& P, int i, int weti, bool judge, double& xfo, double& yfo, double& px,
+                                   double& py) {
   typedef Mesh<R> Mh;
   const R half = (R)0.5, one = (R)1.0;
   R xf = 0, yf = 0;
@@ -392,7 +409,6 @@ __device__ inline void advave_cell(const Dev& P, int i, double& xfo, double& yfo
   const R epor = (R)P.epor[i], iucp = (R)P.iucp[i];
   const Grad<R> gi = load_grad<R>(P, i);
   const R ui = (R)P.ua[i], vi = (R)P.va[i];
-  const int weti = P.iswetce[i] * P.iswetc[i];
   const double ged1 = P.grav_e[i] * P.d1[i];
   if constexpr (!LIM) {
     // Each edge as the cell sees it: its own side from the values above, sums that commute
@@ -411,7 +427,7 @@ __device__ inline void advave_cell(const Dev& P, int i, double& xfo, double& yfo
       const int side = (bits >> s) & 1, o = os[s];
       const size_t q = (size_t)s * n1 + i;
       const double edx = P.ce_dx[q], edy = P.ce_dy[q];
-      if (weti == 1 || P.iswetce[o] * P.iswetc[o] == 1) {
+      if (weti == 1 || wet_other(P, judge, i, s, o, xs[s], xs[(s + 1) % 3])) {
         const R dij = (R)(0.5 * (dn[s] + dn[(s + 1) % 3]));
         R xi, yi, xo, yo, dx, dy;
         if constexpr (sizeof(R) == 4) {
@@ -570,8 +586,13 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 8 : (LIM ? 1 : 5)) k_ext
     P.vark[i] = P.va[i];
     P.elrk1[i] = P.el1[i];
   }
-  if (parts & EC_N2E)
-    P.elf1[i] = ONE_THIRD * (P.elf[P.nv[i]] + P.elf[P.nv[n1 + i]] + P.elf[P.nv[2 * n1 + i]]);
+  double elf1;
+  if (parts & EC_N2E) {
+    elf1 = ONE_THIRD * (P.elf[P.nv[i]] + P.elf[P.nv[n1 + i]] + P.elf[P.nv[2 * n1 + i]]);
+    P.elf1[i] = elf1;
+  }
+  const int weti = P.iswetce[i] * ((parts & EC_WET) ? wet_cell<false>(P, i, elf1) : P.iswetc[i]);
+  if (!(parts & (EC_N2E | EC_WET))) elf1 = P.elf1[i];
   double fob = 0.0;
   if (parts & EC_FLUXOBN) {
     fob = fluxobn_cell(P, i, K);
@@ -581,7 +602,7 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 8 : (LIM ? 1 : 5)) k_ext
   }
   double xf, yf, px, py;
   if (parts & (EC_ADVAVE | EC_INT_ADVAVE)) {
-    advave_cell<R, LIM>(P, i, xf, yf, px, py);
+    advave_cell<R, LIM>(P, i, weti, parts & EC_WET, xf, yf, px, py);
     if (P.isbce[i] == 2) {
       if (P.gcy) {  // advave_edge_gcy.F
         xf = xf + fob * P.ua[i] * P.iucp[i];
@@ -621,7 +642,7 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 8 : (LIM ? 1 : 5)) k_ext
     double uaf, vaf;
     if (parts & EC_EXTUV) {
       // EXTUV_EDGE(K) (extuv_edge.F:106-163)
-      if (P.iswetce[i] * P.iswetc[i] == 1) {
+      if (weti == 1) {
         double ramp = sched_row(P)[P.sl.ramp_ext(iext)];
         double wus = P.have_wind ? P.wsx[i] * ramp * 0.001 : 0.0;
         double wvs = P.have_wind ? P.wsy[i] * ramp * 0.001 : 0.0;
@@ -630,8 +651,8 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 8 : (LIM ? 1 : 5)) k_ext
         double resy = P.ady2d[i] + yf + P.dry2d[i] + py + P.cor[i] * P.ua[i] * P.d1[i] * P.art[i] -
                       (wvs + P.wvbot[i]) * P.art[i];
         double a = dAlphaRK[K];
-        uaf = (P.uark[i] * (P.h1[i] + P.elrk1[i]) - a * P.dte * resx / P.art[i]) / (P.h1[i] + P.elf1[i]);
-        vaf = (P.vark[i] * (P.h1[i] + P.elrk1[i]) - a * P.dte * resy / P.art[i]) / (P.h1[i] + P.elf1[i]);
+        uaf = (P.uark[i] * (P.h1[i] + P.elrk1[i]) - a * P.dte * resx / P.art[i]) / (P.h1[i] + elf1);
+        vaf = (P.vark[i] * (P.h1[i] + P.elrk1[i]) - a * P.dte * resy / P.art[i]) / (P.h1[i] + elf1);
       } else {
         uaf = 0.0;
         vaf = 0.0;
@@ -654,7 +675,7 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 8 : (LIM ? 1 : 5)) k_ext
     }
     P.uaf[i] = uaf;
     P.vaf[i] = vaf;
-    if (parts & EC_FINISH) ext_update_cell(P, i, K, uaf, vaf);
+    if (parts & EC_FINISH) ext_update_cell(P, i, K, elf1, uaf, vaf);
   }
 }
 
@@ -692,10 +713,16 @@ __device__ __forceinline__ void ext_cell_c(const Dev& P, const int i, int iext, 
     P.elrk1[i] = ld1<CS>(P.el1 + i);
   }
   double elf1 = 0.0;
+  int wetc;
+  if (parts & EC_WET) {
+    wetc = wet_cell<CS>(P, i, elf1);
+  } else {
+    wetc = P.iswetc[i];
+  }
   if (parts & EC_N2E) {
     elf1 = ONE_THIRD * (P.elf[ld1<CS>(P.nv + i)] + P.elf[ld1<CS>(P.nv + n1 + i)] + P.elf[ld1<CS>(P.nv + 2 * n1 + i)]);
     P.elf1[i] = elf1;
-  } else if (parts & (EC_EXTUV | EC_FINISH)) {
+  } else if (!(parts & EC_WET) && (parts & (EC_EXTUV | EC_FINISH))) {
     elf1 = ld1<CS>(P.elf1 + i);
   }
   double fob = 0.0;
@@ -705,7 +732,7 @@ __device__ __forceinline__ void ext_cell_c(const Dev& P, const int i, int iext, 
   } else if (isbce == 2) {
     fob = P.fluxobn[i];
   }
-  const int weti = P.iswetce[i] * P.iswetc[i];
+  const int weti = P.iswetce[i] * wetc;
   const double d1i = ld1<CS>(P.d1 + i);
   // {COR*ART, ART, H1, GRAV_E}: formed by the internal-step call below, read by the stages
   const double4 e1 = (parts & EC_INT_ADVAVE) ? make_double4(0.0, 0.0, 0.0, P.grav_e[i]) : ld1<CS>(P.f.exc1 + i);
@@ -729,7 +756,7 @@ __device__ __forceinline__ void ext_cell_c(const Dev& P, const int i, int iext, 
       const double dltxc = v2.x - v1.x, dltyc = v2.y - v1.y;
       const float dij = (float)(0.5 * (P.d[j1] + P.d[j2]));
       const double elij = 0.5 * (P.el[j1] + P.el[j2]);
-      if (weti == 1 || P.iswetce[o] * P.iswetc[o] == 1) {
+      if (weti == 1 || wet_other(P, parts & EC_WET, i, s, o, j1, j2)) {
         const float4 go4 = P.f.g2d4[o];
         const float vco = VC[o];
         const double2 xyo = P.f.xyc[o];
@@ -1400,7 +1427,7 @@ __global__ void k_ext_update(const Dev P, int K) {
     P.ua[i] = u;
     P.va[i] = v;
     if (P.wetting_drying_on) P.iswetce[i] = P.iswetc[i];
-    ext_update_cell(P, i, K, u, v);
+    ext_update_cell(P, i, K, P.elf1[i], u, v);
   }
 }
 
