@@ -1257,6 +1257,9 @@ int fvg_set_precision(fvg_handle* h, int32_t mode) {
     if ((rc = dalloc(h, (float**)&f.trie, 2 * (size_t)P.trie_n))) return fail(rc);
     if ((rc = dalloc(h, (float**)&f.a1u4, 4 * n1))) return fail(rc);
     if ((rc = dalloc(h, (float**)&f.a2u4, 4 * n1))) return fail(rc);
+    // the allocations were cleared on the default stream, which the handle's stream does not
+    // wait for by itself
+    CK(cudaStreamSynchronize(cudaStreamLegacy));
     launch_make_f32(P, h->stream);
     CK(cudaGetLastError());
     // records of the compact stage kernel, used where the mesh's edge metrics are the ones
@@ -1270,6 +1273,7 @@ int fvg_set_precision(fvg_handle* h, int32_t mode) {
     if ((rc = dalloc(h, &f.cflag, n1))) return fail(rc);
     int* d_bad = nullptr;
     if ((rc = dalloc(h, &d_bad, 1))) return fail(rc);
+    CK(cudaStreamSynchronize(cudaStreamLegacy));
     launch_make_compact(P, h->stream, d_bad);
     CK(cudaGetLastError());
     int bad = -1;

@@ -246,7 +246,8 @@ int fvg_mlp_create(uint64_t seed, fvg_mlp** out) {
   for (int p = OW2; p < OB2; ++p) h[p] = nd(rng) * std::sqrt(2.f / MH);
   for (int p = OW3; p < OB3; ++p) h[p] = nd(rng) * std::sqrt(1.f / MH);
   if (cudaMemcpy(q->par, h.data(), NPAR * sizeof(float), cudaMemcpyHostToDevice) != cudaSuccess ||
-      cudaMemset(q->m, 0, NPAR * sizeof(float)) != cudaSuccess || cudaMemset(q->v, 0, NPAR * sizeof(float)) != cudaSuccess)
+      cudaMemsetAsync(q->m, 0, NPAR * sizeof(float), q->stream) != cudaSuccess ||
+      cudaMemsetAsync(q->v, 0, NPAR * sizeof(float), q->stream) != cudaSuccess)
     return fail(FVG_ERR_CUDA);
   *out = q;
   return FVG_OK;
@@ -277,8 +278,8 @@ int fvg_mlp_set_params(fvg_mlp* q, const float* host, int32_t n) {
   if (!q || !host || n != NPAR) return FVG_ERR_ARG;
   MK(cudaStreamSynchronize(q->stream));
   MK(cudaMemcpy(q->par, host, NPAR * sizeof(float), cudaMemcpyHostToDevice));
-  MK(cudaMemset(q->m, 0, NPAR * sizeof(float)));
-  MK(cudaMemset(q->v, 0, NPAR * sizeof(float)));
+  MK(cudaMemsetAsync(q->m, 0, NPAR * sizeof(float), q->stream));
+  MK(cudaMemsetAsync(q->v, 0, NPAR * sizeof(float), q->stream));
   q->step = 0;
   return FVG_OK;
 }
