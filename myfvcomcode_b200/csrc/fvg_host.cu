@@ -508,7 +508,6 @@ int fvg_create(const fvg_mesh* m, const fvg_params* prm, const fvg_forcing* f, f
   // ---- mesh upload ----
 #define UPD(dst, src, n) if ((rc = upload(h, (double**)&P.dst, src, n))) return fail(rc)
 #define UPI(dst, src, n) if ((rc = upload(h, (int**)&P.dst, src, n))) return fail(rc)
-#define UP3(dst, src, rows, str) if ((rc = upload3(h, (double**)&P.dst, src, rows, KB, str))) return fail(rc)
   UPD(vx, m->vx, m1); UPD(vy, m->vy, m1); UPD(h, m->h, m1); UPD(art1, m->art1, m1); UPD(art2, m->art2, m1);
   UPD(grav_n, m->grav_n, m1); UPD(nn_hvc, m->nn_hvc, m1); UPD(phpn, m->phpn, m1);
   UPI(isonb, m->isonb, m1); UPI(ntsn, m->ntsn, m1); UPI(ntve, m->ntve, m1);
@@ -517,7 +516,6 @@ int fvg_create(const fvg_mesh* m, const fvg_params* prm, const fvg_forcing* f, f
   P.trie_n = (int)(m1 * m->trie_cols);
   UPD(dltxecec, m->dltxecec, m1 * m->trie_cols); UPD(dltyecec, m->dltyecec, m1 * m->trie_cols);
   UPD(dltxnec, m->dltxnec, m1 * m->trie_cols); UPD(dltynec, m->dltynec, m1 * m->trie_cols);
-  UP3(z, m->z, m1, ms); UP3(zz, m->zz, m1, ms); UP3(dz, m->dz, m1, ms); UP3(dzz, m->dzz, m1, ms);
   UPD(xc, m->xc, n1); UPD(yc, m->yc, n1); UPD(art, m->art, n1); UPD(cor, m->cor, n1);
   UPD(grav_e, m->grav_e, n1); UPD(cc_hvc, m->cc_hvc, n1); UPD(cc_sponge, m->cc_sponge, n1);
   UPD(cc_z0b, m->cc_z0b, n1); UPD(epor, m->epor, n1); UPD(iucp, m->iucp, n1);
@@ -534,7 +532,32 @@ int fvg_create(const fvg_mesh* m, const fvg_params* prm, const fvg_forcing* f, f
     UPI(nbe4, nb4.data(), nb4.size());
   }
   UPD(a1u, m->a1u, n1 * 4); UPD(a2u, m->a2u, n1 * 4); UPD(awx, m->awx, n1 * 3); UPD(awy, m->awy, n1 * 3);
-  UP3(z1, m->z1, n1, ns); UP3(zz1, m->zz1, n1, ns); UP3(dz1, m->dz1, n1, ns); UP3(dzz1, m->dzz1, n1, ns);
+  // sigma arrays: one table of KB values where every node (cell) has the same levels
+  auto sigma = [&](Sigma& d, const double* src, size_t rows, size_t stride) -> int {
+    bool same = true;
+    for (int k = 0; k < KB && same; ++k) {
+      const double* p = src + (size_t)k * rows;
+      for (size_t i = 2; i < rows; ++i)
+        if (std::memcmp(p + i, p + 1, sizeof(double)) != 0) { same = false; break; }
+    }
+    double* q = nullptr;
+    int r;
+    if (same) {
+      std::vector<double> t(KB);
+      for (int k = 0; k < KB; ++k) t[k] = src[(size_t)k * rows + 1];
+      r = upload(h, &q, t.data(), (size_t)KB);
+    } else {
+      r = upload3(h, &q, src, rows, KB, stride);
+    }
+    d.a = q;
+    d.stride = same ? 1u : (unsigned)stride;
+    d.mask = same ? 0u : ~0u;
+    return r;
+  };
+  if ((rc = sigma(P.z, m->z, m1, ms)) || (rc = sigma(P.zz, m->zz, m1, ms)) || (rc = sigma(P.dz, m->dz, m1, ms)) ||
+      (rc = sigma(P.dzz, m->dzz, m1, ms)) || (rc = sigma(P.z1, m->z1, n1, ns)) || (rc = sigma(P.zz1, m->zz1, n1, ns)) ||
+      (rc = sigma(P.dz1, m->dz1, n1, ns)) || (rc = sigma(P.dzz1, m->dzz1, n1, ns)))
+    return fail(rc);
   UPI(iec, m->iec, e1 * 2); UPI(ienode, m->ienode, e1 * 2); UPI(isbc, m->isbc, e1);
   UPD(xijc, m->xijc, e1); UPD(yijc, m->yijc, e1); UPD(dltxc, m->dltxc, e1); UPD(dltyc, m->dltyc, e1);
   UPI(niec, m->niec, v1 * 2); UPI(ntrg, m->ntrg, v1); UPD(dltxe, m->dltxe, v1); UPD(dltye, m->dltye, v1);

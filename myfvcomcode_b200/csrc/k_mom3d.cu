@@ -57,8 +57,8 @@ __global__ void k_cell_pre(const Dev P, int parts) {
   const int KBM1 = P.KBM1;
   if (parts & CP_ADJUST1) {
     double uac = 0.0, vac = 0.0;
-    for (int k = 1; k <= KBM1; ++k) uac = uac + P.u[C3(P, i, k)] * P.dz1[C3(P, i, k)];
-    for (int k = 1; k <= KBM1; ++k) vac = vac + P.v[C3(P, i, k)] * P.dz1[C3(P, i, k)];
+    for (int k = 1; k <= KBM1; ++k) uac = uac + P.u[C3(P, i, k)] * P.dz1(i, k);
+    for (int k = 1; k <= KBM1; ++k) vac = vac + P.v[C3(P, i, k)] * P.dz1(i, k);
     double du = 1.0 * (P.ua[i] - uac), dv = 1.0 * (P.va[i] - vac);
     for (int k = 1; k <= KBM1; ++k) {
       P.u[C3(P, i, k)] = P.u[C3(P, i, k)] + du;
@@ -88,7 +88,7 @@ __global__ void k_cell_pre(const Dev P, int parts) {
   }
   if (parts & CP_BROUGH) {
     const double VK2 = 0.160;
-    double zb = P.zz1[C3(P, i, KBM1)] - P.z1[C3(P, i, P.KB)];
+    double zb = P.zz1(i, KBM1) - P.z1(i, P.KB);
     double lg = (P.dt1[i] > 3.0) ? log(zb * P.dt1[i] / P.cc_z0b[i]) : log(zb * 3.0 / P.cc_z0b[i]);
     double cbc = VK2 / (lg * lg);
     if (cbc < P.cbcmin) cbc = P.cbcmin;
@@ -96,7 +96,7 @@ __global__ void k_cell_pre(const Dev P, int parts) {
     double ub = P.u[C3(P, i, KBM1)], vb = P.v[C3(P, i, KBM1)];
     double btps = cbc * sqrt(ub * ub + vb * vb);
     double wu = -btps * ub, wv = -btps * vb;
-    double cff = 0.75 * P.dz1[C3(P, i, KBM1)] * P.d1[i];
+    double cff = 0.75 * P.dz1(i, KBM1) * P.d1[i];
     wu = (wu >= 0.0 ? 1.0 : -1.0) * fmin(fabs(wu), fabs(ub * cff / P.dti));
     wv = (wv >= 0.0 ? 1.0 : -1.0) * fmin(fabs(wv), fabs(vb * cff / P.dti));
     P.wubot[i] = wu;
@@ -281,10 +281,10 @@ __device__ inline void river3(const Dev& P, int i, int k, double& x, double& y) 
     double temp;
     if (P.river_location == 0) {
       int j = P.inodeq[ii];
-      temp = 0.5 * P.qdis[ii] * vq * vq * vlctyq / P.dz[N3(P, j, k)];
+      temp = 0.5 * P.qdis[ii] * vq * vq * vlctyq / P.dz(j, k);
     } else {
       int i1 = P.icellq[ii];
-      temp = P.qdis[ii] * vq * vq * vlctyq / P.dz1[C3(P, i1, k)];
+      temp = P.qdis[ii] * vq * vq * vlctyq / P.dz1(i1, k);
     }
     x = x - temp * P.cos_angleq[ii];
     y = y - temp * P.sin_angleq[ii];
@@ -326,7 +326,7 @@ __global__ void __launch_bounds__(256) k_advection3d(const Dev P) {
     const int ia = ci.y, ib = ci.z;
     if (!(P.iswetct[ia] * P.iswetc[ia] == 1 || P.iswetct[ib] * P.iswetc[ib] == 1)) continue;
     const int j1 = ci.w, j2 = P.ce_j2[q];
-    R dij = (R)(0.5 * (P.dt[j1] * P.dz[N3(P, j1, k)] + P.dt[j2] * P.dz[N3(P, j2, k)]));
+    R dij = (R)(0.5 * (P.dt[j1] * P.dz(j1, k) + P.dt[j2] * P.dz(j2, k)));
     EdgeFlux<R> f = edge_flux3<R>(P, q, ia, ib, k, dij, false);
     R isb = (R)isbc;
     R tp = (R)((double)(float)(1 - isbc) * P.epor[i]);
@@ -386,8 +386,8 @@ __global__ void k_baropg(const Dev P, int do_baropg, int do_sums) {
         }
         const size_t c = C3(P, i, k);
         rhoc[b] = P.rho[c] - P.rmean[c];
-        zz[b] = P.zz1[c];
-        dz[b] = P.dz1[c];
+        zz[b] = P.zz1(i, k);
+        dz[b] = P.dz1(i, k);
       }
 #pragma unroll
       for (int b = 0; b < kB; ++b) {
@@ -476,8 +476,8 @@ __global__ void k_adjust2(const Dev P, int parts) {
   if (wet) {
     for (int k = 1; k <= P.KBM1; ++k) {
       size_t q = C3(P, i, k);
-      ut = ut + P.u[q] * P.dz1[q];
-      vt = vt + P.v[q] * P.dz1[q];
+      ut = ut + P.u[q] * P.dz1(i, k);
+      vt = vt + P.v[q] * P.dz1(i, k);
     }
     ut = ut * dt1;
     vt = vt * dt1;
@@ -506,7 +506,7 @@ __global__ void k_adjust2(const Dev P, int parts) {
       P.u[q] = uu;
       P.v[q] = vv;
     }
-    const double dij = dt1 * P.dz1[q];
+    const double dij = dt1 * P.dz1(i, k);
     double* F = P.he_vflux + (size_t)(k - 1) * P.ncvs + i;
     for (int s = 0; s < 3; ++s) F[(size_t)s * P.ns] = dij * (-uu * dy[s] + vv * dx[s]);
   }
@@ -574,7 +574,7 @@ __global__ void k_vertvl_col(const Dev P, int parts) {
     if (P.iswetnt[i] * P.iswetn[i] == 1) {
       double dd = P.d[i] - P.dt[i];
       for (int k = 1; k <= KBM1; ++k) {
-        wk = wk + P.scr_xflux[N3(P, i, k)] / P.art1[i] + P.dz[N3(P, i, k)] * dd / P.dti;
+        wk = wk + P.scr_xflux[N3(P, i, k)] / P.art1[i] + P.dz(i, k) * dd / P.dti;
         P.wts[N3(P, i, k + 1)] = wk;
       }
     } else {
@@ -583,7 +583,7 @@ __global__ void k_vertvl_col(const Dev P, int parts) {
     }
     double wkb = wk;
     if (fabs(wkb - wb) > 1.0e-8 && P.isonb[i] != 2) {
-      double tmp1 = P.elf[i] * (double)(float)KBM1 - (wkb - wb) * P.dti / P.dz[N3(P, i, 1)];
+      double tmp1 = P.elf[i] * (double)(float)KBM1 - (wkb - wb) * P.dti / P.dz(i, 1);
       tmp1 = tmp1 / (double)(float)KBM1;
       P.dtfa[i] = tmp1 + P.h[i];
       for (int k = 2; k <= KB; ++k) {
@@ -694,25 +694,26 @@ __device__ inline void adv_uv_tail(const Dev& P, int i, int k, R xr, R yr, R vmr
   y = y + py;
   size_t q = C3(P, i, k);
   if (wet) {
-    const double *U = P.u, *V = P.v, *W = P.w, *DZ1 = P.dz1;
+    const double *U = P.u, *V = P.v, *W = P.w;
+    const double z = P.dz1(i, k), zm = k > 1 ? P.dz1(i, k - 1) : 0.0, zp = k < P.KBM1 ? P.dz1(i, k + 1) : 0.0;
     double xfv, yfv;
     if (k == 1) {
       size_t qp = C3(P, i, k + 1);
-      xfv = -W[qp] * (U[q] * DZ1[qp] + U[qp] * DZ1[q]) / (DZ1[q] + DZ1[qp]);
-      yfv = -W[qp] * (V[q] * DZ1[qp] + V[qp] * DZ1[q]) / (DZ1[q] + DZ1[qp]);
+      xfv = -W[qp] * (U[q] * zp + U[qp] * z) / (z + zp);
+      yfv = -W[qp] * (V[q] * zp + V[qp] * z) / (z + zp);
     } else if (k == P.KBM1) {
       size_t qm = C3(P, i, k - 1);
-      xfv = W[q] * (U[q] * DZ1[qm] + U[qm] * DZ1[q]) / (DZ1[q] + DZ1[qm]);
-      yfv = W[q] * (V[q] * DZ1[qm] + V[qm] * DZ1[q]) / (DZ1[q] + DZ1[qm]);
+      xfv = W[q] * (U[q] * zm + U[qm] * z) / (z + zm);
+      yfv = W[q] * (V[q] * zm + V[qm] * z) / (z + zm);
     } else {
       size_t qm = C3(P, i, k - 1), qp = C3(P, i, k + 1);
-      xfv = W[q] * (U[q] * DZ1[qm] + U[qm] * DZ1[q]) / (DZ1[q] + DZ1[qm]) -
-            W[qp] * (U[q] * DZ1[qp] + U[qp] * DZ1[q]) / (DZ1[q] + DZ1[qp]);
-      yfv = W[q] * (V[q] * DZ1[qm] + V[qm] * DZ1[q]) / (DZ1[q] + DZ1[qm]) -
-            W[qp] * (V[q] * DZ1[qp] + V[qp] * DZ1[q]) / (DZ1[q] + DZ1[qp]);
+      xfv = W[q] * (U[q] * zm + U[qm] * z) / (z + zm) -
+            W[qp] * (U[q] * zp + U[qp] * z) / (z + zp);
+      yfv = W[q] * (V[q] * zm + V[qm] * z) / (z + zm) -
+            W[qp] * (V[q] * zp + V[qp] * z) / (z + zp);
     }
-    x = x + xfv * P.art[i] + P.drhox[q] - P.cor[i] * V[q] * P.dt1[i] * DZ1[q] * P.art[i];
-    y = y + yfv * P.art[i] + P.drhoy[q] + P.cor[i] * U[q] * P.dt1[i] * DZ1[q] * P.art[i];
+    x = x + xfv * P.art[i] + P.drhox[q] - P.cor[i] * V[q] * P.dt1[i] * z * P.art[i];
+    y = y + yfv * P.art[i] + P.drhoy[q] + P.cor[i] * U[q] * P.dt1[i] * z * P.art[i];
   }
   if (P.isbce[i] == 2) { x = 0.0; y = 0.0; }
   river3(P, i, k, x, y);
@@ -746,7 +747,7 @@ __global__ void __launch_bounds__(256) k_adv_uv(const Dev P) {
   double px = 0.0, py = 0.0;
   const R epor = (R)P.epor[i], three = (R)3.0;
   R xr = 0, yr = 0, vmr = 0;
-  const double dz1i = P.dz1[C3(P, i, k)];
+  const double dz1i = P.dz1(i, k);
   const double gdd = P.grav_e[i] * P.dt1[i] * dz1i;
   for (int s = 0; s < 3; ++s) {
     const size_t q = (size_t)s * n1 + i;
@@ -755,7 +756,7 @@ __global__ void __launch_bounds__(256) k_adv_uv(const Dev P) {
     const int ia = ci.y, ib = ci.z;
     const int j1 = ci.w, j2 = P.ce_j2[q];
     double elij = 0.5 * (P.egf[j1] + P.egf[j2]);
-    R dij = (R)(0.5 * (P.dt[j1] * P.dz[N3(P, j1, k)] + P.dt[j2] * P.dz[N3(P, j2, k)]));
+    R dij = (R)(0.5 * (P.dt[j1] * P.dz(j1, k) + P.dt[j2] * P.dz(j2, k)));
     if (P.iswetct[ia] * P.iswetc[ia] == 1 || P.iswetct[ib] * P.iswetc[ib] == 1) {
       EdgeFlux<R> f = edge_flux3<R>(P, q, ia, ib, k, dij, true);
       vmr = vmr + f.viscof;
@@ -833,24 +834,24 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? (UV ? 6 : 7) : 4) k_mom3
     dt1 = P.dt1[i];
     d1 = P.d1[i];
     gd = P.grav_e[i] * dt1;
-    z = P.dz1[C3(P, i, kb)];
+    z = P.dz1(i, kb);
     if (kb > 1) {
       const size_t qm = C3(P, i, kb - 1);
       um = P.u[qm];
       vm = P.v[qm];
-      zm = P.dz1[qm];
+      zm = P.dz1(i, kb - 1);
       const double wk = P.w[C3(P, i, kb)];
       xtop = wk * (ui_d * zm + um * z) / (z + zm);
       ytop = wk * (vi_d * zm + vm * z) / (z + zm);
     }
   }
   for (int k = kb; k <= ke; ++k) {
-    const size_t base = C3(P, 0, k), nbase = N3(P, 0, k);
-    const double *U = P.u + base, *V = P.v + base, *DZ = P.dz + nbase;
+    const size_t base = C3(P, 0, k);
+    const double *U = P.u + base, *V = P.v + base;
     const G3<R> gi = load_g3<R>(P, i, k);
     const R* VC = Mh::vc3(P) + base;
     const R vci = VC[i], ui = (R)ui_d, vi = (R)vi_d;
-    const double dd[3] = {dts[0] * DZ[xs[0]], dts[1] * DZ[xs[1]], dts[2] * DZ[xs[2]]};
+    const double dd[3] = {dts[0] * P.dz(xs[0], k), dts[1] * P.dz(xs[1], k), dts[2] * P.dz(xs[2], k)};
     const double gdd = gd * z;
     R xr = 0, yr = 0, vmr = 0;
     double px = 0.0, py = 0.0;
@@ -952,7 +953,7 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? (UV ? 6 : 7) : 4) k_mom3
       const size_t qp = q + P.ns;
       up = P.u[qp];
       vp = P.v[qp];
-      zp = P.dz1[qp];
+      zp = P.dz1(i, k + 1);
       const double wk = P.w[qp], zs = z + zp;
       xbot = wk * (ui_d * zp + up * z) / zs;
       ybot = wk * (vi_d * zp + vp * z) / zs;
@@ -1109,7 +1110,7 @@ __global__ void __launch_bounds__(kTileCells, sizeof(R) == 4 ? 6 : 4) k_mom3d_st
     for (int q = tid; q < ne; q += nt) {
       if (!s_ok[q]) continue;
       const int lab = s_j[2 * EC + q], la = lab & 0xffff, lb = lab >> 16;
-      const R dij = (R)(0.5 * (s_dt[q] * P.dz[N3(P, s_j[q], k)] + s_dt[EC + q] * P.dz[N3(P, s_j[EC + q], k)]));
+      const R dij = (R)(0.5 * (s_dt[q] * P.dz(s_j[q], k) + s_dt[EC + q] * P.dz(s_j[EC + q], k)));
       const R ga[4] = {s_c[2 * CC + la], s_c[3 * CC + la], s_c[4 * CC + la], s_c[5 * CC + la]};
       const R gb[4] = {s_c[2 * CC + lb], s_c[3 * CC + lb], s_c[4 * CC + lb], s_c[5 * CC + lb]};
       const EdgeFlux<R> f = edge_flux_staged<R>(P, s_c[la], s_c[CC + la], ga, s_c[lb], s_c[CC + lb], gb,
@@ -1128,7 +1129,7 @@ __global__ void __launch_bounds__(kTileCells, sizeof(R) == 4 ? 6 : 4) k_mom3d_st
     R xr = 0, yr = 0, vmr = 0;
     double px = 0.0, py = 0.0, dz1i = 0.0, gdd = 0.0;
     if (UV) {
-      dz1i = P.dz1[C3(P, i, k)];
+      dz1i = P.dz1(i, k);
       gdd = P.grav_e[i] * P.dt1[i] * dz1i;
     }
 #pragma unroll
@@ -1235,10 +1236,10 @@ __global__ void __launch_bounds__(128) k_vdif_uv(const Dev P, int parts) {
       const double d1 = P.d1[i];
       // A(K) uses KM1(K+1) with DZ1(K), DZZ1(K); C(K) uses KM1(K) with DZ1(K), DZZ1(K-1).
       auto Acoef = [&](int kk) {
-        return -DTI * (P.km1[C3(P, i, kk + 1)] + P.umol) / (P.dz1[C3(P, i, kk)] * P.dzz1[C3(P, i, kk)] * d1 * d1);
+        return -DTI * (P.km1[C3(P, i, kk + 1)] + P.umol) / (P.dz1(i, kk) * P.dzz1(i, kk) * d1 * d1);
       };
       auto Ccoef = [&](int kk) {
-        return -DTI * (P.km1[C3(P, i, kk)] + P.umol) / (P.dz1[C3(P, i, kk)] * P.dzz1[C3(P, i, kk - 1)] * d1 * d1);
+        return -DTI * (P.km1[C3(P, i, kk)] + P.umol) / (P.dz1(i, kk) * P.dzz1(i, kk - 1) * d1 * d1);
       };
       int n1 = P.N + 1;
       int it1 = P.isonb[P.nv[i]], it2 = P.isonb[P.nv[n1 + i]], it3 = P.isonb[P.nv[2 * n1 + i]];
@@ -1247,8 +1248,8 @@ __global__ void __launch_bounds__(128) k_vdif_uv(const Dev P, int parts) {
       double wus = P.wusurf[i], wvs = P.wvsurf[i];
       vhu[1] = a1 / (a1 - 1.0);
       vhv[1] = a1 / (a1 - 1.0);
-      vhpu[1] = (-DTI * wus * tmp / (-P.dz1[C3(P, i, 1)] * d1) - P.uf[C3(P, i, 1)]) / (a1 - 1.0);
-      vhpv[1] = (-DTI * wvs * tmp / (-P.dz1[C3(P, i, 1)] * d1) - P.vf[C3(P, i, 1)]) / (a1 - 1.0);
+      vhpu[1] = (-DTI * wus * tmp / (-P.dz1(i, 1) * d1) - P.uf[C3(P, i, 1)]) / (a1 - 1.0);
+      vhpv[1] = (-DTI * wvs * tmp / (-P.dz1(i, 1) * d1) - P.vf[C3(P, i, 1)]) / (a1 - 1.0);
       // the forward elimination; the loads of four levels are issued before their steps
       auto step = [&](int k, double ak, double ck, double uk, double vk) {
         double pu = 1.0 / (ak + ck * (1.0 - vhu[k - 1]) - 1.0);
@@ -1276,7 +1277,7 @@ __global__ void __launch_bounds__(128) k_vdif_uv(const Dev P, int parts) {
       double tps = P.cbc[i] * sqrt(ub * ub + vb * vb);
       P.tps[i] = tps;
       double cb = Ccoef(KBM1);
-      double dzb = P.dz1[C3(P, i, KBM1)];
+      double dzb = P.dz1(i, KBM1);
       double ufk = (cb * vhpu[KBM2] - P.uf[C3(P, i, KBM1)]) / (tps * DTI / (-dzb * d1) - 1.0 - (vhu[KBM2] - 1.0) * cb);
       double vfk = (cb * vhpv[KBM2] - P.vf[C3(P, i, KBM1)]) / (tps * DTI / (-dzb * d1) - 1.0 - (vhv[KBM2] - 1.0) * cb);
       finish(KBM1, ufk, vfk);
@@ -1325,7 +1326,7 @@ __global__ void __launch_bounds__(128) k_vdif_uv(const Dev P, int parts) {
       double etf1aa = ONE_THIRD * (P.el[j1] + P.el[j2] + P.el[j3]);
       for (int k = 1; k <= KBM1; ++k) {
         size_t q = C3(P, i, k);
-        double zz = P.zz1[q];
+        double zz = P.zz1(i, k);
         double ww1 = 0.5 * (P.w[q] + P.w[C3(P, i, k + 1)]) + P.u[q] * (zz * dddx + dedx) + P.v[q] * (zz * dddy + dedy);
         double ww2 = (zz + 1.0) * (etf1aa - P.et1[i]) / DTI;
         P.ww[q] = ww1 + ww2;
@@ -1385,7 +1386,7 @@ __global__ void __launch_bounds__(128) k_phy_rhoz(const Dev P) {
   const int M1 = P.KBM1;
   double X[kMaxKB], A[kMaxKB];
   for (int k = 1; k <= M1; ++k) {
-    X[k - 1] = P.zz[N3(P, i, k)] * P.dt[i] + P.et[i];
+    X[k - 1] = P.zz(i, k) * P.dt[i] + P.et[i];
     A[k - 1] = P.rho1[N3(P, i, k)];
   }
   int j = 0;
@@ -1420,13 +1421,13 @@ __global__ void __launch_bounds__(128) k_phy_baropg(const Dev P) {
   }
   auto emit = [&](int k, double bx, double by) {
     const size_t q = C3(P, i, k);
-    const double dz1 = P.dz1[q];
+    const double dz1 = P.dz1(i, k);
     P.drhox[q] = -bx * dt1 * dz1 * art * ramp;
     P.drhoy[q] = -by * dt1 * dz1 * art * ramp;
   };
   auto target = [&](int k) {
-    return (P.zz[N3(P, j1, k)] * P.dt[j1] + P.et[j1] + (P.zz[N3(P, j2, k)] * P.dt[j2] + P.et[j2]) +
-            (P.zz[N3(P, j3, k)] * P.dt[j3] + P.et[j3])) / 3.;
+    return (P.zz(j1, k) * P.dt[j1] + P.et[j1] + (P.zz(j2, k) * P.dt[j2] + P.et[j2]) +
+            (P.zz(j3, k) * P.dt[j3] + P.et[j3])) / 3.;
   };
   if (ntmp <= 1) {
     double bx = 0.0, by = 0.0;

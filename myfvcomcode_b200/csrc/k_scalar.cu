@@ -192,7 +192,8 @@ __global__ void __launch_bounds__(256) k_grad(const Dev P, int which) {
     R vf;
     if (which == 0) {
       const size_t qm = N3(P, i, k - 1);
-      vf = (R)((P.viscofh[q] * P.dz[qm] + P.viscofh[qm] * P.dz[q]) / (P.dz[q] + P.dz[qm]));
+      const double za = P.dz(i, k - 1), zb = P.dz(i, k);
+      vf = (R)((P.viscofh[q] * za + P.viscofh[qm] * zb) / (zb + za));
     } else {
       vf = (R)P.viscofh[q];
     }
@@ -214,42 +215,42 @@ __global__ void __launch_bounds__(256) k_grad(const Dev P, int which) {
 // Vertical-neighbour bound of FCT on sigma layers (fct_t.F:78-97) and on interfaces
 // (fct_q2.F:73-92).
 __device__ inline void fct_layer_bounds(const Dev& P, int i, int k, const double* F, double& fmax_, double& fmin_) {
-  const double* DZ = P.dz;
+  const double z = P.dz(i, k), zm = k > 1 ? P.dz(i, k - 1) : 0.0, zp = k < P.KBM1 ? P.dz(i, k + 1) : 0.0;
   size_t q = N3(P, i, k);
   if (k == 1) {
     size_t qp = N3(P, i, k + 1);
-    double a = (F[q] * DZ[qp] + F[qp] * DZ[q]) / (DZ[q] + DZ[qp]);
+    double a = (F[q] * zp + F[qp] * z) / (z + zp);
     fmax_ = fmax(fmax_, a);
     fmin_ = fmin(fmin_, a);
   } else if (k == P.KBM1) {
     size_t qm = N3(P, i, k - 1);
-    double a = (F[q] * DZ[qm] + F[qm] * DZ[q]) / (DZ[q] + DZ[qm]);
+    double a = (F[q] * zm + F[qm] * z) / (z + zm);
     fmax_ = fmax(fmax_, a);
     fmin_ = fmin(fmin_, a);
   } else {
     size_t qm = N3(P, i, k - 1), qp = N3(P, i, k + 1);
-    double a = (F[q] * DZ[qm] + F[qm] * DZ[q]) / (DZ[q] + DZ[qm]);
-    double b = (F[q] * DZ[qp] + F[qp] * DZ[q]) / (DZ[q] + DZ[qp]);
+    double a = (F[q] * zm + F[qm] * z) / (z + zm);
+    double b = (F[q] * zp + F[qp] * z) / (z + zp);
     fmax_ = fmax(fmax(fmax_, a), b);
     fmin_ = fmin(fmin(fmin_, a), b);
   }
 }
 __device__ inline void fct_level_bounds(const Dev& P, int i, int k, const double* F, double& fmax_, double& fmin_) {
-  const double* DZZ = P.dzz;
+  const double z = P.dzz(i, k), zm = P.dzz(i, k - 1), zmm = k > 2 ? P.dzz(i, k - 2) : 0.0;
   size_t q = N3(P, i, k), qm = N3(P, i, k - 1), qp = N3(P, i, k + 1);
   if (k == 2) {
-    double a = (F[q] * DZZ[q] + F[qp] * DZZ[qm]) / (DZZ[q] + DZZ[qm]);
+    double a = (F[q] * z + F[qp] * zm) / (z + zm);
     fmax_ = fmax(fmax_, a);
     fmin_ = fmin(fmin_, a);
   } else if (k == P.KBM1) {
     size_t qmm = N3(P, i, k - 2);
-    double a = (F[q] * DZZ[qmm] + F[qm] * DZZ[qm]) / (DZZ[qm] + DZZ[qmm]);
+    double a = (F[q] * zmm + F[qm] * zm) / (zm + zmm);
     fmax_ = fmax(fmax_, a);
     fmin_ = fmin(fmin_, a);
   } else {
     size_t qmm = N3(P, i, k - 2);
-    double a = (F[q] * DZZ[qmm] + F[qm] * DZZ[qm]) / (DZZ[qm] + DZZ[qmm]);
-    double b = (F[q] * DZZ[q] + F[qp] * DZZ[qm]) / (DZZ[q] + DZZ[qm]);
+    double a = (F[q] * zmm + F[qm] * zm) / (zm + zmm);
+    double b = (F[q] * z + F[qp] * zm) / (z + zm);
     fmax_ = fmax(fmax(fmax_, a), b);
     fmin_ = fmin(fmin(fmin_, a), b);
   }
@@ -286,14 +287,14 @@ __device__ inline void he_cell_load(const Dev& P, int c, int k, HeCell<R>& hc) {
   size_t ck = C3(P, c, k);
   if (MODE == 0) {
     size_t ckm = C3(P, c, k - 1);
-    const double za = P.dz1[ckm], zb = P.dz1[ck], zs = zb + za;
+    const double za = P.dz1(c, k - 1), zb = P.dz1(c, k), zs = zb + za;
     hc.uq = (R)((P.u[ck] * za + P.u[ckm] * zb) / zs);
     hc.vq = (R)((P.v[ck] * za + P.v[ckm] * zb) / zs);
-    hc.dtij = (R)(P.dt1[c] * P.dzz1[ckm]);
+    hc.dtij = (R)(P.dt1[c] * P.dzz1(c, k - 1));
   } else {
     hc.uq = (R)P.u[ck];
     hc.vq = (R)P.v[ck];
-    hc.dtij = (R)(P.dt1[c] * P.dz1[ck]);
+    hc.dtij = (R)(P.dt1[c] * P.dz1(c, k));
   }
 }
 
@@ -505,8 +506,8 @@ __global__ void __launch_bounds__(256) k_gather_q(const Dev P, int parts) {
     if (wet) {
       size_t qm = N3(P, i, k - 1), qp = N3(P, i, k + 1);
       double temp = P.wts[qm] * Q[qm] - P.wts[qp] * Q[qp];
-      x = x + temp * P.art1[i] * P.dzz[qm] / (P.dz[qm] + P.dz[q]);
-      qf = (Q[q] - x / P.art1[i] * (P.dti / (P.dt[i] * P.dzz[qm]))) * (P.dt[i] / P.d[i]);
+      x = x + temp * P.art1[i] * P.dzz(i, k - 1) / (P.dz(i, k - 1) + P.dz(i, k));
+      qf = (Q[q] - x / P.art1[i] * (P.dti / (P.dt[i] * P.dzz(i, k - 1)))) * (P.dt[i] / P.d[i]);
     } else {
       qf = Q[q];
     }
@@ -649,16 +650,16 @@ __global__ void __launch_bounds__(256, 4) k_vdif_q_levels(const Dev P) {
     double boygr = 0.0, prod = 0.0, lk;
     if (k >= 2 && k <= KBM1) {
       if (wet) {
-        boygr = P.grav_n[i] * (P.rho1[n3(k - 1)] - P.rho1[q]) / (P.dzz[n3(k - 1)] * d);
+        boygr = P.grav_n[i] * (P.rho1[n3(k - 1)] - P.rho1[q]) / (P.dzz(i, k - 1) * d);
         prod = P.km[q] * 0.0 * pow(.5 * (-boygr + fabs(boygr)), 1.5);
         double uk, vk;
         ring_mean(k, uk, vk);
-        const double den = P.dzz[n3(k - 1)] * d;
+        const double den = P.dzz(i, k - 1) * d;
         const double shear2 = ((uk - ukm1) * (uk - ukm1) + (vk - vkm1) * (vk - vkm1)) / (den * den);
         if (AUX & 1) {
           // the network's inputs: inside the envelope or not, then transformed,
           // standardised and rounded to BF16 as the MMA takes them
-          const float fv[CLOS_IN] = {(float)boygr, (float)shear2, (float)d, (float)P.z[q], (float)sqrt(utau2),
+          const float fv[CLOS_IN] = {(float)boygr, (float)shear2, (float)d, (float)P.z(i, k), (float)sqrt(utau2),
                                      (float)sqrt(sqrt(wub * wub + wvb * wvb)), (float)q2, (float)q2l};
           uint32_t packed[4];
           for (int f = 0; f < CLOS_IN; ++f) {
@@ -675,7 +676,7 @@ __global__ void __launch_bounds__(256, 4) k_vdif_q_levels(const Dev P) {
           samp(0, k, boygr);
           samp(1, k, shear2);
           samp(2, k, d);
-          samp(3, k, P.z[q]);
+          samp(3, k, P.z(i, k));
           samp(4, k, sqrt(utau2));
           samp(5, k, sqrt(sqrt(wub * wub + wvb * wvb)));
           samp(6, k, q2);
@@ -688,7 +689,7 @@ __global__ void __launch_bounds__(256, 4) k_vdif_q_levels(const Dev P) {
       }
       // length scale and its limits (vdif_q.F:300-331)
       lk = q2l / q2;
-      if (P.z[q] > -0.5) lk = fmax(lk, KAPPA * l0);
+      if (P.z(i, k) > -0.5) lk = fmax(lk, KAPPA * l0);
       if (boygr < 0.0) {
         double lmax = sqrt(fabs(GH_MIN) * q2 / (-boygr + SMALL));
         lk = fmin(lk, lmax);
@@ -709,7 +710,7 @@ __global__ void __launch_bounds__(256, 4) k_vdif_q_levels(const Dev P) {
     P.vq_gh[q] = gh;
     P.vq_dtef[q] = dtef;
     if (wet && k >= 2 && k <= KBM1) {
-      const double x = (1. / fabs(P.z[q] - P.z[n3(1)]) + 1. / fabs(P.z[q] - P.z[n3(KB)])) * lk / (d * KAPPA);
+      const double x = (1. / fabs(P.z(i, k) - P.z(i, 1)) + 1. / fabs(P.z(i, k) - P.z(i, KB))) * lk / (d * KAPPA);
       P.vq_dtefl[q] = dtef * (1. + E2 * (x * x));
     }
   }
@@ -744,8 +745,8 @@ __global__ void __launch_bounds__(128) k_vdif_q_sweep(const Dev P) {
   double* QF = q2l ? P.q2lf : P.q2f;
   // the coefficients of level k: A, C, the diagonal term and the source of the equation
   auto coef = [&](int k, double& a, double& c, double& e, double& r, double& qf) {
-    a = -0.5 * DTI * (P.kq[n3(k + 1)] + P.kq[n3(k)] + 2.0 * P.umol) / (P.dzz[n3(k - 1)] * P.dz[n3(k)] * d * d);
-    c = -0.5 * DTI * (P.kq[n3(k - 1)] + P.kq[n3(k)] + 2.0 * P.umol) / (P.dzz[n3(k - 1)] * P.dz[n3(k - 1)] * d * d);
+    a = -0.5 * DTI * (P.kq[n3(k + 1)] + P.kq[n3(k)] + 2.0 * P.umol) / (P.dzz(i, k - 1) * P.dz(i, k) * d * d);
+    c = -0.5 * DTI * (P.kq[n3(k - 1)] + P.kq[n3(k)] + 2.0 * P.umol) / (P.dzz(i, k - 1) * P.dz(i, k - 1) * d * d);
     if (q2l) {
       e = DTI * P.vq_dtefl[n3(k)] + 1.;
       r = DTI * (-P.vq_prod[n3(k)] * P.l[n3(k)] * E1);
@@ -883,24 +884,24 @@ __global__ void __launch_bounds__(256) k_gather_ts(const Dev P, int parts) {
     size_t q = N3(P, i, k);
     double ff;
     if (wet) {
-      const double* DZ = P.dz;
+      const double z = P.dz(i, k), zm = k > 1 ? P.dz(i, k - 1) : 0.0, zp = k < P.KBM1 ? P.dz(i, k + 1) : 0.0;
       double temp;
       if (k == 1) {
         size_t qp = N3(P, i, k + 1);
-        temp = -P.wts[qp] * (F1[q] * DZ[qp] + F1[qp] * DZ[q]) / (DZ[q] + DZ[qp]);
+        temp = -P.wts[qp] * (F1[q] * zp + F1[qp] * z) / (z + zp);
       } else if (k == P.KBM1) {
         size_t qm = N3(P, i, k - 1);
-        temp = P.wts[q] * (F1[q] * DZ[qm] + F1[qm] * DZ[q]) / (DZ[q] + DZ[qm]);
+        temp = P.wts[q] * (F1[q] * zm + F1[qm] * z) / (z + zm);
       } else {
         size_t qm = N3(P, i, k - 1), qp = N3(P, i, k + 1);
-        temp = P.wts[q] * (F1[q] * DZ[qm] + F1[qm] * DZ[q]) / (DZ[q] + DZ[qm]) -
-               P.wts[qp] * (F1[q] * DZ[qp] + F1[qp] * DZ[q]) / (DZ[q] + DZ[qp]);
+        temp = P.wts[q] * (F1[q] * zm + F1[qm] * z) / (z + zm) -
+               P.wts[qp] * (F1[q] * zp + F1[qp] * z) / (z + zp);
       }
       if (P.isonb[i] == 2)
         x = temp * P.art1[i];
       else
         x = x + temp * P.art1[i];
-      ff = (F1[q] - x / P.art1[i] * (P.dti / (P.dt[i] * DZ[q]))) * (P.dt[i] / P.dtfa[i]);
+      ff = (F1[q] - x / P.art1[i] * (P.dti / (P.dt[i] * z))) * (P.dt[i] / P.dtfa[i]);
     } else {
       ff = F1[q];
     }
@@ -964,8 +965,8 @@ __global__ void __launch_bounds__(128) k_vdif_ts(const Dev P, int parts) {
   const double DTI = P.dti, UMOLPR = P.umol * 1.e0, GW = 0.0;
   const double d = P.d[i];
   auto n3 = [&](int k) { return N3(P, i, k); };
-  auto AF = [&](int k) { double fkh = P.kh[n3(k + 1)]; return -DTI * (fkh + UMOLPR) / (P.dz[n3(k)] * P.dzz[n3(k)] * d * d); };
-  auto CF = [&](int k) { double fkh = P.kh[n3(k)]; return -DTI * (fkh + UMOLPR) / (P.dz[n3(k)] * P.dzz[n3(k - 1)] * d * d); };
+  auto AF = [&](int k) { double fkh = P.kh[n3(k + 1)]; return -DTI * (fkh + UMOLPR) / (P.dz(i, k) * P.dzz(i, k) * d * d); };
+  auto CF = [&](int k) { double fkh = P.kh[n3(k)]; return -DTI * (fkh + UMOLPR) / (P.dz(i, k) * P.dzz(i, k - 1) * d * d); };
   const double khbottom = P.kh[n3(KBM1)];
   const bool update = P.iswetn[i] * P.iswetnt[i] == 1;
   {
@@ -988,13 +989,13 @@ __global__ void __launch_bounds__(128) k_vdif_ts(const Dev P, int parts) {
     // RAD at level k; zero without heating
     auto RAD = [&](int k) {
       if (!heat) return 0.0;
-      const double zdep = P.z[n3(k)] * d;
+      const double zdep = P.z(i, k) * d;
       return swradf * (P.rheat * exp(zdep / P.zeta1) + (1 - P.rheat) * exp(zdep / P.zeta2));
     };
     double rad_k = RAD(1), rad_k1 = RAD(2);
     double af1 = AF(1);
     vhf[1] = af1 / (af1 - 1.);
-    vhpf[1] = -DTI * (sasurf + wfsurf - swradf + rad_k - rad_k1) / (-P.dz[n3(1)] * d) - F[n3(1)];
+    vhpf[1] = -DTI * (sasurf + wfsurf - swradf + rad_k - rad_k1) / (-P.dz(i, 1) * d) - F[n3(1)];
     vhpf[1] = vhpf[1] / (af1 - 1.);
     // level k's coefficients and source, then its step of the (serial) recurrence; the
     // loads of four levels are issued before their steps
@@ -1004,7 +1005,7 @@ __global__ void __launch_bounds__(128) k_vdif_ts(const Dev P, int parts) {
       af = AF(k);
       cf = CF(k);
       fk = F[n3(k)];
-      r = DTI * (rad_k - rad_k1) / (d * P.dz[n3(k)]);
+      r = DTI * (rad_k - rad_k1) / (d * P.dz(i, k));
     };
     auto step = [&](int k, double af, double cf, double fk, double r) {
       double p = 1. / (af + cf * (1. - vhf[k - 1]) - 1.);
@@ -1040,7 +1041,7 @@ __global__ void __launch_bounds__(128) k_vdif_ts(const Dev P, int parts) {
       }
       double cfb = CF(KBM1);
       const double rad_b = RAD(KBM1), rad_kb = RAD(KB);
-      double ff = (cfb * vhpf[KBM2] - F[n3(KBM1)] - GW + DTI * (rad_b - rad_kb - tmp) / (d * P.dz[n3(KBM1)])) /
+      double ff = (cfb * vhpf[KBM2] - F[n3(KBM1)] - GW + DTI * (rad_b - rad_kb - tmp) / (d * P.dz(i, KBM1))) /
                   (cfb * (1. - vhf[KBM2]) - 1.);
       F[n3(KBM1)] = ff;
       for (int k = 2; k <= KBM1; ++k) {
@@ -1097,8 +1098,8 @@ __global__ void __launch_bounds__(64) k_bcond_ts_obc(const Dev P, int parts) {
   if (live) {
     f1 = F1[q];
     fnext = FF1[q1];
-    term[0][k - 1] = f1 * P.dz[q];
-    term[1][k - 1] = fnext * P.dz[q1];
+    term[0][k - 1] = f1 * P.dz(j, k);
+    term[1][k - 1] = fnext * P.dz(j1, k);
     term[2][k - 1] = XO[(size_t)(k - 1) * (P.iobcn + 1) + ob];
   }
   __syncthreads();
@@ -1208,8 +1209,8 @@ __global__ void k_budget_partial(const Dev P, double* part) {
     double dd = P.d[i] * P.art1[i];
     double ct = 0.0, cs = 0.0;
     for (int k = 1; k <= P.KBM1; ++k) {
-      ct = ct + P.t1[N3(P, i, k)] * P.dz[N3(P, i, k)];
-      cs = cs + P.s1[N3(P, i, k)] * P.dz[N3(P, i, k)];
+      ct = ct + P.t1[N3(P, i, k)] * P.dz(i, k);
+      cs = cs + P.s1[N3(P, i, k)] * P.dz(i, k);
     }
     v = v + dd;
     hh = hh + ct * dd;
