@@ -53,8 +53,8 @@ struct fvg_handle {
   cudaGraph_t graph = nullptr;
   bool use_graph = true;
   int clos_grid = 148;
-  // compact external stage of the precision form: allowed (tuning key "compact") and
-  // possible (the mesh check of fvg_set_precision passed)
+  // external stages on the packed records: allowed (tuning key "compact") and possible (the
+  // mesh's edge metrics are the ones its coordinates define, no limiter)
   int compact_allowed = 1;
   int compact_ok = 0;
   // resident external loop: allowed (tuning key "ext_loop"), possible (the device launches
@@ -265,8 +265,7 @@ struct Marker {
 // Whether the external loop runs as one resident kernel (k_ext_loop).
 bool use_ext_loop(const fvg_handle* h) {
   const Dev& P = h->P;
-  if (!h->ext_loop || !h->loop_ok || P.limiter) return false;
-  if (P.prec && !P.f.compact) return false;
+  if (!h->ext_loop || !h->loop_ok || !P.xform) return false;
   return (long)std::max(P.M, P.N) <= (long)kLoopThreads * P.nsm;
 }
 
@@ -295,7 +294,7 @@ void enqueue_internal_step(fvg_handle* h, cudaStream_t s, Marker mk = Marker(), 
   launch_ext_prep(P, s);
   if (P.limiter) launch_alfa2(P, s);
   mk.mark(s, G_BAROPG);
-  launch_ext_cell(P, s, 1, 1, EC_INT_ADVAVE | EC_COMPACT);
+  launch_ext_cell(P, s, 1, 1, EC_INT_ADVAVE);
   launch_int_reset(P, s);
   mk.mark(s, G_INT_ADVAVE);
   // The ISPLIT x 4 Runge-Kutta stages.  Instead of copying UAF to UA and ISWETC to
@@ -314,7 +313,11 @@ void enqueue_internal_step(fvg_handle* h, cudaStream_t s, Marker mk = Marker(), 
     if (done) cudaEventRecord(done, s);
     mk.mark(s, G_EXT_CELL);
   }
-  for (int iext = 1; iext <= p.isplit && !loop; ++iext) {
+  for (int st = 0; st < 4 * p.isplit && !loop && P.xform; ++st) {
+    launch_ext_stage(P, s, st);
+    mk.mark(s, G_EXT_CELL);
+  }
+  for (int iext = 1; iext <= p.isplit && !P.xform; ++iext) {
     for (int K = 1; K <= 4; ++K, ++stage) {
       Dev Q = P;
       if (stage & 1) {
@@ -335,8 +338,7 @@ void enqueue_internal_step(fvg_handle* h, cudaStream_t s, Marker mk = Marker(), 
       if (P.limiter) launch_alfa2(Q, s);
       launch_ext_cell(Q, s, iext, K,
                       (!p.wetting_drying_on ? EC_N2E : P.limiter ? 0 : EC_WET) | EC_FLUXOBN | EC_ADVAVE | EC_EXTUV |
-                          EC_BC2 | (K == 1 ? EC_COPY_RK : 0) | EC_FINISH | EC_COMPACT |
-                          (iext == p.isplit && K == 4 ? EC_LAST : 0),
+                          EC_BC2 | (K == 1 ? EC_COPY_RK : 0) | EC_FINISH,
                       P.limiter ? 0 : 1);
       mk.mark(s, G_EXT_CELL);
     }
@@ -573,6 +575,7 @@ int fvg_create(const fvg_mesh* m, const fvg_params* prm, const fvg_forcing* f, f
   }
 
   // ---- gather lists ----
+  std::vector<int> lo;  // the other cells and the flags of the packed stages (loopo)
   {
     std::vector<std::vector<int>> nl(m1), cl(n1);
     for (int he = 1; he <= m->ncv; ++he) {
@@ -631,8 +634,16 @@ int fvg_create(const fvg_mesh* m, const fvg_params* prm, const fvg_forcing* f, f
     }
     // the resident external loop: the neighbours' nodes off the edges, the cells' least H
     {
-      std::vector<int> far(3 * n1, 0), lx(4 * n1, 0), lo(4 * n1, 0);
+      // half-edges of each cell in ascending order, as their positions take them
+      std::vector<int> ch3(3 * n1, 0), cn(n1, 0);
+      for (int he = 1; he <= m->ncv; ++he) {
+        const int c = m->ntrg[he];
+        if (cn[c] < 3) ch3[3 * c + cn[c]++] = he;
+      }
+      std::vector<int> far(3 * n1, 0), lx(4 * n1, 0);
+      lo.assign(4 * n1, 0);
       std::vector<double> hm(n1, 0.0);
+      h->compact_ok = P.limiter == 0;
       for (size_t i = 1; i < n1; ++i) {
         // the node common to two slots' edges
         auto common = [&](int sa, int sb) {
@@ -654,8 +665,21 @@ int fvg_create(const fvg_mesh* m, const fvg_params* prm, const fvg_forcing* f, f
           bits |= side << sl | (m->isbc[e] != 0 ? 1 : 0) << (3 + sl);
           lo[4 * i + sl] = side == 0 ? m->iec[e1 + e] : m->iec[e];
           lx[4 * i + sl] = x[sl];
+          const int j1 = m->ienode[e], j2 = m->ienode[e1 + e], ia = m->iec[e], ib = m->iec[e1 + e];
+          if (j1 != x[sl]) bits |= 1 << (8 + sl);
+          // the metrics that the packed stages form from the coordinates
+          const double xij = (m->vx[j1] + m->vx[j2]) / 2.0, yij = (m->vy[j1] + m->vy[j2]) / 2.0;
+          if (xij - m->xc[ia] != m->xijc[e] - m->xc[ia] || yij - m->yc[ia] != m->yijc[e] - m->yc[ia] ||
+              xij - m->xc[ib] != m->xijc[e] - m->xc[ib] || yij - m->yc[ib] != m->yijc[e] - m->yc[ib] ||
+              m->vx[j2] - m->vx[j1] != m->dltxc[e] || m->vy[j2] - m->vy[j1] != m->dltyc[e])
+            h->compact_ok = 0;
+          const int he = ch3[3 * i + sl];
+          if (he == 0 || m->dltxe[he] != xij - m->xc[i] || m->dltye[he] != yij - m->yc[i]) h->compact_ok = 0;
         }
         lx[4 * i + 3] = bits;
+        const double iu = m->iucp[i], ep = m->epor[i];
+        if (!(iu == 0.0 || iu == 1.0) || !(ep == 0.0 || ep == 1.0)) h->compact_ok = 0;
+        lo[4 * i + 3] = (m->isbce[i] & 3) | (m->cc_sponge[i] != 0.0 ? 16 : 0) | (ep == 1.0 ? 32 : 0) | (iu == 1.0 ? 64 : 0);
         hm[i] = std::fmin(std::fmin(m->h[m->nv[i]], m->h[m->nv[n1 + i]]), m->h[m->nv[2 * n1 + i]]);
         for (int sl = 0; sl < 3; ++sl) {
           const int code = cl[i][sl], e = code >> 1;
@@ -668,7 +692,13 @@ int fvg_create(const fvg_mesh* m, const fvg_params* prm, const fvg_forcing* f, f
       }
       UPI(wfar, far.data(), far.size());
       UPI(loopx, lx.data(), lx.size());
-      UPI(loopo, lo.data(), lo.size());
+      std::vector<double> xy(2 * m1), cxy(2 * n1);
+      for (size_t i = 0; i < m1; ++i) { xy[2 * i] = m->vx[i]; xy[2 * i + 1] = m->vy[i]; }
+      for (size_t i = 0; i < n1; ++i) { cxy[2 * i] = m->xc[i]; cxy[2 * i + 1] = m->yc[i]; }
+      if ((rc = upload(h, (double**)&P.vxy, xy.data(), xy.size()))) return fail(rc);
+      if ((rc = upload(h, (double**)&P.xyc, cxy.data(), cxy.size()))) return fail(rc);
+      if ((rc = dalloc(h, (double**)&P.exd, 12 * n1))) return fail(rc);
+      if ((rc = dalloc(h, (double**)&P.xrk, 2 * n1))) return fail(rc);
       if ((rc = dalloc(h, (double**)&P.xuv, 4 * n1))) return fail(rc);
       if ((rc = dalloc(h, (double**)&P.xnd, 2 * m1))) return fail(rc);
       if ((rc = dalloc(h, &P.xg, 4 * n1))) return fail(rc);
@@ -787,6 +817,8 @@ int fvg_create(const fvg_mesh* m, const fvg_params* prm, const fvg_forcing* f, f
     build_csr(co, ptr, ent);
     UPI(node_obc, node_obc.data(), m1); UPI(obc_kind, kind.data(), o1);
     UPI(cell_obc_ptr, ptr.data(), ptr.size()); UPI(cell_obc, ent.data(), ent.size());
+    for (size_t i = 1; i < n1; ++i)
+      if (ptr[i + 1] > ptr[i]) lo[4 * i + 3] |= 8;
     UPI(i_obc_n, m->i_obc_n, o1); UPI(next_obc, m->next_obc, o1);
     UPD(dltn_obc, m->dltn_obc, o1); UPD(fluxf_obc, m->fluxf_obc, o1 * 2);
     size_t nt = h->ntide;
@@ -838,6 +870,9 @@ int fvg_create(const fvg_mesh* m, const fvg_params* prm, const fvg_forcing* f, f
     UPI(node_riv_ptr, ptr.data(), ptr.size()); UPI(node_riv, ent.data(), ent.size());
     build_csr(cr, ptr, ent);
     UPI(cell_riv_ptr, ptr.data(), ptr.size()); UPI(cell_riv, ent.data(), ent.size());
+    for (size_t i = 1; i < n1; ++i)
+      if (ptr[i + 1] > ptr[i]) lo[4 * i + 3] |= 4;
+    UPI(loopo, lo.data(), lo.size());
     UPI(cell_bcriv, bcriv.data(), n1); UPI(riv_skip, skip.data(), m1);
     UPI(inodeq, m->inodeq, q1); UPI(icellq, m->icellq, q1); UPI(n_icellq, m->n_icellq, q1 * 2);
     UPD(rdisq, m->rdisq, q1 * 2); UPD(qarea, m->qarea, q1); UPD(vqdist, m->vqdist, q1 * (KB - 1));
@@ -961,6 +996,7 @@ int fvg_create(const fvg_mesh* m, const fvg_params* prm, const fvg_forcing* f, f
     h->err = "device synchronize failed after create";
     return fail(FVG_ERR_CUDA);
   }
+  h->P.xform = h->compact_ok;
   *out = h;
   return FVG_OK;
 }
@@ -1239,6 +1275,11 @@ int fvg_set_forcing(fvg_handle* h, const fvg_forcing* f) {
   return FVG_OK;
 }
 
+static void set_xform(fvg_handle* h) {
+  h->P.xform = h->compact_ok && h->compact_allowed;
+  h->P.f.compact = h->P.prec == FVG_PREC_FP32_FLUX && h->P.xform;
+}
+
 int fvg_set_precision(fvg_handle* h, int32_t mode) {
   if (!h) return FVG_ERR_ARG;
   if (mode != FVG_PREC_FP64 && mode != FVG_PREC_FP32_FLUX) { h->err = "unknown precision mode"; return FVG_ERR_ARG; }
@@ -1285,27 +1326,12 @@ int fvg_set_precision(fvg_handle* h, int32_t mode) {
     CK(cudaStreamSynchronize(cudaStreamLegacy));
     launch_make_f32(P, h->stream);
     CK(cudaGetLastError());
-    // records of the compact stage kernel, used where the mesh's edge metrics are the ones
-    // its coordinates define (checked here, bit for bit)
-    if ((rc = dalloc(h, (int**)&f.slot4, 4 * 3 * n1))) return fail(rc);
-    if ((rc = dalloc(h, (double**)&f.vxy, 2 * ((size_t)P.M + 1)))) return fail(rc);
-    if ((rc = dalloc(h, (double**)&f.xyc, 2 * n1))) return fail(rc);
-    if ((rc = dalloc(h, (float**)&f.artcc, 2 * n1))) return fail(rc);
     if ((rc = dalloc(h, (double**)&f.exc0, 4 * n1))) return fail(rc);
     if ((rc = dalloc(h, (double**)&f.exc1, 4 * n1))) return fail(rc);
-    if ((rc = dalloc(h, &f.cflag, n1))) return fail(rc);
-    int* d_bad = nullptr;
-    if ((rc = dalloc(h, &d_bad, 1))) return fail(rc);
     CK(cudaStreamSynchronize(cudaStreamLegacy));
-    launch_make_compact(P, h->stream, d_bad);
-    CK(cudaGetLastError());
-    int bad = -1;
-    CK(cudaMemcpyAsync(&bad, d_bad, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
-    CK(cudaStreamSynchronize(h->stream));
-    h->compact_ok = (bad == 0 && !P.limiter && !P.gcy) ? 1 : 0;
   }
   P.prec = mode;
-  P.f.compact = (mode == FVG_PREC_FP32_FLUX && h->compact_ok) ? h->compact_allowed : 0;
+  set_xform(h);
   // The captured step holds the other precision's kernels: capture again.
   CK(cudaStreamSynchronize(h->stream));
   if (h->gexec) { cudaGraphExecDestroy(h->gexec); h->gexec = nullptr; }
@@ -1427,7 +1453,7 @@ int fvg_set_tuning(fvg_handle* h, const char* key, int32_t value) {
     h->P.staged = value;
   } else if (k == "compact") {
     h->compact_allowed = value != 0;
-    h->P.f.compact = (h->P.prec == FVG_PREC_FP32_FLUX && h->compact_ok) ? h->compact_allowed : 0;
+    set_xform(h);
   } else if (k == "stream_hints") {
     h->P.ldcs = value != 0;
   } else if (k == "ext_grid") {

@@ -61,21 +61,11 @@ struct F32 {
   float4 *a1u4, *a2u4;
   // Least-squares gradient of UA, VA per cell packed: {UX, UY, VX, VY}
   float4* g2d4;
-  // Compact external stage (compact != 0; set up by fvg_set_precision after checking that
-  // the mesh's edge metrics are the ones its node and cell coordinates define, bit for
-  // bit: DLTXC = VX(IENODE2)-VX(IENODE1), XIJC = (VX(IENODE1)+VX(IENODE2))/2, DLTXE =
-  // XIJC-XC of the half-edge's cell, the same in y).  slot4: per (slot s, cell c) at
-  // s*(N+1)+c {code, the other cell, IENODE1, IENODE2}; vxy {VX, VY} per node; xyc {XC, YC}
-  // per cell; artcc {ART, CC_HVC} in FP32; exc0 per internal step {ADX2D+DRX2D-WUBOT*ART,
-  // ADY2D+DRY2D-WVBOT*ART, 0.001*WSX*ART, 0.001*WSY*ART}; exc1 {COR*ART, ART, H1, GRAV_E};
-  // cflag: ISBCE in bits 0-1, IUCP = 1 bit 2, EPOR = 1 bit 3, river momentum entries bit
-  // 4, open-boundary flux entries bit 5, a sponge coefficient bit 6.
+  // compact: the external stages run on the packed records (Dev::xform) in this form.  exc0
+  // per internal step {ADX2D+DRX2D-WUBOT*ART, ADY2D+DRY2D-WVBOT*ART, 0.001*WSX*ART,
+  // 0.001*WSY*ART}; exc1 {COR*ART, ART, H1, GRAV_E}.
   int compact;
-  int4* slot4;
-  double2 *vxy, *xyc;
-  float2* artcc;
   double4 *exc0, *exc1;
-  int* cflag;
 };
 
 // Input and output scaling of the learned closure's network, and the training envelope.
@@ -217,15 +207,26 @@ struct Dev {
   // obf: the specified elevation of open-boundary node ob at stage st (0..4*ISPLIT-1) of
   // the current internal step, at st*(IOBCN+1) + ob (k_ext_prep).
   double* obf;
-  // The resident external loop (k_ext_loop).  loopx, per cell: its nodes X0, X1, X2 in the
-  // order in which slot s is the edge X(s), X(s+1 mod 3), and w: bit s the cell's side of
-  // slot s, bit 3+s its ISBC, bits 6-7 the place of NV(c,3) among X; loopo, per cell the
-  // other cell of slots 0, 1, 2; wfar, per slot and cell (s*(N+1) + c) the node of the other
-  // cell that is off the edge (0: none); hmin, per cell the smallest H of its nodes.
-  // Exchanged inside the loop: xuv {UA, VA} and xw (ISWETC), each in two buffers of N+1; xg
-  // the FP64 gradients (four per cell), xvc ART*|grad|*CC_HVC in the form's type, xnd
-  // {EL, D} per node.  bar: the grid barrier's counter; bar_err (pinned host memory), set
-  // when a wait ran out.  loop_cells, loop_nodes: cells and nodes per block.
+  // The external stages' packed records (k_ext_loop, k_stage_node, k_stage_cell; and k_mom3d).
+  // loopx, per cell: its nodes X0, X1, X2 in the order in which slot s is the edge X(s),
+  // X(s+1 mod 3), and w: bit s the cell's side of slot s, bit 3+s its ISBC, bits 6-7 the place
+  // of NV(c,3) among X, bit 8+s set where IENODE(e,1) is X(s+1); loopo, per cell the other cell
+  // of slots 0, 1, 2, and w: ISBCE in bits 0-1, river momentum entries bit 2, open-boundary
+  // flux entries bit 3, a sponge coefficient bit 4, EPOR = 1 bit 5, IUCP = 1 bit 6.
+  // xform: the stages form the edge geometry from vxy {VX, VY} and xyc {XC, YC} (DLTXC =
+  // VX(IENODE2)-VX(IENODE1), XIJC = (VX(IENODE1)+VX(IENODE2))/2, DLTXE = XIJC-XC), which
+  // fvg_create found equal to the mesh's own metrics bit for bit; 0 where it did not, or
+  // where a limiter is on: the general kernels then run.
+  // wfar, per slot and cell (s*(N+1) + c) the node of the other cell that is off the edge (0:
+  // none); hmin, per cell the smallest H of its nodes.  exd: EXTUV's fixed terms in FP64, six
+  // planes of N+1 pairs (store_fixed); xrk the pairs UARK, VARK.  Exchanged between cells and
+  // nodes of a stage: xuv {UA, VA} and xw (ISWETC), each in two buffers of N+1; xg the FP64
+  // gradients (four per cell), xvc ART*|grad|*CC_HVC in the form's type, xnd {EL, D} per node.
+  // bar: the resident loop's grid barrier; bar_err (pinned host memory), set when a wait ran
+  // out.  loop_cells, loop_nodes: its cells and nodes per block.
+  int xform;
+  const double2 *vxy, *xyc;
+  double2 *exd, *xrk;
   const int4 *loopx, *loopo;
   double2 *xuv, *xnd;
   double *xg, *xvc;
@@ -301,9 +302,9 @@ struct Dev {
   // so that the arrays gathered from neighbours stay in L2 between stages (tuning key
   // "stream_hints"); results do not depend on it.
   int ldcs;
-  // Blocks per SM of the compact stage kernel's grid-stride launch (tuning key
-  // "ext_grid", default 8: one full wave whose threads walk the cells); 0: one thread per
-  // cell.  nsm: the device's SM count.
+  // Most blocks per SM of the stage cell kernel's launch (tuning key "ext_grid", default 8):
+  // a larger mesh runs as one full wave whose threads walk the cells; 0: one thread per cell.
+  // nsm: the device's SM count.
   int ext_grid, nsm;
 };
 
@@ -442,7 +443,6 @@ template <> struct Mesh<double> {
   __device__ static double dltxc(const Dev& P, int e) { return P.dltxc[e]; }
   __device__ static double dltyc(const Dev& P, int e) { return P.dltyc[e]; }
   __device__ static double art(const Dev& P, int c) { return P.art[c]; }
-  __device__ static double2 artcc(const Dev& P, int c) { return make_double2(P.art[c], P.cc_hvc[c]); }
   __device__ static double cc_hvc(const Dev& P, int c) { return P.cc_hvc[c]; }
   __device__ static double a1u(const Dev& P, size_t q) { return P.a1u[q]; }
   __device__ static double a2u(const Dev& P, size_t q) { return P.a2u[q]; }
@@ -471,7 +471,6 @@ template <> struct Mesh<float> {
   __device__ static float dltxc(const Dev& P, int e) { return P.f.dltxc[e]; }
   __device__ static float dltyc(const Dev& P, int e) { return P.f.dltyc[e]; }
   __device__ static float art(const Dev& P, int c) { return P.f.art[c]; }
-  __device__ static float2 artcc(const Dev& P, int c) { return P.f.artcc[c]; }  // {ART, CC_HVC}
   __device__ static float cc_hvc(const Dev& P, int c) { return P.f.cc_hvc[c]; }
   __device__ static float a1u(const Dev& P, size_t q) { return P.f.a1u[q]; }
   __device__ static float a2u(const Dev& P, size_t q) { return P.f.a2u[q]; }
@@ -542,12 +541,9 @@ enum ExtNodeParts { EN_EXTEL = 1, EN_BC = 2, EN_COPY_ELRK = 4, EN_GRAD = 8, EN_F
 // EC_FINISH: end with the cell part of the stage's update (EL1, D1, the stage sums, the
 // next stage's continuity fluxes from the new UAF, VAF), UA/VA being swapped with
 // UAF/VAF between stages instead of copied.
-// EC_COMPACT: the stage loop of an internal step may use the compact FP32 kernel (when
-// F32::compact is set); EC_LAST: the last stage of that loop (the compact kernel writes
-// ADVUA, ADVVA, PSTX, PSTY only there and in the internal-step ADVAVE call).
 // EC_WET: WET_JUDGE's cell part first (no limiter, whose alfa kernel needs the flags before).
 enum ExtCellParts { EC_N2E = 1, EC_FLUXOBN = 2, EC_ADVAVE = 4, EC_EXTUV = 8, EC_BC2 = 16, EC_COPY_RK = 32,
-                    EC_INT_ADVAVE = 64, EC_FINISH = 128, EC_COMPACT = 256, EC_LAST = 512, EC_WET = 1024 };
+                    EC_INT_ADVAVE = 64, EC_FINISH = 128, EC_WET = 256 };
 void launch_ext_finish(const Dev& P, cudaStream_t s, int K, int wet_prev);
 // pdl: launched as a programmatic dependent of the previous kernel in the stream (the
 // fused external loop); the kernel waits for that kernel's completion before it touches
@@ -560,11 +556,9 @@ void launch_alfa2(const Dev& P, cudaStream_t s);
 void launch_ext_update(const Dev& P, cudaStream_t s, int K);
 void launch_begin_step(const Dev& P, cudaStream_t s);
 void launch_ext_loop(const Dev& P, cudaStream_t s);
+void launch_ext_stage(const Dev& P, cudaStream_t s, int st);
 void launch_ext_prep(const Dev& P, cudaStream_t s);
 void launch_make_f32(const Dev& P, cudaStream_t s);
-// Fill the compact external stage's records and count (into *mismatch, device memory)
-// the mesh metrics that differ from the ones the coordinates define.
-void launch_make_compact(const Dev& P, cudaStream_t s, int* mismatch);
 void launch_closure(const Dev& P, cudaStream_t s, int* err, int grid);
 void launch_vdif_q_shallow(const Dev& P, cudaStream_t s);
 size_t closure_smem_bytes();
@@ -621,6 +615,7 @@ using fvg::Dev;
 void launch_alfa2(const Dev& P, cudaStream_t s);
 void launch_ext_cell(const Dev& P, cudaStream_t s, int iext, int K, int parts, int pdl);
 void launch_ext_loop(const Dev& P, cudaStream_t s);
+void launch_ext_stage(const Dev& P, cudaStream_t s, int st);
 void launch_grad3(const Dev& P, cudaStream_t s);
 void launch_advection3d(const Dev& P, cudaStream_t s);
 void launch_adv_uv(const Dev& P, cudaStream_t s);

@@ -571,6 +571,27 @@ __device__ inline void bc_solid(const Dev& P, int i, int rj, double& uu, double&
   }
 }
 
+// EXTUV's terms that stay fixed over the coming external loop, packed for its stages.  FP64:
+// six pairs per cell (exd), read as they are.  FP32 form: summed in FP64 (exc0, exc1), which
+// that form's rounding allows.
+template <typename R>
+__device__ inline void store_fixed(const Dev& P, int i, double adx, double ady) {
+  const size_t n1 = P.N + 1;
+  const double art = P.art[i], wx = P.have_wind ? P.wsx[i] : 0.0, wy = P.have_wind ? P.wsy[i] : 0.0;
+  if constexpr (sizeof(R) == 4) {
+    P.f.exc0[i] = make_double4(adx + P.drx2d[i] - P.wubot[i] * art, ady + P.dry2d[i] - P.wvbot[i] * art,
+                               0.001 * wx * art, 0.001 * wy * art);
+    P.f.exc1[i] = make_double4(P.cor[i] * art, art, P.h1[i], P.grav_e[i]);
+  } else {
+    P.exd[i] = make_double2(adx, P.drx2d[i]);
+    P.exd[n1 + i] = make_double2(ady, P.dry2d[i]);
+    P.exd[2 * n1 + i] = make_double2(P.wubot[i], P.wvbot[i]);
+    P.exd[3 * n1 + i] = make_double2(wx, wy);
+    P.exd[4 * n1 + i] = make_double2(P.cor[i], art);
+    P.exd[5 * n1 + i] = make_double2(P.h1[i], P.grav_e[i]);
+  }
+}
+
 // -------------------------------------------------------------------------------------
 // Per-cell part of one RK stage.  EC_INT_ADVAVE is the internal-step call of ADVAVE
 // followed by ADX2D -= ADVUA (internal_step.F:387-392).
@@ -629,8 +650,10 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 8 : (LIM ? 1 : 5)) k_ext
     P.pstx[i] = px;
     P.psty[i] = py;
     if (parts & EC_INT_ADVAVE) {
-      P.adx2d[i] = P.adx2d[i] - xf;
-      P.ady2d[i] = P.ady2d[i] - yf;
+      const double adx = P.adx2d[i] - xf, ady = P.ady2d[i] - yf;
+      P.adx2d[i] = adx;
+      P.ady2d[i] = ady;
+      if (P.xform) store_fixed<R>(P, i, adx, ady);
     }
   } else {
     xf = P.advua[i];
@@ -679,259 +702,502 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 8 : (LIM ? 1 : 5)) k_ext
   }
 }
 
-#ifdef FVG_F32_TU
+
 // -------------------------------------------------------------------------------------
-// Compact cell kernel of the precision form's stage loop (F32::compact; no limiter, GCN).
-// The same steps as k_ext_cell<float, false> -- FLUX_OBN, ADVAVE's edge loop in FP32 with
-// the FP64 surface-slope pressure gradient, EXTUV_EDGE and BCOND_GCN(2) in FP64, the cell
-// part of the stage's update -- over smaller records:
-//   * a slot is {code, other cell, IENODE1, IENODE2}; the edge's geometry is formed in FP64
-//     from the node and cell coordinates (XIJC = (VX1+VX2)/2, DLTXC = VX2-VX1, the offsets
-//     XIJC-XC rounded once to FP32, DLTXE = XIJC-XC of this cell for the continuity flux),
-//     values fvg_set_precision has checked equal, bit for bit, to the mesh's own metrics;
-//   * EXTUV's terms that stay fixed over the external loop are summed once per internal
-//     step (exc0, exc1, written by the internal-step ADVAVE call of this kernel), so that a
-//     stage reads five FP64 values per cell for them instead of thirteen;
-//   * ADVUA, ADVVA, PSTX, PSTY, which no later stage reads, are stored by the last stage
-//     (EC_LAST) and the internal-step call only.
+// The external stages on packed records (Dev::xform), two phases per Runge-Kutta stage:
+//   node phase   the update of the previous stage, EXTEL_EDGE and the boundary elevation of
+//                a node; the least-squares gradient of a cell and its viscosity term
+//                ART*|grad|*CC_HVC, which its neighbours' edges share;
+//   cell phase   WET_JUDGE's cell part (a dry cell forms its neighbours' flags itself),
+//                ADVAVE, EXTUV, BCOND_GCN(2) and the update of a cell.
+// A stage waits on loads, not on arithmetic or bandwidth, so a phase loads all it needs before
+// it computes: values of neighbours and nodes are packed in pairs (xuv, xg, xnd), the edge
+// geometry is formed from coordinates (seven pairs instead of twenty-four doubles), EXTUV's
+// fixed terms are pairs too.  ISWETN, DTFA, EL and D, which nothing inside the loop reads from
+// their own arrays, are left to k_ext_finish; ADVUA, ADVVA, PSTX, PSTY to the last stage.  In
+// FP64 every value is formed as the general stage kernels form it, with the sums that commute
+// taken in the cell's own order: results are theirs bit for bit.
+//
+// k_ext_loop runs the whole external loop as one kernel, for meshes with at most one cell and
+// one node per thread of a grid of one block per SM (launched cooperatively, so that all its
+// blocks are resident), with a grid barrier behind each phase: there a stage kernel is one wave
+// behind a launch, and 80 to 120 launches were half of the step.  k_stage_node and k_stage_cell
+// are the same phases as kernels, for larger meshes.
 // -------------------------------------------------------------------------------------
-// 64 registers (eight blocks per SM): held to 80 registers, six blocks, it measured slower
-// (1.89 against 1.76 ms per step).
-// CS: the records the stage reads once (flags, slots, EXTUV's fixed terms, the Runge-Kutta
-// start values, the cell's own D1/ELF1/EL1) are loaded evict-first (ld1), so that what
-// neighbours gather (UA, VA, the gradients, ART/CC_HVC, XC/YC, the nodes' VX/VY, D, EL,
-// the wet flags) keeps its L2 lines between stages.
-template <bool CS>
-__device__ __forceinline__ void ext_cell_c(const Dev& P, const int i, int iext, int K, int parts) {
-  const size_t n1 = P.N + 1;
-  const int fl = ld1<CS>(P.f.cflag + i);
-  const int isbce = fl & 3;
-  const double ua_i = P.ua[i], va_i = P.va[i];
-  if (parts & EC_COPY_RK) {
-    P.uark[i] = ua_i;
-    P.vark[i] = va_i;
-    P.elrk1[i] = ld1<CS>(P.el1 + i);
-  }
-  double elf1 = 0.0;
-  int wetc;
-  if (parts & EC_WET) {
-    wetc = wet_cell<CS>(P, i, elf1);
+// A load of what other threads exchange: in L2 inside the resident loop, whose L1 lines go
+// stale; through L1 in the stage kernels, where neighbouring cells share it.
+template <bool RES, class T>
+__device__ __forceinline__ T ldx(const T* p) {
+  if constexpr (RES) return __ldcg(p);
+  return *p;
+}
+template <typename R, bool RES>
+__device__ __forceinline__ Grad<R> ld_xg(const Dev& P, int c) {
+  if constexpr (sizeof(R) == 4) {
+    const float4 a = ldx<RES>(P.f.g2d4 + c);
+    return Grad<R>{a.x, a.y, a.z, a.w};
   } else {
-    wetc = P.iswetc[i];
+    const double2* g = reinterpret_cast<const double2*>(P.xg) + 2 * (size_t)c;
+    const double2 a = ldx<RES>(g), b = ldx<RES>(g + 1);
+    return Grad<R>{a.x, a.y, b.x, b.y};
   }
-  if (parts & EC_N2E) {
-    elf1 = ONE_THIRD * (P.elf[ld1<CS>(P.nv + i)] + P.elf[ld1<CS>(P.nv + n1 + i)] + P.elf[ld1<CS>(P.nv + 2 * n1 + i)]);
-    P.elf1[i] = elf1;
-  } else if (!(parts & EC_WET) && (parts & (EC_EXTUV | EC_FINISH))) {
-    elf1 = ld1<CS>(P.elf1 + i);
+}
+template <typename R>
+__device__ __forceinline__ void st_xg(const Dev& P, int c, const Grad<R>& g) {
+  if constexpr (sizeof(R) == 4) {
+    P.f.g2d4[c] = make_float4(g.ux, g.uy, g.vx, g.vy);
+  } else {
+    double2* q = reinterpret_cast<double2*>(P.xg) + 2 * (size_t)c;
+    q[0] = make_double2(g.ux, g.uy);
+    q[1] = make_double2(g.vx, g.vy);
   }
-  double fob = 0.0;
-  if (parts & EC_FLUXOBN) {
-    if (fl & 32) fob = fluxobn_cell(P, i, K);
-    if ((fl & 32) || isbce == 2) P.fluxobn[i] = fob;
-  } else if (isbce == 2) {
-    fob = P.fluxobn[i];
+}
+
+// Gradient and viscosity term of cell c (neighbours nb) with velocity u, v at stage st.
+template <typename R, bool CS, bool RES>
+__device__ __forceinline__ Grad<R> grad_job(const Dev& P, int c, int st, double u, double v, R& vc) {
+  typedef Mesh<R> Mh;
+  const double2* const uv = P.xuv + (st & 1) * (size_t)(P.N + 1);
+  int k1, k2, k3;
+  R A[4], B[4];
+  lsq_coef<R, CS>(P, c, k1, k2, k3, A, B);
+  const double2 b1 = ldx<RES>(uv + k1), b2 = ldx<RES>(uv + k2), b3 = ldx<RES>(uv + k3);
+  const R art = Mh::art(P, c), cc = Mh::cc_hvc(P, c), half = (R)0.5;
+  R u1 = (R)b1.x, u2 = (R)b2.x, u3 = (R)b3.x, v1 = (R)b1.y, v2 = (R)b2.y, v3 = (R)b3.y;
+  if (P.gcy && (k1 == 0 || k2 == 0 || k3 == 0)) {
+    double gu, gv;
+    if (k1 == 0) { ghost_uv1(P, u, v, c, 1, gu, gv); u1 = (R)gu; v1 = (R)gv; }
+    if (k2 == 0) { ghost_uv1(P, u, v, c, 2, gu, gv); u2 = (R)gu; v2 = (R)gv; }
+    if (k3 == 0) { ghost_uv1(P, u, v, c, 3, gu, gv); u3 = (R)gu; v3 = (R)gv; }
   }
-  const int weti = P.iswetce[i] * wetc;
-  const double d1i = ld1<CS>(P.d1 + i);
-  // {COR*ART, ART, H1, GRAV_E}: formed by the internal-step call below, read by the stages
-  const double4 e1 = (parts & EC_INT_ADVAVE) ? make_double4(0.0, 0.0, 0.0, P.grav_e[i]) : ld1<CS>(P.f.exc1 + i);
-  double xf = 0.0, yf = 0.0, px = 0.0, py = 0.0;
-  if (parts & (EC_ADVAVE | EC_INT_ADVAVE)) {
-    const float half = 0.5f, one = 1.0f;
-    const double ged1 = e1.w * d1i;
-    const float4 gi4 = P.f.g2d4[i];
-    const float* VC = reinterpret_cast<const float*>(P.xvc);
-    const float vci = VC[i];
-    const double2 xyi = P.f.xyc[i];
-    const float ui = (float)ua_i, vi = (float)va_i;
-    const float epor = (fl & 8) ? 1.0f : 0.0f, iucp = (fl & 4) ? 1.0f : 0.0f;
-    float xr = 0.f, yr = 0.f;
+  Grad<R> g;
+  g.ux = dot4(A[0], (R)u, A[1], u1, A[2], u2, A[3], u3);
+  g.uy = dot4(B[0], (R)u, B[1], u1, B[2], u2, B[3], u3);
+  g.vx = dot4(A[0], (R)v, A[1], v1, A[2], v2, A[3], v3);
+  g.vy = dot4(B[0], (R)v, B[1], v1, B[2], v2, B[3], v3);
+  st_xg<R>(P, c, g);
+  vc = art * sqrt(g.ux * g.ux + g.vy * g.vy + half * ((g.uy + g.vx) * (g.uy + g.vx))) * cc;
+  reinterpret_cast<R*>(P.xvc)[c] = vc;
+  return g;
+}
+
+// What the resident loop keeps of a node between stages; the launched phases load it.
+struct NodeKeep {
+  double elf, el, elrk, d, egf, h, art1, riv[2];
+  int ob, kind, nhe, nriv;
+};
+// EXTEL_EDGE, the boundary elevation and the previous stage's update of node i.  RES: the
+// resident loop, whose z lives in registers.
+template <bool CS, bool RES>
+__device__ __forceinline__ void node_phase(const Dev& P, int i, int st, NodeKeep& z) {
+  const int K = st % 4 + 1;
+  const size_t ms = P.ms;
+  if constexpr (!RES) {
+    z.ob = ld1<CS>(P.node_obc + i);
+    z.nhe = ld1<CS>(P.node_he_ptr + i + 1) - ld1<CS>(P.node_he_ptr + i);
+    z.h = ld1<CS>(P.h + i);
+    z.art1 = ld1<CS>(P.art1 + i);
+    z.elf = st > 0 ? P.elf[i] : 0.0;
+    z.el = st == 0 ? P.el[i] : 0.0;
+    z.d = st == 0 ? P.d[i] : 0.0;
+    z.elrk = st > 0 ? ld1<CS>(P.elrk + i) : 0.0;
+    z.egf = K == 4 ? ld1<CS>(P.egf + i) : 0.0;
+    z.nriv = P.numqbc > 0 ? P.node_riv_ptr[i + 1] - P.node_riv_ptr[i] : 0;
+  }
+  double x = 0.0;
+  const int* L = P.node_vpos_ell + i;
+  int j = 0;
+  for (; j + 6 <= z.nhe; j += 6) {
+    int e[6];
+    double f[6];
 #pragma unroll
-    for (int s = 0; s < 3; ++s) {
-      const int4 sl = ld1<CS>(P.f.slot4 + (size_t)s * n1 + i);  // {code, other cell, IENODE1, IENODE2}
-      const int code = sl.x, side = code & 1, o = sl.y, j1 = sl.z, j2 = sl.w;
-      const double2 v1 = P.f.vxy[j1], v2 = P.f.vxy[j2];
-      const double xijc = (v1.x + v2.x) / 2.0, yijc = (v1.y + v2.y) / 2.0;
-      const double dltxc = v2.x - v1.x, dltyc = v2.y - v1.y;
-      const float dij = (float)(0.5 * (P.d[j1] + P.d[j2]));
-      const double elij = 0.5 * (P.el[j1] + P.el[j2]);
-      if (weti == 1 || wet_other(P, parts & EC_WET, i, s, o, j1, j2)) {
-        const float4 go4 = P.f.g2d4[o];
-        const float vco = VC[o];
-        const double2 xyo = P.f.xyc[o];
-        const float uo = (float)P.ua[o], vo = (float)P.va[o];
-        const float xoi = (float)(xijc - xyi.x), yoi = (float)(yijc - xyi.y);
-        const float xoo = (float)(xijc - xyo.x), yoo = (float)(yijc - xyo.y);
-        // side 0: this cell is IA; side 1: this cell is IB
-        const float4 ga = side == 0 ? gi4 : go4, gb = side == 0 ? go4 : gi4;
-        const float uia = side == 0 ? ui : uo, via = side == 0 ? vi : vo;
-        const float uib = side == 0 ? uo : ui, vib = side == 0 ? vo : vi;
-        const float xa = side == 0 ? xoi : xoo, ya = side == 0 ? yoi : yoo;
-        const float xb = side == 0 ? xoo : xoi, yb = side == 0 ? yoo : yoi;
-        // ga = {UX, UY, VX, VY} of IA, gb of IB
-        const float uij1 = uia + ga.x * xa + ga.y * ya;
-        const float vij1 = via + ga.z * xa + ga.w * ya;
-        const float uij2 = uib + gb.x * xb + gb.y * yb;
-        const float vij2 = vib + gb.z * xb + gb.w * yb;
-        const float uij = half * (uij1 + uij2);
-        const float vij = half * (vij1 + vij2);
-        const float dx = (float)dltxc, dy = (float)dltyc;
-        const float un = -uij * dy + vij * dx;
-        float viscof = (float)P.fact * half * (vci + vco);
-        if (P.fm1 != 0.0) viscof += (float)P.fm1 * half * (P.f.artcc[i].y + P.f.artcc[o].y);
-        if (P.hprnu != 1.0) viscof = viscof / (float)P.hprnu;
-        const float txx = (ga.x + gb.x) * viscof;
-        const float tyy = (ga.w + gb.w) * viscof;
-        const float txy = half * (ga.y + gb.y + ga.z + gb.z) * viscof;
-        const float fxx = dij * (txx * dy - txy * dx);
-        const float fyy = dij * (txy * dy - tyy * dx);
-        const float sg = fsign1(un);
-        const float xadv = dij * un * ((one - sg) * uij2 + (one + sg) * uij1) * half;
-        const float yadv = dij * un * ((one - sg) * vij2 + (one + sg) * vij1) * half;
-        const float nb = one - (float)((code >> 1) & 1);
-        if (side == 0) {
-          xr = xr + (xadv + fxx * epor) * nb * iucp;
-          yr = yr + (yadv + fyy * epor) * nb * iucp;
-        } else {
-          xr = xr - (xadv + fxx * epor) * nb * iucp;
-          yr = yr - (yadv + fyy * epor) * nb * iucp;
-        }
-      }
-      if (side == 0) {
-        px = px - ged1 * elij * dltyc;
-        py = py + ged1 * elij * dltxc;
-      } else {
-        px = px + ged1 * elij * dltyc;
-        py = py - ged1 * elij * dltxc;
-      }
+    for (int q = 0; q < 6; ++q) e[q] = ld1<CS>(L + (j + q) * ms);
+#pragma unroll
+    for (int q = 0; q < 6; ++q) f[q] = ldx<RES>(P.exf2d + (e[q] >> 1));
+#pragma unroll
+    for (int q = 0; q < 6; ++q) x = (e[q] & 1) ? x + f[q] : x - f[q];
+  }
+  for (; j + 2 <= z.nhe; j += 2) {
+    const int e0 = ld1<CS>(L + j * ms), e1 = ld1<CS>(L + (j + 1) * ms);
+    const double f0 = ldx<RES>(P.exf2d + (e0 >> 1)), f1 = ldx<RES>(P.exf2d + (e1 >> 1));
+    x = (e0 & 1) ? x + f0 : x - f0;
+    x = (e1 & 1) ? x + f1 : x - f1;
+  }
+  if (j < z.nhe) {
+    const int e0 = ld1<CS>(L + j * ms);
+    const double f0 = ldx<RES>(P.exf2d + (e0 >> 1));
+    x = (e0 & 1) ? x + f0 : x - f0;
+  }
+  if (st > 0) {
+    // the previous stage's clamp (WET_JUDGE) and update (ext_update_node)
+    if (P.wetting_drying_on) z.elf = fmax(z.elf, -z.h + P.min_depth);
+    z.el = z.elf;
+    z.d = z.h + z.elf;
+    if (K == 4) {  // previous stage 3
+      z.egf = z.egf + z.elf / (double)P.isplit;
+      if constexpr (!RES) P.egf[i] = z.egf;
     }
-    const float w = (float)weti;
-    xf = (double)(xr * w);
-    yf = (double)(yr * w);
-    if (isbce == 2) {
-      const double iu = (fl & 4) ? 1.0 : 0.0;
-      xf = (xf + fob * ua_i) * iu;
-      yf = (yf + fob * va_i) * iu;
-    }
-    if (fl & 16) {
-      for (int q = P.cell_riv_ptr[i]; q < P.cell_riv_ptr[i + 1]; ++q) {
-        int k = P.cell_riv[q] >> 1;
-        double vlctyq = P.qdis[k] / P.qarea[k];
-        if (P.river_location == 0) {
-          xf = xf - 0.5 * P.qdis[k] * vlctyq * P.cos_angleq[k];
-          yf = yf - 0.5 * P.qdis[k] * vlctyq * P.sin_angleq[k];
-        } else {
-          double temp = P.qdis[k] * vlctyq;
-          xf = xf - temp * P.cos_angleq[k];
-          yf = yf - temp * P.sin_angleq[k];
-        }
-      }
-    }
-    if (parts & (EC_LAST | EC_INT_ADVAVE)) {
-      P.advua[i] = xf;
-      P.advva[i] = yf;
-      P.pstx[i] = px;
-      P.psty[i] = py;
-    }
-    if (parts & EC_INT_ADVAVE) {
-      // ADX2D -= ADVUA (internal_step.F:387-392), then EXTUV's fixed terms of the coming
-      // external loop
-      const double adx = P.adx2d[i] - xf, ady = P.ady2d[i] - yf;
-      P.adx2d[i] = adx;
-      P.ady2d[i] = ady;
-      const double art = P.art[i];
-      const double wx = P.have_wind ? 0.001 * P.wsx[i] * art : 0.0;
-      const double wy = P.have_wind ? 0.001 * P.wsy[i] * art : 0.0;
-      P.f.exc0[i] = make_double4(adx + P.drx2d[i] - P.wubot[i] * art, ady + P.dry2d[i] - P.wvbot[i] * art, wx, wy);
-      P.f.exc1[i] = make_double4(P.cor[i] * art, art, P.h1[i], P.grav_e[i]);
+    if (K == 1 && z.ob > 0) {
+      const double tmp = -(z.elf - z.elrk) * z.art1 / P.dte - P.xflux_obcn[z.ob];
+      P.uard_obcn[z.ob] = P.uard_obcn[z.ob] + tmp / (double)(float)P.isplit;
     }
   }
-  if (parts & (EC_EXTUV | EC_BC2)) {
-    double uaf = 0.0, vaf = 0.0;
-    if (parts & EC_EXTUV) {
-      if (weti == 1) {
-        const double4 e0 = ld1<CS>(P.f.exc0 + i);
-        const double ramp = sched_row(P)[P.sl.ramp_ext(iext)];
-        const double resx = e0.x + xf + px - e1.x * va_i * d1i - ramp * e0.z;
-        const double resy = e0.y + yf + py + e1.x * ua_i * d1i - ramp * e0.w;
-        const double a = dAlphaRK[K];
-        const double uark = (parts & EC_COPY_RK) ? ua_i : ld1<CS>(P.uark + i);
-        const double vark = (parts & EC_COPY_RK) ? va_i : ld1<CS>(P.vark + i);
-        const double elrk1 = (parts & EC_COPY_RK) ? ld1<CS>(P.el1 + i) : ld1<CS>(P.elrk1 + i);
-        uaf = (uark * (e1.z + elrk1) - a * P.dte * resx / e1.y) / (e1.z + elf1);
-        vaf = (vark * (e1.z + elrk1) - a * P.dte * resy / e1.y) / (e1.z + elf1);
-      }
-      if (fl & 64) {
-        const double sp = P.cc_sponge[i];
-        uaf = uaf / (1.0 + sp * (uaf * uaf));
-        vaf = vaf / (1.0 + sp * (vaf * vaf));
+  if (K == 1) {
+    z.elrk = z.el;
+    if constexpr (!RES) P.elrk[i] = z.elrk;
+  }
+  if (z.ob > 0) {
+    P.xflux_obcn[z.ob] = x;
+    x = 0.0;
+  }
+  if (z.nriv > 0) {
+    int q0 = P.node_riv_ptr[i];
+    if constexpr (RES) {
+      x = x - z.riv[0];
+      if (z.nriv > 1) x = x - z.riv[1];
+      q0 += 2;
+    }
+    for (int q = q0; q < P.node_riv_ptr[i + 1]; ++q) {
+      const int r = P.node_riv[q], jr = r >> 1;
+      x = x - (P.river_location == 0 ? P.qdis[jr] : P.qdis[jr] * P.rdisq[(size_t)(r & 1) * (P.numqbc + 1) + jr]);
+    }
+  }
+  const double alpha = dAlphaRK[K], dtk = alpha * P.dte;
+  z.elf = z.elrk - dtk * x / z.art1;
+  if (z.ob > 0) {
+    if constexpr (!RES) z.kind = P.obc_kind[z.ob];
+    if (z.kind == 1) {
+      if (P.obc_elev_on) z.elf = P.obf[(size_t)st * (P.iobcn + 1) + z.ob];
+      z.elf = add_rn(z.elrk, mul_rn(alpha, z.elf - z.elrk));
+    } else if (z.kind == 2) {
+      z.elf = 0.0;
+    }
+    if constexpr (RES) P.elrk[i] = z.elrk;
+  }
+  P.elf[i] = z.elf;
+  P.xnd[i] = make_double2(z.el, z.d);
+}
+
+// What the resident loop keeps of a cell between stages; the launched phases load it.
+template <typename R>
+struct CellKeep {
+  int4 xn, oo;  // loopx, loopo
+  double u, v;
+  Grad<R> g;
+  R vc;
+  // the resident loop's river and open-boundary entries (up to two of each)
+  int bcriv, nobc, nriv, ob[2], obn[2];
+  double obf[2], rvx[2], rvy[2];
+};
+template <typename R, bool CS, bool RES>
+__device__ __forceinline__ void cell_phase(const Dev& P, int c, int st, CellKeep<R>& z) {
+  typedef Mesh<R> Mh;
+  const R half = (R)0.5, one = (R)1.0;
+  const int iext = st / 4 + 1, K = st % 4 + 1, last = 4 * P.isplit - 1;
+  const size_t n1 = P.N + 1, ns = P.ns;
+  const double2* const uv = P.xuv + (st & 1) * n1;
+  double2* const uvn = P.xuv + ((st + 1) & 1) * n1;
+  int* const wn = P.xw + (st & 1) * n1;
+  const int* const wp = P.xw + ((st + 1) & 1) * n1;
+  const R* const xvc = reinterpret_cast<const R*>(P.xvc);
+  const bool wd = P.wetting_drying_on != 0;
+  if constexpr (!RES) {
+    z.xn = ld1<CS>(P.loopx + c);
+    z.oo = ld1<CS>(P.loopo + c);
+  }
+  // RES: everything the phase reads is loaded before its arithmetic and its stores; the
+  // launched phase, with many warps per SM and fewer registers, loads coordinates and fixed
+  // terms where they are used
+  const int xs[3] = {z.xn.x, z.xn.y, z.xn.z}, os[3] = {z.oo.x, z.oo.y, z.oo.z};
+  const int bits = z.xn.w, fl = z.oo.w, isbce = fl & 3;
+  double2 nd[3], ou[3], nx[3], cx[3];
+  double en[3], hn3[3];
+  Grad<R> go[3];
+  R vo[3];
+#pragma unroll
+  for (int s = 0; s < 3; ++s) {
+    nd[s] = ldx<RES>(P.xnd + xs[s]);
+    en[s] = ldx<RES>(P.elf + xs[s]);
+    if constexpr (RES) {
+      ou[s] = ldx<RES>(uv + os[s]);
+      go[s] = ld_xg<R, RES>(P, os[s]);
+      vo[s] = ldx<RES>(xvc + os[s]);
+    }
+  }
+  if constexpr (!RES) {
+    const double2 own = uv[c];
+    z.u = own.x;
+    z.v = own.y;
+    z.g = ld_xg<R, RES>(P, c);
+    z.vc = xvc[c];
+  }
+  const double2 ci = P.xyc[c];
+#pragma unroll
+  for (int s = 0; s < 3; ++s) {
+    if constexpr (RES) {
+      nx[s] = P.vxy[xs[s]];
+      cx[s] = P.xyc[os[s]];
+    }
+    hn3[s] = wd ? P.h[xs[s]] : 0.0;
+  }
+  const double u = z.u, v = z.v;
+  const double d1i = ld1<CS>(P.d1 + c);
+  const double2 rk = K == 1 ? make_double2(u, v) : ld1<CS>(P.xrk + c);
+  const double elrk1 = ld1<CS>((K == 1 ? P.el1 : P.elrk1) + c);
+  const int wce = wp[c], wci = wd ? 0 : P.iswetc[c];  // ISWETCE; ISWETC where it is fixed
+  const double hmin = wd ? ld1<CS>(P.hmin + c) : 0.0;
+  const double uard = K == 3 ? ld1<CS>(P.uard + c) : 0.0, vard = K == 3 ? ld1<CS>(P.vard + c) : 0.0;
+  const double ramp = sched_row(P)[P.sl.ramp_ext(iext)];
+  // EXTUV's terms that stay fixed over the loop (store_fixed)
+  double4 e0, e1;
+  double2 ax2, ay2, wb, ws;
+  double art, cor, h1i, grav;
+  if constexpr (sizeof(R) == 4) {
+    e1 = ld1<CS>(P.f.exc1 + c);
+    cor = e1.x;
+    art = e1.y;
+    h1i = e1.z;
+    grav = e1.w;
+  } else {
+    const double2 hg = ld1<CS>(P.exd + 5 * n1 + c);
+    h1i = hg.x;
+    grav = hg.y;
+  }
+  auto load_fixed = [&]() {
+    if constexpr (sizeof(R) == 4) {
+      e0 = ld1<CS>(P.f.exc0 + c);
+    } else {
+      ax2 = ld1<CS>(P.exd + c);
+      ay2 = ld1<CS>(P.exd + n1 + c);
+      wb = ld1<CS>(P.exd + 2 * n1 + c);
+      ws = ld1<CS>(P.exd + 3 * n1 + c);
+      const double2 ca = ld1<CS>(P.exd + 4 * n1 + c);
+      cor = ca.x;
+      art = ca.y;
+    }
+  };
+  if constexpr (RES) load_fixed();
+  const double ged1 = grav * d1i;
+  // WET_JUDGE's cell part, or N2E2D; the mean in NV order (its last node's place in bits)
+  const int k3 = (bits >> 6) & 3;
+  double cl[3] = {en[0], en[1], en[2]};
+  int wetc = wci;
+  if (wd) {
+    const double md = P.min_depth;
+    const double dtmp = fmax(fmax(en[0], en[1]), en[2]) + hmin;
+    wetc = ((dtmp - md) < 1.0e-5) ? 0 : 1;
+#pragma unroll
+    for (int s = 0; s < 3; ++s) cl[s] = fmax(en[s], -hn3[s] + md);
+  }
+  const double l3 = k3 == 0 ? cl[0] : (k3 == 1 ? cl[1] : cl[2]);
+  const double l12 = k3 == 0 ? cl[1] + cl[2] : (k3 == 1 ? cl[0] + cl[2] : cl[0] + cl[1]);
+  const double elf1 = ONE_THIRD * (l12 + l3);
+  const int weti = wce * wetc;
+  // FLUX_OBN
+  double fob = 0.0;
+  if (fl & 8) {
+    if (RES && z.nobc <= 2) {
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        if (q < z.nobc) {
+          const int j = z.obn[q];
+          const double ej0 = ldx<RES>(P.elf + j);
+          const double ej = wd ? fmax(ej0, -P.h[j] + P.min_depth) : ej0;
+          const double flux =
+              -(ej - ldx<RES>(P.elrk + j)) * P.art1[j] / (dAlphaRK[K] * P.dte) - ldx<RES>(P.xflux_obcn + z.ob[q]);
+          fob = fob + z.obf[q] * flux;
+        }
       }
     } else {
-      uaf = P.uaf[i];
-      vaf = P.vaf[i];
+      fob = fluxobn_cell(P, c, K);
     }
-    if (parts & EC_BC2) {
-      if (isbce == 3) { uaf = 0.0; vaf = 0.0; }
-      if (isbce == 1) bc_solid(P, i, P.cell_bcriv[i], uaf, vaf);
-    }
-    P.uaf[i] = uaf;
-    P.vaf[i] = vaf;
-    if (parts & EC_FINISH) {
-      // cell part of the stage's update (ext_update_cell) with DLTXE, DLTYE = XIJC-XC
-      P.el1[i] = elf1;
-      const double dd1 = e1.z + elf1;
-      P.d1[i] = dd1;
-      if (K == 3) {
-        P.uard[i] = ld1<CS>(P.uard + i) + uaf * dd1;
-        P.vard[i] = ld1<CS>(P.vard + i) + vaf * dd1;
-      }
-      const double2 xyi = P.f.xyc[i];
+  }
+  if ((fl & 8) || st == 0) P.fluxobn[c] = fob;
+  if (K == 1) {
+    P.elrk1[c] = elrk1;
+    P.xrk[c] = rk;
+  }
+  R xr = 0, yr = 0;
+  double px = 0.0, py = 0.0;
+  double exx[3], exy[3];  // XIJC-XC, YIJC-YC of the cell, which are DLTXE, DLTYE too
+  const R epor = (fl & 32) ? one : (R)0, iucp = (fl & 64) ? one : (R)0;
+  const R ui = (R)u, vi = (R)v, vci = z.vc;
+  const Grad<R> gi = z.g;
 #pragma unroll
-      for (int s = 0; s < 3; ++s) {
-        const int4 sl = ld1<CS>(P.f.slot4 + (size_t)s * n1 + i);
-        const double2 v1 = P.f.vxy[sl.z], v2 = P.f.vxy[sl.w];
-        const double dxe = (v1.x + v2.x) / 2.0 - xyi.x, dye = (v1.y + v2.y) / 2.0 - xyi.y;
-        P.exf2d[(size_t)s * P.ns + i] = dd1 * (-uaf * dye + vaf * dxe);
+  for (int s = 0; s < 3; ++s) {
+    const int side = (bits >> s) & 1, isbc = (bits >> (3 + s)) & 1, turn = (bits >> (8 + s)) & 1, o = os[s];
+    const double2 na = nd[s], nbb = nd[(s + 1) % 3];
+    const double2 v1 = RES ? nx[s] : P.vxy[xs[s]], v2 = RES ? nx[(s + 1) % 3] : P.vxy[xs[(s + 1) % 3]];
+    const double xij = (v1.x + v2.x) * 0.5, yij = (v1.y + v2.y) * 0.5;
+    const double edx = turn ? v1.x - v2.x : v2.x - v1.x, edy = turn ? v1.y - v2.y : v2.y - v1.y;
+    exx[s] = xij - ci.x;
+    exy[s] = yij - ci.y;
+    const R dij = (R)(0.5 * (na.y + nbb.y));
+    const double elij = 0.5 * (na.x + nbb.x);
+    bool on = weti == 1;
+    if (!on) {
+      // a dry cell: the neighbour's flags of the stage before and of this one
+      int wo = wp[o];
+      if (wd && o != 0) {
+        const double e = fmax(fmax(en[s], en[(s + 1) % 3]), ldx<RES>(P.elf + P.wfar[(size_t)s * n1 + c]));
+        wo = wo * (((e + P.hmin[o]) - P.min_depth) < 1.0e-5 ? 0 : 1);
+      } else {
+        wo = wo * (wd ? wn[0] : P.iswetc[o]);
       }
+      on = wo == 1;
+    }
+    if (on) {
+      const R dx = (R)edx, dy = (R)edy;
+      const double2 co = RES ? cx[s] : P.xyc[o];
+      const R xi = (R)exx[s], yi = (R)exy[s], xo = (R)(xij - co.x), yo = (R)(yij - co.y);
+      const double2 uvo = RES ? ou[s] : uv[o];
+      const Grad<R> gs = RES ? go[s] : ld_xg<R, RES>(P, o);
+      const R uo = (R)uvo.x, vv = (R)uvo.y, vco = RES ? vo[s] : xvc[o];
+      const R uown = ui + gi.ux * xi + gi.uy * yi, vown = vi + gi.vx * xi + gi.vy * yi;
+      const R uoth = uo + gs.ux * xo + gs.uy * yo, voth = vv + gs.vx * xo + gs.vy * yo;
+      const R uij = half * (uown + uoth), vij = half * (vown + voth);
+      const R un = -uij * dy + vij * dx;
+      R viscof = (R)P.fact * half * (vci + vco);
+      viscof = viscof + (R)P.fm1 * half * (P.fm1 != 0.0 ? Mh::cc_hvc(P, c) + Mh::cc_hvc(P, o) : (R)0);
+      if (P.hprnu != 1.0) viscof = viscof / (R)P.hprnu;
+      const R vxa = side ? gs.vx : gi.vx, vxb = side ? gi.vx : gs.vx;
+      const R txx = (gi.ux + gs.ux) * viscof;
+      const R tyy = (gi.vy + gs.vy) * viscof;
+      const R txy = half * (gi.uy + gs.uy + vxa + vxb) * viscof;
+      const R fxx = dij * (txx * dy - txy * dx);
+      const R fyy = dij * (txy * dy - tyy * dx);
+      const R sg = fsign1(un), sgo = side ? -sg : sg;
+      const R xadv = dij * un * ((one - sgo) * uoth + (one + sgo) * uown) * half;
+      const R yadv = dij * un * ((one - sgo) * voth + (one + sgo) * vown) * half;
+      const R nbd = one - (R)isbc;
+      const R ax = (xadv + fxx * epor) * nbd * iucp, ay = (yadv + fyy * epor) * nbd * iucp;
+      xr = side ? xr - ax : xr + ax;
+      yr = side ? yr - ay : yr + ay;
+    }
+    const double tx = ged1 * elij * edy, ty = ged1 * elij * edx;
+    px = side ? px + tx : px - tx;
+    py = side ? py - ty : py + ty;
+  }
+  const R w = (R)weti;
+  double xf = (double)(xr * w), yf = (double)(yr * w);
+  if (isbce == 2) {
+    const double iu = (fl & 64) ? 1.0 : 0.0;
+    if (P.gcy) {
+      xf = xf + fob * u * iu;
+      yf = yf + fob * v * iu;
+    } else {
+      xf = (xf + fob * u) * iu;
+      yf = (yf + fob * v) * iu;
     }
   }
-}
-
-// One cell per thread (WALK false), or a grid-stride walk over the cells with a grid of
-// Dev::ext_grid blocks per SM (WALK true).
-template <bool CS, bool WALK>
-__global__ void __launch_bounds__(128, 8) k_ext_cell_c(const Dev P, int iext, int K, int parts) {
-  pdl_enter();
-  if constexpr (WALK) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x + 1; i <= P.N; i += gridDim.x * blockDim.x)
-      ext_cell_c<CS>(P, i, iext, K, parts);
-  } else {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
-    if (i <= P.N) ext_cell_c<CS>(P, i, iext, K, parts);
+  if (fl & 4) {
+    int q0 = P.cell_riv_ptr[c];
+    if constexpr (RES) {
+      xf = xf - z.rvx[0];
+      yf = yf - z.rvy[0];
+      if (z.nriv > 1) {
+        xf = xf - z.rvx[1];
+        yf = yf - z.rvy[1];
+      }
+      q0 += 2;
+    }
+    for (int q = q0; q < P.cell_riv_ptr[c + 1]; ++q) {
+      const int k = P.cell_riv[q] >> 1;
+      const double vl = P.qdis[k] / P.qarea[k];
+      const double t = P.river_location == 0 ? 0.5 * P.qdis[k] * vl : P.qdis[k] * vl;
+      xf = xf - t * P.cos_angleq[k];
+      yf = yf - t * P.sin_angleq[k];
+    }
+  }
+  if (st == last) {
+    P.advua[c] = xf;
+    P.advva[c] = yf;
+    P.pstx[c] = px;
+    P.psty[c] = py;
+  }
+  double uaf = 0.0, vaf = 0.0;
+  if (weti == 1) {
+    const double a = dAlphaRK[K];
+    if constexpr (!RES) load_fixed();
+    double resx, resy;
+    if constexpr (sizeof(R) == 4) {
+      resx = e0.x + xf + px - cor * v * d1i - ramp * e0.z;
+      resy = e0.y + yf + py + cor * u * d1i - ramp * e0.w;
+    } else {
+      const double wus = P.have_wind ? ws.x * ramp * 0.001 : 0.0;
+      const double wvs = P.have_wind ? ws.y * ramp * 0.001 : 0.0;
+      resx = ax2.x + xf + ax2.y + px - cor * v * d1i * art - (wus + wb.x) * art;
+      resy = ay2.x + yf + ay2.y + py + cor * u * d1i * art - (wvs + wb.y) * art;
+    }
+    uaf = (rk.x * (h1i + elrk1) - a * P.dte * resx / art) / (h1i + elf1);
+    vaf = (rk.y * (h1i + elrk1) - a * P.dte * resy / art) / (h1i + elf1);
+  }
+  if (fl & 16) {
+    const double sp = P.cc_sponge[c];
+    uaf = uaf / (1.0 + sp * (uaf * uaf));
+    vaf = vaf / (1.0 + sp * (vaf * vaf));
+  }
+  if (isbce == 3 && !P.gcy) { uaf = 0.0; vaf = 0.0; }
+  if (isbce == 1) {
+    const int rj = RES ? z.bcriv : P.cell_bcriv[c];
+    if (!P.gcy || rj > 0) bc_solid(P, c, rj, uaf, vaf);
+  }
+  z.u = uaf;
+  z.v = vaf;
+  uvn[c] = make_double2(uaf, vaf);
+  wn[c] = wd ? wetc : wce;
+  P.el1[c] = elf1;
+  const double dd1 = h1i + elf1;
+  P.d1[c] = dd1;
+  if (K == 3) {
+    P.uard[c] = uard + uaf * dd1;
+    P.vard[c] = vard + vaf * dd1;
+  }
+#pragma unroll
+  for (int s = 0; s < 3; ++s) P.exf2d[(size_t)s * ns + c] = dd1 * (-uaf * exy[s] + vaf * exx[s]);
+  if (st == last) {
+    // as the general loop leaves its arrays before k_ext_finish
+    P.elf1[c] = elf1;
+    P.ua[c] = uaf;
+    P.va[c] = vaf;
+    P.uark[c] = rk.x;
+    P.vark[c] = rk.y;
+    if (wd) P.iswetce[c] = wetc;
   }
 }
-#endif  // FVG_F32_TU
 
-// -------------------------------------------------------------------------------------
-// The external loop of one internal step (ISPLIT x 4 Runge-Kutta stages) as one resident
-// kernel, for meshes with at most one cell and one node per thread of a grid of one block
-// per SM, launched cooperatively so that all its blocks are resident.  There a stage kernel
-// is one wave of dependent loads behind a launch, and 80 to 120 of them were half of the
-// step.  A stage is two phases with a grid barrier behind each:
-//   node phase   the update of the previous stage, EXTEL_EDGE and the boundary elevation of
-//                the thread's node; the least-squares gradient of the thread's cell and its
-//                viscosity term ART*|grad|*CC_HVC, which its neighbours' edges share;
-//   cell phase   WET_JUDGE's cell part (a dry cell forms its neighbours' flags itself),
-//                ADVAVE, EXTUV, BCOND_GCN(2) and the update of the thread's cell.
-// What bounds a stage is the chain of loads behind a barrier, so a phase's addresses are
-// all known when it begins: the thread keeps its neighbours' and nodes' numbers, the river
-// and open-boundary entries are resolved before the loop, and what is exchanged between
-// threads goes through packed arrays read in L2 (xuv, xg, xvc, xnd, ELF, exf2d).  ISWETN is
-// left to the closing kernel: nothing inside the loop reads it.  In FP64 every value is
-// formed as the stage kernels form it, with the sums that commute taken in the cell's own
-// order: results are theirs bit for bit.
-// -------------------------------------------------------------------------------------
+// One job per thread: nodes 1..M, then the cells' gradients.
+template <typename R, bool CS>
+__global__ void __launch_bounds__(256, 5) k_stage_node(const Dev P, int st) {
+  pdl_enter();
+  const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
+  if (i > P.M) {
+    const int c = i - P.M;
+    if (c > P.N) return;
+    const double2 own = P.xuv[(st & 1) * (size_t)(P.N + 1) + c];
+    R vc;
+    grad_job<R, CS, false>(P, c, st, own.x, own.y, vc);
+  } else {
+    NodeKeep z;
+    node_phase<CS, false>(P, i, st, z);
+  }
+}
+// Resident blocks per SM of the stage cell kernel.
+template <typename R>
+constexpr int kStageBlocks = sizeof(R) == 4 ? 7 : 5;
+// WALK: one wave of blocks whose threads walk the cells.
+template <typename R, bool CS, bool WALK>
+__global__ void __launch_bounds__(128, kStageBlocks<R>) k_stage_cell(const Dev P, int st) {
+  pdl_enter();
+  int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
+  do {
+    if (i > P.N) return;
+    CellKeep<R> z;
+    cell_phase<R, CS, false>(P, i, st, z);
+    i += gridDim.x * blockDim.x;
+  } while (WALK);
+}
+
 // Barrier over the grid: every block adds one to the counter (zeroed by k_begin_step) and
 // waits until all have.  The wait is bounded; a block whose wait runs out reports it and
 // leaves, and so do the others in their turn.
@@ -954,464 +1220,74 @@ __device__ __forceinline__ bool grid_barrier(const Dev& P, unsigned target) {
   return __syncthreads_and(ok);
 }
 
-// The loop's exchange arrays by arithmetic type: the gradient record of a cell.
-template <typename R>
-__device__ __forceinline__ Grad<R> ld_xg(const Dev& P, int c) {
-  if constexpr (sizeof(R) == 4) {
-    const float4 a = __ldcg(P.f.g2d4 + c);
-    return Grad<R>{a.x, a.y, a.z, a.w};
-  } else {
-    const double2* g = reinterpret_cast<const double2*>(P.xg) + 2 * (size_t)c;
-    const double2 a = __ldcg(g), b = __ldcg(g + 1);
-    return Grad<R>{a.x, a.y, b.x, b.y};
-  }
-}
-template <typename R>
-__device__ __forceinline__ void st_xg(const Dev& P, int c, const Grad<R>& g) {
-  if constexpr (sizeof(R) == 4) {
-    P.f.g2d4[c] = make_float4(g.ux, g.uy, g.vx, g.vy);
-  } else {
-    double2* q = reinterpret_cast<double2*>(P.xg) + 2 * (size_t)c;
-    q[0] = make_double2(g.ux, g.uy);
-    q[1] = make_double2(g.vx, g.vy);
-  }
-}
-
 template <typename R, int T>
 __global__ void __launch_bounds__(T, 1) k_ext_loop(const __grid_constant__ Dev P) {
-  typedef Mesh<R> Mh;
-  const R half = (R)0.5, one = (R)1.0;
   const int tid = threadIdx.x;
   const int c = blockIdx.x * P.loop_cells + tid + 1, i = blockIdx.x * P.loop_nodes + tid + 1;
   const bool hc = tid < P.loop_cells && c <= P.N, hn = tid < P.loop_nodes && i <= P.M;
-  const size_t n1 = P.N + 1, ns = P.ns, ms = P.ms;
-  R* const xvc = reinterpret_cast<R*>(P.xvc);
-  const bool wd = P.wetting_drying_on != 0;
-
-  // ---- the thread's cell: neighbours, nodes, flags ----
-  int4 xn = make_int4(0, 0, 0, 0), oo = xn, nb = xn;
-  int isbce = 0, bcriv = 0, nobc = 0, nriv = 0;
-  int ob_[2] = {0, 0}, obn[2] = {0, 0};
-  double obf[2] = {0.0, 0.0}, rvx[2] = {0.0, 0.0}, rvy[2] = {0.0, 0.0};
-  double u = 0.0, v = 0.0;
+  CellKeep<R> z;
   if (hc) {
-    xn = P.loopx[c];  // nodes X0, X1, X2: slot s is the edge X(s), X(s+1); bits, see loopx
-    oo = P.loopo[c];  // the other cell of slots 0, 1, 2
-    nb = P.nbe4[c];
-    isbce = P.isbce[c];
-    if (isbce == 1) bcriv = P.cell_bcriv[c];
-    const int q0 = P.cell_obc_ptr[c], q1 = P.cell_obc_ptr[c + 1];
-    nobc = q1 - q0;
-    if (nobc <= 2)
-      for (int q = 0; q < nobc; ++q) {
+    z.xn = P.loopx[c];
+    z.oo = P.loopo[c];
+    z.bcriv = (z.oo.w & 3) == 1 ? P.cell_bcriv[c] : 0;
+    const int q0 = P.cell_obc_ptr[c];
+    z.nobc = P.cell_obc_ptr[c + 1] - q0;
+    for (int q = 0; q < 2; ++q) {
+      z.ob[q] = z.obn[q] = 0;
+      z.obf[q] = z.rvx[q] = z.rvy[q] = 0.0;
+      if (q < z.nobc) {
         const int code = P.cell_obc[q0 + q];
-        ob_[q] = code >> 1;
-        obn[q] = P.i_obc_n[code >> 1];
-        obf[q] = P.fluxf_obc[(size_t)(code & 1) * (P.iobcn + 1) + (code >> 1)];
-      }
-    else
-      P.fluxobn[c] = 0.0;
-    if (nobc == 0) P.fluxobn[c] = 0.0;
-    const int r0 = P.cell_riv_ptr[c];
-    nriv = P.cell_riv_ptr[c + 1] - r0;
-    for (int q = 0; q < nriv && q < 2; ++q) {
-      const int k = P.cell_riv[r0 + q] >> 1;
-      const double vlctyq = P.qdis[k] / P.qarea[k];
-      if (P.river_location == 0) {
-        rvx[q] = 0.5 * P.qdis[k] * vlctyq * P.cos_angleq[k];
-        rvy[q] = 0.5 * P.qdis[k] * vlctyq * P.sin_angleq[k];
-      } else {
-        const double temp = P.qdis[k] * vlctyq;
-        rvx[q] = temp * P.cos_angleq[k];
-        rvy[q] = temp * P.sin_angleq[k];
+        z.ob[q] = code >> 1;
+        z.obn[q] = P.i_obc_n[code >> 1];
+        z.obf[q] = P.fluxf_obc[(size_t)(code & 1) * (P.iobcn + 1) + (code >> 1)];
       }
     }
-    u = P.ua[c];
-    v = P.va[c];
-    P.xuv[c] = make_double2(u, v);
-    P.xw[n1 + c] = P.iswetce[c];
+    const int r0 = P.cell_riv_ptr[c];
+    z.nriv = P.cell_riv_ptr[c + 1] - r0;
+    for (int q = 0; q < z.nriv && q < 2; ++q) {
+      const int k = P.cell_riv[r0 + q] >> 1;
+      const double vlctyq = P.qdis[k] / P.qarea[k];
+      const double t = P.river_location == 0 ? 0.5 * P.qdis[k] * vlctyq : P.qdis[k] * vlctyq;
+      z.rvx[q] = t * P.cos_angleq[k];
+      z.rvy[q] = t * P.sin_angleq[k];
+    }
+    z.u = P.ua[c];
+    z.v = P.va[c];
   }
-  if (blockIdx.x == 0 && tid == 0) {
-    // the ghost cell 0 of both buffers
-    P.xuv[0] = make_double2(P.ua[0], P.va[0]);
-    P.xuv[n1] = make_double2(P.uaf[0], P.vaf[0]);
-    P.xw[0] = P.iswetc[0];
-    P.xw[n1] = P.iswetce[0];
-    const Grad<R> g = load_grad<R>(P, 0);
-    st_xg<R>(P, 0, g);
-    xvc[0] = Mh::art(P, 0) * sqrt(g.ux * g.ux + g.vy * g.vy + half * ((g.uy + g.vx) * (g.uy + g.vx))) * Mh::cc_hvc(P, 0);
-  }
-  // ---- the thread's node ----
-  double elf = 0.0, el = 0.0, elrk = 0.0, dn = 0.0, egf = 0.0, hnode = 0.0, art1 = 1.0;
-  double nrv[2] = {0.0, 0.0};
-  int ob = 0, kind = 0, nhe = 0, nnriv = 0;
+  NodeKeep y;
   if (hn) {
-    elf = P.elf[i];
-    el = P.el[i];
-    dn = P.d[i];
-    egf = P.egf[i];
-    hnode = P.h[i];
-    art1 = P.art1[i];
-    ob = P.node_obc[i];
-    if (ob > 0) kind = P.obc_kind[ob];
-    nhe = P.node_he_ptr[i + 1] - P.node_he_ptr[i];
+    y.elf = P.elf[i];
+    y.el = P.el[i];
+    y.d = P.d[i];
+    y.elrk = 0.0;
+    y.egf = P.egf[i];
+    y.h = P.h[i];
+    y.art1 = P.art1[i];
+    y.ob = P.node_obc[i];
+    y.kind = y.ob > 0 ? P.obc_kind[y.ob] : 0;
+    y.nhe = P.node_he_ptr[i + 1] - P.node_he_ptr[i];
     const int r0 = P.node_riv_ptr[i];
-    nnriv = P.node_riv_ptr[i + 1] - r0;
-    for (int q = 0; q < nnriv && q < 2; ++q) {
+    y.nriv = P.node_riv_ptr[i + 1] - r0;
+    y.riv[0] = y.riv[1] = 0.0;
+    for (int q = 0; q < y.nriv && q < 2; ++q) {
       const int r = P.node_riv[r0 + q], j = r >> 1;
-      nrv[q] = P.river_location == 0 ? P.qdis[j] : P.qdis[j] * P.rdisq[(size_t)(r & 1) * (P.numqbc + 1) + j];
+      y.riv[q] = P.river_location == 0 ? P.qdis[j] : P.qdis[j] * P.rdisq[(size_t)(r & 1) * (P.numqbc + 1) + j];
     }
   }
   unsigned target = 0;
-  if (!grid_barrier(P, target += gridDim.x)) return;
-
   const int nst = 4 * P.isplit;
   for (int st = 0; st < nst; ++st) {
-    const int iext = st / 4 + 1, K = st % 4 + 1;
-    const double2* const uv = P.xuv + (st & 1) * n1;
-    double2* const uvn = P.xuv + ((st + 1) & 1) * n1;
-    int* const wn = P.xw + (st & 1) * n1;
-    const int* const wp = P.xw + ((st + 1) & 1) * n1;
-    // ================= node phase =================
-    double2 b1, b2, b3;
-    R A[4], B[4];
-    R gart = 0, gcc = 0;
-    if (hc) {
-      b1 = __ldcg(uv + nb.x);
-      b2 = __ldcg(uv + nb.y);
-      b3 = __ldcg(uv + nb.z);
-      int k1, k2, k3;
-      lsq_coef<R>(P, c, k1, k2, k3, A, B);
-      gart = Mh::art(P, c);
-      gcc = Mh::cc_hvc(P, c);
-    }
-    if (hn) {
-      double x = 0.0;
-      const int* L = P.node_vpos_ell + i;
-      int j = 0;
-      for (; j + 6 <= nhe; j += 6) {
-        int e[6];
-        double f[6];
-#pragma unroll
-        for (int q = 0; q < 6; ++q) e[q] = L[(j + q) * ms];
-#pragma unroll
-        for (int q = 0; q < 6; ++q) f[q] = __ldcg(P.exf2d + (e[q] >> 1));
-#pragma unroll
-        for (int q = 0; q < 6; ++q) x = (e[q] & 1) ? x + f[q] : x - f[q];
-      }
-      for (; j + 2 <= nhe; j += 2) {
-        const int e0 = L[j * ms], e1 = L[(j + 1) * ms];
-        const double f0 = __ldcg(P.exf2d + (e0 >> 1)), f1 = __ldcg(P.exf2d + (e1 >> 1));
-        x = (e0 & 1) ? x + f0 : x - f0;
-        x = (e1 & 1) ? x + f1 : x - f1;
-      }
-      if (j < nhe) {
-        const int e0 = L[j * ms];
-        const double f0 = __ldcg(P.exf2d + (e0 >> 1));
-        x = (e0 & 1) ? x + f0 : x - f0;
-      }
-      if (st > 0) {
-        // the previous stage's clamp (WET_JUDGE) and update (ext_update_node)
-        if (wd) elf = fmax(elf, -hnode + P.min_depth);
-        el = elf;
-        dn = hnode + elf;
-        if (K == 4) egf = egf + elf / (double)P.isplit;  // previous stage 3
-        if (K == 1 && ob > 0) {
-          const double tmp = -(elf - elrk) * art1 / P.dte - P.xflux_obcn[ob];
-          P.uard_obcn[ob] = P.uard_obcn[ob] + tmp / (double)(float)P.isplit;
-        }
-      }
-      if (K == 1) elrk = el;
-      if (ob > 0) {
-        P.xflux_obcn[ob] = x;
-        x = 0.0;
-      }
-      if (nnriv > 0) {
-        x = x - nrv[0];
-        if (nnriv > 1) x = x - nrv[1];
-        for (int q = P.node_riv_ptr[i] + 2; q < P.node_riv_ptr[i + 1]; ++q) {
-          const int r = P.node_riv[q], jr = r >> 1;
-          x = x - (P.river_location == 0 ? P.qdis[jr] : P.qdis[jr] * P.rdisq[(size_t)(r & 1) * (P.numqbc + 1) + jr]);
-        }
-      }
-      const double alpha = dAlphaRK[K], dtk = alpha * P.dte;
-      elf = elrk - dtk * x / art1;
-      if (ob > 0) {
-        if (kind == 1) {
-          if (P.obc_elev_on) elf = P.obf[(size_t)st * (P.iobcn + 1) + ob];
-          elf = add_rn(elrk, mul_rn(alpha, elf - elrk));
-        } else if (kind == 2) {
-          elf = 0.0;
-        }
-        P.elrk[i] = elrk;
-      }
-      P.elf[i] = elf;
-      P.xnd[i] = make_double2(el, dn);
-    }
-    Grad<R> gi = {0, 0, 0, 0};
-    R vci = 0;
-    if (hc) {
-      R u1 = (R)b1.x, u2 = (R)b2.x, u3 = (R)b3.x, v1 = (R)b1.y, v2 = (R)b2.y, v3 = (R)b3.y;
-      if (P.gcy && (nb.x == 0 || nb.y == 0 || nb.z == 0)) {
-        double gu, gv;
-        if (nb.x == 0) { ghost_uv1(P, u, v, c, 1, gu, gv); u1 = (R)gu; v1 = (R)gv; }
-        if (nb.y == 0) { ghost_uv1(P, u, v, c, 2, gu, gv); u2 = (R)gu; v2 = (R)gv; }
-        if (nb.z == 0) { ghost_uv1(P, u, v, c, 3, gu, gv); u3 = (R)gu; v3 = (R)gv; }
-      }
-      gi.ux = dot4(A[0], (R)u, A[1], u1, A[2], u2, A[3], u3);
-      gi.uy = dot4(B[0], (R)u, B[1], u1, B[2], u2, B[3], u3);
-      gi.vx = dot4(A[0], (R)v, A[1], v1, A[2], v2, A[3], v3);
-      gi.vy = dot4(B[0], (R)v, B[1], v1, B[2], v2, B[3], v3);
-      st_xg<R>(P, c, gi);
-      vci = gart * sqrt(gi.ux * gi.ux + gi.vy * gi.vy + half * ((gi.uy + gi.vx) * (gi.uy + gi.vx))) * gcc;
-      xvc[c] = vci;
-    }
+    if (hn) node_phase<false, true>(P, i, st, y);
+    if (hc) z.g = grad_job<R, false, true>(P, c, st, z.u, z.v, z.vc);
     if (!grid_barrier(P, target += gridDim.x)) return;
-    // ================= cell phase =================
-    if (hc) {
-      const int xs[3] = {xn.x, xn.y, xn.z}, os[3] = {oo.x, oo.y, oo.z};
-      const int bits = xn.w;
-      // everything the phase reads is loaded before its arithmetic and its stores
-      double2 nd[3], ou[3];
-      double en[3], hn3[3], edx[3], edy[3], hgx[3], hgy[3];
-      Grad<R> go[3];
-      R vo[3], xi[3], yi[3], xo[3], yo[3];
-#pragma unroll
-      for (int s = 0; s < 3; ++s) {
-        nd[s] = __ldcg(P.xnd + xs[s]);
-        en[s] = __ldcg(P.elf + xs[s]);
-        ou[s] = __ldcg(uv + os[s]);
-        go[s] = ld_xg<R>(P, os[s]);
-        vo[s] = __ldcg(xvc + os[s]);
-      }
-#pragma unroll
-      for (int s = 0; s < 3; ++s) {
-        const int side = (bits >> s) & 1;
-        const size_t q = (size_t)s * n1 + c, pos = (size_t)s * ns + c;
-        hn3[s] = P.h[xs[s]];
-        if constexpr (sizeof(R) == 4) {
-          const float4 G = P.f.ce_geo[q];  // XOA, YOA, XOB, YOB
-          xi[s] = side ? G.z : G.x;
-          yi[s] = side ? G.w : G.y;
-          xo[s] = side ? G.x : G.z;
-          yo[s] = side ? G.y : G.w;
-        } else {
-          xi[s] = (side ? P.ce_xob : P.ce_xoa)[q];
-          yi[s] = (side ? P.ce_yob : P.ce_yoa)[q];
-          xo[s] = (side ? P.ce_xoa : P.ce_xob)[q];
-          yo[s] = (side ? P.ce_yoa : P.ce_yob)[q];
-        }
-        edx[s] = P.ce_dx[q];
-        edy[s] = P.ce_dy[q];
-        hgx[s] = Mesh<double>::hg(P, 0, pos);
-        hgy[s] = Mesh<double>::hg(P, 1, pos);
-      }
-      const double d1i = P.d1[c], h1i = P.h1[c], grav = P.grav_e[c], hmin = P.hmin[c], sp = P.cc_sponge[c];
-      const double iu = P.iucp[c];
-      const R epor = (R)P.epor[c], iucp = (R)iu;
-      const double uark = K == 1 ? u : P.uark[c], vark = K == 1 ? v : P.vark[c];
-      const double elrk1 = (K == 1 ? P.el1 : P.elrk1)[c];
-      const int wce = wp[c], wci = wd ? 0 : P.iswetc[c];  // ISWETCE; ISWETC where it is fixed
-      const double uard = K == 3 ? P.uard[c] : 0.0, vard = K == 3 ? P.vard[c] : 0.0;
-      const double ramp = sched_row(P)[P.sl.ramp_ext(iext)];
-      // EXTUV's terms that stay fixed over the loop; in the FP32 form summed by the
-      // internal-step ADVAVE call (exc0, exc1)
-      double4 e0 = make_double4(0.0, 0.0, 0.0, 0.0), e1 = e0;
-      double adx = 0.0, ady = 0.0, drx = 0.0, dry = 0.0, wbx = 0.0, wby = 0.0, wsx = 0.0, wsy = 0.0, art, cor;
-      if constexpr (sizeof(R) == 4) {
-        e0 = P.f.exc0[c];
-        e1 = P.f.exc1[c];
-        art = e1.y;
-        cor = e1.x;
-      } else {
-        adx = P.adx2d[c];
-        ady = P.ady2d[c];
-        drx = P.drx2d[c];
-        dry = P.dry2d[c];
-        wbx = P.wubot[c];
-        wby = P.wvbot[c];
-        art = P.art[c];
-        cor = P.cor[c];
-        if (P.have_wind) {
-          wsx = P.wsx[c];
-          wsy = P.wsy[c];
-        }
-      }
-      const double ged1 = grav * d1i;
-      // WET_JUDGE's cell part, or N2E2D; the mean in NV order (its last node's place in bits)
-      const int k3 = (bits >> 6) & 3;
-      double cl[3] = {en[0], en[1], en[2]};
-      int wetc = wci;
-      if (wd) {
-        const double md = P.min_depth;
-        const double dtmp = fmax(fmax(en[0], en[1]), en[2]) + hmin;
-        wetc = ((dtmp - md) < 1.0e-5) ? 0 : 1;
-#pragma unroll
-        for (int s = 0; s < 3; ++s) cl[s] = fmax(en[s], -hn3[s] + md);
-      }
-      const double l3 = k3 == 0 ? cl[0] : (k3 == 1 ? cl[1] : cl[2]);
-      const double l12 = k3 == 0 ? cl[1] + cl[2] : (k3 == 1 ? cl[0] + cl[2] : cl[0] + cl[1]);
-      const double elf1 = ONE_THIRD * (l12 + l3);
-      const int weti = wce * wetc;
-      // FLUX_OBN
-      double fob = 0.0;
-      if (nobc > 0) {
-        if (nobc <= 2) {
-#pragma unroll
-          for (int q = 0; q < 2; ++q) {
-            if (q < nobc) {
-              const int j = obn[q];
-              const double ej0 = __ldcg(P.elf + j);
-              const double ej = wd ? fmax(ej0, -P.h[j] + P.min_depth) : ej0;
-              const double flux =
-                  -(ej - __ldcg(P.elrk + j)) * P.art1[j] / (dAlphaRK[K] * P.dte) - __ldcg(P.xflux_obcn + ob_[q]);
-              fob = fob + obf[q] * flux;
-            }
-          }
-        } else {
-          fob = fluxobn_cell(P, c, K);
-        }
-        P.fluxobn[c] = fob;
-      }
-      if (K == 1) {
-        P.elrk1[c] = elrk1;
-        P.uark[c] = u;
-        P.vark[c] = v;
-      }
-      R xr = 0, yr = 0;
-      double px = 0.0, py = 0.0;
-      const R ui = (R)u, vi = (R)v;
-#pragma unroll
-      for (int s = 0; s < 3; ++s) {
-        const int side = (bits >> s) & 1, isbc = (bits >> (3 + s)) & 1, o = os[s];
-        const size_t q = (size_t)s * n1 + c;
-        const double2 na = nd[s], nbb = nd[(s + 1) % 3];
-        const R dij = (R)(0.5 * (na.y + nbb.y));
-        const double elij = 0.5 * (na.x + nbb.x);
-        bool on = weti == 1;
-        if (!on) {
-          // a dry cell: the neighbour's flags of the stage before and of this one
-          int wo = wp[o];
-          if (wd && o != 0) {
-            const double e = fmax(fmax(en[s], en[(s + 1) % 3]), __ldcg(P.elf + P.wfar[q]));
-            wo = wo * (((e + P.hmin[o]) - P.min_depth) < 1.0e-5 ? 0 : 1);
-          } else {
-            wo = wo * (wd ? P.xw[(st & 1) * n1] : P.iswetc[o]);
-          }
-          on = wo == 1;
-        }
-        const R dx = (R)edx[s], dy = (R)edy[s];
-        if (on) {
-          const R uo = (R)ou[s].x, vv = (R)ou[s].y;
-          const R uown = ui + gi.ux * xi[s] + gi.uy * yi[s], vown = vi + gi.vx * xi[s] + gi.vy * yi[s];
-          const R uoth = uo + go[s].ux * xo[s] + go[s].uy * yo[s], voth = vv + go[s].vx * xo[s] + go[s].vy * yo[s];
-          const R uij = half * (uown + uoth), vij = half * (vown + voth);
-          const R un = -uij * dy + vij * dx;
-          R viscof = (R)P.fact * half * (vci + vo[s]);
-          viscof = viscof + (R)P.fm1 * half * (P.fm1 != 0.0 ? gcc + Mh::cc_hvc(P, o) : (R)0);
-          if (P.hprnu != 1.0) viscof = viscof / (R)P.hprnu;
-          const R vxa = side ? go[s].vx : gi.vx, vxb = side ? gi.vx : go[s].vx;
-          const R txx = (gi.ux + go[s].ux) * viscof;
-          const R tyy = (gi.vy + go[s].vy) * viscof;
-          const R txy = half * (gi.uy + go[s].uy + vxa + vxb) * viscof;
-          const R fxx = dij * (txx * dy - txy * dx);
-          const R fyy = dij * (txy * dy - tyy * dx);
-          const R sg = fsign1(un), sgo = side ? -sg : sg;
-          const R xadv = dij * un * ((one - sgo) * uoth + (one + sgo) * uown) * half;
-          const R yadv = dij * un * ((one - sgo) * voth + (one + sgo) * vown) * half;
-          const R nbd = one - (R)isbc;
-          const R ax = (xadv + fxx * epor) * nbd * iucp, ay = (yadv + fyy * epor) * nbd * iucp;
-          xr = side ? xr - ax : xr + ax;
-          yr = side ? yr - ay : yr + ay;
-        }
-        const double tx = ged1 * elij * edy[s], ty = ged1 * elij * edx[s];
-        px = side ? px + tx : px - tx;
-        py = side ? py - ty : py + ty;
-      }
-      const R w = (R)weti;
-      double xf = (double)(xr * w), yf = (double)(yr * w);
-      if (isbce == 2) {
-        if (P.gcy) {
-          xf = xf + fob * u * iu;
-          yf = yf + fob * v * iu;
-        } else {
-          xf = (xf + fob * u) * iu;
-          yf = (yf + fob * v) * iu;
-        }
-      }
-      if (nriv > 0) {
-        xf = xf - rvx[0];
-        yf = yf - rvy[0];
-        if (nriv > 1) {
-          xf = xf - rvx[1];
-          yf = yf - rvy[1];
-        }
-        for (int q = P.cell_riv_ptr[c] + 2; q < P.cell_riv_ptr[c + 1]; ++q) {
-          const int k = P.cell_riv[q] >> 1;
-          const double vl = P.qdis[k] / P.qarea[k];
-          const double t = P.river_location == 0 ? 0.5 * P.qdis[k] * vl : P.qdis[k] * vl;
-          xf = xf - t * P.cos_angleq[k];
-          yf = yf - t * P.sin_angleq[k];
-        }
-      }
-      if (st == nst - 1) {
-        P.advua[c] = xf;
-        P.advva[c] = yf;
-        P.pstx[c] = px;
-        P.psty[c] = py;
-      }
-      double uaf = 0.0, vaf = 0.0;
-      if (weti == 1) {
-        const double a = dAlphaRK[K];
-        double resx, resy;
-        if constexpr (sizeof(R) == 4) {
-          resx = e0.x + xf + px - cor * v * d1i - ramp * e0.z;
-          resy = e0.y + yf + py + cor * u * d1i - ramp * e0.w;
-        } else {
-          const double wus = P.have_wind ? wsx * ramp * 0.001 : 0.0;
-          const double wvs = P.have_wind ? wsy * ramp * 0.001 : 0.0;
-          resx = adx + xf + drx + px - cor * v * d1i * art - (wus + wbx) * art;
-          resy = ady + yf + dry + py + cor * u * d1i * art - (wvs + wby) * art;
-        }
-        uaf = (uark * (h1i + elrk1) - a * P.dte * resx / art) / (h1i + elf1);
-        vaf = (vark * (h1i + elrk1) - a * P.dte * resy / art) / (h1i + elf1);
-      }
-      if (sp != 0.0) {
-        uaf = uaf / (1.0 + sp * (uaf * uaf));
-        vaf = vaf / (1.0 + sp * (vaf * vaf));
-      }
-      if (isbce == 3 && !P.gcy) { uaf = 0.0; vaf = 0.0; }
-      if (isbce == 1 && (!P.gcy || bcriv > 0)) bc_solid(P, c, bcriv, uaf, vaf);
-      u = uaf;
-      v = vaf;
-      uvn[c] = make_double2(u, v);
-      if (wd) wn[c] = wetc;
-      else wn[c] = wce;
-      P.el1[c] = elf1;
-      const double dd1 = h1i + elf1;
-      P.d1[c] = dd1;
-      if (K == 3) {
-        P.uard[c] = uard + u * dd1;
-        P.vard[c] = vard + v * dd1;
-      }
-#pragma unroll
-      for (int s = 0; s < 3; ++s) P.exf2d[(size_t)s * ns + c] = dd1 * (-u * hgy[s] + v * hgx[s]);
-      if (st == nst - 1) {
-        // as the launched loop leaves its arrays before k_ext_finish
-        P.elf1[c] = elf1;
-        P.ua[c] = u;
-        P.va[c] = v;
-        if (wd) P.iswetce[c] = wetc;
-      }
-    }
+    if (hc) cell_phase<R, false, true>(P, c, st, z);
     if (st < nst - 1 && !grid_barrier(P, target += gridDim.x)) return;
   }
   if (hn) {
-    P.el[i] = el;
-    P.d[i] = dn;
-    P.dtfa[i] = dn;
-    P.egf[i] = egf;
-    P.elrk[i] = elrk;
+    P.el[i] = y.el;
+    P.d[i] = y.d;
+    P.egf[i] = y.egf;
+    P.elrk[i] = y.elrk;
   }
 }
 
@@ -1469,6 +1345,24 @@ __global__ void k_ext_prep(const Dev P) {
   if (i > P.N) return;
   store_grad<false>(P, i);
   store_exf(P, i);
+  if (P.xform) {
+    // the stages' exchange buffers: the loop reads buffer 0 first, and its flags in buffer 1
+    const size_t n1 = P.N + 1;
+    P.xuv[i] = make_double2(P.ua[i], P.va[i]);
+    P.xw[n1 + i] = P.iswetce[i];
+    if (i == 1) {  // the ghost cell 0 of both buffers, its gradient and viscosity
+      P.xuv[0] = make_double2(P.ua[0], P.va[0]);
+      P.xuv[n1] = make_double2(P.uaf[0], P.vaf[0]);
+      P.xw[0] = P.iswetc[0];
+      P.xw[n1] = P.iswetce[0];
+      if (!P.prec) {
+        P.xg[0] = P.g2d[0][0];
+        P.xg[1] = P.g2d[1][0];
+        P.xg[2] = P.g2d[2][0];
+        P.xg[3] = P.g2d[3][0];
+      }
+    }
+  }
 }
 
 // Start of an internal step: advance the schedule slot, then BCOND_GCN(8,0)'s river ramp
@@ -1561,48 +1455,6 @@ void launch_make_f32(const Dev& P, cudaStream_t s) {
   if ((size_t)P.N + 1 > npk) npk = P.N + 1;
   k_pack_he_f32<<<nblk(npk, 256), 256, 0, s>>>(P);
 }
-#ifndef FVG_F32_TU
-// Records of the compact stage kernel, and the count of mesh metrics that differ from the
-// values the kernel forms from the coordinates (then the compact kernel is not used).
-__global__ void k_make_compact(const Dev P, int* mismatch) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i <= P.M) P.f.vxy[i] = make_double2(P.vx[i], P.vy[i]);
-  if (i > P.N) return;
-  P.f.xyc[i] = make_double2(P.xc[i], P.yc[i]);
-  P.f.artcc[i] = make_float2((float)P.art[i], (float)P.cc_hvc[i]);
-  if (i == 0) return;
-  const size_t n1 = P.N + 1;
-  int bad = 0;
-  for (int s = 0; s < 3; ++s) {
-    const size_t q = (size_t)s * n1 + i;
-    const int code = P.ce_code[q], ia = P.ce_ia[q], ib = P.ce_ib[q], j1 = P.ce_j1[q], j2 = P.ce_j2[q];
-    const int side = code & 1;
-    if ((side == 0 ? ia : ib) != i) ++bad;
-    P.f.slot4[q] = make_int4(code, side == 0 ? ib : ia, j1, j2);
-    const double xijc = (P.vx[j1] + P.vx[j2]) / 2.0, yijc = (P.vy[j1] + P.vy[j2]) / 2.0;
-    if (xijc - P.xc[ia] != P.ce_xoa[q] || yijc - P.yc[ia] != P.ce_yoa[q]) ++bad;
-    if (xijc - P.xc[ib] != P.ce_xob[q] || yijc - P.yc[ib] != P.ce_yob[q]) ++bad;
-    if (P.vx[j2] - P.vx[j1] != P.ce_dx[q] || P.vy[j2] - P.vy[j1] != P.ce_dy[q]) ++bad;
-    const size_t pos = (size_t)s * P.ns + i;
-    if (P.hg[pos] != xijc - P.xc[i] || P.hg[P.ncvs + pos] != yijc - P.yc[i]) ++bad;
-  }
-  const double iu = P.iucp[i], ep = P.epor[i];
-  if (!(iu == 0.0 || iu == 1.0) || !(ep == 0.0 || ep == 1.0)) ++bad;
-  int fl = P.isbce[i] & 3;
-  if (iu == 1.0) fl |= 4;
-  if (ep == 1.0) fl |= 8;
-  if (P.cell_riv_ptr[i + 1] > P.cell_riv_ptr[i]) fl |= 16;
-  if (P.cell_obc_ptr[i + 1] > P.cell_obc_ptr[i]) fl |= 32;
-  if (P.cc_sponge[i] != 0.0) fl |= 64;
-  P.f.cflag[i] = fl;
-  if (bad) atomicAdd(mismatch, bad);
-}
-void launch_make_compact(const Dev& P, cudaStream_t s, int* mismatch) {
-  const int n = (P.M > P.N ? P.M : P.N) + 1;
-  k_make_compact<<<nblk(n, 256), 256, 0, s>>>(P, mismatch);
-}
-#endif
-
 void launch_wet_judge(const Dev& P, cudaStream_t s) {
   k_wet_cells<false><<<nblk(P.N, 256), 256, 0, s>>>(P);
   k_wet_nodes<<<nblk(P.M, 256), 256, 0, s>>>(P);
@@ -1614,19 +1466,6 @@ void launch_wet_cells(const Dev& P, cudaStream_t s, int pdl) {
 void launch_ext_cell(const Dev& P, cudaStream_t s, int iext, int K, int parts, int pdl) {
   FVG_F32_FORWARD(launch_ext_cell(P, s, iext, K, parts, pdl));
   void (*k)(const Dev, int, int, int);
-#ifdef FVG_F32_TU
-  if ((parts & EC_COMPACT) && P.f.compact && !P.limiter && !P.gcy) {
-    const int b = col_threads(P, P.N, 128), nb = nblk(P.N, b);
-    if (P.ext_grid > 0 && nb > P.ext_grid * P.nsm) {
-      launch_maybe_pdl(pdl, P.ldcs ? k_ext_cell_c<true, true> : k_ext_cell_c<false, true>, dim3(P.ext_grid * P.nsm),
-                       dim3(128), s, P, iext, K, parts);
-    } else {
-      launch_maybe_pdl(pdl, P.ldcs ? k_ext_cell_c<true, false> : k_ext_cell_c<false, false>, dim3(nb), dim3(b), s,
-                       P, iext, K, parts);
-    }
-    return;
-  }
-#endif
   k = P.limiter ? k_ext_cell<RF, true> : k_ext_cell<RF, false>;
   const int b = col_threads(P, P.N, 128);
   launch_maybe_pdl(pdl, k, dim3(nblk(P.N, b)), dim3(b), s, P, iext, K, parts);
@@ -1657,14 +1496,30 @@ static void loop_launch(const Dev& P, cudaStream_t s, int grid) {
 void launch_ext_loop(const Dev& P, cudaStream_t s) {
   FVG_F32_FORWARD(launch_ext_loop(P, s));
   const int need = nblk(P.N > P.M ? P.N : P.M, P.nsm);
-  const int t = need <= 128 ? 128 : need <= 288 ? 288 : kLoopThreads;
+  const int t = need <= 128 ? 128 : need <= 256 ? 256 : kLoopThreads;
   Dev Q = P;
   const int grid = t > 128 ? P.nsm : nblk(P.N > P.M ? P.N : P.M, t);
   Q.loop_cells = nblk(P.N, grid);
   Q.loop_nodes = nblk(P.M, grid);
   if (t == 128) loop_launch<128>(Q, s, grid);
-  else if (t == 288) loop_launch<288>(Q, s, grid);
+  else if (t == 256) loop_launch<256>(Q, s, grid);
   else loop_launch<kLoopThreads>(Q, s, grid);
+}
+// Stage st of the launched loop: its two phases as kernels, each a programmatic dependent of
+// the one before (not the first).
+void launch_ext_stage(const Dev& P, cudaStream_t s, int st) {
+  FVG_F32_FORWARD(launch_ext_stage(P, s, st));
+  const int n = P.M + P.N, bn = col_threads(P, n, 256);
+  launch_maybe_pdl(st > 0, P.ldcs ? k_stage_node<RF, true> : k_stage_node<RF, false>, dim3(nblk(n, bn)), dim3(bn), s,
+                   P, st);
+  const int b = col_threads(P, P.N, 128), nb = nblk(P.N, b);
+  const int wave = (P.ext_grid < kStageBlocks<RF> ? P.ext_grid : kStageBlocks<RF>)*P.nsm;
+  if (P.ext_grid > 0 && nb > wave)
+    launch_maybe_pdl(1, P.ldcs ? k_stage_cell<RF, true, true> : k_stage_cell<RF, false, true>, dim3(wave), dim3(b), s, P,
+                     st);
+  else
+    launch_maybe_pdl(1, P.ldcs ? k_stage_cell<RF, true, false> : k_stage_cell<RF, false, false>, dim3(nb), dim3(b), s, P,
+                     st);
 }
 void launch_begin_step(const Dev& P, cudaStream_t s) { k_begin_step<<<1, 32, 0, s>>>(P, 1); }
 void launch_set_qdis(const Dev& P, cudaStream_t s) { k_begin_step<<<1, 32, 0, s>>>(P, 0); }
