@@ -725,6 +725,7 @@ int fvg_create(const fvg_mesh* m, const fvg_params* prm, const fvg_forcing* f, f
       UPI(tl.edges, tb.edges.data(), tb.edges.size());
       UPI(tl.slots, tb.slots.data(), tb.slots.size());
       P.staged = 1;
+      if (ext_loop_setup() || fvg_f32::ext_loop_setup()) h->loop_ok = 0;
       if (staged_setup() || fvg_f32::staged_setup()) {
         h->err = "cannot configure the staged momentum kernels";
         return fail(FVG_ERR_CUDA);

@@ -556,6 +556,7 @@ void launch_alfa2(const Dev& P, cudaStream_t s);
 void launch_ext_update(const Dev& P, cudaStream_t s, int K);
 void launch_begin_step(const Dev& P, cudaStream_t s);
 void launch_ext_loop(const Dev& P, cudaStream_t s);
+int ext_loop_setup();
 void launch_ext_stage(const Dev& P, cudaStream_t s, int st);
 void launch_ext_prep(const Dev& P, cudaStream_t s);
 void launch_make_f32(const Dev& P, cudaStream_t s);
@@ -615,6 +616,7 @@ using fvg::Dev;
 void launch_alfa2(const Dev& P, cudaStream_t s);
 void launch_ext_cell(const Dev& P, cudaStream_t s, int iext, int K, int parts, int pdl);
 void launch_ext_loop(const Dev& P, cudaStream_t s);
+int ext_loop_setup();
 void launch_ext_stage(const Dev& P, cudaStream_t s, int st);
 void launch_grad3(const Dev& P, cudaStream_t s);
 void launch_advection3d(const Dev& P, cudaStream_t s);

@@ -753,16 +753,57 @@ __device__ __forceinline__ void st_xg(const Dev& P, int c, const Grad<R>& g) {
   }
 }
 
+// What a thread of the resident loop reads every stage and nothing changes in between, in
+// shared memory, one column per thread (T threads): a grid barrier empties L1, and these were
+// half of a phase's loads from L2.  Pairs: VX,VY of X0..X2, XC,YC of the cell and of the other
+// cells, EXTUV's fixed terms; doubles: hmin, H of X0..X2, CC_SPONGE; the gradient's
+// coefficients, ART and CC_HVC in the form's type; the first kLoopList entries of the node's
+// half-edge list and the cell's NBE.
+constexpr int kLoopList = 14;
+template <typename R, int T>
+struct LoopShared {
+  double2 p2[13][T];
+  double p1[5][T];
+  // the cell's own state, written back after the last stage: D1, EL1, ELRK1, UARK, VARK, UARD, VARD
+  double own[7][T];
+  R ab[10][T];
+  int list[kLoopList][T];
+  int nb[3][T];
+};
+template <typename R, int T>
+__device__ __forceinline__ LoopShared<R, T>& loop_shared() {
+  extern __shared__ __align__(16) unsigned char loop_sm[];
+  return *reinterpret_cast<LoopShared<R, T>*>(loop_sm);
+}
+
 // Gradient and viscosity term of cell c (neighbours nb) with velocity u, v at stage st.
-template <typename R, bool CS, bool RES>
+// T: threads per block of the resident loop, 0 in a stage kernel.
+template <typename R, bool CS, int T>
 __device__ __forceinline__ Grad<R> grad_job(const Dev& P, int c, int st, double u, double v, R& vc) {
   typedef Mesh<R> Mh;
+  constexpr bool RES = T > 0;
   const double2* const uv = P.xuv + (st & 1) * (size_t)(P.N + 1);
   int k1, k2, k3;
-  R A[4], B[4];
-  lsq_coef<R, CS>(P, c, k1, k2, k3, A, B);
+  R A[4], B[4], art, cc;
+  if constexpr (RES) {
+    const LoopShared<R, T>& sm = loop_shared<R, T>();
+    k1 = sm.nb[0][threadIdx.x];
+    k2 = sm.nb[1][threadIdx.x];
+    k3 = sm.nb[2][threadIdx.x];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      A[j] = sm.ab[j][threadIdx.x];
+      B[j] = sm.ab[4 + j][threadIdx.x];
+    }
+    art = sm.ab[8][threadIdx.x];
+    cc = sm.ab[9][threadIdx.x];
+  } else {
+    lsq_coef<R, CS>(P, c, k1, k2, k3, A, B);
+    art = Mh::art(P, c);
+    cc = Mh::cc_hvc(P, c);
+  }
   const double2 b1 = ldx<RES>(uv + k1), b2 = ldx<RES>(uv + k2), b3 = ldx<RES>(uv + k3);
-  const R art = Mh::art(P, c), cc = Mh::cc_hvc(P, c), half = (R)0.5;
+  const R half = (R)0.5;
   R u1 = (R)b1.x, u2 = (R)b2.x, u3 = (R)b3.x, v1 = (R)b1.y, v2 = (R)b2.y, v3 = (R)b3.y;
   if (P.gcy && (k1 == 0 || k2 == 0 || k3 == 0)) {
     double gu, gv;
@@ -788,8 +829,9 @@ struct NodeKeep {
 };
 // EXTEL_EDGE, the boundary elevation and the previous stage's update of node i.  RES: the
 // resident loop, whose z lives in registers.
-template <bool CS, bool RES>
+template <typename R, bool CS, int T>
 __device__ __forceinline__ void node_phase(const Dev& P, int i, int st, NodeKeep& z) {
+  constexpr bool RES = T > 0;
   const int K = st % 4 + 1;
   const size_t ms = P.ms;
   if constexpr (!RES) {
@@ -807,6 +849,20 @@ __device__ __forceinline__ void node_phase(const Dev& P, int i, int st, NodeKeep
   double x = 0.0;
   const int* L = P.node_vpos_ell + i;
   int j = 0;
+  if constexpr (RES) {
+    // the list's first entries at once
+    const LoopShared<R, T>& sm = loop_shared<R, T>();
+    int e[kLoopList];
+    double f[kLoopList];
+#pragma unroll
+    for (int q = 0; q < kLoopList; ++q) e[q] = q < z.nhe ? sm.list[q][threadIdx.x] : 0;
+#pragma unroll
+    for (int q = 0; q < kLoopList; ++q) f[q] = q < z.nhe ? ldx<RES>(P.exf2d + (e[q] >> 1)) : 0.0;
+#pragma unroll
+    for (int q = 0; q < kLoopList; ++q)
+      if (q < z.nhe) x = (e[q] & 1) ? x + f[q] : x - f[q];
+    j = kLoopList;
+  }
   for (; j + 6 <= z.nhe; j += 6) {
     int e[6];
     double f[6];
@@ -886,12 +942,15 @@ struct CellKeep {
   Grad<R> g;
   R vc;
   // the resident loop's river and open-boundary entries (up to two of each)
-  int bcriv, nobc, nriv, ob[2], obn[2];
+  int bcriv, nobc, nriv, wce, wci, ob[2], obn[2];
   double obf[2], rvx[2], rvy[2];
 };
-template <typename R, bool CS, bool RES>
+template <typename R, bool CS, int T>
 __device__ __forceinline__ void cell_phase(const Dev& P, int c, int st, CellKeep<R>& z) {
   typedef Mesh<R> Mh;
+  constexpr bool RES = T > 0;
+  LoopShared<R, RES ? T : 1>& sm = loop_shared<R, RES ? T : 1>();
+  const int me = RES ? threadIdx.x : 0;
   const R half = (R)0.5, one = (R)1.0;
   const int iext = st / 4 + 1, K = st % 4 + 1, last = 4 * P.isplit - 1;
   const size_t n1 = P.N + 1, ns = P.ns;
@@ -905,12 +964,12 @@ __device__ __forceinline__ void cell_phase(const Dev& P, int c, int st, CellKeep
     z.xn = ld1<CS>(P.loopx + c);
     z.oo = ld1<CS>(P.loopo + c);
   }
-  // RES: everything the phase reads is loaded before its arithmetic and its stores; the
-  // launched phase, with many warps per SM and fewer registers, loads coordinates and fixed
-  // terms where they are used
+  // RES: what other threads wrote is loaded before the arithmetic and the stores, the rest comes
+  // from shared memory; the launched phase, with many warps per SM and fewer registers, loads
+  // the neighbours where they are used
   const int xs[3] = {z.xn.x, z.xn.y, z.xn.z}, os[3] = {z.oo.x, z.oo.y, z.oo.z};
   const int bits = z.xn.w, fl = z.oo.w, isbce = fl & 3;
-  double2 nd[3], ou[3], nx[3], cx[3];
+  double2 nd[3], ou[3];
   double en[3], hn3[3];
   Grad<R> go[3];
   R vo[3];
@@ -931,52 +990,60 @@ __device__ __forceinline__ void cell_phase(const Dev& P, int c, int st, CellKeep
     z.g = ld_xg<R, RES>(P, c);
     z.vc = xvc[c];
   }
-  const double2 ci = P.xyc[c];
+  const double2 ci = RES ? sm.p2[3][me] : P.xyc[c];
 #pragma unroll
-  for (int s = 0; s < 3; ++s) {
-    if constexpr (RES) {
-      nx[s] = P.vxy[xs[s]];
-      cx[s] = P.xyc[os[s]];
-    }
-    hn3[s] = wd ? P.h[xs[s]] : 0.0;
-  }
+  for (int s = 0; s < 3; ++s) hn3[s] = RES ? sm.p1[1 + s][me] : (wd ? P.h[xs[s]] : 0.0);
   const double u = z.u, v = z.v;
-  const double d1i = ld1<CS>(P.d1 + c);
-  const double2 rk = K == 1 ? make_double2(u, v) : ld1<CS>(P.xrk + c);
-  const double elrk1 = ld1<CS>((K == 1 ? P.el1 : P.elrk1) + c);
-  const int wce = wp[c], wci = wd ? 0 : P.iswetc[c];  // ISWETCE; ISWETC where it is fixed
-  const double hmin = wd ? ld1<CS>(P.hmin + c) : 0.0;
-  const double uard = K == 3 ? ld1<CS>(P.uard + c) : 0.0, vard = K == 3 ? ld1<CS>(P.vard + c) : 0.0;
+  const double d1i = RES ? sm.own[0][me] : ld1<CS>(P.d1 + c);
+  const double2 rk = K == 1 ? make_double2(u, v)
+                            : (RES ? make_double2(sm.own[3][me], sm.own[4][me]) : ld1<CS>(P.xrk + c));
+  const double elrk1 = RES ? sm.own[K == 1 ? 1 : 2][me] : ld1<CS>((K == 1 ? P.el1 : P.elrk1) + c);
+  const int wce = RES ? z.wce : wp[c], wci = wd ? 0 : (RES ? z.wci : P.iswetc[c]);  // ISWETCE; a fixed ISWETC
+  const double hmin = RES ? sm.p1[0][me] : (wd ? ld1<CS>(P.hmin + c) : 0.0);
+  double uard = 0.0, vard = 0.0;
+  if (!RES && K == 3) {
+    uard = ld1<CS>(P.uard + c);
+    vard = ld1<CS>(P.vard + c);
+  }
   const double ramp = sched_row(P)[P.sl.ramp_ext(iext)];
   // EXTUV's terms that stay fixed over the loop (store_fixed)
   double4 e0, e1;
   double2 ax2, ay2, wb, ws;
   double art, cor, h1i, grav;
   if constexpr (sizeof(R) == 4) {
-    e1 = ld1<CS>(P.f.exc1 + c);
+    if constexpr (RES) {
+      const double2 a = sm.p2[9][me], b = sm.p2[10][me];
+      e1 = make_double4(a.x, a.y, b.x, b.y);
+    } else {
+      e1 = ld1<CS>(P.f.exc1 + c);
+    }
     cor = e1.x;
     art = e1.y;
     h1i = e1.z;
     grav = e1.w;
   } else {
-    const double2 hg = ld1<CS>(P.exd + 5 * n1 + c);
+    const double2 hg = RES ? sm.p2[12][me] : ld1<CS>(P.exd + 5 * n1 + c);
     h1i = hg.x;
     grav = hg.y;
   }
   auto load_fixed = [&]() {
     if constexpr (sizeof(R) == 4) {
-      e0 = ld1<CS>(P.f.exc0 + c);
+      if constexpr (RES) {
+        const double2 a = sm.p2[7][me], b = sm.p2[8][me];
+        e0 = make_double4(a.x, a.y, b.x, b.y);
+      } else {
+        e0 = ld1<CS>(P.f.exc0 + c);
+      }
     } else {
-      ax2 = ld1<CS>(P.exd + c);
-      ay2 = ld1<CS>(P.exd + n1 + c);
-      wb = ld1<CS>(P.exd + 2 * n1 + c);
-      ws = ld1<CS>(P.exd + 3 * n1 + c);
-      const double2 ca = ld1<CS>(P.exd + 4 * n1 + c);
+      ax2 = RES ? sm.p2[7][me] : ld1<CS>(P.exd + c);
+      ay2 = RES ? sm.p2[8][me] : ld1<CS>(P.exd + n1 + c);
+      wb = RES ? sm.p2[9][me] : ld1<CS>(P.exd + 2 * n1 + c);
+      ws = RES ? sm.p2[10][me] : ld1<CS>(P.exd + 3 * n1 + c);
+      const double2 ca = RES ? sm.p2[11][me] : ld1<CS>(P.exd + 4 * n1 + c);
       cor = ca.x;
       art = ca.y;
     }
   };
-  if constexpr (RES) load_fixed();
   const double ged1 = grav * d1i;
   // WET_JUDGE's cell part, or N2E2D; the mean in NV order (its last node's place in bits)
   const int k3 = (bits >> 6) & 3;
@@ -1014,8 +1081,14 @@ __device__ __forceinline__ void cell_phase(const Dev& P, int c, int st, CellKeep
   }
   if ((fl & 8) || st == 0) P.fluxobn[c] = fob;
   if (K == 1) {
-    P.elrk1[c] = elrk1;
-    P.xrk[c] = rk;
+    if constexpr (RES) {
+      sm.own[2][me] = elrk1;
+      sm.own[3][me] = u;
+      sm.own[4][me] = v;
+    } else {
+      P.elrk1[c] = elrk1;
+      P.xrk[c] = rk;
+    }
   }
   R xr = 0, yr = 0;
   double px = 0.0, py = 0.0;
@@ -1027,7 +1100,8 @@ __device__ __forceinline__ void cell_phase(const Dev& P, int c, int st, CellKeep
   for (int s = 0; s < 3; ++s) {
     const int side = (bits >> s) & 1, isbc = (bits >> (3 + s)) & 1, turn = (bits >> (8 + s)) & 1, o = os[s];
     const double2 na = nd[s], nbb = nd[(s + 1) % 3];
-    const double2 v1 = RES ? nx[s] : P.vxy[xs[s]], v2 = RES ? nx[(s + 1) % 3] : P.vxy[xs[(s + 1) % 3]];
+    const double2 v1 = RES ? sm.p2[s][me] : P.vxy[xs[s]];
+    const double2 v2 = RES ? sm.p2[(s + 1) % 3][me] : P.vxy[xs[(s + 1) % 3]];
     const double xij = (v1.x + v2.x) * 0.5, yij = (v1.y + v2.y) * 0.5;
     const double edx = turn ? v1.x - v2.x : v2.x - v1.x, edy = turn ? v1.y - v2.y : v2.y - v1.y;
     exx[s] = xij - ci.x;
@@ -1048,7 +1122,7 @@ __device__ __forceinline__ void cell_phase(const Dev& P, int c, int st, CellKeep
     }
     if (on) {
       const R dx = (R)edx, dy = (R)edy;
-      const double2 co = RES ? cx[s] : P.xyc[o];
+      const double2 co = RES ? sm.p2[4 + s][me] : P.xyc[o];
       const R xi = (R)exx[s], yi = (R)exy[s], xo = (R)(xij - co.x), yo = (R)(yij - co.y);
       const double2 uvo = RES ? ou[s] : uv[o];
       const Grad<R> gs = RES ? go[s] : ld_xg<R, RES>(P, o);
@@ -1118,7 +1192,7 @@ __device__ __forceinline__ void cell_phase(const Dev& P, int c, int st, CellKeep
   double uaf = 0.0, vaf = 0.0;
   if (weti == 1) {
     const double a = dAlphaRK[K];
-    if constexpr (!RES) load_fixed();
+    load_fixed();
     double resx, resy;
     if constexpr (sizeof(R) == 4) {
       resx = e0.x + xf + px - cor * v * d1i - ramp * e0.z;
@@ -1133,7 +1207,7 @@ __device__ __forceinline__ void cell_phase(const Dev& P, int c, int st, CellKeep
     vaf = (rk.y * (h1i + elrk1) - a * P.dte * resy / art) / (h1i + elf1);
   }
   if (fl & 16) {
-    const double sp = P.cc_sponge[c];
+    const double sp = RES ? sm.p1[4][me] : P.cc_sponge[c];
     uaf = uaf / (1.0 + sp * (uaf * uaf));
     vaf = vaf / (1.0 + sp * (vaf * vaf));
   }
@@ -1145,13 +1219,24 @@ __device__ __forceinline__ void cell_phase(const Dev& P, int c, int st, CellKeep
   z.u = uaf;
   z.v = vaf;
   uvn[c] = make_double2(uaf, vaf);
-  wn[c] = wd ? wetc : wce;
-  P.el1[c] = elf1;
+  if (wd) wn[c] = wetc;
+  else if (!RES || st < 2) wn[c] = wce;
   const double dd1 = h1i + elf1;
-  P.d1[c] = dd1;
-  if (K == 3) {
-    P.uard[c] = uard + uaf * dd1;
-    P.vard[c] = vard + vaf * dd1;
+  if constexpr (RES) {
+    z.wce = wd ? wetc : wce;
+    sm.own[0][me] = dd1;
+    sm.own[1][me] = elf1;
+    if (K == 3) {
+      sm.own[5][me] = sm.own[5][me] + uaf * dd1;
+      sm.own[6][me] = sm.own[6][me] + vaf * dd1;
+    }
+  } else {
+    P.el1[c] = elf1;
+    P.d1[c] = dd1;
+    if (K == 3) {
+      P.uard[c] = uard + uaf * dd1;
+      P.vard[c] = vard + vaf * dd1;
+    }
   }
 #pragma unroll
   for (int s = 0; s < 3; ++s) P.exf2d[(size_t)s * ns + c] = dd1 * (-uaf * exy[s] + vaf * exx[s]);
@@ -1163,6 +1248,13 @@ __device__ __forceinline__ void cell_phase(const Dev& P, int c, int st, CellKeep
     P.uark[c] = rk.x;
     P.vark[c] = rk.y;
     if (wd) P.iswetce[c] = wetc;
+    if constexpr (RES) {
+      P.el1[c] = elf1;
+      P.d1[c] = dd1;
+      P.elrk1[c] = elrk1;
+      P.uard[c] = sm.own[5][me];
+      P.vard[c] = sm.own[6][me];
+    }
   }
 }
 
@@ -1176,10 +1268,10 @@ __global__ void __launch_bounds__(256, 5) k_stage_node(const Dev P, int st) {
     if (c > P.N) return;
     const double2 own = P.xuv[(st & 1) * (size_t)(P.N + 1) + c];
     R vc;
-    grad_job<R, CS, false>(P, c, st, own.x, own.y, vc);
+    grad_job<R, CS, 0>(P, c, st, own.x, own.y, vc);
   } else {
     NodeKeep z;
-    node_phase<CS, false>(P, i, st, z);
+    node_phase<R, CS, 0>(P, i, st, z);
   }
 }
 // Resident blocks per SM of the stage cell kernel.
@@ -1193,7 +1285,7 @@ __global__ void __launch_bounds__(128, kStageBlocks<R>) k_stage_cell(const Dev P
   do {
     if (i > P.N) return;
     CellKeep<R> z;
-    cell_phase<R, CS, false>(P, i, st, z);
+    cell_phase<R, CS, 0>(P, i, st, z);
     i += gridDim.x * blockDim.x;
   } while (WALK);
 }
@@ -1220,11 +1312,14 @@ __device__ __forceinline__ bool grid_barrier(const Dev& P, unsigned target) {
   return __syncthreads_and(ok);
 }
 
-template <typename R, int T>
+// SPLIT: the block's first half of threads holds its cells and the second half its nodes, so
+// that the two jobs of a node phase run side by side on different warps.
+template <typename R, int T, bool SPLIT>
 __global__ void __launch_bounds__(T, 1) k_ext_loop(const __grid_constant__ Dev P) {
-  const int tid = threadIdx.x;
-  const int c = blockIdx.x * P.loop_cells + tid + 1, i = blockIdx.x * P.loop_nodes + tid + 1;
-  const bool hc = tid < P.loop_cells && c <= P.N, hn = tid < P.loop_nodes && i <= P.M;
+  const int tid = threadIdx.x, tn = SPLIT ? tid - T / 2 : tid;
+  const int c = blockIdx.x * P.loop_cells + tid + 1, i = blockIdx.x * P.loop_nodes + tn + 1;
+  const bool hc = tid < P.loop_cells && c <= P.N, hn = tn >= 0 && tn < P.loop_nodes && i <= P.M;
+  LoopShared<R, T>& sm = loop_shared<R, T>();
   CellKeep<R> z;
   if (hc) {
     z.xn = P.loopx[c];
@@ -1253,6 +1348,43 @@ __global__ void __launch_bounds__(T, 1) k_ext_loop(const __grid_constant__ Dev P
     }
     z.u = P.ua[c];
     z.v = P.va[c];
+    const size_t n1 = P.N + 1;
+    const int xs[3] = {z.xn.x, z.xn.y, z.xn.z}, os[3] = {z.oo.x, z.oo.y, z.oo.z};
+    z.wce = P.iswetce[c];
+    z.wci = P.iswetc[c];
+    sm.own[0][tid] = P.d1[c];
+    sm.own[1][tid] = P.el1[c];
+    sm.own[5][tid] = P.uard[c];
+    sm.own[6][tid] = P.vard[c];
+    sm.p2[3][tid] = P.xyc[c];
+    sm.p1[0][tid] = P.hmin[c];
+    sm.p1[4][tid] = P.cc_sponge[c];
+    for (int s = 0; s < 3; ++s) {
+      sm.p2[s][tid] = P.vxy[xs[s]];
+      sm.p2[4 + s][tid] = P.xyc[os[s]];
+      sm.p1[1 + s][tid] = P.h[xs[s]];
+    }
+    if constexpr (sizeof(R) == 4) {
+      const double4 e0 = P.f.exc0[c], e1 = P.f.exc1[c];
+      sm.p2[7][tid] = make_double2(e0.x, e0.y);
+      sm.p2[8][tid] = make_double2(e0.z, e0.w);
+      sm.p2[9][tid] = make_double2(e1.x, e1.y);
+      sm.p2[10][tid] = make_double2(e1.z, e1.w);
+    } else {
+      for (int q = 0; q < 6; ++q) sm.p2[7 + q][tid] = P.exd[q * n1 + c];
+    }
+    int k1, k2, k3;
+    R A[4], B[4];
+    lsq_coef<R>(P, c, k1, k2, k3, A, B);
+    sm.nb[0][tid] = k1;
+    sm.nb[1][tid] = k2;
+    sm.nb[2][tid] = k3;
+    for (int j = 0; j < 4; ++j) {
+      sm.ab[j][tid] = A[j];
+      sm.ab[4 + j][tid] = B[j];
+    }
+    sm.ab[8][tid] = Mesh<R>::art(P, c);
+    sm.ab[9][tid] = Mesh<R>::cc_hvc(P, c);
   }
   NodeKeep y;
   if (hn) {
@@ -1266,6 +1398,7 @@ __global__ void __launch_bounds__(T, 1) k_ext_loop(const __grid_constant__ Dev P
     y.ob = P.node_obc[i];
     y.kind = y.ob > 0 ? P.obc_kind[y.ob] : 0;
     y.nhe = P.node_he_ptr[i + 1] - P.node_he_ptr[i];
+    for (int q = 0; q < kLoopList && q < y.nhe; ++q) sm.list[q][tid] = P.node_vpos_ell[q * (size_t)P.ms + i];
     const int r0 = P.node_riv_ptr[i];
     y.nriv = P.node_riv_ptr[i + 1] - r0;
     y.riv[0] = y.riv[1] = 0.0;
@@ -1277,10 +1410,10 @@ __global__ void __launch_bounds__(T, 1) k_ext_loop(const __grid_constant__ Dev P
   unsigned target = 0;
   const int nst = 4 * P.isplit;
   for (int st = 0; st < nst; ++st) {
-    if (hn) node_phase<false, true>(P, i, st, y);
-    if (hc) z.g = grad_job<R, false, true>(P, c, st, z.u, z.v, z.vc);
+    if (hn) node_phase<R, false, T>(P, i, st, y);
+    if (hc) z.g = grad_job<R, false, T>(P, c, st, z.u, z.v, z.vc);
     if (!grid_barrier(P, target += gridDim.x)) return;
-    if (hc) cell_phase<R, false, true>(P, c, st, z);
+    if (hc) cell_phase<R, false, T>(P, c, st, z);
     if (st < nst - 1 && !grid_barrier(P, target += gridDim.x)) return;
   }
   if (hn) {
@@ -1478,32 +1611,47 @@ void launch_ext_finish(const Dev& P, cudaStream_t s, int K, int wet_prev) {
   int n = P.M > P.N ? P.M : P.N;
   k_ext_finish<<<nblk(n, 256), 256, 0, s>>>(P, K, wet_prev);
 }
-template <int T>
+template <int T, bool SPLIT>
 static void loop_launch(const Dev& P, cudaStream_t s, int grid) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(T);
+  cfg.dynamicSmemBytes = sizeof(LoopShared<RF, T>);
   cfg.stream = s;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeCooperative;
   at[0].val.cooperative = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, k_ext_loop<RF, T>, P);
-}
-// One block per SM at most; the smallest block that then holds a cell and a node per thread,
-// so that the threads of a small mesh spread over the SMs.
-void launch_ext_loop(const Dev& P, cudaStream_t s) {
-  FVG_F32_FORWARD(launch_ext_loop(P, s));
-  const int need = nblk(P.N > P.M ? P.N : P.M, P.nsm);
-  const int t = need <= 128 ? 128 : need <= 256 ? 256 : kLoopThreads;
   Dev Q = P;
-  const int grid = t > 128 ? P.nsm : nblk(P.N > P.M ? P.N : P.M, t);
   Q.loop_cells = nblk(P.N, grid);
   Q.loop_nodes = nblk(P.M, grid);
-  if (t == 128) loop_launch<128>(Q, s, grid);
-  else if (t == 256) loop_launch<256>(Q, s, grid);
-  else loop_launch<kLoopThreads>(Q, s, grid);
+  cudaLaunchKernelEx(&cfg, k_ext_loop<RF, T, SPLIT>, Q);
+}
+// Shared memory of the resident loop's blocks (once, before any launch or capture); 0 on success.
+template <int T, bool SPLIT>
+static int loop_attr() {
+  return cudaFuncSetAttribute(k_ext_loop<RF, T, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)sizeof(LoopShared<RF, T>)) == cudaSuccess
+             ? 0
+             : 1;
+}
+int ext_loop_setup() { return loop_attr<256, true>() | loop_attr<256, false>() | loop_attr<kLoopThreads, false>(); }
+// One block per SM at most, the smallest that then holds a cell and a node per thread, so that
+// the threads spread over the SMs.  256 threads take 250 registers each and spill nothing; up
+// to 128 cells per SM they leave half of the threads to the nodes.  One cluster of sixteen
+// blocks with its hardware barrier in place of the grid's measured no faster (2,121 nodes 492
+// against 491 us per step): a phase waits on its own loads and arithmetic more than on the
+// barrier.
+void launch_ext_loop(const Dev& P, cudaStream_t s) {
+  FVG_F32_FORWARD(launch_ext_loop(P, s));
+  const int most = P.N > P.M ? P.N : P.M, need = nblk(most, P.nsm);
+  if (need <= 128)
+    loop_launch<256, true>(P, s, nblk(most, 128));
+  else if (need <= 256)
+    loop_launch<256, false>(P, s, P.nsm);
+  else
+    loop_launch<kLoopThreads, false>(P, s, P.nsm);
 }
 // Stage st of the launched loop: its two phases as kernels, each a programmatic dependent of
 // the one before (not the first).
