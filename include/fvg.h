@@ -327,7 +327,11 @@ int fvg_closure_status(fvg_handle* h, int32_t* columns_on_network, int32_t* wait
    "ext_loop"     = 1 (default): the external loop of a mesh of at most 384 cells per SM runs
                    as one resident cooperative kernel (no limiter; the FP32-flux form with
                    the compact kernel's records); 0 launches every stage.  FP64 results do
-                   not depend on it; fvg_get_tuning reports whether it is in use. */
+                   not depend on it; fvg_get_tuning reports whether it is in use;
+   "branches"     = 1 (default): up to 20 million cell-layers the independent parts of a step
+                   (BAROPG beside ADVECTION; momentum, turbulence and tracers after VERTVL)
+                   run beside one another on streams of the handle; 0 one after another.
+                   Results do not depend on it (bit for bit). */
 int fvg_set_tuning(fvg_handle* h, const char* key, int32_t value);
 int fvg_get_tuning(const fvg_handle* h, const char* key, int32_t* value);
 

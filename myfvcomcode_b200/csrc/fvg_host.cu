@@ -21,6 +21,12 @@ using namespace fvg;
 
 namespace {
 
+// Most cell-layers of a mesh whose step runs in branches (use_branches): they measured faster
+// at every size (175 nodes x 5 layers 431 -> 396 us per step, 50k x 30 FP64 3249 -> 3038, 200k x
+// 30 10821 -> 10577), but cost the tracers' own flux scratch, 48 bytes per cell-layer (24 in
+// FP32), which a large ensemble would rather hold members in.
+constexpr long kBranchCells = 20000000;
+
 const double kPI2 = 2.0 * 3.141592653589793238;
 
 struct FieldDesc {
@@ -61,6 +67,15 @@ struct fvg_handle {
   // cooperatively)
   int ext_loop = 1;
   int loop_ok = 0;
+  // side branches of a step (use_branches): allowed (tuning key "branches"), their streams,
+  // fork and join events, and the tracers' own flux scratch in FP64 and FP32
+  int branches = 1;
+  cudaStream_t side[2] = {nullptr, nullptr};
+  cudaEvent_t ev[7] = {};
+  double2* ex2_ts = nullptr;
+  double* gvn_ts = nullptr;
+  float2* ex2f_ts = nullptr;
+  float* npk_ts = nullptr;
 };
 
 #define CK(call)                                                                      \
@@ -269,6 +284,13 @@ bool use_ext_loop(const fvg_handle* h) {
   return (long)std::max(P.M, P.N) <= (long)kLoopThreads * P.nsm;
 }
 
+// Whether the independent parts of a step run as branches beside one another: BAROPG beside
+// ADVECTION; after VERTVL the momentum, the turbulence and the tracers.  Their kernels fill
+// the chip only on large meshes.
+bool use_branches(const fvg_handle* h) {
+  return h->branches && h->ex2_ts && (!h->P.prec || h->ex2f_ts);
+}
+
 // One INTERNAL_STEP as a kernel sequence (internal_step.F:115-1590).
 // after: in a group, the event of the model before (its resident external loop is done, if
 // it has one), which this model's loop waits for, so that no two cooperative grids of one
@@ -279,18 +301,28 @@ void enqueue_internal_step(fvg_handle* h, cudaStream_t s, Marker mk = Marker(), 
   const fvg_params& p = h->prm;
   const int spc = p.scalar_positivity_control ? AD_FCT : 0;
   mk.mark(s, -1);
+  // Branches: stream b runs beside s from a fork to a join.  A profile keeps one order.
+  const bool br = use_branches(h) && !mk.ev;
+  cudaStream_t b1 = br ? h->side[0] : s, b2 = br ? h->side[1] : s;
+  auto chain = [&](cudaStream_t later, cudaStream_t first, int e) {
+    if (later == first) return;
+    cudaEventRecord(h->ev[e], first);
+    cudaStreamWaitEvent(later, h->ev[e], 0);
+  };
   launch_begin_step(P, s);
+  const bool zlev = !p.barotropic && P.baropg_z, sigma = !p.barotropic && !P.baropg_z;
+  if (br && sigma) {
+    chain(b1, s, 0);
+    launch_baropg(P, b1, 1, 0);
+  }
   launch_cell_pre(P, s, CP_ADJUST1 | CP_BC5 | CP_BCOND8 | CP_BROUGH);
   mk.mark(s, G_CELL_PRE);
   launch_grad3(P, s);
   launch_advection3d(P, s);
   mk.mark(s, G_ADV3D);
-  if (!p.barotropic && P.baropg_z) {
-    launch_phy_baropg(P, s);
-    launch_baropg(P, s, 0, 1);
-  } else {
-    launch_baropg(P, s, !p.barotropic, 1);
-  }
+  if (zlev) launch_phy_baropg(P, s);
+  if (br && sigma) chain(s, b1, 1);
+  launch_baropg(P, s, sigma && !br, 1);
   launch_ext_prep(P, s);
   if (P.limiter) launch_alfa2(P, s);
   mk.mark(s, G_BAROPG);
@@ -351,33 +383,51 @@ void enqueue_internal_step(fvg_handle* h, cudaStream_t s, Marker mk = Marker(), 
   mk.mark(s, G_VV_FLUX);
   launch_vertvl_col(P, s, VC_WTS | VC_WD2 | (p.barotropic || P.baropg_z ? 0 : VC_RHO_ROUNDTRIP) | VC_BOT_NODE);
   mk.mark(s, G_VV_COL);
-  launch_w_viscofh(P, s, 1, 1);
+  launch_w_viscofh(P, s, 1, 1, 1);
   mk.mark(s, G_W_VISC);
+  const int ts = (p.temperature_active ? AD_T : 0) | (p.salinity_active ? AD_S : 0);
+  chain(b1, s, 2);
+  if (ts) chain(b2, s, 3);
+  // momentum
   launch_grad3(P, s);
   launch_adv_uv(P, s);
   mk.mark(s, G_ADV_UV);
-  launch_vdif_uv(P, s, VU_VDIF | VU_BC3 | VU_WREAL);
+  launch_vdif_uv(P, s, VU_VDIF | VU_BC3 | VU_WREAL | VU_NO_STRESS);
   mk.mark(s, G_VDIF_UV);
-  launch_grad(P, s, 0);
+  // turbulence
+  launch_grad(P, b1, 0);
   mk.mark(s, G_GRAD_Q);
-  launch_adv_q(P, s, AD_Q2 | AD_Q2L | spc);
+  launch_adv_q(P, b1, AD_Q2 | AD_Q2L | spc);
   mk.mark(s, G_ADV_Q);
-  launch_vdif_q(P, s, 1);
+  launch_vdif_q(P, b1, 1);
   mk.mark(s, G_VDIF_Q);
   if (P.closure) {
-    launch_closure(P, s, P.clos_err, h->clos_grid);
+    launch_closure(P, b1, P.clos_err, h->clos_grid);
     mk.mark(s, G_CLOSURE);
   }
-  int ts = (p.temperature_active ? AD_T : 0) | (p.salinity_active ? AD_S : 0);
+  // tracers; VDIF_TS takes the new KH
   if (ts) {
-    launch_grad(P, s, 1);
+    Dev Q = P;
+    if (br) {
+      Q.ex2 = h->ex2_ts;
+      Q.gvn = h->gvn_ts;
+      if (P.prec) {
+        Q.f.ex2 = h->ex2f_ts;
+        Q.f.npk = h->npk_ts;
+      }
+    }
+    launch_grad(Q, b2, 1);
     mk.mark(s, G_GRAD_TS);
-    launch_adv_ts(P, s, ts | spc);
+    launch_adv_ts(Q, b2, ts | spc);
     mk.mark(s, G_ADV_TS);
-    launch_vdif_ts(P, s, ts);
+    chain(b2, b1, 4);
+    launch_vdif_ts(P, b2, ts);
     mk.mark(s, G_VDIF_TS);
-    launch_bcond_ts(P, s, ts);
+    launch_bcond_ts(P, b2, ts);
     mk.mark(s, G_BCOND_TS);
+    chain(s, b2, 5);
+  } else {
+    chain(s, b1, 6);
   }
   int fin = FI_KM1 | FI_SHIFT | (p.temperature_active ? FI_T : 0) | (p.salinity_active ? FI_S : 0) |
             (p.barotropic ? 0 : FI_DENS);
@@ -975,6 +1025,14 @@ int fvg_create(const fvg_mesh* m, const fvg_params* prm, const fvg_forcing* f, f
   if ((rc = dalloc(h, &P.vc3, ns * KB))) return fail(rc);
   if ((rc = dalloc(h, (double**)&P.ex2, (size_t)P.ncvs * KB * 2))) return fail(rc);
   P.he_vflux = (double*)P.ex2;
+  if ((long)N * (KB - 1) <= kBranchCells) {
+    if ((rc = dalloc(h, (double**)&h->ex2_ts, (size_t)P.ncvs * KB * 2))) return fail(rc);
+    if ((rc = dalloc(h, &h->gvn_ts, ms * KB))) return fail(rc);
+    for (auto& q : h->side)
+      if (cudaStreamCreateWithFlags(&q, cudaStreamNonBlocking) != cudaSuccess) return fail(FVG_ERR_CUDA);
+    for (auto& e : h->ev)
+      if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) return fail(FVG_ERR_CUDA);
+  }
 
   // ---- schedule ----
   h->sched_cap = 256;
@@ -1011,6 +1069,10 @@ void fvg_destroy(fvg_handle* h) {
   if (h->h_sched) cudaFreeHost(h->h_sched);
   if (h->h_ctl) cudaFreeHost(h->h_ctl);
   if (h->stream) cudaStreamDestroy(h->stream);
+  for (auto q : h->side)
+    if (q) cudaStreamDestroy(q);
+  for (auto e : h->ev)
+    if (e) cudaEventDestroy(e);
   delete h;
 }
 
@@ -1305,6 +1367,10 @@ int fvg_set_precision(fvg_handle* h, int32_t mode) {
     }
     if ((rc = dalloc(h, &f.npk, ms * KB * 16))) return fail(rc);
     if ((rc = dalloc(h, (float**)&f.ex2, (size_t)P.ncvs * KB * 2))) return fail(rc);
+    if (h->ex2_ts) {
+      if ((rc = dalloc(h, (float**)&h->ex2f_ts, (size_t)P.ncvs * KB * 2))) return fail(rc);
+      if ((rc = dalloc(h, &h->npk_ts, ms * KB * 16))) return fail(rc);
+    }
     if ((rc = dalloc(h, &f.xo, 2 * e1))) return fail(rc);
     if ((rc = dalloc(h, &f.yo, 2 * e1))) return fail(rc);
     if ((rc = dalloc(h, &f.dltxc, e1))) return fail(rc);
@@ -1462,6 +1528,8 @@ int fvg_set_tuning(fvg_handle* h, const char* key, int32_t value) {
     h->P.ext_grid = value;
   } else if (k == "ext_loop") {
     h->ext_loop = value != 0;
+  } else if (k == "branches") {
+    h->branches = value != 0;
   } else {
     h->err = "unknown tuning key " + k;
     return FVG_ERR_ARG;
@@ -1483,6 +1551,7 @@ int fvg_get_tuning(const fvg_handle* h, const char* key, int32_t* value) {
   else if (k == "stream_hints") *value = h->P.ldcs;
   else if (k == "ext_grid") *value = h->P.ext_grid;
   else if (k == "ext_loop") *value = use_ext_loop(h);
+  else if (k == "branches") *value = use_branches(h);
   else return FVG_ERR_ARG;
   return FVG_OK;
 }

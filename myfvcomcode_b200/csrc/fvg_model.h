@@ -585,10 +585,12 @@ void launch_adjust2(const Dev& P, cudaStream_t s, int parts);
 void launch_vertvl_flux(const Dev& P, cudaStream_t s);
 enum VertvlColParts { VC_WTS = 1, VC_WD2 = 2, VC_RHO_ROUNDTRIP = 4, VC_BOT_NODE = 8 };
 void launch_vertvl_col(const Dev& P, cudaStream_t s, int parts);
-void launch_w_viscofh(const Dev& P, cudaStream_t s, int do_w, int do_visc);
+// do_stress: with W also the bottom stress that VDIF_UV leaves (vdif_uv.F:172-182), which
+// depends on the lowest layer's U, V alone, so that VDIF_Q need not wait for VDIF_UV.
+void launch_w_viscofh(const Dev& P, cudaStream_t s, int do_w, int do_visc, int do_stress = 0);
 void launch_adv_uv(const Dev& P, cudaStream_t s);
 int staged_setup();  // shared-memory limit of the tile-staged momentum kernels; 0 on success
-enum VdifUvParts { VU_VDIF = 1, VU_BC3 = 2, VU_WREAL = 4 };
+enum VdifUvParts { VU_VDIF = 1, VU_BC3 = 2, VU_WREAL = 4, VU_NO_STRESS = 8 };
 void launch_vdif_uv(const Dev& P, cudaStream_t s, int parts);
 
 // ---------------- scalars and turbulence (k_scalar.cu) ----------------

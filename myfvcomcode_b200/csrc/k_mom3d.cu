@@ -623,7 +623,7 @@ __global__ void k_vertvl_col(const Dev P, int parts) {
 // W = N2E(WTS)*ISWETC (vertvl_edge.F:552-563) on cells, and VISCOF_H (viscofh.F:58-122)
 // on nodes, one thread per (entity, layer).
 // -------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) k_w_viscofh(const Dev P, int do_w, int do_visc) {
+__global__ void __launch_bounds__(256) k_w_viscofh(const Dev P, int do_w, int do_visc, int do_stress) {
   int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
   int kb, ke;
   col_range(P, 1, P.KB, kb, ke);
@@ -632,6 +632,17 @@ __global__ void __launch_bounds__(256) k_w_viscofh(const Dev P, int do_w, int do
   if (do_w && i <= P.N) {
     double w = ONE_THIRD * (P.wts[N3(P, P.nv[i], k)] + P.wts[N3(P, P.nv[n1 + i], k)] + P.wts[N3(P, P.nv[2 * n1 + i], k)]);
     P.w[C3(P, i, k)] = (double)(float)P.iswetc[i] * w;
+    if (do_stress && k == P.KBM1) {
+      double wx = 0.0, wy = 0.0;
+      if (P.iswetc[i] == 1) {
+        const double ub = P.u[C3(P, i, k)], vb = P.v[C3(P, i, k)];
+        const double tps = P.cbc[i] * sqrt(ub * ub + vb * vb);
+        wx = -tps * ub;
+        wy = -tps * vb;
+      }
+      P.wubot[i] = wx;
+      P.wvbot[i] = wy;
+    }
   }
   if (do_visc && i <= P.M && k <= P.KBM1) {
     const double* U = P.u + C3(P, 0, k);
@@ -1287,13 +1298,17 @@ __global__ void __launch_bounds__(128) k_vdif_uv(const Dev P, int parts) {
         vfk = (vhv[ki] * vfk + vhpv[ki]);
         finish(ki, ufk, vfk);
       }
-      P.wubot[i] = -tps * ub;
-      P.wvbot[i] = -tps * vb;
+      if (!(parts & VU_NO_STRESS)) {
+        P.wubot[i] = -tps * ub;
+        P.wvbot[i] = -tps * vb;
+      }
     } else {
       for (int k = 2; k <= KBM1; ++k) finish(KB - k, 0.0, 0.0);
       if (fused) finish(KBM1, P.uf[C3(P, i, KBM1)], P.vf[C3(P, i, KBM1)]);
-      P.wubot[i] = 0.0;
-      P.wvbot[i] = 0.0;
+      if (!(parts & VU_NO_STRESS)) {
+        P.wubot[i] = 0.0;
+        P.wvbot[i] = 0.0;
+      }
     }
     if (!fused) {
       for (int k = 1; k <= KBM1; ++k) {
@@ -1523,10 +1538,10 @@ void launch_vertvl_col(const Dev& P, cudaStream_t s, int parts) {
   const int b = col_threads(P, P.M, 128);
   k_vertvl_col<<<nblk(P.M, b), b, 0, s>>>(P, parts);
 }
-void launch_w_viscofh(const Dev& P, cudaStream_t s, int do_w, int do_visc) {
+void launch_w_viscofh(const Dev& P, cudaStream_t s, int do_w, int do_visc, int do_stress) {
   int n = P.M > P.N ? P.M : P.N;
   const Dev Q = col_shape(P, n, P.KB);
-  k_w_viscofh<<<col_grid(Q, n, P.KB), Q.col_bc, 0, s>>>(Q, do_w, do_visc);
+  k_w_viscofh<<<col_grid(Q, n, P.KB), Q.col_bc, 0, s>>>(Q, do_w, do_visc, do_stress);
 }
 void launch_adv_uv(const Dev& P, cudaStream_t s) {
   FVG_F32_FORWARD(launch_adv_uv(P, s));

@@ -63,3 +63,28 @@ def test_resident_loop_fp32_flux(name):
         assert np.abs(x - y).max() <= 1e-5 * np.abs(y).max(), f
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32flux"])
+def test_branches_equal_one_order(precision):
+    from myfvcomcode_b200.engine import Fvcom, Group
+    models = [Fvcom(_case("coast")) for _ in range(3)]
+    for m in models:
+        m.set_precision(precision)
+    models[1].set_tuning("branches", 0)
+    assert [m.get_tuning("branches") for m in models] == [1, 0, 1]
+    models[0].run(6)
+    models[1].run(6)
+    grp = Group([models[2]])
+    grp.run(6)
+    for f in FIELDS + ("v", "s1", "km", "kh", "uf", "rho", "wubot", "tps"):
+        for m in (models[0], models[2]):
+            assert np.array_equal(m.get(f), models[1].get(f)), f
+    # plain launches on the same streams
+    models[0].use_graph(False)
+    models[0].run(2)
+    models[1].run(2)
+    assert np.array_equal(models[0].get("t1"), models[1].get("t1"))
+    grp.close()
+    for m in models:
+        m.close()
