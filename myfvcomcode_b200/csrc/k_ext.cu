@@ -1274,9 +1274,12 @@ __global__ void __launch_bounds__(256, 5) k_stage_node(const Dev P, int st) {
     node_phase<R, CS, 0>(P, i, st, z);
   }
 }
-// Resident blocks per SM of the stage cell kernel.
+// Resident blocks per SM of the stage cell kernel, external mode of a step: FP64 four blocks of
+// 128 registers 2,524 us against five of 96 (spilling 100 bytes) 2,905 (200k nodes; 50k 1,024
+// against 1,122); FP32 six 923, seven 966, eight 996, five 1,005 (50k; 200k 2,302, 2,267,
+// 2,447, 2,200).
 template <typename R>
-constexpr int kStageBlocks = sizeof(R) == 4 ? 7 : 5;
+constexpr int kStageBlocks = sizeof(R) == 4 ? 6 : 4;
 // WALK: one wave of blocks whose threads walk the cells.
 template <typename R, bool CS, bool WALK>
 __global__ void __launch_bounds__(128, kStageBlocks<R>) k_stage_cell(const Dev P, int st) {
