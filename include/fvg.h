@@ -306,10 +306,11 @@ int fvg_closure_status(fvg_handle* h, int32_t* columns_on_network, int32_t* wait
    "col_layers"  = consecutive layers each thread walks, 1..KB (default 8);
                    until one of the two is set, a launch that would not fill the chip
                    takes fewer layers per thread, then fewer threads per block;
-   "compact"     = 1 (default) lets the precision form's Runge-Kutta stages use the
-                   compact cell kernel where fvg_set_precision found the mesh's edge metrics
-                   to be the ones its coordinates define; 0 keeps the general kernel.
-                   fvg_get_tuning("compact") reports whether the compact kernel is in use;
+   "compact"     = 1 (default) lets the Runge-Kutta stages run on packed records where
+                   fvg_create found the mesh's edge metrics to be the ones its coordinates
+                   define (a limited scheme in FP64 only); 0 keeps the general kernels.  FP64
+                   results do not depend on it.  fvg_get_tuning("compact") reports whether
+                   the precision form uses them;
    "staged"      = 2 runs ADVECTION_EDGE_GCN and ADV_UV_EDGE_GCN (LIMITED_NO, GCN) as the
                    tile-staged kernels (neighbour cells in shared memory, each edge
                    evaluated once per tile); 1 (default) and 0 one thread per cell, which
@@ -325,8 +326,8 @@ int fvg_closure_status(fvg_handle* h, int32_t* columns_on_network, int32_t* wait
                    partly filled last wave is left; 0 launches one thread per cell.
                    Results do not depend on it;
    "ext_loop"     = 1 (default): the external loop of a mesh of at most 384 cells per SM runs
-                   as one resident cooperative kernel (no limiter; the FP32-flux form with
-                   the compact kernel's records); 0 launches every stage.  FP64 results do
+                   as one resident cooperative kernel (with "compact" in use or possible);
+                   0 launches every stage.  FP64 results do
                    not depend on it; fvg_get_tuning reports whether it is in use;
    "branches"     = 1 (default): up to 20 million cell-layers the independent parts of a step
                    (BAROPG beside ADVECTION; momentum, turbulence and tracers after VERTVL)

@@ -60,7 +60,7 @@ struct fvg_handle {
   bool use_graph = true;
   int clos_grid = 148;
   // external stages on the packed records: allowed (tuning key "compact") and possible (the
-  // mesh's edge metrics are the ones its coordinates define, no limiter)
+  // mesh's edge metrics are the ones its coordinates define)
   int compact_allowed = 1;
   int compact_ok = 0;
   // resident external loop: allowed (tuning key "ext_loop"), possible (the device launches
@@ -693,7 +693,7 @@ int fvg_create(const fvg_mesh* m, const fvg_params* prm, const fvg_forcing* f, f
       std::vector<int> far(3 * n1, 0), lx(4 * n1, 0);
       lo.assign(4 * n1, 0);
       std::vector<double> hm(n1, 0.0);
-      h->compact_ok = P.limiter == 0;
+      h->compact_ok = 1;
       for (size_t i = 1; i < n1; ++i) {
         // the node common to two slots' edges
         auto common = [&](int sa, int sb) {
@@ -753,6 +753,7 @@ int fvg_create(const fvg_mesh* m, const fvg_params* prm, const fvg_forcing* f, f
       if ((rc = dalloc(h, (double**)&P.xnd, 2 * m1))) return fail(rc);
       if ((rc = dalloc(h, &P.xg, 4 * n1))) return fail(rc);
       if ((rc = dalloc(h, &P.xvc, n1))) return fail(rc);
+      if (P.limiter && (rc = dalloc(h, (double**)&P.xal, 2 * n1))) return fail(rc);
       if ((rc = dalloc(h, &P.xw, 2 * n1))) return fail(rc);
       if ((rc = dalloc(h, &P.obf, (size_t)4 * prm->isplit * (m->iobcn + 1)))) return fail(rc);
       UPD(hmin, hm.data(), n1);
@@ -1266,8 +1267,10 @@ int32_t fvg_kernels_per_step(const fvg_handle* h) {
   if (!h) return -1;
   const fvg_params& p = h->prm;
   int n = 1 + 1 + 2 + 2 + 2;                                // begin, cell_pre, grad3+adv3d, baropg+prep, int advave+reset
-  n += (use_ext_loop(h) ? 1 : p.isplit * 4 * (2 + (p.wetting_drying_on && p.limiter ? 1 : 0))) + 1; // RK stages, closing update
-  if (p.limiter) n += p.isplit * 4 + 1 + 2;                  // slope limiters: stages, ADVAVE, 3-D
+  n += (use_ext_loop(h) ? 1 : p.isplit * 4 * (2 + (p.limiter ? 1 : 0) +
+                                              (p.wetting_drying_on && p.limiter && !h->P.xform ? 1 : 0))) + 1;
+                                                           // RK stages (with slope limiters), closing update
+  if (p.limiter) n += 1 + 2;                               // slope limiters: ADVAVE, 3-D
   if (p.baropg_z && !p.barotropic) n += 2;                   // PHY_BAROPG's two kernels
   n += 1 + 1 + 1 + 1 + 2 + 1;                              // adjust2, vertvl x2, w/viscofh, grad3+adv_uv, vdif_uv
   n += 7;                                                  // grad_q, adv_q (2 phases), vdif_q (4 passes)
@@ -1339,7 +1342,7 @@ int fvg_set_forcing(fvg_handle* h, const fvg_forcing* f) {
 }
 
 static void set_xform(fvg_handle* h) {
-  h->P.xform = h->compact_ok && h->compact_allowed;
+  h->P.xform = h->compact_ok && h->compact_allowed && !(h->P.limiter && h->P.prec);
   h->P.f.compact = h->P.prec == FVG_PREC_FP32_FLUX && h->P.xform;
 }
 

@@ -213,10 +213,11 @@ struct Dev {
   // of NV(c,3) among X, bit 8+s set where IENODE(e,1) is X(s+1); loopo, per cell the other cell
   // of slots 0, 1, 2, and w: ISBCE in bits 0-1, river momentum entries bit 2, open-boundary
   // flux entries bit 3, a sponge coefficient bit 4, EPOR = 1 bit 5, IUCP = 1 bit 6.
+  // xal: UALFA, VALFA of a limited scheme (FP64).
   // xform: the stages form the edge geometry from vxy {VX, VY} and xyc {XC, YC} (DLTXC =
   // VX(IENODE2)-VX(IENODE1), XIJC = (VX(IENODE1)+VX(IENODE2))/2, DLTXE = XIJC-XC), which
-  // fvg_create found equal to the mesh's own metrics bit for bit; 0 where it did not, or
-  // where a limiter is on: the general kernels then run.
+  // fvg_create found equal to the mesh's own metrics bit for bit; 0 where it did not: the
+  // general kernels then run.
   // wfar, per slot and cell (s*(N+1) + c) the node of the other cell that is off the edge (0:
   // none); hmin, per cell the smallest H of its nodes.  exd: EXTUV's fixed terms in FP64, six
   // planes of N+1 pairs (store_fixed); xrk the pairs UARK, VARK.  Exchanged between cells and
@@ -228,7 +229,7 @@ struct Dev {
   const double2 *vxy, *xyc;
   double2 *exd, *xrk;
   const int4 *loopx, *loopo;
-  double2 *xuv, *xnd;
+  double2 *xuv, *xnd, *xal;
   double *xg, *xvc;
   int* xw;
   int loop_cells, loop_nodes;

@@ -776,6 +776,21 @@ __device__ __forceinline__ LoopShared<R, T>& loop_shared() {
   return *reinterpret_cast<LoopShared<R, T>*>(loop_sm);
 }
 
+// ISWETCE*ISWETC of cell o on the other side of slot s of a dry cell c at a stage with flag
+// buffers wp (the stage before) and wn (this one): the neighbour's flag of this stage is formed
+// from its three nodes, e the larger ELF of the edge's two, as WET_JUDGE forms it.
+template <bool RES>
+__device__ __forceinline__ bool stage_wet_other(const Dev& P, int c, int s, int o, const int* wp, const int* wn, double e) {
+  int wo = wp[o];
+  if (P.wetting_drying_on && o != 0) {
+    const double m = fmax(e, ldx<RES>(P.elf + P.wfar[(size_t)s * (P.N + 1) + c]));
+    wo = wo * (((m + P.hmin[o]) - P.min_depth) < 1.0e-5 ? 0 : 1);
+  } else {
+    wo = wo * (P.wetting_drying_on ? wn[0] : P.iswetc[o]);
+  }
+  return wo == 1;
+}
+
 // Gradient and viscosity term of cell c (neighbours nb) with velocity u, v at stage st.
 // T: threads per block of the resident loop, 0 in a stage kernel.
 template <typename R, bool CS, int T>
@@ -934,6 +949,46 @@ __device__ __forceinline__ void node_phase(const Dev& P, int i, int st, NodeKeep
   P.xnd[i] = make_double2(z.el, z.d);
 }
 
+// Slope limiters UALFA, VALFA of cell c for the limited ADVAVE (advave_edge_gcn.F:141-318), a
+// phase of its own between the two: WET_JUDGE's cell flag, then the cell's three edges with a
+// wet side, from its own gradient g and the two cells' velocities.
+template <typename R, bool CS, int T>
+__device__ __forceinline__ void alfa_phase(const Dev& P, int c, int st, const int4 xn, const int4 oo, int wce, double u,
+                                           double v, const Grad<R>& g) {
+  constexpr bool RES = T > 0;
+  const size_t n1 = P.N + 1;
+  const double2* const uv = P.xuv + (st & 1) * n1;
+  const int* const wp = P.xw + ((st + 1) & 1) * n1;
+  const int* const wn = P.xw + (st & 1) * n1;
+  const bool wd = P.wetting_drying_on != 0;
+  const int xs[3] = {xn.x, xn.y, xn.z}, os[3] = {oo.x, oo.y, oo.z};
+  double2 ou[3];
+  double en[3];
+#pragma unroll
+  for (int s = 0; s < 3; ++s) {
+    ou[s] = ldx<RES>(uv + os[s]);
+    en[s] = ldx<RES>(P.elf + xs[s]);
+  }
+  int wetc = wd ? 0 : P.iswetc[c];
+  if (wd) {
+    const double dtmp = fmax(fmax(en[0], en[1]), en[2]) + P.hmin[c];
+    wetc = ((dtmp - P.min_depth) < 1.0e-5) ? 0 : 1;
+  }
+  const bool wet = wce * wetc == 1;
+  const double2 ci = P.xyc[c];
+  R au = (R)1, av = (R)1;
+#pragma unroll
+  for (int s = 0; s < 3; ++s) {
+    const int o = os[s];
+    if (!(wet || stage_wet_other<RES>(P, c, s, o, wp, wn, fmax(en[s], en[(s + 1) % 3])))) continue;
+    const double2 v1 = P.vxy[xs[s]], v2 = P.vxy[xs[(s + 1) % 3]];
+    const R x = (R)((v1.x + v2.x) * 0.5 - ci.x), y = (R)((v1.y + v2.y) * 0.5 - ci.y);
+    lim_alfa<R>(fabs((R)u - (R)ou[s].x), g.ux * x + g.uy * y, au);
+    lim_alfa<R>(fabs((R)v - (R)ou[s].y), g.vx * x + g.vy * y, av);
+  }
+  P.xal[c] = make_double2(au, av);
+}
+
 // What the resident loop keeps of a cell between stages; the launched phases load it.
 template <typename R>
 struct CellKeep {
@@ -945,7 +1000,7 @@ struct CellKeep {
   int bcriv, nobc, nriv, wce, wci, ob[2], obn[2];
   double obf[2], rvx[2], rvy[2];
 };
-template <typename R, bool CS, int T>
+template <typename R, bool CS, int T, bool LIM>
 __device__ __forceinline__ void cell_phase(const Dev& P, int c, int st, CellKeep<R>& z) {
   typedef Mesh<R> Mh;
   constexpr bool RES = T > 0;
@@ -1109,17 +1164,7 @@ __device__ __forceinline__ void cell_phase(const Dev& P, int c, int st, CellKeep
     const R dij = (R)(0.5 * (na.y + nbb.y));
     const double elij = 0.5 * (na.x + nbb.x);
     bool on = weti == 1;
-    if (!on) {
-      // a dry cell: the neighbour's flags of the stage before and of this one
-      int wo = wp[o];
-      if (wd && o != 0) {
-        const double e = fmax(fmax(en[s], en[(s + 1) % 3]), ldx<RES>(P.elf + P.wfar[(size_t)s * n1 + c]));
-        wo = wo * (((e + P.hmin[o]) - P.min_depth) < 1.0e-5 ? 0 : 1);
-      } else {
-        wo = wo * (wd ? wn[0] : P.iswetc[o]);
-      }
-      on = wo == 1;
-    }
+    if (!on) on = stage_wet_other<RES>(P, c, s, o, wp, wn, fmax(en[s], en[(s + 1) % 3]));
     if (on) {
       const R dx = (R)edx, dy = (R)edy;
       const double2 co = RES ? sm.p2[4 + s][me] : P.xyc[o];
@@ -1127,8 +1172,17 @@ __device__ __forceinline__ void cell_phase(const Dev& P, int c, int st, CellKeep
       const double2 uvo = RES ? ou[s] : uv[o];
       const Grad<R> gs = RES ? go[s] : ld_xg<R, RES>(P, o);
       const R uo = (R)uvo.x, vv = (R)uvo.y, vco = RES ? vo[s] : xvc[o];
-      const R uown = ui + gi.ux * xi + gi.uy * yi, vown = vi + gi.vx * xi + gi.vy * yi;
-      const R uoth = uo + gs.ux * xo + gs.uy * yo, voth = vv + gs.vx * xo + gs.vy * yo;
+      R uown, vown, uoth, voth;
+      if constexpr (LIM) {
+        const double2 ai = ldx<RES>(P.xal + c), ao = ldx<RES>(P.xal + o);
+        lim_faces<R>(P.limiter, ui, uo, gi.ux * xi + gi.uy * yi, gs.ux * xo + gs.uy * yo, ai.x, ao.x, uown, uoth);
+        lim_faces<R>(P.limiter, vi, vv, gi.vx * xi + gi.vy * yi, gs.vx * xo + gs.vy * yo, ai.y, ao.y, vown, voth);
+      } else {
+        uown = ui + gi.ux * xi + gi.uy * yi;
+        vown = vi + gi.vx * xi + gi.vy * yi;
+        uoth = uo + gs.ux * xo + gs.uy * yo;
+        voth = vv + gs.vx * xo + gs.vy * yo;
+      }
       const R uij = half * (uown + uoth), vij = half * (vown + voth);
       const R un = -uij * dy + vij * dx;
       R viscof = (R)P.fact * half * (vci + vco);
@@ -1281,16 +1335,27 @@ __global__ void __launch_bounds__(256, 5) k_stage_node(const Dev P, int st) {
 template <typename R>
 constexpr int kStageBlocks = sizeof(R) == 4 ? 6 : 4;
 // WALK: one wave of blocks whose threads walk the cells.
-template <typename R, bool CS, bool WALK>
+template <typename R, bool CS, bool WALK, bool LIM>
 __global__ void __launch_bounds__(128, kStageBlocks<R>) k_stage_cell(const Dev P, int st) {
   pdl_enter();
   int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
   do {
     if (i > P.N) return;
     CellKeep<R> z;
-    cell_phase<R, CS, 0>(P, i, st, z);
+    cell_phase<R, CS, 0, LIM>(P, i, st, z);
     i += gridDim.x * blockDim.x;
   } while (WALK);
+}
+
+template <typename R, bool CS>
+__global__ void __launch_bounds__(128) k_stage_alfa(const Dev P, int st) {
+  pdl_enter();
+  const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
+  if (i > P.N) return;
+  const size_t n1 = P.N + 1;
+  const double2 own = P.xuv[(st & 1) * n1 + i];
+  alfa_phase<R, CS, 0>(P, i, st, ld1<CS>(P.loopx + i), ld1<CS>(P.loopo + i), P.xw[((st + 1) & 1) * n1 + i], own.x, own.y,
+                       ld_xg<R, false>(P, i));
 }
 
 // Barrier over the grid: every block adds one to the counter (zeroed by k_begin_step) and
@@ -1317,7 +1382,7 @@ __device__ __forceinline__ bool grid_barrier(const Dev& P, unsigned target) {
 
 // SPLIT: the block's first half of threads holds its cells and the second half its nodes, so
 // that the two jobs of a node phase run side by side on different warps.
-template <typename R, int T, bool SPLIT>
+template <typename R, int T, bool SPLIT, bool LIM>
 __global__ void __launch_bounds__(T, 1) k_ext_loop(const __grid_constant__ Dev P) {
   const int tid = threadIdx.x, tn = SPLIT ? tid - T / 2 : tid;
   const int c = blockIdx.x * P.loop_cells + tid + 1, i = blockIdx.x * P.loop_nodes + tn + 1;
@@ -1416,7 +1481,11 @@ __global__ void __launch_bounds__(T, 1) k_ext_loop(const __grid_constant__ Dev P
     if (hn) node_phase<R, false, T>(P, i, st, y);
     if (hc) z.g = grad_job<R, false, T>(P, c, st, z.u, z.v, z.vc);
     if (!grid_barrier(P, target += gridDim.x)) return;
-    if (hc) cell_phase<R, false, T>(P, c, st, z);
+    if constexpr (LIM) {
+      if (hc) alfa_phase<R, false, T>(P, c, st, z.xn, z.oo, z.wce, z.u, z.v, z.g);
+      if (!grid_barrier(P, target += gridDim.x)) return;
+    }
+    if (hc) cell_phase<R, false, T, LIM>(P, c, st, z);
     if (st < nst - 1 && !grid_barrier(P, target += gridDim.x)) return;
   }
   if (hn) {
@@ -1491,6 +1560,7 @@ __global__ void k_ext_prep(const Dev P) {
       P.xuv[n1] = make_double2(P.uaf[0], P.vaf[0]);
       P.xw[0] = P.iswetc[0];
       P.xw[n1] = P.iswetce[0];
+      if (P.limiter) P.xal[0] = make_double2(1.0, 1.0);
       if (!P.prec) {
         P.xg[0] = P.g2d[0][0];
         P.xg[1] = P.g2d[1][0];
@@ -1614,6 +1684,10 @@ void launch_ext_finish(const Dev& P, cudaStream_t s, int K, int wet_prev) {
   int n = P.M > P.N ? P.M : P.N;
   k_ext_finish<<<nblk(n, 256), 256, 0, s>>>(P, K, wet_prev);
 }
+// A limited scheme runs on the packed records in FP64 only.  LIMITED_1's clamp is
+// discontinuous: the packed FP32 form's rounding (a few 1e-9 of the fields) would switch it on
+// other edges, so that form keeps the general kernels.
+constexpr bool kLimited = sizeof(RF) == 8;
 template <int T, bool SPLIT>
 static void loop_launch(const Dev& P, cudaStream_t s, int grid) {
   cudaLaunchConfig_t cfg = {};
@@ -1629,15 +1703,20 @@ static void loop_launch(const Dev& P, cudaStream_t s, int grid) {
   Dev Q = P;
   Q.loop_cells = nblk(P.N, grid);
   Q.loop_nodes = nblk(P.M, grid);
-  cudaLaunchKernelEx(&cfg, k_ext_loop<RF, T, SPLIT>, Q);
+  void (*k)(const Dev) = k_ext_loop<RF, T, SPLIT, false>;
+  if constexpr (kLimited) {
+    if (P.limiter) k = k_ext_loop<RF, T, SPLIT, true>;
+  }
+  cudaLaunchKernelEx(&cfg, k, Q);
 }
 // Shared memory of the resident loop's blocks (once, before any launch or capture); 0 on success.
 template <int T, bool SPLIT>
 static int loop_attr() {
-  return cudaFuncSetAttribute(k_ext_loop<RF, T, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)sizeof(LoopShared<RF, T>)) == cudaSuccess
-             ? 0
-             : 1;
+  int bad = 0;
+  for (auto k : {k_ext_loop<RF, T, SPLIT, false>, k_ext_loop<RF, T, SPLIT, kLimited>})
+    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(LoopShared<RF, T>)) != cudaSuccess)
+      bad = 1;
+  return bad;
 }
 int ext_loop_setup() { return loop_attr<256, true>() | loop_attr<256, false>() | loop_attr<kLoopThreads, false>(); }
 // One block per SM at most, the smallest that then holds a cell and a node per thread, so that
@@ -1664,13 +1743,19 @@ void launch_ext_stage(const Dev& P, cudaStream_t s, int st) {
   launch_maybe_pdl(st > 0, P.ldcs ? k_stage_node<RF, true> : k_stage_node<RF, false>, dim3(nblk(n, bn)), dim3(bn), s,
                    P, st);
   const int b = col_threads(P, P.N, 128), nb = nblk(P.N, b);
+  if constexpr (kLimited) {
+    if (P.limiter)
+      launch_maybe_pdl(1, P.ldcs ? k_stage_alfa<RF, true> : k_stage_alfa<RF, false>, dim3(nb), dim3(b), s, P, st);
+  }
   const int wave = (P.ext_grid < kStageBlocks<RF> ? P.ext_grid : kStageBlocks<RF>)*P.nsm;
-  if (P.ext_grid > 0 && nb > wave)
-    launch_maybe_pdl(1, P.ldcs ? k_stage_cell<RF, true, true> : k_stage_cell<RF, false, true>, dim3(wave), dim3(b), s, P,
-                     st);
-  else
-    launch_maybe_pdl(1, P.ldcs ? k_stage_cell<RF, true, false> : k_stage_cell<RF, false, false>, dim3(nb), dim3(b), s, P,
-                     st);
+  const bool walk = P.ext_grid > 0 && nb > wave;
+  auto k = [&](auto lim) {
+    constexpr bool L = decltype(lim)::value;
+    return walk ? (P.ldcs ? k_stage_cell<RF, true, true, L> : k_stage_cell<RF, false, true, L>)
+                : (P.ldcs ? k_stage_cell<RF, true, false, L> : k_stage_cell<RF, false, false, L>);
+  };
+  launch_maybe_pdl(1, P.limiter ? k(std::bool_constant<kLimited>()) : k(std::false_type()), dim3(walk ? wave : nb),
+                   dim3(b), s, P, st);
 }
 void launch_begin_step(const Dev& P, cudaStream_t s) { k_begin_step<<<1, 32, 0, s>>>(P, 1); }
 void launch_set_qdis(const Dev& P, cudaStream_t s) { k_begin_step<<<1, 32, 0, s>>>(P, 0); }

@@ -19,13 +19,14 @@ def _case(name):
     if name == "channel_wide":  # 148 blocks of 128 threads are not enough: the next block size
         return cases.estuary_channel(nx=170, ny=60, kb=4, lx=34000.0, ly=12000.0, IRAMP=10)
     ghost = name == "coast_ghost"
-    npts = {"coast": 1500, "coast_ghost": 1500, "coast_large": 25000}[name]
+    npts = {"coast_large": 25000}.get(name, 1500)
+    more = {"coast_limited_1": dict(LIMITER="LIMITED_1"), "coast_limited_2": dict(LIMITER="LIMITED_2")}.get(name, {})
     return cases.coastal_mesh(npts=npts, kb=5, lx=20000.0, ly=10000.0, seed=7, IRAMP=2, dte=0.5 if npts > 2000 else 2.0,
-                              ghost_cells="GCY1" if ghost else "GCN")
+                              ghost_cells="GCY1" if ghost else "GCN", **more)
 
 
 @pytest.mark.parametrize("name", ["channel_node_river", "channel_edge_river", "channel_wide", "coast", "coast_ghost",
-                                  "coast_large"])
+                                  "coast_large", "coast_limited_1", "coast_limited_2"])
 def test_resident_loop_equals_launched_loop(name):
     from myfvcomcode_b200.engine import Fvcom
     case = _case(name)
@@ -36,6 +37,13 @@ def test_resident_loop_equals_launched_loop(name):
     b.run(8)
     for f in FIELDS:
         assert np.array_equal(a.get(f), b.get(f)), f
+    # the packed stages against the general stage kernels
+    c = Fvcom(case)
+    c.set_tuning("compact", 0)
+    c.run(8)
+    for f in FIELDS:
+        assert np.array_equal(b.get(f), c.get(f)), f
+    c.close()
     # one step without the graph
     a.use_graph(False)
     a.run(1)
