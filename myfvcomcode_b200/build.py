@@ -22,7 +22,7 @@ LIB = os.path.join(HERE, "lib", "libfvg.so")
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
     "-lineinfo", "-O3", "--fmad=false", "-std=c++17",
-    "-Xcompiler", "-fPIC,-O2", "-shared",
+    "-Xcompiler", "-fPIC,-O3", "-shared",
 ]
 
 
