@@ -991,7 +991,7 @@ int fvg_create(const fvg_mesh* m, const fvg_params* prm, const fvg_forcing* f, f
     }
   if ((rc = dalloc(h, &P.gvn, ms * KB))) return fail(rc);
   if ((rc = dalloc(h, &P.budget, 3 + 3 * 148))) return fail(rc);
-  for (double** pp : {&P.vq_prod, &P.vq_gh, &P.vq_dtef, &P.vq_dtefl})
+  for (double** pp : {&P.vq_prod, &P.vq_gh, &P.vq_stf, &P.vq_dtef, &P.vq_dtefl})
     if ((rc = dalloc(h, pp, ms * KB))) return fail(rc);
   if ((rc = dalloc(h, &P.vq_ut, ms))) return fail(rc);
   P.ncvs = (int)(3 * ns);  // half-edge arrays by position, pos = slot*ns + cell

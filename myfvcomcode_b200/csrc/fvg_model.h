@@ -247,8 +247,8 @@ struct Dev {
   double *gt[2][6];  // ADV_T / ADV_S: the same six per tracer
   double* gvn;       // VISCOFH*NN_HVC of the half-edge fluxes, per node and layer or level (FP64 form)
   double* budget;                            // 3 doubles
-  // VDIF_Q between its passes: PROD, GH, DTEF, the q2l DTEF (node 3-D) and UTAU2 (node)
-  double *vq_prod, *vq_gh, *vq_dtef, *vq_dtefl, *vq_ut;
+  // VDIF_Q between its passes: PROD, GH, STF, DTEF, the q2l DTEF (node 3-D) and UTAU2 (node)
+  double *vq_prod, *vq_gh, *vq_stf, *vq_dtef, *vq_dtefl, *vq_ut;
   double2* ex2;                              // half-edge fluxes of both tracers (ncvs x KB, by position)
   // VERTVL_EDGE's EXFLUX of each half-edge position and layer, at (k-1)*ncvs + pos; it
   // lives in the allocation of ex2, which is free between ADJUST2D3D and the next advection.

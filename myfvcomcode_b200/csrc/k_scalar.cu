@@ -651,7 +651,7 @@ __global__ void __launch_bounds__(256, 4) k_vdif_q_levels(const Dev P) {
     if (k >= 2 && k <= KBM1) {
       if (wet) {
         boygr = P.grav_n[i] * (P.rho1[n3(k - 1)] - P.rho1[q]) / (P.dzz(i, k - 1) * d);
-        prod = P.km[q] * 0.0 * pow(.5 * (-boygr + fabs(boygr)), 1.5);
+        // the reference's internal-wave term carries a weight of zero and is not evaluated
         double uk, vk;
         ring_mean(k, uk, vk);
         const double den = P.dzz(i, k - 1) * d;
@@ -682,7 +682,7 @@ __global__ void __launch_bounds__(256, 4) k_vdif_q_levels(const Dev P) {
           samp(6, k, q2);
           samp(7, k, q2l);
         }
-        prod = prod + P.km[q] * SEF * ((uk - ukm1) * (uk - ukm1) + (vk - vkm1) * (vk - vkm1)) / (den * den);
+        prod = P.km[q] * SEF * ((uk - ukm1) * (uk - ukm1) + (vk - vkm1) * (vk - vkm1)) / (den * den);
         prod = prod + P.kh[q] * boygr;
         ukm1 = uk;
         vkm1 = vk;
@@ -708,6 +708,7 @@ __global__ void __launch_bounds__(256, 4) k_vdif_q_levels(const Dev P) {
     const double dtef = sqrt(q2) / (B1 * lk + SMALL) * stf;
     P.vq_prod[q] = prod;
     P.vq_gh[q] = gh;
+    P.vq_stf[q] = stf;
     P.vq_dtef[q] = dtef;
     if (wet && k >= 2 && k <= KBM1) {
       const double x = (1. / fabs(P.z(i, k) - P.z(i, 1)) + 1. / fabs(P.z(i, k) - P.z(i, KB))) * lk / (d * KAPPA);
@@ -815,9 +816,7 @@ __global__ void __launch_bounds__(256) k_vdif_q_coef(const Dev P, int copy_back)
       continue;
     }
     const double gh = P.vq_gh[q];
-    double stf = 1.0;
-    if (gh < 0.0) stf = 1.0 - F4(0.9) * pow(gh / GHC, 1.5);
-    if (gh < GHC) stf = F4(0.1);
+    const double stf = P.vq_stf[q];
     double coef1 = A2 * (1.0 - 6.0 * A1 / B1 * stf);
     double coef2 = 3.0 * A2 * B2 / stf + 18.0 * A1 * A2;
     double coef3 = A1 * (1.0 - 3.0 * C1 - 6.0 * A1 / B1 * stf);
