@@ -320,12 +320,15 @@ inline int col_threads(const Dev& P, long n, int most) {
 // The launch shape of a column-tiled kernel over n entities and nl layers: the default
 // shape (col_bc threads, each walking col_lc layers) amortises the entity's index chain
 // over its layers, but a thread then runs that many layers one after the other, which is
-// the whole time of a kernel that does not fill the chip.  Below about four blocks per SM
-// the chunk is halved until there are, then the block.
+// the whole time of a kernel that does not fill the chip, and a few long blocks end in a wave
+// that is nearly empty.  Below twelve blocks per SM the chunk is halved until there are, then
+// the block.  Four -> twelve blocks: 50 k nodes x 30 layers, grad_ts 146 -> 129 us, vdif_q 248 ->
+// 236, grad_q 137 -> 127; 20 k x 19, w_viscofh 46 -> 33; 200 k keeps the full chunk, which is
+// the faster there (step 9840 against 10610 us with half of it).
 inline Dev col_shape(const Dev& P, int n, int nl) {
   Dev Q = P;
   if (!P.col_auto) return Q;
-  const long want = 4L * P.nsm;
+  const long want = 12L * P.nsm;
   while (Q.col_lc > 1 && (long)((n + Q.col_bc - 1) / Q.col_bc) * ((nl + Q.col_lc - 1) / Q.col_lc) < want)
     Q.col_lc = (Q.col_lc + 1) / 2;
   while (Q.col_bc > 32 && (long)((n + Q.col_bc - 1) / Q.col_bc) * ((nl + Q.col_lc - 1) / Q.col_lc) < P.nsm)

@@ -888,9 +888,11 @@ __global__ void __launch_bounds__(256) k_adv_uv(const Dev P) {
 //   * ADV_UV's vertical flux through a layer's lower interface is the next layer's upper one.
 // The terms and their order are the reference's: FP64 results are bit for bit those of the
 // per-edge evaluation.
+// Blocks per SM: in FP64 five for ADVECTION (703 -> 659 us at 200 k nodes x 30 layers against
+// four), four for ADV_UV, where five gain 2 % at 200 k and lose 10 % at 6 k; in FP32 seven and six.
 // -------------------------------------------------------------------------------------
 template <typename R, bool UV>
-__global__ void __launch_bounds__(128, sizeof(R) == 4 ? (UV ? 6 : 7) : 4) k_mom3d(const Dev P) {
+__global__ void __launch_bounds__(128, sizeof(R) == 4 ? (UV ? 6 : 7) : (UV ? 4 : 5)) k_mom3d(const Dev P) {
   typedef Mesh<R> Mh;
   const R half = (R)0.5, one = (R)1.0, three = (R)3.0;
   const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;

@@ -366,8 +366,13 @@ __device__ inline R he_flux(const HeCell<R>& hc, const HeGeo<R>& g, int flip, co
   return exflux;
 }
 
+// Largest block of k_he_adv.  The FP32 form takes 64 registers and eight blocks per SM: 200 k
+// nodes, six -> eight blocks, ADV_Q 716 -> 682 us.  In FP64 five blocks (96 registers) suit T and
+// S (28 bytes spilled); Q2 and Q2L, with the level interpolation, spill 72 and keep four (ADV_Q
+// 1186 against 1258 us).
+constexpr int kHeThreads = 128;
 template <typename R, int MODE>
-__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 3 : 2) k_he_adv(const Dev P, int parts) {
+__global__ void __launch_bounds__(kHeThreads, sizeof(R) == 4 ? 8 : (MODE == 1 ? 5 : 4)) k_he_adv(const Dev P, int parts) {
   typedef typename Mesh<R>::R2 R2;
   int c = blockIdx.x * blockDim.x + threadIdx.x + 1;
   if (c > P.N) return;
@@ -447,7 +452,13 @@ __global__ void __launch_bounds__(64) k_obc_xflux(const Dev P, int parts) {
 
 // Signed sum of a node's half-edge fluxes on layer k, both tracers, in ascending
 // half-edge order (the order of the reference's scatter into XFLUX).
-// The loads are issued four entries at a time (codes, then fluxes) and added in order.
+// The loads are issued kHeBat entries at a time (codes, then fluxes) and added in order; a
+// node of six cells has twelve.  Four, six and eight entries with the node gathers at 200 k
+// nodes x 30 layers: ADV_Q 1094, 1090, 1085 us in FP64, 751, 722, 716 in FP32.
+constexpr int kHeBat = 8;
+// Largest block of the node gathers.  Four FP64 and six FP32 blocks per SM leave them 128 and
+// 80 registers; six and seven spill 140 and 76 bytes (FP64 step 9900 against 9840 us).
+constexpr int kGatherThreads = 128;
 template <typename R>
 __device__ inline double2 gather_he(const Dev& P, int i, int n, int k) {
   typedef typename Mesh<R>::R2 R2;
@@ -464,62 +475,108 @@ __device__ inline double2 gather_he(const Dev& P, int i, int n, int k) {
       x1 = x1 + e.y;
     }
   };
-  int j = 0;
-  for (; j + 4 <= n; j += 4) {
-    const int c0 = L[j * ms], c1 = L[(j + 1) * ms], c2 = L[(j + 2) * ms], c3 = L[(j + 3) * ms];
-    const R2 e0 = EX[c0 >> 1], e1 = EX[c1 >> 1], e2 = EX[c2 >> 1], e3 = EX[c3 >> 1];
-    add(c0, e0);
-    add(c1, e1);
-    add(c2, e2);
-    add(c3, e3);
-  }
-  for (; j < n; ++j) {
-    const int c = L[j * ms];
-    add(c, EX[c >> 1]);
+  for (int j = 0; j < n; j += kHeBat) {
+    int c[kHeBat];
+    R2 e[kHeBat];
+#pragma unroll
+    for (int b = 0; b < kHeBat; ++b) c[b] = L[(j + b < n ? j + b : j) * ms];
+#pragma unroll
+    for (int b = 0; b < kHeBat; ++b) e[b] = EX[c[b] >> 1];
+#pragma unroll
+    for (int b = 0; b < kHeBat; ++b)
+      if (j + b < n) add(c[b], e[b]);
   }
   return make_double2((double)x0, (double)x1);
 }
 
 // Phase 2 of ADV_Q(Q2,Q2F)/ADV_Q(Q2L,Q2LF) (adv_q.F:114-401) with FCT_Q2/FCT_Q2L.
+// Latency bounds the node gathers (30 % of the issue slots at 28 % occupancy), so a layer's loads
+// of both tracers stand before its first store, and what two neighbouring layers share -- the
+// values beside the interface, the value on it (the lower layer's upper bound is the same sum
+// with its two terms swapped) and the vertical flux through it -- is formed once and handed
+// down.  That and the node's quotients taken out of the loop halve the divisions (14 -> 7 per
+// layer in the T/S gather).  At 200 k nodes x 30 layers ADV_Q went 1187 -> 1086 us and ADV_TS
+// 1125 -> 1009 in FP64, 802 -> 682 and 805 -> 653 in FP32 (with k_he_adv's blocks).
 template <typename R>
-__global__ void __launch_bounds__(256) k_gather_q(const Dev P, int parts) {
+__global__ void __launch_bounds__(kGatherThreads, sizeof(R) == 4 ? 6 : 4) k_gather_q(const Dev P, int parts) {
   int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
   if (i > P.M) return;
   int kb, ke;
   col_range(P, 2, P.KBM1, kb, ke);
+  if (kb > ke) return;
   const bool wet = P.iswetn[i] * P.iswetnt[i] == 1;
-  const int nhe = P.node_he_ptr[i + 1] - P.node_he_ptr[i];
-  for (int k = kb; k <= ke; ++k) {
-  const double2 xs = gather_he<R>(P, i, nhe, k);
-  for (int t = 0; t < 2; ++t) {
-    if (!(parts & (t == 0 ? AD_Q2 : AD_Q2L))) continue;
-    const double* Q = (t == 0 ? P.q2 : P.q2l);
-    double* QF = (t == 0 ? P.q2f : P.q2lf);
-    if (k == 2) {
-      // QF = 0 on every level before the interior levels are set (adv_q.F:114)
-      QF[N3(P, i, 1)] = 0.0;
-      QF[N3(P, i, P.KB)] = 0.0;
+  const bool fct = (parts & AD_FCT) && !P.riv_skip[i];
+  const int nhe = P.node_he_ptr[i + 1] - P.node_he_ptr[i], KBM1 = P.KBM1;
+  const double art1 = P.art1[i], dt = P.dt[i], dr = dt / P.d[i];
+  const bool on[2] = {(parts & AD_Q2) != 0, (parts & AD_Q2L) != 0};
+  const double* Q[2] = {P.q2, P.q2l};
+  double* QF[2] = {P.q2f, P.q2lf};
+  // f, fp: Q on levels k and k+1; wf, wfm: WTS*Q on levels k and k-1; face: the bound between
+  // levels k-1 and k, which is level k-1's lower and level k's upper one
+  double f[2], wf[2], wfm[2], face[2] = {0.0, 0.0};
+  {
+    const size_t q = N3(P, i, kb), qm = N3(P, i, kb - 1);
+    const double w = P.wts[q], wm = P.wts[qm];
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+      if (!on[t]) continue;
+      const double fm = Q[t][qm];
+      f[t] = Q[t][q];
+      wfm[t] = wm * fm;
+      wf[t] = w * f[t];
+      if (fct && kb > 2) {
+        const double zm = P.dzz(i, kb - 1), zmm = P.dzz(i, kb - 2);
+        face[t] = (f[t] * zmm + fm * zm) / (zm + zmm);
+      }
     }
-    double x = t == 0 ? xs.x : xs.y;
-    size_t q = N3(P, i, k);
-    double qf;
-    if (wet) {
-      size_t qm = N3(P, i, k - 1), qp = N3(P, i, k + 1);
-      double temp = P.wts[qm] * Q[qm] - P.wts[qp] * Q[qp];
-      x = x + temp * P.art1[i] * P.dzz(i, k - 1) / (P.dz(i, k - 1) + P.dz(i, k));
-      qf = (Q[q] - x / P.art1[i] * (P.dti / (P.dt[i] * P.dzz(i, k - 1)))) * (P.dt[i] / P.d[i]);
-    } else {
-      qf = Q[q];
-    }
-    if ((parts & AD_FCT) && !P.riv_skip[i]) {
-      double qmin, qmax;
-      NodeRec<R>::minmax(P, 0, t, q, qmin, qmax);
-      fct_level_bounds(P, i, k, Q, qmax, qmin);
-      if (qmin - qf > 0.0) qf = qmin;
-      if (qf - qmax > 0.0) qf = qmax;
-    }
-    QF[q] = qf;
   }
+  for (int k = kb; k <= ke; ++k) {
+    const size_t q = N3(P, i, k), qp = N3(P, i, k + 1);
+    const double z = P.dzz(i, k), zm = P.dzz(i, k - 1), zl = P.dz(i, k - 1) + P.dz(i, k);
+    const double wp = P.wts[qp];
+    double fp[2], qmin[2], qmax[2];
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+      if (!on[t]) continue;
+      fp[t] = Q[t][qp];
+      if (fct) NodeRec<R>::minmax(P, 0, t, q, qmin[t], qmax[t]);
+    }
+    const double2 xs = gather_he<R>(P, i, nhe, k);
+    const double rt = P.dti / (dt * zm);
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+      if (!on[t]) continue;
+      if (k == 2) {
+        // QF = 0 on every level before the interior levels are set (adv_q.F:114)
+        QF[t][N3(P, i, 1)] = 0.0;
+        QF[t][N3(P, i, P.KB)] = 0.0;
+      }
+      double x = t == 0 ? xs.x : xs.y;
+      const double wfp = wp * fp[t];
+      double qf = f[t];
+      if (wet) {
+        const double temp = wfm[t] - wfp;
+        x = x + temp * art1 * zm / zl;
+        qf = (f[t] - x / art1 * rt) * dr;
+      }
+      if (fct) {
+        if (k > 2) {
+          qmax[t] = fmax(qmax[t], face[t]);
+          qmin[t] = fmin(qmin[t], face[t]);
+        }
+        if (k == 2 || k < KBM1) {
+          face[t] = (f[t] * z + fp[t] * zm) / (z + zm);
+          qmax[t] = fmax(qmax[t], face[t]);
+          qmin[t] = fmin(qmin[t], face[t]);
+        }
+        if (qmin[t] - qf > 0.0) qf = qmin[t];
+        if (qf - qmax[t] > 0.0) qf = qmax[t];
+      }
+      QF[t][q] = qf;
+      wfm[t] = wf[t];
+      wf[t] = wfp;
+      f[t] = fp[t];
+    }
   }
 }
 
@@ -866,56 +923,86 @@ __global__ void __launch_bounds__(256) k_turb_update(const Dev P) {
 // fct_s.F:50-108) on the same (node, layer) thread.
 // -------------------------------------------------------------------------------------
 template <typename R>
-__global__ void __launch_bounds__(256) k_gather_ts(const Dev P, int parts) {
+__global__ void __launch_bounds__(kGatherThreads, sizeof(R) == 4 ? 6 : 4) k_gather_ts(const Dev P, int parts) {
   int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
   if (i > P.M) return;
   int kb, ke;
   col_range(P, 1, P.KBM1, kb, ke);
+  if (kb > ke) return;
   const bool wet = P.iswetn[i] * P.iswetnt[i] == 1;
-  const int nhe = P.node_he_ptr[i + 1] - P.node_he_ptr[i];
-  for (int k = kb; k <= ke; ++k) {
-  const double2 xs = gather_he<R>(P, i, nhe, k);
-  for (int t = 0; t < 2; ++t) {
-    if (!(parts & (t == 0 ? AD_T : AD_S))) continue;
-    const double* F1 = (t == 0 ? P.t1 : P.s1);
-    double* FF1 = (t == 0 ? P.tf1 : P.sf1);
-    double x = t == 0 ? xs.x : xs.y;
-    size_t q = N3(P, i, k);
-    double ff;
-    if (wet) {
-      const double z = P.dz(i, k), zm = k > 1 ? P.dz(i, k - 1) : 0.0, zp = k < P.KBM1 ? P.dz(i, k + 1) : 0.0;
-      double temp;
-      if (k == 1) {
-        size_t qp = N3(P, i, k + 1);
-        temp = -P.wts[qp] * (F1[q] * zp + F1[qp] * z) / (z + zp);
-      } else if (k == P.KBM1) {
-        size_t qm = N3(P, i, k - 1);
-        temp = P.wts[q] * (F1[q] * zm + F1[qm] * z) / (z + zm);
-      } else {
-        size_t qm = N3(P, i, k - 1), qp = N3(P, i, k + 1);
-        temp = P.wts[q] * (F1[q] * zm + F1[qm] * z) / (z + zm) -
-               P.wts[qp] * (F1[q] * zp + F1[qp] * z) / (z + zp);
+  const bool fct = (parts & AD_FCT) && !P.riv_skip[i];
+  const bool open = P.isonb[i] == 2;
+  const int nhe = P.node_he_ptr[i + 1] - P.node_he_ptr[i], KBM1 = P.KBM1;
+  const double art1 = P.art1[i], dt = P.dt[i], dr = dt / P.dtfa[i];
+  const bool on[2] = {(parts & AD_T) != 0, (parts & AD_S) != 0};
+  const double* F1[2] = {P.t1, P.s1};
+  double* FF1[2] = {P.tf1, P.sf1};
+  // f, fp: the tracer on layers k and k+1; face, flux: the value on the interface between layers
+  // k-1 and k and the vertical flux through it, layer k-1's lower and layer k's upper ones
+  double f[2], face[2] = {0.0, 0.0}, flux[2] = {0.0, 0.0};
+  {
+    const size_t q = N3(P, i, kb);
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+      if (!on[t]) continue;
+      f[t] = F1[t][q];
+      if (kb > 1) {
+        const double z = P.dz(i, kb), zm = P.dz(i, kb - 1);
+        const double sum = f[t] * zm + F1[t][N3(P, i, kb - 1)] * z;
+        face[t] = sum / (z + zm);
+        flux[t] = P.wts[q] * sum / (z + zm);
       }
-      if (P.isonb[i] == 2)
-        x = temp * P.art1[i];
-      else
-        x = x + temp * P.art1[i];
-      ff = (F1[q] - x / P.art1[i] * (P.dti / (P.dt[i] * z))) * (P.dt[i] / P.dtfa[i]);
-    } else {
-      ff = F1[q];
     }
-    if (parts & AD_FCT) {
-      if (!P.riv_skip[i]) {
-        double fmn, fmx;
-        NodeRec<R>::minmax(P, 1, t, q, fmn, fmx);
-        fct_layer_bounds(P, i, k, F1, fmx, fmn);
-        if (fmn - ff > 0.0) ff = fmn;
-        if (ff - fmx > 0.0) ff = fmx;
-      }
-      if (t == 1 && ff < 0.0) ff = 0.0;
-    }
-    FF1[q] = ff;
   }
+  for (int k = kb; k <= ke; ++k) {
+    const size_t q = N3(P, i, k), qp = N3(P, i, k + 1);
+    const double z = P.dz(i, k), zp = k < KBM1 ? P.dz(i, k + 1) : 0.0;
+    const bool lower = k == 1 || k < KBM1;
+    const double wp = lower ? P.wts[qp] : 0.0;
+    double fp[2], fmn[2], fmx[2];
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+      if (!on[t]) continue;
+      fp[t] = lower ? F1[t][qp] : 0.0;
+      if (fct) NodeRec<R>::minmax(P, 1, t, q, fmn[t], fmx[t]);
+    }
+    const double2 xs = gather_he<R>(P, i, nhe, k);
+    const double rt = P.dti / (dt * z);
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+      if (!on[t]) continue;
+      double x = t == 0 ? xs.x : xs.y;
+      const double up = flux[t], fa = face[t];
+      if (lower) {
+        const double sum = f[t] * zp + fp[t] * z;
+        face[t] = sum / (z + zp);
+        flux[t] = wp * sum / (z + zp);
+      }
+      double ff = f[t];
+      if (wet) {
+        const double temp = k == 1 ? -flux[t] : (lower ? up - flux[t] : up);
+        if (open)
+          x = temp * art1;
+        else
+          x = x + temp * art1;
+        ff = (f[t] - x / art1 * rt) * dr;
+      }
+      if (fct) {
+        if (k > 1) {
+          fmx[t] = fmax(fmx[t], fa);
+          fmn[t] = fmin(fmn[t], fa);
+        }
+        if (lower) {
+          fmx[t] = fmax(fmx[t], face[t]);
+          fmn[t] = fmin(fmn[t], face[t]);
+        }
+        if (fmn[t] - ff > 0.0) ff = fmn[t];
+        if (ff - fmx[t] > 0.0) ff = fmx[t];
+      }
+      if ((parts & AD_FCT) && t == 1 && ff < 0.0) ff = 0.0;
+      FF1[t][q] = ff;
+      f[t] = fp[t];
+    }
   }
 }
 
@@ -1239,7 +1326,10 @@ void launch_grad(const Dev& P, cudaStream_t s, int which) {
 void launch_adv_q(const Dev& P, cudaStream_t s, int parts) {
   FVG_F32_FORWARD(launch_adv_q(P, s, parts));
   const int nl = P.KBM1 - 1;
-  const Dev Q = col_shape(P, P.N, nl), G = col_shape(P, P.M, nl);
+  Dev Q = col_shape(P, P.N, nl);
+  if (Q.col_bc > kHeThreads) Q.col_bc = kHeThreads;
+  Dev G = col_shape(P, P.M, nl);
+  if (G.col_bc > kGatherThreads) G.col_bc = kGatherThreads;
   k_he_adv<RF, 0><<<col_grid(Q, P.N, nl), Q.col_bc, 0, s>>>(Q, parts);
   k_gather_q<RF><<<col_grid(G, P.M, nl), G.col_bc, 0, s>>>(G, parts);
 }
@@ -1267,7 +1357,10 @@ void launch_turb_update(const Dev& P, cudaStream_t s) {
 }
 void launch_adv_ts(const Dev& P, cudaStream_t s, int parts) {
   FVG_F32_FORWARD(launch_adv_ts(P, s, parts));
-  const Dev Q = col_shape(P, P.N, P.KBM1), G = col_shape(P, P.M, P.KBM1);
+  Dev Q = col_shape(P, P.N, P.KBM1);
+  if (Q.col_bc > kHeThreads) Q.col_bc = kHeThreads;
+  Dev G = col_shape(P, P.M, P.KBM1);
+  if (G.col_bc > kGatherThreads) G.col_bc = kGatherThreads;
   k_he_adv<RF, 1><<<col_grid(Q, P.N, P.KBM1), Q.col_bc, 0, s>>>(Q, parts);
   if (P.iobcn > 0) k_obc_xflux<RF><<<dim3(nblk(P.iobcn, 64), P.KBM1, 2), 64, 0, s>>>(P, parts);
   k_gather_ts<RF><<<col_grid(G, P.M, P.KBM1), G.col_bc, 0, s>>>(G, parts);
