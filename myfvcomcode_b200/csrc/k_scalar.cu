@@ -694,24 +694,35 @@ __global__ void __launch_bounds__(256, 4) k_vdif_q_levels(const Dev P) {
   double ukm1 = 0.0, vkm1 = 0.0;
   if (wet && kb <= KBM1) ring_mean(kb >= 2 ? kb - 1 : 1, ukm1, vkm1);
   bool chunk_inside = wet;  // every interior level of this chunk inside the closure's envelope
+  double rhom = kb >= 2 ? P.rho1[n3(kb - 1)] : 0.0;  // RHO1 above the level
   for (int k = kb; k <= ke; ++k) {
     const size_t q = n3(k);
+    const bool inner = k >= 2 && k <= KBM1;
+    // the level's loads stand before its first store, which none of them could pass otherwise
+    // (200 k nodes x 30 layers: VDIF_Q 839 -> 800 us)
+    const double rho = P.rho1[q], q20 = Q2[q], q2l0 = Q2L[q];
+    double q2f = 1.0, q2lf = 1.0, km = 0.0, kh = 0.0, uk = 0.0, vk = 0.0;
+    if (inner) {
+      q2f = P.q2f[q];
+      q2lf = P.q2lf[q];
+      km = P.km[q];
+      kh = P.kh[q];
+      if (wet) ring_mean(k, uk, vk);
+    }
     // positivity of the previous Q2F/Q2LF (vdif_q.F:144-149)
-    if (k >= 2 && k <= KBM1 && (P.q2f[q] <= SMALL || P.q2lf[q] <= SMALL)) {
+    if (inner && (q2f <= SMALL || q2lf <= SMALL)) {
       P.q2f[q] = SMALL;
       P.q2lf[q] = SMALL;
     }
-    const double q2 = fabs(Q2[q] + SMALL);
-    double q2l = fabs(Q2L[q]);
+    const double q2 = fabs(q20 + SMALL);
+    double q2l = fabs(q2l0);
     Q2[q] = q2;
     double boygr = 0.0, prod = 0.0, lk;
     if (k >= 2 && k <= KBM1) {
       if (wet) {
-        boygr = P.grav_n[i] * (P.rho1[n3(k - 1)] - P.rho1[q]) / (P.dzz(i, k - 1) * d);
-        // the reference's internal-wave term carries a weight of zero and is not evaluated
-        double uk, vk;
-        ring_mean(k, uk, vk);
         const double den = P.dzz(i, k - 1) * d;
+        boygr = P.grav_n[i] * (rhom - rho) / den;
+        // the reference's internal-wave term carries a weight of zero and is not evaluated
         const double shear2 = ((uk - ukm1) * (uk - ukm1) + (vk - vkm1) * (vk - vkm1)) / (den * den);
         if (AUX & 1) {
           // the network's inputs: inside the envelope or not, then transformed,
@@ -739,8 +750,8 @@ __global__ void __launch_bounds__(256, 4) k_vdif_q_levels(const Dev P) {
           samp(6, k, q2);
           samp(7, k, q2l);
         }
-        prod = P.km[q] * SEF * ((uk - ukm1) * (uk - ukm1) + (vk - vkm1) * (vk - vkm1)) / (den * den);
-        prod = prod + P.kh[q] * boygr;
+        prod = km * SEF * ((uk - ukm1) * (uk - ukm1) + (vk - vkm1) * (vk - vkm1)) / (den * den);
+        prod = prod + kh * boygr;
         ukm1 = uk;
         vkm1 = vk;
       }
@@ -767,6 +778,7 @@ __global__ void __launch_bounds__(256, 4) k_vdif_q_levels(const Dev P) {
     P.vq_gh[q] = gh;
     P.vq_stf[q] = stf;
     P.vq_dtef[q] = dtef;
+    rhom = rho;
     if (wet && k >= 2 && k <= KBM1) {
       const double x = (1. / fabs(P.z(i, k) - P.z(i, 1)) + 1. / fabs(P.z(i, k) - P.z(i, KB))) * lk / (d * KAPPA);
       P.vq_dtefl[q] = dtef * (1. + E2 * (x * x));
@@ -1241,9 +1253,10 @@ __device__ inline double dens2(double S, double T) {
 // -------------------------------------------------------------------------------------
 // End of the internal step: T1=TF1, S1=SF1, N2E3D to T/S, DENS2 with N2E3D(RHO1,RHO),
 // N2E3D(KM,KM1), U=UF, V=VF, ET=EL, DT=D, ET1=EL1, DT1=D1, WD_UPDATE(3)
-// (internal_step.F:1053-1590).  Threads over (max(M,N)+1) x KB.
+// (internal_step.F:1053-1590).  Threads over (max(M,N)+1) x KB, or over the nodes alone
+// (cells = 0) where k_final_cells follows.
 // -------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) k_final(const Dev P, int parts) {
+__global__ void __launch_bounds__(256) k_final(const Dev P, int parts, int cells) {
   int i = blockIdx.x * 32 + threadIdx.x;
   int k = blockIdx.y * 8 + threadIdx.y + 1;
   if (k > P.KB) return;
@@ -1260,7 +1273,7 @@ __global__ void __launch_bounds__(256) k_final(const Dev P, int parts) {
       if (P.wetting_drying_on) P.iswetnt[i] = P.iswetn[i];
     }
   }
-  if (i >= 1 && i <= P.N) {
+  if (cells && i >= 1 && i <= P.N) {
     const size_t n1 = P.N + 1;
     int a = P.nv[i], b = P.nv[n1 + i], c = P.nv[2 * n1 + i];
     size_t qa = N3(P, a, k), qb = N3(P, b, k), qc = N3(P, c, k);
@@ -1283,6 +1296,62 @@ __global__ void __launch_bounds__(256) k_final(const Dev P, int parts) {
         if (P.wetting_drying_on) P.iswetct[i] = P.iswetc[i];
       }
     }
+  }
+}
+
+// The cells' part of k_final alone, after k_final has written RHO1: one thread per cell walks a
+// chunk of levels, the inputs of kFinBat levels loaded before they are stored.  In one kernel
+// a cell cannot read RHO1 that another block writes and evaluates the density of its three
+// nodes itself, seven evaluations per node instead of one, which bound it (98 us at 50 k nodes x 30
+// layers for about 270 MB, 41 us at the copy rate).  kFinSplit: from this many cells x levels
+// on the second launch pays.  One kernel and two: 4 k cells x 11 levels 10.2 and 11.6 us, 12 k x 24
+// 16.8 and 19.4, 39 k x 20 33.0 and 27.7, 99 k x 31 98 and 77, 396 k x 31 398 and 279.
+constexpr int kFinBat = 2;
+constexpr long kFinSplit = 500000;
+__global__ void __launch_bounds__(128) k_final_cells(const Dev P, int parts) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
+  if (i > P.N) return;
+  int kb, ke;
+  col_range(P, 1, P.KB, kb, ke);
+  const size_t n1 = P.N + 1;
+  const int nd[3] = {P.nv[i], P.nv[n1 + i], P.nv[2 * n1 + i]};
+  const bool ft = parts & FI_T, fs = parts & FI_S, fd = parts & FI_DENS, fk = parts & FI_KM1, fu = parts & FI_SHIFT;
+  for (int k0 = kb; k0 <= ke; k0 += kFinBat) {
+    double t[kFinBat][3], s[kFinBat][3], r[kFinBat][3], m[kFinBat][3], u[kFinBat], v[kFinBat];
+#pragma unroll
+    for (int b = 0; b < kFinBat; ++b) {
+      const int k = k0 + b <= ke ? k0 + b : ke;
+#pragma unroll
+      for (int j = 0; j < 3; ++j) {
+        const size_t q = N3(P, nd[j], k);
+        if (ft) t[b][j] = P.tf1[q];
+        if (fs) s[b][j] = P.sf1[q];
+        if (fd) r[b][j] = P.rho1[q];
+        if (fk) m[b][j] = P.km[q];
+      }
+      if (fu) {
+        u[b] = P.uf[C3(P, i, k)];
+        v[b] = P.vf[C3(P, i, k)];
+      }
+    }
+#pragma unroll
+    for (int b = 0; b < kFinBat; ++b) {
+      if (k0 + b > ke) break;
+      const size_t q = C3(P, i, k0 + b);
+      if (ft) P.t[q] = ONE_THIRD * (t[b][0] + t[b][1] + t[b][2]);
+      if (fs) P.s[q] = ONE_THIRD * (s[b][0] + s[b][1] + s[b][2]);
+      if (fd) P.rho[q] = ONE_THIRD * (r[b][0] + r[b][1] + r[b][2]);
+      if (fk) P.km1[q] = ONE_THIRD * (m[b][0] + m[b][1] + m[b][2]);
+      if (fu) {
+        P.u[q] = u[b];
+        P.v[q] = v[b];
+      }
+    }
+  }
+  if (fu && kb == 1) {
+    P.et1[i] = P.el1[i];
+    P.dt1[i] = P.d1[i];
+    if (P.wetting_drying_on) P.iswetct[i] = P.iswetc[i];
   }
 }
 
@@ -1381,9 +1450,14 @@ void launch_bcond_ts(const Dev& P, cudaStream_t s, int parts) {
   if (P.iobcn > 0) k_bcond_ts_obc<<<dim3(P.iobcn, 2), 64, 0, s>>>(P, parts);
 }
 void launch_final(const Dev& P, cudaStream_t s, int parts) {
-  int n = (P.M > P.N ? P.M : P.N) + 1;
+  const bool split = (long)P.N * P.KB >= kFinSplit;
+  const int n = (split ? P.M : P.M > P.N ? P.M : P.N) + 1;
   dim3 b(32, 8), g(nblk(n, 32), nblk(P.KB, 8));
-  k_final<<<g, b, 0, s>>>(P, parts);
+  k_final<<<g, b, 0, s>>>(P, parts, split ? 0 : 1);
+  if (!split) return;
+  Dev Q = col_shape(P, P.N, P.KB);
+  if (Q.col_bc > 128) Q.col_bc = 128;
+  k_final_cells<<<col_grid(Q, P.N, P.KB), Q.col_bc, 0, s>>>(Q, parts);
 }
 void launch_budget(const Dev& P, cudaStream_t s) {
   const int nb = 148;
