@@ -321,8 +321,8 @@ int fvg_closure_status(fvg_handle* h, int32_t* columns_on_network, int32_t* wait
                    Runge-Kutta start values) evict-first in L2, so that the arrays they
                    gather from neighbours stay in L2 from one stage to the next; 0 plain
                    loads.  A cache hint only: results do not depend on it (bit for bit);
-   "ext_grid"     = blocks per SM (1..8, default 8) of the external loop's compact cell
-                   kernel, launched as one wave whose threads walk the cells so that no
+   "ext_grid"     = blocks per SM (1..8, default 8) of the external loop's stage cell
+                   kernel at most, launched as one wave whose threads walk the cells so that no
                    partly filled last wave is left; 0 launches one thread per cell.
                    Results do not depend on it;
    "ext_loop"     = 1 (default): the external loop of a mesh of at most 384 cells per SM runs

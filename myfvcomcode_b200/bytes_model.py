@@ -31,9 +31,8 @@ def ledger(grid, isplit, wet_dry, precision="fp64", compact=False):
     control-volume metrics read by the flux kernels.  FP64 state is counted at 8 bytes
     in both forms (ADVX/ADVY, UF/VF/VISCOFM and DZ1 among them).
 
-    ``compact`` (precision form only): the Runge-Kutta stages' cell kernel is the compact
-    one, whose records replace the slot table's metrics and EXTUV's fixed inputs (see
-    ``ext_cell_compact``).
+    ``compact``: the Runge-Kutta stages run on the packed records (``ext_stage``); one launch
+    of group ext_cell is then one stage, its node and its cell kernel, wet judgement included.
     """
     s = sizes(grid)
     M, N, NE, NCV, K, KB = s["M"], s["N"], s["NE"], s["NCV"], s["K"], s["KB"]
@@ -62,11 +61,13 @@ def ledger(grid, isplit, wet_dry, precision="fp64", compact=False):
     g["ext_node"] = (M * (I + I + 3 * D) + halfedge_csr + NCV * (I + 2 * D) + N * 3 * D + M * 5 * D + wet_node, st)
     g["ext_cell"] = (N * (cell_lsq // N + 22 * D + 4 * X + 6 * I) + N * 8 * D + edge_geo + pg_extra
                      + M * 4 * D + N * (6 * D + 3 * I), st)
-    if compact and precision == "fp32flux":
-        g["ext_cell"] = (ext_cell_compact(N, M, isplit), st)
     g["ext_update"] = (M * (6 * D + I) + N * (10 * D + (2 * I if wet_dry else 0)), 1)
     if wet_dry:
         g["wet_judge"] = (N * (3 * I + I + D) + M * D, st)
+    if compact:
+        g["ext_cell"] = (ext_stage(N, M, NCV, X, isplit, wet_dry), st)
+        g.pop("ext_node")
+        g.pop("wet_judge", None)
     # ---- 3-D, once per internal step ----
     g["cell_pre"] = (N * K * 4 * D + N * K * D + N * 12 * D, 1)              # U,V rw; DZ1; 2-D
     # U, V read and ADVX, ADVY written per cell and layer (FP64 in both forms)
@@ -98,20 +99,26 @@ def ledger(grid, isplit, wet_dry, precision="fp64", compact=False):
     return g
 
 
-def ext_cell_compact(N, M, isplit):
-    """Bytes of one launch of the compact stage kernel, averaged over the 4*ISPLIT stages.
+def ext_stage(N, M, NCV, X, isplit, wet_dry):
+    """Bytes of one stage on the packed records, averaged over the 4*ISPLIT stages.
 
-    Per cell: the flag word, UA, VA, the two wet flags, D1, the packed FP32 gradient
-    {UX, UY, VX, VY}, {ART, CC_HVC} in FP32, {XC, YC}, three 16-byte slots, the two
-    32-byte records of EXTUV's terms, UARK, VARK, ELRK1, ELF1 read; UAF, VAF, EL1, D1
-    and the three half-edge continuity fluxes written.  Per node: {VX, VY}, D, EL read.
-    The first stage of each external step also reads EL1 and writes UARK, VARK, ELRK1
-    (instead of reading them); the last stage writes ADVUA, ADVVA, PSTX, PSTY.
+    Node kernel, per node: open-boundary slot, list pointer, H, ART1, ELF, ELRK read, ELF and
+    {EL, D} written, its list and the half-edge continuity fluxes; per cell: NBE, A1U/A2U,
+    ART, CC_HVC, {UA, VA} read, the gradient and ART*|grad|*CC_HVC written.
+    Cell kernel, per cell: the two 16-byte topology records, {UA, VA}, the gradient and its
+    viscosity part, {XC, YC}, D1, UARK/VARK, ELRK1, EXTUV's fixed terms (64 bytes in FP32,
+    96 in FP64) read, {UA, VA}, D1 and three half-edge fluxes written; per node {VX, VY},
+    {EL, D}, ELF.  With wetting and drying the flag read and written, the cell's smallest H
+    and the node's H.  The third stage also updates UARD, VARD; the fourth EGF; the first
+    writes the start values that the others read; the last writes ADVUA, ADVVA, PSTX, PSTY.
     """
-    per_cell = I + 2 * D + 2 * I + D + 16 + 8 + 16 + 3 * 16 + 2 * 32 + 4 * D + 4 * D + 3 * D
-    st = 4 * isplit
-    extra = (isplit * D + 4 * D) / st
-    return int(N * (per_cell + extra) + M * (16 + 2 * D))
+    fixed = 64 if X == 4 else 96
+    node = M * (2 * I + 4 * D + D + 2 * D) + 2 * NCV * I + NCV * D + N * (3 * I + 10 * X + 2 * D + 5 * X)
+    cell = N * (32 + 2 * D + 5 * X + 2 * D + D + 2 * D + D + fixed + 2 * D + D + 3 * D) + M * (2 * D + 2 * D + D)
+    if wet_dry:
+        cell += N * (2 * I + D) + M * D
+    extra = (isplit * (N * (4 * D + D) + M * 3 * D) + N * 4 * D) / (4 * isplit)
+    return int(node + cell + extra)
 
 
 def step_bytes(grid, isplit, wet_dry, precision="fp64", compact=False):

@@ -3,6 +3,8 @@
 //   k_wet_*      WET_JUDGE                                      (wetting/drying only)
 //   k_ext_cell   N2E2D + FLUX_OBN + ADVAVE_EDGE_GCN + EXTUV_EDGE + BCOND_GCN(2,K)  (per cell)
 //   k_ext_update external_step.F:333-436 (EL=ELF, D, D1, UA=UAF, UARD/EGF sums)
+// and, on meshes whose metrics are the ones their coordinates define, the same on packed records:
+//   k_stage_node, k_stage_cell (one stage), k_ext_loop (every stage of an internal step)
 // Reference: FVCOM_source/external_step.F:30-443 and the routines cited per kernel.
 // Arithmetic is kept in the reference's expression order; the library is compiled with
 // --fmad=false so no multiply-add is contracted.
