@@ -57,6 +57,7 @@ struct fvg_handle {
   int* h_ctl = nullptr;       // pinned
   cudaGraphExec_t gexec = nullptr;
   cudaGraph_t graph = nullptr;
+  unsigned version = 0;  // counts the changes that make a captured step stale (regraph)
   bool use_graph = true;
   int clos_grid = 148;
   // external stages on the packed records: allowed (tuning key "compact") and possible (the
@@ -88,6 +89,14 @@ struct fvg_handle {
   } while (0)
 
 namespace {
+
+// The captured step no longer holds what a step launches: it is captured again on the next one,
+// and so is the graph of a group that the model belongs to (fvg_handle::version).
+void regraph(fvg_handle* h) {
+  ++h->version;
+  if (h->gexec) { cudaGraphExecDestroy(h->gexec); h->gexec = nullptr; }
+  if (h->graph) { cudaGraphDestroy(h->graph); h->graph = nullptr; }
+}
 
 template <class T>
 int dalloc(fvg_handle* h, T** p, size_t n) {
@@ -1404,8 +1413,7 @@ int fvg_set_precision(fvg_handle* h, int32_t mode) {
   set_xform(h);
   // The captured step holds the other precision's kernels: capture again.
   CK(cudaStreamSynchronize(h->stream));
-  if (h->gexec) { cudaGraphExecDestroy(h->gexec); h->gexec = nullptr; }
-  if (h->graph) { cudaGraphDestroy(h->graph); h->graph = nullptr; }
+  regraph(h);
   return FVG_OK;
 }
 
@@ -1416,11 +1424,7 @@ int fvg_set_closure(fvg_handle* h, int32_t mode, const float* params, int32_t np
   if (!h) return FVG_ERR_ARG;
   Dev& P = h->P;
   CK(cudaStreamSynchronize(h->stream));
-  auto regraph = [&]() {
-    if (h->gexec) { cudaGraphExecDestroy(h->gexec); h->gexec = nullptr; }
-    if (h->graph) { cudaGraphDestroy(h->graph); h->graph = nullptr; }
-  };
-  if (mode == 0) { P.closure = 0; regraph(); return FVG_OK; }
+  if (mode == 0) { P.closure = 0; regraph(h); return FVG_OK; }
   if (mode != 1 || !params || nparams != fvg_mlp_num_params() || !norm || nnorm != FVG_CLOSURE_NORM_FLOATS) {
     h->err = "fvg_set_closure: bad mode, parameter or scaling vector";
     return FVG_ERR_ARG;
@@ -1470,7 +1474,7 @@ int fvg_set_closure(fvg_handle* h, int32_t mode, const float* params, int32_t np
   nm.teps = norm[54];
   P.clos_norm = nm;
   P.closure = 1;
-  regraph();
+  regraph(h);
   return FVG_OK;
 }
 
@@ -1501,8 +1505,7 @@ int fvg_closure_sample(fvg_handle* h, float* dev_buf, int64_t cap) {
   CK(cudaStreamSynchronize(h->stream));
   if (dev_buf != h->P.clos_samp) {
     h->P.clos_samp = dev_buf;
-    if (h->gexec) { cudaGraphExecDestroy(h->gexec); h->gexec = nullptr; }
-    if (h->graph) { cudaGraphDestroy(h->graph); h->graph = nullptr; }
+    regraph(h);
   }
   return FVG_OK;
 }
@@ -1539,8 +1542,7 @@ int fvg_set_tuning(fvg_handle* h, const char* key, int32_t value) {
   }
   // The captured step holds the old launch shapes: capture again on the next step.
   CK(cudaStreamSynchronize(h->stream));
-  if (h->gexec) { cudaGraphExecDestroy(h->gexec); h->gexec = nullptr; }
-  if (h->graph) { cudaGraphDestroy(h->graph); h->graph = nullptr; }
+  regraph(h);
   return FVG_OK;
 }
 
@@ -1710,6 +1712,7 @@ struct fvg_group {
   cudaStream_t stream = nullptr;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t gexec = nullptr;
+  std::vector<unsigned> version;  // fvg_handle::version of each model at the capture
   std::vector<cudaEvent_t> ev;  // fork event, one join event per model, one per resident loop
   std::string err;
 };
@@ -1734,6 +1737,10 @@ static void group_free(fvg_group* g) {
   } while (0)
 
 static int group_capture(fvg_group* g) {
+  if (g->gexec) { cudaGraphExecDestroy(g->gexec); g->gexec = nullptr; }
+  if (g->graph) { cudaGraphDestroy(g->graph); g->graph = nullptr; }
+  g->version.clear();
+  for (const fvg_handle* h : g->hs) g->version.push_back(h->version);
   GK(cudaStreamBeginCapture(g->stream, cudaStreamCaptureModeThreadLocal));
   GK(cudaEventRecord(g->ev[0], g->stream));
   cudaEvent_t after = nullptr;
@@ -1772,7 +1779,9 @@ static int group_steps(fvg_group* g, int32_t nsteps, double* ms) {
       if (rc) { g->err = h->err; return rc; }
       GK(cudaStreamSynchronize(h->stream));
     }
-    if (!g->gexec) {
+    bool stale = !g->gexec;
+    for (size_t q = 0; q < g->hs.size() && !stale; ++q) stale = g->version[q] != g->hs[q]->version;
+    if (stale) {
       int rc = group_capture(g);
       if (rc) return rc;
     }
