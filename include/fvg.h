@@ -218,7 +218,9 @@ int fvg_get_ifield(fvg_handle* h, const char* name, int32_t* dst, int64_t count)
 /* Element count of a field, or -1 for an unknown name. */
 int64_t fvg_field_size(const fvg_handle* h, const char* name);
 
-/* Model clock: IINT of the last completed internal step and ExtTime in seconds. */
+/* Model clock: IINT of the last completed internal step and ExtTime in seconds.  After a step
+   that returned FVG_ERR_TIMEOUT for the external loop (see fvg_run) the state counts as set
+   again with this call. */
 int fvg_set_clock(fvg_handle* h, int32_t iint, double ext_time);
 int fvg_get_clock(const fvg_handle* h, int32_t* iint, double* ext_time);
 
@@ -232,7 +234,12 @@ int fvg_external_step(fvg_handle* h, int32_t iext);
    mod_force.F:14341, :11229, :13415): tidal constituents (same NTIDE as at creation),
    river discharge/T/S and surface stress; NULL members are left unchanged. */
 int fvg_set_forcing(fvg_handle* h, const fvg_forcing* f);
-/* n consecutive internal steps; replayed from a captured CUDA graph after the first. */
+/* n consecutive internal steps; replayed from a captured CUDA graph after the first.
+   FVG_ERR_TIMEOUT: a bounded device wait ran out, of the learned closure (see
+   fvg_closure_status) or of the external loop ("ext_loop_polls" of fvg_set_tuning).  After the
+   latter the clock has advanced by the steps that were queued, the state is that of a half-done
+   stage, and every later step of the handle is refused with the same status until the state's
+   fields have been set again and fvg_set_clock has been called. */
 int fvg_run(fvg_handle* h, int32_t nsteps);
 /* One reference routine (enum fvg_routine) on the current state, for parity checks. */
 int fvg_run_routine(fvg_handle* h, int32_t routine, int32_t arg);
@@ -329,6 +336,9 @@ int fvg_closure_status(fvg_handle* h, int32_t* columns_on_network, int32_t* wait
                    as one resident cooperative kernel (with "compact" in use or possible);
                    0 launches every stage.  FP64 results do
                    not depend on it; fvg_get_tuning reports whether it is in use;
+   "ext_loop_polls" = most polls of a grid barrier of that kernel (default 4194304, about
+                   two seconds; 0: no wait at all); a barrier that takes more ends the
+                   call with FVG_ERR_TIMEOUT (see fvg_run);
    "branches"     = 1 (default): up to 20 million cell-layers the independent parts of a step
                    (BAROPG beside ADVECTION; momentum, turbulence and tracers after VERTVL)
                    run beside one another on streams of the handle; 0 one after another.

@@ -27,6 +27,11 @@ namespace {
 // FP32), which a large ensemble would rather hold members in.
 constexpr long kBranchCells = 20000000;
 
+// Most polls of a grid barrier of the resident external loop (about two seconds).  A phase
+// takes microseconds; what the wait has to outlast is a block that starts late behind the
+// kernels of other models on the card.
+constexpr int kLoopPolls = 1 << 22;
+
 const double kPI2 = 2.0 * 3.141592653589793238;
 
 struct FieldDesc {
@@ -1057,6 +1062,7 @@ int fvg_create(const fvg_mesh* m, const fvg_params* prm, const fvg_forcing* f, f
     if ((rc = dalloc(h, &ctl, 4))) return fail(rc);
     P.ctl = ctl;
     if ((rc = dalloc(h, &P.bar, 32))) return fail(rc);
+    P.bar_polls = kLoopPolls;
     P.bar_err = h->h_ctl + 1;  // pinned memory, written by the device only on an error
     *P.bar_err = 0;
   }
@@ -1130,6 +1136,12 @@ int fvg_get_ifield(fvg_handle* h, const char* name, int32_t* dst, int64_t count)
 
 int fvg_set_clock(fvg_handle* h, int32_t iint, double ext_time) {
   if (!h) return FVG_ERR_ARG;
+  if (h->h_ctl[1] != 0) {  // the state has been set again after a wait that ran out
+    CK(cudaStreamSynchronize(h->stream));
+    CK(cudaMemsetAsync(h->P.bar, 0, sizeof(unsigned), h->stream));
+    CK(cudaStreamSynchronize(h->stream));
+    h->h_ctl[1] = 0;
+  }
   h->iint = iint;
   h->ext_time = ext_time;
   return FVG_OK;
@@ -1175,12 +1187,12 @@ static void finish_chunk(fvg_handle* h, int c) {
   h->ramp = h->prm.iramp != 0 ? std::tanh((double)h->iint / (double)h->prm.iramp) : 1.0;
 }
 
-// A grid barrier of the resident external loop whose bounded wait ran out, read once the
-// steps have run.
+// A grid barrier of the resident external loop whose bounded wait ran out, read while the
+// stream is idle.  The state is then that of a half-done stage: no step runs on it until it has
+// been set again and fvg_set_clock clears the word.
 static int loop_check(fvg_handle* h) {
-  if (!h->h_ctl || h->h_ctl[1] == 0) return FVG_OK;
-  h->h_ctl[1] = 0;
-  h->err = "external loop: a bounded wait of its grid barrier ran out";
+  if (h->h_ctl[1] == 0) return FVG_OK;
+  h->err = "external loop: a bounded wait of its grid barrier ran out; set the state and the clock again";
   return FVG_ERR_TIMEOUT;
 }
 
@@ -1208,6 +1220,7 @@ static int run_steps(fvg_handle* h, int32_t nsteps, int mode, double* group_ms, 
   while (done < nsteps) {
     int c = std::min(h->sched_cap, nsteps - done);
     CK(cudaStreamSynchronize(h->stream));
+    { int rc = loop_check(h); if (rc) return rc; }
     { int rc = prep_chunk(h, c); if (rc) return rc; }
     if (total_ms) CK(cudaEventRecord(t0, h->stream));
     std::vector<cudaEvent_t> ev;
@@ -1534,6 +1547,9 @@ int fvg_set_tuning(fvg_handle* h, const char* key, int32_t value) {
     h->P.ext_grid = value;
   } else if (k == "ext_loop") {
     h->ext_loop = value != 0;
+  } else if (k == "ext_loop_polls") {
+    if (value < 0) { h->err = "ext_loop_polls must not be negative"; return FVG_ERR_ARG; }
+    h->P.bar_polls = value;
   } else if (k == "branches") {
     h->branches = value != 0;
   } else {
@@ -1556,6 +1572,7 @@ int fvg_get_tuning(const fvg_handle* h, const char* key, int32_t* value) {
   else if (k == "stream_hints") *value = h->P.ldcs;
   else if (k == "ext_grid") *value = h->P.ext_grid;
   else if (k == "ext_loop") *value = use_ext_loop(h);
+  else if (k == "ext_loop_polls") *value = h->P.bar_polls;
   else if (k == "branches") *value = use_branches(h);
   else return FVG_ERR_ARG;
   return FVG_OK;
@@ -1774,6 +1791,10 @@ static int group_steps(fvg_group* g, int32_t nsteps, double* ms) {
     const int c = std::min(cap, nsteps - done);
     GK(cudaStreamSynchronize(g->stream));
     for (fvg_handle* h : g->hs) {
+      int rc = loop_check(h);
+      if (rc) { g->err = h->err; return rc; }
+    }
+    for (fvg_handle* h : g->hs) {
       GK(cudaStreamSynchronize(h->stream));
       int rc = prep_chunk(h, c);
       if (rc) { g->err = h->err; return rc; }
@@ -1795,10 +1816,10 @@ static int group_steps(fvg_group* g, int32_t nsteps, double* ms) {
       total += f;
     }
     GK(cudaStreamSynchronize(g->stream));
+    for (fvg_handle* h : g->hs) finish_chunk(h, c);  // every model's steps have run
     for (fvg_handle* h : g->hs) {
       int rc = loop_check(h);
       if (rc) { g->err = h->err; return rc; }
-      finish_chunk(h, c);
     }
     done += c;
   }

@@ -91,6 +91,9 @@ constexpr int kTileCells = 128;
 // Largest block of the resident external loop (one block per SM, a cell and a node per
 // thread).
 constexpr int kLoopThreads = 384;
+// Top bit of the loop's barrier counter: a wait ran out (the count stays far below it, three
+// barriers a stage and one arrival per block).
+constexpr unsigned kBarStopped = 0x80000000u;
 struct Tiles {
   int n, cap_cells, cap_edges;
   const int *ptr, *nc, *eptr, *cells;
@@ -223,8 +226,9 @@ struct Dev {
   // planes of N+1 pairs (store_fixed); xrk the pairs UARK, VARK.  Exchanged between cells and
   // nodes of a stage: xuv {UA, VA} and xw (ISWETC), each in two buffers of N+1; xg the FP64
   // gradients (four per cell), xvc ART*|grad|*CC_HVC in the form's type, xnd {EL, D} per node.
-  // bar: the resident loop's grid barrier; bar_err (pinned host memory), set when a wait ran
-  // out.  loop_cells, loop_nodes: its cells and nodes per block.
+  // bar: the resident loop's grid barrier, whose waits take at most bar_polls polls (tuning key
+  // "ext_loop_polls"); bar_err (pinned host memory), set when a wait ran out.  loop_cells,
+  // loop_nodes: its cells and nodes per block.
   int xform;
   const double2 *vxy, *xyc;
   double2 *exd, *xrk;
@@ -236,6 +240,7 @@ struct Dev {
   const int* wfar;
   const double* hmin;
   unsigned* bar;
+  int bar_polls;
   int* bar_err;
   // open boundary
   double *xflux_obcn, *uard_obcn, *xflux_obc_t, *xflux_obc_s;

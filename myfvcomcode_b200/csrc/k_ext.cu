@@ -1361,21 +1361,21 @@ __global__ void __launch_bounds__(128) k_stage_alfa(const Dev P, int st) {
 }
 
 // Barrier over the grid: every block adds one to the counter (zeroed by k_begin_step) and
-// waits until all have.  The wait is bounded; a block whose wait runs out reports it and
-// leaves, and so do the others in their turn.
-constexpr long kBarSpin = 1L << 22;
+// waits until all have, for at most bar_polls polls.  A block whose wait runs out reports it,
+// sets the counter's top bit and leaves; the others leave at that bit, and so do the loops of
+// the steps already queued behind (k_begin_step keeps it), whose state is that of a half-done
+// stage.
 __device__ __forceinline__ bool grid_barrier(const Dev& P, unsigned target) {
   __syncthreads();
   int ok = 1;
   if (threadIdx.x == 0) {
     asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(P.bar) : "memory");
     unsigned seen = 0;
-    long it = 0;
-    do {
+    for (int it = 0; it < P.bar_polls && seen < target; ++it)
       asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(P.bar) : "memory");
-    } while (seen < target && ++it < kBarSpin);
-    if (seen < target) {
+    if (seen < target || (seen & kBarStopped)) {
       ok = 0;
+      asm volatile("red.relaxed.gpu.global.or.b32 [%0], %1;" ::"l"(P.bar), "r"(kBarStopped) : "memory");
       *P.bar_err = 1;
     }
   }
@@ -1579,7 +1579,7 @@ __global__ void k_begin_step(const Dev P, int advance) {
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
   int slot = P.ctl[0] + advance;
   P.ctl[0] = slot;
-  *P.bar = 0;
+  *P.bar = *P.bar & kBarStopped;
   double ramp = P.sched[(size_t)slot * P.sl.len];
   for (int j = 1; j <= P.numqbc; ++j) P.qdis[j] = P.qdis0[j] * ramp;
 }
