@@ -1550,6 +1550,11 @@ __global__ void k_ext_prep(const Dev P) {
     for (int q = i - 1; q < 4 * P.isplit * P.iobcn; q += gridDim.x * blockDim.x)
       tide_entry(P, q / P.iobcn, q % P.iobcn + 1);
   if (i > P.N) return;
+  if (i == 1) {
+    // the viscosity beside a boundary edge, in the form's type: the other form's values lie over it
+    if (P.prec) reinterpret_cast<float*>(P.xvc)[0] = 0.f;
+    else P.xvc[0] = 0.0;
+  }
   store_grad<false>(P, i);
   store_exf(P, i);
   if (P.xform) {
@@ -1557,7 +1562,7 @@ __global__ void k_ext_prep(const Dev P) {
     const size_t n1 = P.N + 1;
     P.xuv[i] = make_double2(P.ua[i], P.va[i]);
     P.xw[n1 + i] = P.iswetce[i];
-    if (i == 1) {  // the ghost cell 0 of both buffers, its gradient and viscosity
+    if (i == 1) {  // the ghost cell 0 of both buffers and its gradient
       P.xuv[0] = make_double2(P.ua[0], P.va[0]);
       P.xuv[n1] = make_double2(P.uaf[0], P.vaf[0]);
       P.xw[0] = P.iswetc[0];
