@@ -1287,20 +1287,21 @@ int32_t fvg_profile_groups(void) { return G_COUNT; }
 
 int32_t fvg_kernels_per_step(const fvg_handle* h) {
   if (!h) return -1;
+  const Dev& P = h->P;
   const fvg_params& p = h->prm;
-  int n = 1 + 1 + 2 + 2 + 2;                                // begin, cell_pre, grad3+adv3d, baropg+prep, int advave+reset
-  n += (use_ext_loop(h) ? 1 : p.isplit * 4 * (2 + (p.limiter ? 1 : 0) +
-                                              (p.wetting_drying_on && p.limiter && !h->P.xform ? 1 : 0))) + 1;
-                                                           // RK stages (with slope limiters), closing update
-  if (p.limiter) n += 1 + 2;                               // slope limiters: ADVAVE, 3-D
-  if (p.baropg_z && !p.barotropic) n += 2;                   // PHY_BAROPG's two kernels
-  n += 1 + 1 + 1 + 1 + 2 + 1;                              // adjust2, vertvl x2, w/viscofh, grad3+adv_uv, vdif_uv
-  n += 7;                                                  // grad_q, adv_q (2 phases), vdif_q (4 passes)
-  if (h->P.closure) n += 3;                                // learned closure (compaction x2, network)
-  if (p.temperature_active || p.salinity_active)           // grad_ts, adv_ts (2 phases and the open
-    n += 4 + (h->P.iobcn > 0 ? 2 : 0) + (h->P.numqbc > 0 ? 1 : 0);  // boundary), vdif_ts, bcond_ts (rivers,
-                                                           // open boundary)
-  n += 1;                                                  // final
+  const int lim = P.limiter ? 1 : 0, wd = p.wetting_drying_on ? 1 : 0;
+  // begin, cell_pre, grad3 + advection3d, baropg (sums), prep, ext_cell (ADVAVE) + reset
+  int n = 1 + 1 + 2 + 1 + 1 + 2;
+  if (!p.barotropic) n += P.baropg_z ? 2 : (use_branches(h) ? 1 : 0);  // PHY_BAROPG; BAROPG beside the sums
+  n += 3 * lim;                                                          // slope limiters: ADVAVE, 3-D twice
+  // the external loop; a stage: node and cell phase, limiters, WET_JUDGE where it is a kernel
+  n += use_ext_loop(h) ? 1 : p.isplit * 4 * (2 + lim + (P.xform ? 0 : lim * wd));
+  n += 1 + 1 + 2 + 1;                                                    // finish, adjust2, vertvl x2, w/viscofh
+  n += 2 + 1;                                                            // grad3 + adv_uv, vdif_uv
+  n += 1 + 2 + 3 + (P.closure ? 3 : 0) + 1;                              // grad_q, adv_q, vdif_q; closure; shallow columns
+  if (p.temperature_active || p.salinity_active)                         // grad_ts, adv_ts, vdif_ts; open boundary; rivers
+    n += 1 + 2 + 1 + (P.iobcn > 0 ? 2 : 0) + (P.numqbc > 0 ? 1 : 0);
+  n += final_launches(P);
   return n;
 }
 const char* fvg_profile_group_name(int32_t g) { return (g >= 0 && g < G_COUNT) ? kGroupNames[g] : ""; }

@@ -615,6 +615,7 @@ void launch_vdif_ts(const Dev& P, cudaStream_t s, int parts);
 void launch_bcond_ts(const Dev& P, cudaStream_t s, int parts);
 enum FinalParts { FI_T = 1, FI_S = 2, FI_DENS = 4, FI_KM1 = 8, FI_SHIFT = 16 };
 void launch_final(const Dev& P, cudaStream_t s, int parts);
+int final_launches(const Dev& P);  // its kernels
 void launch_budget(const Dev& P, cudaStream_t s);
 
 }  // namespace fvg

@@ -1449,8 +1449,10 @@ void launch_bcond_ts(const Dev& P, cudaStream_t s, int parts) {
   if (P.numqbc > 0) k_bcond_ts_riv<<<P.KBM1, 128, 0, s>>>(P);
   if (P.iobcn > 0) k_bcond_ts_obc<<<dim3(P.iobcn, 2), 64, 0, s>>>(P, parts);
 }
+static bool final_split(const Dev& P) { return (long)P.N * P.KB >= kFinSplit; }
+int final_launches(const Dev& P) { return final_split(P) ? 2 : 1; }
 void launch_final(const Dev& P, cudaStream_t s, int parts) {
-  const bool split = (long)P.N * P.KB >= kFinSplit;
+  const bool split = final_split(P);
   const int n = (split ? P.M : P.M > P.N ? P.M : P.N) + 1;
   dim3 b(32, 8), g(nblk(n, 32), nblk(P.KB, 8));
   k_final<<<g, b, 0, s>>>(P, parts, split ? 0 : 1);
