@@ -23,9 +23,11 @@ namespace {
 
 // Most cell-layers of a mesh whose step runs in branches (use_branches): they measured faster
 // at every size (175 nodes x 5 layers 431 -> 396 us per step, 50k x 30 FP64 3249 -> 3038, 200k x
-// 30 10821 -> 10577), but cost the tracers' own flux scratch, 48 bytes per cell-layer (24 in
-// FP32), which a large ensemble would rather hold members in.
+// 30 10821 -> 10577), but cost the tracers' own flux scratch (branch_bytes: about 56 bytes per
+// cell-layer, 1.1 GB at this size), which a large ensemble would rather hold members in: it is
+// taken only while kBranchShare times as much memory is free on the card.
 constexpr long kBranchCells = 20000000;
+constexpr size_t kBranchShare = 16;
 
 // Most polls of a grid barrier of the resident external loop (about two seconds).  A phase
 // takes microseconds; what the wait has to outlast is a block that starts late behind the
@@ -74,14 +76,11 @@ struct fvg_handle {
   int ext_loop = 1;
   int loop_ok = 0;
   // side branches of a step (use_branches): allowed (tuning key "branches"), their streams,
-  // fork and join events, and the tracers' own flux scratch in FP64 and FP32
+  // fork and join events, and the tracers' own flux scratch (branch_bytes; none: one order)
   int branches = 1;
   cudaStream_t side[2] = {nullptr, nullptr};
   cudaEvent_t ev[7] = {};
-  double2* ex2_ts = nullptr;
-  double* gvn_ts = nullptr;
-  float2* ex2f_ts = nullptr;
-  float* npk_ts = nullptr;
+  void* ts_scratch = nullptr;
 };
 
 #define CK(call)                                                                      \
@@ -103,11 +102,59 @@ void regraph(fvg_handle* h) {
   if (h->graph) { cudaGraphDestroy(h->graph); h->graph = nullptr; }
 }
 
+// The tracers' own scratch while the turbulence uses the handle's: the half-edge fluxes and then
+// VISCOFH*NN_HVC in FP64, the fluxes and then the node records in the FP32 form, in one
+// allocation that serves the form in use.
+size_t branch_bytes(const Dev& P) {
+  const size_t ex2 = (size_t)P.ncvs * P.KB, node = (size_t)P.ms * P.KB;
+  return std::max(ex2 * sizeof(double2) + node * sizeof(double), ex2 * sizeof(float2) + node * 16 * sizeof(float));
+}
+Dev branch_dev(const fvg_handle* h) {
+  Dev Q = h->P;
+  const size_t ex2 = (size_t)Q.ncvs * Q.KB;
+  if (Q.prec) {
+    Q.f.ex2 = (float2*)h->ts_scratch;
+    Q.f.npk = (float*)(Q.f.ex2 + ex2);
+  } else {
+    Q.ex2 = (double2*)h->ts_scratch;
+    Q.gvn = (double*)(Q.ex2 + ex2);
+  }
+  return Q;
+}
+// Take the scratch where the mesh is not too large and the card not too full; without it the
+// step runs in one order.
+void take_branches(fvg_handle* h) {
+  const Dev& P = h->P;
+  if (h->ts_scratch || (long)P.N * P.KBM1 > kBranchCells) return;
+  size_t room = 0, total = 0;
+  const size_t bytes = branch_bytes(P);
+  if (cudaMemGetInfo(&room, &total) != cudaSuccess || room / kBranchShare < bytes) return;
+  bool ok = true;
+  for (auto& q : h->side) ok = ok && (q || cudaStreamCreateWithFlags(&q, cudaStreamNonBlocking) == cudaSuccess);
+  for (auto& e : h->ev) ok = ok && (e || cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess);
+  if (ok && cudaMalloc(&h->ts_scratch, bytes) != cudaSuccess) h->ts_scratch = nullptr;
+  if (h->ts_scratch) cudaMemsetAsync(h->ts_scratch, 0, bytes, h->stream);
+  cudaGetLastError();  // one order then, and no error
+}
+// Give it back; the captured step (regraph) must not use it again.
+void drop_branches(fvg_handle* h) {
+  if (!h->ts_scratch) return;
+  cudaStreamSynchronize(h->stream);
+  regraph(h);
+  cudaFree(h->ts_scratch);
+  h->ts_scratch = nullptr;
+}
+
 template <class T>
 int dalloc(fvg_handle* h, T** p, size_t n) {
   void* q = nullptr;
   size_t bytes = (n == 0 ? 1 : n) * sizeof(T);
   cudaError_t e = cudaMalloc(&q, bytes);
+  if (e == cudaErrorMemoryAllocation && h->ts_scratch) {  // what the handle needs goes before its branches
+    cudaGetLastError();
+    drop_branches(h);
+    e = cudaMalloc(&q, bytes);
+  }
   if (e != cudaSuccess) {
     h->err = std::string("cudaMalloc: ") + cudaGetErrorString(e);
     return FVG_ERR_NOMEM;
@@ -301,9 +348,7 @@ bool use_ext_loop(const fvg_handle* h) {
 // Whether the independent parts of a step run as branches beside one another: BAROPG beside
 // ADVECTION; after VERTVL the momentum, the turbulence and the tracers.  Their kernels fill
 // the chip only on large meshes.
-bool use_branches(const fvg_handle* h) {
-  return h->branches && h->ex2_ts && (!h->P.prec || h->ex2f_ts);
-}
+bool use_branches(const fvg_handle* h) { return h->branches && h->ts_scratch; }
 
 // One INTERNAL_STEP as a kernel sequence (internal_step.F:115-1590).
 // after: in a group, the event of the model before (its resident external loop is done, if
@@ -421,15 +466,7 @@ void enqueue_internal_step(fvg_handle* h, cudaStream_t s, Marker mk = Marker(), 
   }
   // tracers; VDIF_TS takes the new KH
   if (ts) {
-    Dev Q = P;
-    if (br) {
-      Q.ex2 = h->ex2_ts;
-      Q.gvn = h->gvn_ts;
-      if (P.prec) {
-        Q.f.ex2 = h->ex2f_ts;
-        Q.f.npk = h->npk_ts;
-      }
-    }
+    const Dev Q = br ? branch_dev(h) : P;
     launch_grad(Q, b2, 1);
     mk.mark(s, G_GRAD_TS);
     launch_adv_ts(Q, b2, ts | spc);
@@ -1040,14 +1077,6 @@ int fvg_create(const fvg_mesh* m, const fvg_params* prm, const fvg_forcing* f, f
   if ((rc = dalloc(h, &P.vc3, ns * KB))) return fail(rc);
   if ((rc = dalloc(h, (double**)&P.ex2, (size_t)P.ncvs * KB * 2))) return fail(rc);
   P.he_vflux = (double*)P.ex2;
-  if ((long)N * (KB - 1) <= kBranchCells) {
-    if ((rc = dalloc(h, (double**)&h->ex2_ts, (size_t)P.ncvs * KB * 2))) return fail(rc);
-    if ((rc = dalloc(h, &h->gvn_ts, ms * KB))) return fail(rc);
-    for (auto& q : h->side)
-      if (cudaStreamCreateWithFlags(&q, cudaStreamNonBlocking) != cudaSuccess) return fail(FVG_ERR_CUDA);
-    for (auto& e : h->ev)
-      if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) return fail(FVG_ERR_CUDA);
-  }
 
   // ---- schedule ----
   h->sched_cap = 256;
@@ -1067,6 +1096,7 @@ int fvg_create(const fvg_mesh* m, const fvg_params* prm, const fvg_forcing* f, f
     *P.bar_err = 0;
   }
   P.sched = h->d_sched;
+  take_branches(h);  // last: what every step needs is there
   if (cudaDeviceSynchronize() != cudaSuccess) {
     h->err = "device synchronize failed after create";
     return fail(FVG_ERR_CUDA);
@@ -1082,6 +1112,7 @@ void fvg_destroy(fvg_handle* h) {
   if (h->gexec) cudaGraphExecDestroy(h->gexec);
   if (h->graph) cudaGraphDestroy(h->graph);
   for (void* p : h->allocs) cudaFree(p);
+  if (h->ts_scratch) cudaFree(h->ts_scratch);
   if (h->h_sched) cudaFreeHost(h->h_sched);
   if (h->h_ctl) cudaFreeHost(h->h_ctl);
   if (h->stream) cudaStreamDestroy(h->stream);
@@ -1393,10 +1424,6 @@ int fvg_set_precision(fvg_handle* h, int32_t mode) {
     }
     if ((rc = dalloc(h, &f.npk, ms * KB * 16))) return fail(rc);
     if ((rc = dalloc(h, (float**)&f.ex2, (size_t)P.ncvs * KB * 2))) return fail(rc);
-    if (h->ex2_ts) {
-      if ((rc = dalloc(h, (float**)&h->ex2f_ts, (size_t)P.ncvs * KB * 2))) return fail(rc);
-      if ((rc = dalloc(h, &h->npk_ts, ms * KB * 16))) return fail(rc);
-    }
     if ((rc = dalloc(h, &f.xo, 2 * e1))) return fail(rc);
     if ((rc = dalloc(h, &f.yo, 2 * e1))) return fail(rc);
     if ((rc = dalloc(h, &f.dltxc, e1))) return fail(rc);
@@ -1553,6 +1580,8 @@ int fvg_set_tuning(fvg_handle* h, const char* key, int32_t value) {
     h->P.bar_polls = value;
   } else if (k == "branches") {
     h->branches = value != 0;
+    if (h->branches) take_branches(h);
+    else drop_branches(h);
   } else {
     h->err = "unknown tuning key " + k;
     return FVG_ERR_ARG;
