@@ -165,6 +165,16 @@ int dalloc(fvg_handle* h, T** p, size_t n) {
   return FVG_OK;
 }
 
+// Free what dalloc gave since it held `held` allocations (a call that failed half-way).
+void free_back_to(fvg_handle* h, size_t held) {
+  cudaStreamSynchronize(h->stream);
+  while (h->allocs.size() > held) {
+    cudaFree(h->allocs.back());
+    h->allocs.pop_back();
+  }
+  cudaGetLastError();
+}
+
 template <class T>
 int upload(fvg_handle* h, T** p, const T* src, size_t n) {
   int rc = dalloc(h, p, n);
@@ -1400,55 +1410,67 @@ static void set_xform(fvg_handle* h) {
   h->P.f.compact = h->P.prec == FVG_PREC_FP32_FLUX && h->P.xform;
 }
 
+// The FP32-flux form's scratch and metrics (the first switch to it).
+static int make_f32(fvg_handle* h) {
+  Dev& P = h->P;
+  int rc;
+  const size_t ms = P.ms, ns = P.ns, KB = P.KB, n1 = P.N + 1, e1 = P.NE + 1;
+  F32& f = P.f;
+  if ((rc = dalloc(h, (float**)&f.g34, 4 * ns * KB))) return rc;
+  if ((rc = dalloc(h, &f.vc3, ns * KB))) return rc;
+  if ((rc = dalloc(h, (float**)&f.g2d4, 4 * n1))) return rc;
+  if (P.limiter) {
+    std::vector<float> ones(std::max(n1, ns * KB), 1.0f);
+    for (int q = 0; q < 2; ++q) {
+      if ((rc = dalloc(h, &f.alfa2[q], n1))) return rc;
+      if ((rc = dalloc(h, &f.alfa3[q], ns * KB))) return rc;
+      CK(cudaMemcpy(f.alfa2[q], ones.data(), n1 * sizeof(float), cudaMemcpyHostToDevice));
+      CK(cudaMemcpy(f.alfa3[q], ones.data(), ns * KB * sizeof(float), cudaMemcpyHostToDevice));
+    }
+  }
+  if ((rc = dalloc(h, &f.npk, ms * KB * 16))) return rc;
+  if ((rc = dalloc(h, (float**)&f.ex2, (size_t)P.ncvs * KB * 2))) return rc;
+  if ((rc = dalloc(h, &f.xo, 2 * e1))) return rc;
+  if ((rc = dalloc(h, &f.yo, 2 * e1))) return rc;
+  if ((rc = dalloc(h, &f.dltxc, e1))) return rc;
+  if ((rc = dalloc(h, &f.dltyc, e1))) return rc;
+  if ((rc = dalloc(h, &f.art, n1))) return rc;
+  if ((rc = dalloc(h, &f.cc_hvc, n1))) return rc;
+  if ((rc = dalloc(h, &f.a1u, 4 * n1))) return rc;
+  if ((rc = dalloc(h, &f.a2u, 4 * n1))) return rc;
+  for (float** pp : {&f.ce_xoa, &f.ce_yoa, &f.ce_xob, &f.ce_yob, &f.ce_dx, &f.ce_dy})
+    if ((rc = dalloc(h, pp, 3 * n1))) return rc;
+  if ((rc = dalloc(h, (float**)&f.ce_geo, 4 * 3 * n1))) return rc;
+  if ((rc = dalloc(h, (float**)&f.ce_dd, 2 * 3 * n1))) return rc;
+  if ((rc = dalloc(h, (float**)&f.hg4, 4 * (size_t)P.ncvs))) return rc;
+  if ((rc = dalloc(h, (float**)&f.hg2, 2 * (size_t)P.ncvs))) return rc;
+  if ((rc = dalloc(h, (float**)&f.trie, 2 * (size_t)P.trie_n))) return rc;
+  if ((rc = dalloc(h, (float**)&f.a1u4, 4 * n1))) return rc;
+  if ((rc = dalloc(h, (float**)&f.a2u4, 4 * n1))) return rc;
+  // the allocations were cleared on the default stream, which the handle's stream does not
+  // wait for by itself
+  CK(cudaStreamSynchronize(cudaStreamLegacy));
+  launch_make_f32(P, h->stream);
+  CK(cudaGetLastError());
+  if ((rc = dalloc(h, (double**)&f.exc0, 4 * n1))) return rc;
+  if ((rc = dalloc(h, (double**)&f.exc1, 4 * n1))) return rc;
+  CK(cudaStreamSynchronize(cudaStreamLegacy));
+  return FVG_OK;
+}
+
 int fvg_set_precision(fvg_handle* h, int32_t mode) {
   if (!h) return FVG_ERR_ARG;
   if (mode != FVG_PREC_FP64 && mode != FVG_PREC_FP32_FLUX) { h->err = "unknown precision mode"; return FVG_ERR_ARG; }
   Dev& P = h->P;
   CK(cudaStreamSynchronize(h->stream));
   if (mode == FVG_PREC_FP32_FLUX && !P.f.ex2) {
-    int rc;
-    const size_t ms = P.ms, ns = P.ns, KB = P.KB, n1 = P.N + 1, e1 = P.NE + 1;
-    F32& f = P.f;
-    auto fail = [&](int r) { return r; };
-    if ((rc = dalloc(h, (float**)&f.g34, 4 * ns * KB))) return fail(rc);
-    if ((rc = dalloc(h, &f.vc3, ns * KB))) return fail(rc);
-    if ((rc = dalloc(h, (float**)&f.g2d4, 4 * n1))) return fail(rc);
-    if (P.limiter) {
-      std::vector<float> ones(std::max(n1, ns * KB), 1.0f);
-      for (int q = 0; q < 2; ++q) {
-        if ((rc = dalloc(h, &f.alfa2[q], n1))) return fail(rc);
-        if ((rc = dalloc(h, &f.alfa3[q], ns * KB))) return fail(rc);
-        CK(cudaMemcpy(f.alfa2[q], ones.data(), n1 * sizeof(float), cudaMemcpyHostToDevice));
-        CK(cudaMemcpy(f.alfa3[q], ones.data(), ns * KB * sizeof(float), cudaMemcpyHostToDevice));
-      }
+    const size_t held = h->allocs.size();
+    const int rc = make_f32(h);
+    if (rc) {  // all or nothing: a later call starts again
+      free_back_to(h, held);
+      P.f = F32{};
+      return rc;
     }
-    if ((rc = dalloc(h, &f.npk, ms * KB * 16))) return fail(rc);
-    if ((rc = dalloc(h, (float**)&f.ex2, (size_t)P.ncvs * KB * 2))) return fail(rc);
-    if ((rc = dalloc(h, &f.xo, 2 * e1))) return fail(rc);
-    if ((rc = dalloc(h, &f.yo, 2 * e1))) return fail(rc);
-    if ((rc = dalloc(h, &f.dltxc, e1))) return fail(rc);
-    if ((rc = dalloc(h, &f.dltyc, e1))) return fail(rc);
-    if ((rc = dalloc(h, &f.art, n1))) return fail(rc);
-    if ((rc = dalloc(h, &f.cc_hvc, n1))) return fail(rc);
-    if ((rc = dalloc(h, &f.a1u, 4 * n1))) return fail(rc);
-    if ((rc = dalloc(h, &f.a2u, 4 * n1))) return fail(rc);
-    for (float** pp : {&f.ce_xoa, &f.ce_yoa, &f.ce_xob, &f.ce_yob, &f.ce_dx, &f.ce_dy})
-      if ((rc = dalloc(h, pp, 3 * n1))) return fail(rc);
-    if ((rc = dalloc(h, (float**)&f.ce_geo, 4 * 3 * n1))) return fail(rc);
-    if ((rc = dalloc(h, (float**)&f.ce_dd, 2 * 3 * n1))) return fail(rc);
-    if ((rc = dalloc(h, (float**)&f.hg4, 4 * (size_t)P.ncvs))) return fail(rc);
-    if ((rc = dalloc(h, (float**)&f.hg2, 2 * (size_t)P.ncvs))) return fail(rc);
-    if ((rc = dalloc(h, (float**)&f.trie, 2 * (size_t)P.trie_n))) return fail(rc);
-    if ((rc = dalloc(h, (float**)&f.a1u4, 4 * n1))) return fail(rc);
-    if ((rc = dalloc(h, (float**)&f.a2u4, 4 * n1))) return fail(rc);
-    // the allocations were cleared on the default stream, which the handle's stream does not
-    // wait for by itself
-    CK(cudaStreamSynchronize(cudaStreamLegacy));
-    launch_make_f32(P, h->stream);
-    CK(cudaGetLastError());
-    if ((rc = dalloc(h, (double**)&f.exc0, 4 * n1))) return fail(rc);
-    if ((rc = dalloc(h, (double**)&f.exc1, 4 * n1))) return fail(rc);
-    CK(cudaStreamSynchronize(cudaStreamLegacy));
   }
   P.prec = mode;
   set_xform(h);
@@ -1475,18 +1497,21 @@ int fvg_set_closure(fvg_handle* h, int32_t mode, const float* params, int32_t np
   int rc;
   if (!P.clos_feat) {
     if (closure_setup_attrs()) { h->err = "cannot configure the closure kernel"; return FVG_ERR_CUDA; }
-    if ((rc = dalloc(h, &P.clos_feat, S))) return rc;
-    // one flag per level chunk and node: at most KB chunks (one level per thread)
-    if ((rc = dalloc(h, &P.clos_envc, (size_t)P.KB * ((size_t)P.M + 1)))) return rc;
-    if ((rc = dalloc(h, &P.clos_env, (size_t)P.M + 1))) return rc;
-    if ((rc = dalloc(h, &P.clos_list, (size_t)P.M + 1))) return rc;
-    if ((rc = dalloc(h, &P.clos_cnt, (size_t)P.M / 1024 + 2))) return rc;
-    if ((rc = dalloc(h, &P.clos_err, 1))) return rc;
+    const size_t held = h->allocs.size();
     float* b = nullptr;
-    if ((rc = dalloc(h, &b, 144))) return rc;
-    P.clos_b = b;
     uint8_t* w = nullptr;
-    if ((rc = dalloc(h, &w, closure_weight_image_bytes()))) return rc;
+    // clos_envc: one flag per level chunk and node, at most KB chunks (one level per thread)
+    if ((rc = dalloc(h, &P.clos_feat, S)) || (rc = dalloc(h, &P.clos_envc, (size_t)P.KB * ((size_t)P.M + 1))) ||
+        (rc = dalloc(h, &P.clos_env, (size_t)P.M + 1)) || (rc = dalloc(h, &P.clos_list, (size_t)P.M + 1)) ||
+        (rc = dalloc(h, &P.clos_cnt, (size_t)P.M / 1024 + 2)) || (rc = dalloc(h, &P.clos_err, 1)) ||
+        (rc = dalloc(h, &b, 144)) || (rc = dalloc(h, &w, closure_weight_image_bytes()))) {
+      free_back_to(h, held);
+      P.clos_feat = nullptr;
+      P.clos_env = nullptr;
+      P.clos_err = nullptr;
+      return rc;
+    }
+    P.clos_b = b;
     P.clos_w = w;
     int dev = 0, nsm = 148;
     cudaGetDevice(&dev);
