@@ -432,13 +432,13 @@ void enqueue_internal_step(fvg_handle* h, cudaStream_t s, Marker mk = Marker(), 
       const int pdl = stage > 0 ? 1 : 0;
       launch_ext_node(Q, s, iext, K, EN_EXTEL | EN_BC | EN_GRAD | EN_TABLE | (K == 1 ? EN_COPY_ELRK : 0) | prev, pdl);
       mk.mark(s, G_EXT_NODE);
-      if (p.wetting_drying_on && P.limiter) {
+      if (p.wetting_drying_on && per_edge(P)) {
         launch_wet_cells(Q, s, 1);  // its node part opens the next stage's node kernel
         mk.mark(s, G_WET);
       }
       if (P.limiter) launch_alfa2(Q, s);
       launch_ext_cell(Q, s, iext, K,
-                      (!p.wetting_drying_on ? EC_N2E : P.limiter ? 0 : EC_WET) | EC_FLUXOBN | EC_ADVAVE | EC_EXTUV |
+                      (!p.wetting_drying_on ? EC_N2E : per_edge(P) ? 0 : EC_WET) | EC_FLUXOBN | EC_ADVAVE | EC_EXTUV |
                           EC_BC2 | (K == 1 ? EC_COPY_RK : 0) | EC_FINISH,
                       P.limiter ? 0 : 1);
       mk.mark(s, G_EXT_CELL);
@@ -755,6 +755,7 @@ int fvg_create(const fvg_mesh* m, const fvg_params* prm, const fvg_forcing* f, f
       lo.assign(4 * n1, 0);
       std::vector<double> hm(n1, 0.0);
       h->compact_ok = 1;
+      P.closed = 3;
       for (size_t i = 1; i < n1; ++i) {
         // the node common to two slots' edges
         auto common = [&](int sa, int sb) {
@@ -770,7 +771,7 @@ int fvg_create(const fvg_mesh* m, const fvg_params* prm, const fvg_forcing* f, f
               seen |= 1 << sl;
               if (j == 2) bits |= sl << 6;
             }
-        if (seen != 7) { h->err = "cell whose three edges are not its sides"; return fail(FVG_ERR_BOUNDS); }
+        if (seen != 7) P.closed &= ~1;
         for (int sl = 0; sl < 3; ++sl) {
           const int e = cl[i][sl] >> 1, side = cl[i][sl] & 1;
           bits |= side << sl | (m->isbc[e] != 0 ? 1 : 0) << (3 + sl);
@@ -801,6 +802,7 @@ int fvg_create(const fvg_mesh* m, const fvg_params* prm, const fvg_forcing* f, f
           }
         }
       }
+      if (!(P.closed & 1)) h->compact_ok = 0;
       UPI(wfar, far.data(), far.size());
       UPI(loopx, lx.data(), lx.size());
       std::vector<double> xy(2 * m1), cxy(2 * n1);
@@ -877,9 +879,15 @@ int fvg_create(const fvg_mesh* m, const fvg_params* prm, const fvg_forcing* f, f
         const int he = chv[3 * i + s2], a = x[s2], b = x[(s2 + 1) % 3];
         const bool straight = m->niec[he] == a && m->niec[v1 + he] == b;
         const bool flip = m->niec[he] == b && m->niec[v1 + he] == a;
-        if (a == b || !(straight || flip)) { h->err = "half-edges of a cell that do not part its three nodes"; return fail(FVG_ERR_BOUNDS); }
+        if (a == b || !(straight || flip)) P.closed &= ~2;
         hex[4 * i + s2] = a;
         hex[4 * i + 3] |= (flip ? 1 : 0) << s2;
+      }
+    }
+    for (size_t i = 1; i < n1; ++i)
+      for (int s2 = 0; s2 < 3; ++s2) {
+        const int he = chv[3 * i + s2];
+        const bool flip = (P.closed & 2) && (hex[4 * i + 3] >> s2 & 1);
         slot[he] = s2;
         const size_t pos = (size_t)s2 * ns + i, pl = 3 * ns, sa = flip ? vi1 : 0, sb = flip ? 0 : vi1;
         hg[pos] = m->dltxe[he];
@@ -889,7 +897,6 @@ int fvg_create(const fvg_mesh* m, const fvg_params* prm, const fvg_forcing* f, f
         hg[4 * pl + pos] = m->dltxncve[sb + he];
         hg[5 * pl + pos] = m->dltyncve[sb + he];
       }
-    }
     UPD(hg, hg.data(), hg.size());
     UPI(hex, hex.data(), hex.size());
     std::vector<std::vector<int>> vl(m1);
@@ -1336,7 +1343,7 @@ int32_t fvg_kernels_per_step(const fvg_handle* h) {
   if (!p.barotropic) n += P.baropg_z ? 2 : (use_branches(h) ? 1 : 0);  // PHY_BAROPG; BAROPG beside the sums
   n += 3 * lim;                                                          // slope limiters: ADVAVE, 3-D twice
   // the external loop; a stage: node and cell phase, limiters, WET_JUDGE where it is a kernel
-  n += use_ext_loop(h) ? 1 : p.isplit * 4 * (2 + lim + (P.xform ? 0 : lim * wd));
+  n += use_ext_loop(h) ? 1 : p.isplit * 4 * (2 + lim + (P.xform || !per_edge(P) ? 0 : wd));
   n += 1 + 1 + 2 + 1;                                                    // finish, adjust2, vertvl x2, w/viscofh
   n += 2 + 1;                                                            // grad3 + adv_uv, vdif_uv
   n += 1 + 2 + 3 + (P.closure ? 3 : 0) + 1;                              // grad_q, adv_q, vdif_q; closure; shallow columns

@@ -164,7 +164,11 @@ struct Dev {
   // side of X(s), DLTXNCVE and DLTYNCVE of the side of X(s+1) (hex).
   const double* hg;
   // Per cell its nodes X0, X1, X2 in the order in which the half-edge of slot s separates
-  // X(s) and X(s+1 mod 3); w: bit s where NIEC(he,1) is X(s+1).
+  // X(s) and X(s+1 mod 3); w: bit s where NIEC(he,1) is X(s+1).  closed: bit 0 where every
+  // cell's three edges go round its three nodes (loopx), bit 1 where its half-edges do (hex);
+  // a mesh whose lists do not is stepped as they say, by the kernels that read each edge's
+  // nodes (per_edge, k_he_adv_listed; hg then has NIEC(he,1) for X(s)).
+  int closed;
   const int4* hex;
   const int *cell_edge;               // cell -> its 3 edges (id*2 + side), ascending id
   // Slot table of the cell edge loops, slot s of cell i at s*(N+1) + i (edges in the order
@@ -314,6 +318,9 @@ struct Dev {
   int ext_grid, nsm;
 };
 
+// Whether the momentum edge fluxes run in the kernels that take an edge's cells, nodes and
+// limiters from its own list entry.
+inline bool per_edge(const Dev& P) { return P.limiter || !(P.closed & 1); }
 // Threads per block of a kernel with one thread per entity: `most`, or fewer (down to one
 // warp) where blocks of `most` would leave SMs without a block.  A small mesh's kernel is
 // a chain of dependent loads, and warps alone on their SMs run it fastest.
@@ -528,6 +535,19 @@ __device__ inline void lim_faces(int limiter, R ua, R ub, R ea, R eb, R alfa_a, 
       f1 = ua;
       f2 = ub;
     }
+  }
+}
+// Face values of an edge between the values ua, ub with gradients (gax, gay), (gbx, gby) over the
+// offsets (xa, ya), (xb, yb): LIMITED_NO's sum, or the limited ones with the limiters alfa[a],
+// alfa[b].
+template <typename R>
+__device__ inline void edge_faces(int limiter, R ua, R ub, R gax, R gay, R xa, R ya, R gbx, R gby, R xb, R yb,
+                                  const R* alfa, size_t a, size_t b, R& f1, R& f2) {
+  if (limiter == 0) {
+    f1 = ua + gax * xa + gay * ya;
+    f2 = ub + gbx * xb + gby * yb;
+  } else {
+    lim_faces<R>(limiter, ua, ub, gax * xa + gay * ya, gbx * xb + gby * yb, alfa[a], alfa[b], f1, f2);
   }
 }
 __device__ inline double2 mk2(double a, double b) { return make_double2(a, b); }

@@ -397,8 +397,8 @@ __device__ inline bool wet_other(const Dev& P, bool judge, int i, int s, int o, 
   return P.iswetce[o] * P.iswetc[o] == 1;
 }
 
-// ADVAVE_EDGE_GCN for one cell (advave_edge_gcn.F:115-1003, LIMITED_NO branch), over the
-// cell's slot table.  The edge fluxes are evaluated in R; the surface-slope pressure
+// ADVAVE_EDGE_GCN for one cell (advave_edge_gcn.F:115-1003), over the cell's slot table.  LIM:
+// each edge by its own list entry (per_edge), with the limited schemes' face values.  The edge fluxes are evaluated in R; the surface-slope pressure
 // gradient PSTX/PSTY stays FP64.
 template <typename R, bool LIM>
 __device__ inline void advave_cell(const Dev& P, int i, int weti, bool judge, double& xfo, double& yfo, double& px,
@@ -495,10 +495,10 @@ __device__ inline void advave_cell(const Dev& P, int i, int weti, bool judge, do
         const Grad<R> ga = load_grad<R>(P, ia), gb = load_grad<R>(P, ib);
         const R xija = Mh::s_xoa(P, q), yija = Mh::s_yoa(P, q);
         const R xijb = Mh::s_xob(P, q), yijb = Mh::s_yob(P, q);
-        lim_faces<R>(P.limiter, (R)P.ua[ia], (R)P.ua[ib], ga.ux * xija + ga.uy * yija, gb.ux * xijb + gb.uy * yijb,
-                     Mh::alfa2(P, 0)[ia], Mh::alfa2(P, 0)[ib], uij1, uij2);
-        lim_faces<R>(P.limiter, (R)P.va[ia], (R)P.va[ib], ga.vx * xija + ga.vy * yija, gb.vx * xijb + gb.vy * yijb,
-                     Mh::alfa2(P, 1)[ia], Mh::alfa2(P, 1)[ib], vij1, vij2);
+        edge_faces<R>(P.limiter, (R)P.ua[ia], (R)P.ua[ib], ga.ux, ga.uy, xija, yija, gb.ux, gb.uy, xijb, yijb,
+                      Mh::alfa2(P, 0), ia, ib, uij1, uij2);
+        edge_faces<R>(P.limiter, (R)P.va[ia], (R)P.va[ib], ga.vx, ga.vy, xija, yija, gb.vx, gb.vy, xijb, yijb,
+                      Mh::alfa2(P, 1), ia, ib, vij1, vij2);
         R uij = half * (uij1 + uij2);
         R vij = half * (vij1 + vij2);
         const auto DD = Mh::s_dd(P, q);
@@ -1679,7 +1679,7 @@ void launch_wet_cells(const Dev& P, cudaStream_t s, int pdl) {
 void launch_ext_cell(const Dev& P, cudaStream_t s, int iext, int K, int parts, int pdl) {
   FVG_F32_FORWARD(launch_ext_cell(P, s, iext, K, parts, pdl));
   void (*k)(const Dev, int, int, int);
-  k = P.limiter ? k_ext_cell<RF, true> : k_ext_cell<RF, false>;
+  k = per_edge(P) ? k_ext_cell<RF, true> : k_ext_cell<RF, false>;
   const int b = col_threads(P, P.N, 128);
   launch_maybe_pdl(pdl, k, dim3(nblk(P.N, b)), dim3(b), s, P, iext, K, parts);
 }

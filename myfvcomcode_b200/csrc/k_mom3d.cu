@@ -251,8 +251,8 @@ __global__ void __launch_bounds__(256) k_alfa3(const Dev P) {
   }
 }
 
-// Limited schemes.  q: the edge's slot in the cell slot table (offsets and DLTXC/DLTYC of the
-// edge).
+// An edge by its own list entry (per_edge).  q: the edge's slot in the cell slot table (offsets
+// and DLTXC/DLTYC of the edge).
 template <typename R>
 __device__ inline EdgeFlux<R> edge_flux3(const Dev& P, size_t q, int ia, int ib, int k, R dij, bool exflux_form) {
   typedef Mesh<R> Mh;
@@ -272,10 +272,10 @@ __device__ inline EdgeFlux<R> edge_flux3(const Dev& P, size_t q, int ia, int ib,
   ga = load_g3<R>(P, ia, k);
   gb = load_g3<R>(P, ib, k);
   const size_t qa = C3(P, ia, k), qb = C3(P, ib, k);
-  lim_faces<R>(P.limiter, (R)U[ia], (R)U[ib], ga.ux * xija + ga.uy * yija, gb.ux * xijb + gb.uy * yijb,
-               Mh::alfa3(P, 0)[qa], Mh::alfa3(P, 0)[qb], uij1, uij2);
-  lim_faces<R>(P.limiter, (R)V[ia], (R)V[ib], ga.vx * xija + ga.vy * yija, gb.vx * xijb + gb.vy * yijb,
-               Mh::alfa3(P, 1)[qa], Mh::alfa3(P, 1)[qb], vij1, vij2);
+  edge_faces<R>(P.limiter, (R)U[ia], (R)U[ib], ga.ux, ga.uy, xija, yija, gb.ux, gb.uy, xijb, yijb, Mh::alfa3(P, 0), qa,
+                qb, uij1, uij2);
+  edge_faces<R>(P.limiter, (R)V[ia], (R)V[ib], ga.vx, ga.vy, xija, yija, gb.vx, gb.vy, xijb, yijb, Mh::alfa3(P, 1), qa,
+                qb, vij1, vij2);
   R uij = half * (uij1 + uij2);
   R vij = half * (vij1 + vij2);
   R viscof1 = arta * sqrt(ga.ux * ga.ux + ga.vy * ga.vy + half * ((ga.uy + ga.vx) * (ga.uy + ga.vx)));
@@ -1460,8 +1460,8 @@ static void launch_alfa3(const Dev& P, cudaStream_t s) {
 template <bool UV>
 static void launch_mom3d(const Dev& P, cudaStream_t s) {
   Dev Q = col_shape(P, P.N, P.KBM1);
-  if (P.limiter) {
-    launch_alfa3(P, s);
+  if (per_edge(P)) {
+    if (P.limiter) launch_alfa3(P, s);
     (UV ? k_adv_uv<RF> : k_advection3d<RF>)<<<col_grid(Q, P.N, P.KBM1), Q.col_bc, 0, s>>>(Q);
     return;
   }

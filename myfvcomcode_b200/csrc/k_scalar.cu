@@ -412,6 +412,37 @@ __global__ void __launch_bounds__(kHeThreads, sizeof(R) == 4 ? 8 : (MODE == 1 ? 
   }
 }
 
+// The same where a cell's half-edges do not go round its nodes (Dev::closed): both nodes of each
+// half-edge from NIEC.
+template <typename R, int MODE>
+__global__ void __launch_bounds__(kHeThreads) k_he_adv_listed(const Dev P, int parts) {
+  typedef typename Mesh<R>::R2 R2;
+  const int c = blockIdx.x * blockDim.x + threadIdx.x + 1;
+  if (c > P.N) return;
+  int kb, ke;
+  col_range(P, MODE == 0 ? 2 : 1, P.KBM1, kb, ke);
+  const bool on[2] = {(parts & (MODE == 0 ? AD_Q2 : AD_T)) != 0, (parts & (MODE == 0 ? AD_Q2L : AD_S)) != 0};
+  HeCell<R> hc;
+  for (int k = kb; k <= ke; ++k) {
+    he_cell_load<R, MODE>(P, c, k, hc);
+    for (int s = 0; s < 3; ++s) {
+      const int he = P.cell_he[3 * c + s], na = P.niec[he], nb = P.niec[P.NCV + 1 + he];
+      const size_t pos = (size_t)s * P.ns + c;
+      const R nna = (R)P.nn_hvc[na], nnb = (R)P.nn_hvc[nb];
+      R e[2] = {0, 0};
+      for (int t = 0; t < 2; ++t) {
+        if (!on[t]) continue;
+        TRec<R> ra = load_trec<R, MODE>(P, na, k, t), rb = load_trec<R, MODE>(P, nb, k, t);
+        const R visc = he_visc<R, MODE>(P, he_vn<R>(P, na, k, nna, ra.vf), he_vn<R>(P, nb, k, nnb, rb.vf), nna, nnb);
+        he_bounds(ra);
+        he_bounds(rb);
+        e[t] = he_flux<R>(hc, he_geo<R>(P, pos), 0, ra, rb, visc, nullptr);
+      }
+      Mesh<R>::ex2(P)[(size_t)(k - 1) * P.ncvs + pos] = mk2(e[0], e[1]);
+    }
+  }
+}
+
 // XFLUX_ADV of one open-boundary node (adv_t.F:510-511, 572-579): the advective parts of
 // its half-edge fluxes, recomputed with the same arithmetic as phase 1.
 template <typename R>
@@ -422,8 +453,8 @@ __device__ inline double obc_xflux_adv(const Dev& P, int i, int k, int t) {
     int he = code >> 1;
     int c = P.ntrg[he];
     const int sl = P.cell_he[3 * c] == he ? 0 : (P.cell_he[3 * c + 1] == he ? 1 : 2);
-    const int4 hx = P.hex[c];
-    const int na = sl == 0 ? hx.x : (sl == 1 ? hx.y : hx.z), nb = sl == 0 ? hx.y : (sl == 1 ? hx.z : hx.x);
+    const int flip = (P.closed & 2) ? (P.hex[c].w >> sl) & 1 : 0, n1 = P.niec[he], n2 = P.niec[P.NCV + 1 + he];
+    const int na = flip ? n2 : n1, nb = flip ? n1 : n2;
     HeCell<R> hc;
     he_cell_load<R, 1>(P, c, k, hc);
     TRec<R> ra = load_trec<R, 1>(P, na, k, t), rb = load_trec<R, 1>(P, nb, k, t);
@@ -432,7 +463,7 @@ __device__ inline double obc_xflux_adv(const Dev& P, int i, int k, int t) {
     he_bounds(ra);
     he_bounds(rb);
     R part;
-    he_flux<R>(hc, he_geo<R>(P, (size_t)sl * P.ns + c), (hx.w >> sl) & 1, ra, rb, visc, &part);
+    he_flux<R>(hc, he_geo<R>(P, (size_t)sl * P.ns + c), flip, ra, rb, visc, &part);
     xa = (code & 1) ? xa - part : xa + part;
   }
   return (double)xa;
@@ -1399,7 +1430,7 @@ void launch_adv_q(const Dev& P, cudaStream_t s, int parts) {
   if (Q.col_bc > kHeThreads) Q.col_bc = kHeThreads;
   Dev G = col_shape(P, P.M, nl);
   if (G.col_bc > kGatherThreads) G.col_bc = kGatherThreads;
-  k_he_adv<RF, 0><<<col_grid(Q, P.N, nl), Q.col_bc, 0, s>>>(Q, parts);
+  ((P.closed & 2) ? k_he_adv<RF, 0> : k_he_adv_listed<RF, 0>)<<<col_grid(Q, P.N, nl), Q.col_bc, 0, s>>>(Q, parts);
   k_gather_q<RF><<<col_grid(G, P.M, nl), G.col_bc, 0, s>>>(G, parts);
 }
 void launch_fct_q(const Dev& P, cudaStream_t s, int parts) {
@@ -1430,7 +1461,7 @@ void launch_adv_ts(const Dev& P, cudaStream_t s, int parts) {
   if (Q.col_bc > kHeThreads) Q.col_bc = kHeThreads;
   Dev G = col_shape(P, P.M, P.KBM1);
   if (G.col_bc > kGatherThreads) G.col_bc = kGatherThreads;
-  k_he_adv<RF, 1><<<col_grid(Q, P.N, P.KBM1), Q.col_bc, 0, s>>>(Q, parts);
+  ((P.closed & 2) ? k_he_adv<RF, 1> : k_he_adv_listed<RF, 1>)<<<col_grid(Q, P.N, P.KBM1), Q.col_bc, 0, s>>>(Q, parts);
   if (P.iobcn > 0) k_obc_xflux<RF><<<dim3(nblk(P.iobcn, 64), P.KBM1, 2), 64, 0, s>>>(P, parts);
   k_gather_ts<RF><<<col_grid(G, P.M, P.KBM1), G.col_bc, 0, s>>>(G, parts);
 }
