@@ -26,7 +26,9 @@ constexpr int kMaxKB = 64;
 // few columns share an SM, so a loop that loads, works and stores layer by layer waits for one
 // round trip to memory per layer.  Eight layers, at 200 k nodes x 30 layers, before -> after:
 // cell_pre 160 -> 135 us, vdif_uv 394 -> 282 (four layers, and one VH for both components),
-// baropg 355 -> 318 (RHO's round trip in the batch), vertvl_col 101 -> 65.
+// baropg 355 -> 318 (RHO's round trip in the batch), vertvl_col 101 -> 65.  k_adjust2 goes layer
+// by layer: in batches of eight 154 -> 162 us there and 10.3 -> 12.3 at 2,121 nodes x 10, against
+// 25 -> 23.5 at 20 k x 20.
 constexpr int kBat = 8;
 __device__ __constant__ double dAlpha3[5] = {0.0, 0.25, 1.0 / 3.0, 0.5, 1.0};
 
@@ -507,63 +509,42 @@ __global__ void k_adjust2(const Dev P, int parts) {
   const bool wet = adj && P.iswetct[i] * P.iswetc[i] == 1;
   const double dt1 = P.dt1[i];
   double ut = 0.0, vt = 0.0;
-  const int KBM1 = P.KBM1;
   if (wet) {
-    for (int k0 = 1; k0 <= KBM1; k0 += kBat) {
-      double ub[kBat], vb[kBat];
-#pragma unroll
-      for (int b = 0; b < kBat; ++b) {
-        const size_t q = C3(P, i, k0 + b <= KBM1 ? k0 + b : KBM1);
-        ub[b] = P.u[q];
-        vb[b] = P.v[q];
-      }
-#pragma unroll
-      for (int b = 0; b < kBat; ++b) {
-        if (k0 + b > KBM1) break;
-        const double z = P.dz1(i, k0 + b);
-        ut = ut + ub[b] * z;
-        vt = vt + vb[b] * z;
-      }
+    for (int k = 1; k <= P.KBM1; ++k) {
+      size_t q = C3(P, i, k);
+      ut = ut + P.u[q] * P.dz1(i, k);
+      vt = vt + P.v[q] * P.dz1(i, k);
     }
     ut = ut * dt1;
     vt = vt * dt1;
   }
-  const bool flux = parts & AJ_HE_FLUX;
-  if (!flux && !wet) return;
-  double dy[3] = {0.0, 0.0, 0.0}, dx[3] = {0.0, 0.0, 0.0};
-  if (flux)
-    for (int s = 0; s < 3; ++s) {
-      const size_t pos = (size_t)s * P.ns + i;
-      dy[s] = Mesh<double>::hg(P, 1, pos);
-      dx[s] = Mesh<double>::hg(P, 0, pos);
+  if (!(parts & AJ_HE_FLUX)) {
+    if (!wet) return;
+    for (int k = 1; k <= P.KBM1; ++k) {
+      size_t q = C3(P, i, k);
+      P.u[q] = P.u[q] - (ut - ud) / dt1;
+      P.v[q] = P.v[q] - (vt - vd) / dt1;
     }
-  const double cu = wet ? (ut - ud) / dt1 : 0.0, cv = wet ? (vt - vd) / dt1 : 0.0;
-  for (int k0 = 1; k0 <= KBM1; k0 += kBat) {
-    double ub[kBat], vb[kBat];
-#pragma unroll
-    for (int b = 0; b < kBat; ++b) {
-      const size_t q = C3(P, i, k0 + b <= KBM1 ? k0 + b : KBM1);
-      ub[b] = P.u[q];
-      vb[b] = P.v[q];
+    return;
+  }
+  double dy[3], dx[3];
+  for (int s = 0; s < 3; ++s) {
+    const size_t pos = (size_t)s * P.ns + i;
+    dy[s] = Mesh<double>::hg(P, 1, pos);
+    dx[s] = Mesh<double>::hg(P, 0, pos);
+  }
+  for (int k = 1; k <= P.KBM1; ++k) {
+    size_t q = C3(P, i, k);
+    double uu = P.u[q], vv = P.v[q];
+    if (wet) {
+      uu = uu - (ut - ud) / dt1;
+      vv = vv - (vt - vd) / dt1;
+      P.u[q] = uu;
+      P.v[q] = vv;
     }
-#pragma unroll
-    for (int b = 0; b < kBat; ++b) {
-      const int k = k0 + b;
-      if (k > KBM1) break;
-      double uu = ub[b], vv = vb[b];
-      if (wet) {
-        const size_t q = C3(P, i, k);
-        uu = uu - cu;
-        vv = vv - cv;
-        P.u[q] = uu;
-        P.v[q] = vv;
-      }
-      if (flux) {
-        const double dij = dt1 * P.dz1(i, k);
-        double* F = P.he_vflux + (size_t)(k - 1) * P.ncvs + i;
-        for (int s = 0; s < 3; ++s) F[(size_t)s * P.ns] = dij * (-uu * dy[s] + vv * dx[s]);
-      }
-    }
+    const double dij = dt1 * P.dz1(i, k);
+    double* F = P.he_vflux + (size_t)(k - 1) * P.ncvs + i;
+    for (int s = 0; s < 3; ++s) F[(size_t)s * P.ns] = dij * (-uu * dy[s] + vv * dx[s]);
   }
 }
 
