@@ -63,7 +63,7 @@ constexpr int TB = 32;    // samples per tile
 constexpr int NT = 256;   // threads per block
 constexpr int PD = 68;    // row stride of activations and weights (floats)
 constexpr int XD = 12;    // row stride of the inputs
-constexpr int kMostBlocks = 296;
+constexpr int kMostBlocks = 296;  // fixed, as the sum over the blocks depends on it
 struct TrainShared {
   float w1t[MI][PD];      // W1T[k][j]
   float w2t[MH][PD];      // W2T[k][j]
@@ -450,7 +450,7 @@ struct fvg_mlp {
   float *par = nullptr, *m = nullptr, *v = nullptr, *part = nullptr, *lpart = nullptr, *grad = nullptr;
   float* loss = nullptr;
   int* idx = nullptr;
-  int idx_cap = 0, part_blocks = 0, step = 0;
+  int idx_cap = 0, part_blocks = 0, step = 0, nsm = 148;
   cudaStream_t stream = nullptr;
   std::string err;
 };
@@ -500,6 +500,9 @@ int fvg_mlp_create(uint64_t seed, fvg_mlp** out) {
           cudaSuccess ||
       cudaFuncSetAttribute(k_mlp_forward, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(ForwardShared)) !=
           cudaSuccess)
+    return fail(FVG_ERR_CUDA);
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&q->nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
     return fail(FVG_ERR_CUDA);
   if (cudaStreamCreateWithFlags(&q->stream, cudaStreamNonBlocking) != cudaSuccess) return fail(FVG_ERR_CUDA);
   for (float** p : {&q->par, &q->m, &q->v, &q->grad})
@@ -596,7 +599,7 @@ int fvg_mlp_train(fvg_mlp* q, const float* x, const float* y, int32_t n, int32_t
 
 int fvg_mlp_forward(fvg_mlp* q, const float* x, int32_t n, float* out) {
   if (!q || !x || !out || n < 1) return FVG_ERR_ARG;
-  k_mlp_forward<<<std::min((n + FR - 1) / FR, 3 * 148), FR, sizeof(ForwardShared), q->stream>>>(q->par, x, n, out);
+  k_mlp_forward<<<std::min((n + FR - 1) / FR, 3 * q->nsm), FR, sizeof(ForwardShared), q->stream>>>(q->par, x, n, out);
   MK(cudaGetLastError());
   MK(cudaStreamSynchronize(q->stream));
   return FVG_OK;
