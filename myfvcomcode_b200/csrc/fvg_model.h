@@ -191,6 +191,7 @@ struct Dev {
   const int *inodeq, *icellq, *n_icellq;
   const double *rdisq, *qarea, *sin_angleq, *cos_angleq, *vqdist, *qdis0, *tdis, *sdis;
   const int *riv_skip;                        // node is an OBC or river node (FCT skip)
+  const int *riv_own;                         // river -> bit 0/1: no later one enters at its first/second node
   const int *cell_bcriv;                      // first river whose inflow cell this is (BCOND_GCN 2/3/5)
   // ----- forcing -----
   const double *wsx, *wsy;
