@@ -468,8 +468,12 @@ static int mlp_parts(fvg_mlp* q, int nblk) {
   if (q->lpart) cudaFree(q->lpart);
   q->part = nullptr;
   q->lpart = nullptr;
-  MK(cudaMalloc(&q->part, (size_t)nblk * NPAR * sizeof(float)));
-  MK(cudaMalloc(&q->lpart, (size_t)nblk * sizeof(float)));
+  q->part_blocks = 0;
+  if (cudaMalloc(&q->part, (size_t)nblk * NPAR * sizeof(float)) != cudaSuccess ||
+      cudaMalloc(&q->lpart, (size_t)nblk * sizeof(float)) != cudaSuccess) {
+    const cudaError_t e = cudaGetLastError();  // reported here, not by the next launch
+    return mlp_cuda(q, e, "cudaMalloc (gradients of the blocks)");
+  }
   q->part_blocks = nblk;
   return FVG_OK;
 }
@@ -572,6 +576,7 @@ int fvg_mlp_train(fvg_mlp* q, const float* x, const float* y, int32_t n, int32_t
   if (n > q->idx_cap) {
     if (q->idx) cudaFree(q->idx);
     q->idx = nullptr;
+    q->idx_cap = 0;
     MK(cudaMalloc(&q->idx, (size_t)n * sizeof(int)));
     q->idx_cap = n;
   }
