@@ -995,15 +995,16 @@ int fvg_create(const fvg_mesh* m, const fvg_params* prm, const fvg_forcing* f, f
     UPI(loopo, lo.data(), lo.size());
     UPI(cell_bcriv, bcriv.data(), n1); UPI(riv_skip, skip.data(), m1);
     // where several rivers enter at a node, the last one's T and S stand
-    std::vector<int> at(m1, 0), own(q1, 0);
+    std::vector<int> last(m1, 0), at(2 * q1, 0);
     for (int j = 1; j <= nq; ++j) {
-      if (prm->river_location == 0) at[m->inodeq[j]] = j;
-      else at[m->n_icellq[j]] = at[m->n_icellq[q1 + j]] = j;
+      at[2 * j] = prm->river_location == 0 ? m->inodeq[j] : m->n_icellq[j];
+      at[2 * j + 1] = prm->river_location == 0 ? 0 : m->n_icellq[q1 + j];
+      last[at[2 * j]] = last[at[2 * j + 1]] = j;
     }
     for (int j = 1; j <= nq; ++j)
-      own[j] = prm->river_location == 0 ? (at[m->inodeq[j]] == j)
-                                        : (at[m->n_icellq[j]] == j) | (at[m->n_icellq[q1 + j]] == j) << 1;
-    UPI(riv_own, own.data(), q1);
+      for (int s = 0; s < 2; ++s)
+        if (last[at[2 * j + s]] != j) at[2 * j + s] = 0;
+    UPI(riv_ts, at.data(), at.size());
     UPI(inodeq, m->inodeq, q1); UPI(icellq, m->icellq, q1); UPI(n_icellq, m->n_icellq, q1 * 2);
     UPD(rdisq, m->rdisq, q1 * 2); UPD(qarea, m->qarea, q1); UPD(vqdist, m->vqdist, q1 * (KB - 1));
     std::vector<double> sq(q1), cq(q1);

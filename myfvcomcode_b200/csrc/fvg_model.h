@@ -191,7 +191,7 @@ struct Dev {
   const int *inodeq, *icellq, *n_icellq;
   const double *rdisq, *qarea, *sin_angleq, *cos_angleq, *vqdist, *qdis0, *tdis, *sdis;
   const int *riv_skip;                        // node is an OBC or river node (FCT skip)
-  const int *riv_own;                         // river -> bit 0/1: no later one enters at its first/second node
+  const int2 *riv_ts;                         // river -> its nodes (0: none, or a later river's too)
   const int *cell_bcriv;                      // first river whose inflow cell this is (BCOND_GCN 2/3/5)
   // ----- forcing -----
   const double *wsx, *wsy;
@@ -536,19 +536,6 @@ __device__ inline void lim_faces(int limiter, R ua, R ub, R ea, R eb, R alfa_a, 
       f1 = ua;
       f2 = ub;
     }
-  }
-}
-// Face values of an edge between the values ua, ub with gradients (gax, gay), (gbx, gby) over the
-// offsets (xa, ya), (xb, yb): LIMITED_NO's sum, or the limited ones with the limiters alfa[a],
-// alfa[b].
-template <typename R>
-__device__ inline void edge_faces(int limiter, R ua, R ub, R gax, R gay, R xa, R ya, R gbx, R gby, R xb, R yb,
-                                  const R* alfa, size_t a, size_t b, R& f1, R& f2) {
-  if (limiter == 0) {
-    f1 = ua + gax * xa + gay * ya;
-    f2 = ub + gbx * xb + gby * yb;
-  } else {
-    lim_faces<R>(limiter, ua, ub, gax * xa + gay * ya, gbx * xb + gby * yb, alfa[a], alfa[b], f1, f2);
   }
 }
 __device__ inline double2 mk2(double a, double b) { return make_double2(a, b); }

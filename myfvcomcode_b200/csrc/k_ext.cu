@@ -397,10 +397,11 @@ __device__ inline bool wet_other(const Dev& P, bool judge, int i, int s, int o, 
   return P.iswetce[o] * P.iswetc[o] == 1;
 }
 
-// ADVAVE_EDGE_GCN for one cell (advave_edge_gcn.F:115-1003), over the cell's slot table.  LIM:
-// each edge by its own list entry (per_edge), with the limited schemes' face values.  The edge fluxes are evaluated in R; the surface-slope pressure
+// ADVAVE_EDGE_GCN for one cell (advave_edge_gcn.F:115-1003), over the cell's slot table.  EDGES:
+// the edges as the cell sees them, or each by its own list entry (per_edge), plain or limited.  The edge fluxes are evaluated in R; the surface-slope pressure
 // gradient PSTX/PSTY stays FP64.
-template <typename R, bool LIM>
+enum Edges { kSeen, kListed, kLimitedEdges };
+template <typename R, Edges EDGES>
 __device__ inline void advave_cell(const Dev& P, int i, int weti, bool judge, double& xfo, double& yfo, double& px,
                                    double& py) {
   typedef Mesh<R> Mh;
@@ -412,7 +413,7 @@ __device__ inline void advave_cell(const Dev& P, int i, int weti, bool judge, do
   const Grad<R> gi = load_grad<R>(P, i);
   const R ui = (R)P.ua[i], vi = (R)P.va[i];
   const double ged1 = P.grav_e[i] * P.d1[i];
-  if constexpr (!LIM) {
+  if constexpr (EDGES == kSeen) {
     // Each edge as the cell sees it: its own side from the values above, sums that commute
     // without regard to the sides, the upwind weights with the side as a sign, and both
     // cells' ART*|grad|*CC_HVC from the gradient job (xvc), so that the values and their
@@ -495,10 +496,17 @@ __device__ inline void advave_cell(const Dev& P, int i, int weti, bool judge, do
         const Grad<R> ga = load_grad<R>(P, ia), gb = load_grad<R>(P, ib);
         const R xija = Mh::s_xoa(P, q), yija = Mh::s_yoa(P, q);
         const R xijb = Mh::s_xob(P, q), yijb = Mh::s_yob(P, q);
-        edge_faces<R>(P.limiter, (R)P.ua[ia], (R)P.ua[ib], ga.ux, ga.uy, xija, yija, gb.ux, gb.uy, xijb, yijb,
-                      Mh::alfa2(P, 0), ia, ib, uij1, uij2);
-        edge_faces<R>(P.limiter, (R)P.va[ia], (R)P.va[ib], ga.vx, ga.vy, xija, yija, gb.vx, gb.vy, xijb, yijb,
-                      Mh::alfa2(P, 1), ia, ib, vij1, vij2);
+        if constexpr (EDGES == kLimitedEdges) {
+          lim_faces<R>(P.limiter, (R)P.ua[ia], (R)P.ua[ib], ga.ux * xija + ga.uy * yija, gb.ux * xijb + gb.uy * yijb,
+                       Mh::alfa2(P, 0)[ia], Mh::alfa2(P, 0)[ib], uij1, uij2);
+          lim_faces<R>(P.limiter, (R)P.va[ia], (R)P.va[ib], ga.vx * xija + ga.vy * yija, gb.vx * xijb + gb.vy * yijb,
+                       Mh::alfa2(P, 1)[ia], Mh::alfa2(P, 1)[ib], vij1, vij2);
+        } else {
+          uij1 = (R)P.ua[ia] + ga.ux * xija + ga.uy * yija;
+          uij2 = (R)P.ua[ib] + gb.ux * xijb + gb.uy * yijb;
+          vij1 = (R)P.va[ia] + ga.vx * xija + ga.vy * yija;
+          vij2 = (R)P.va[ib] + gb.vx * xijb + gb.vy * yijb;
+        }
         R uij = half * (uij1 + uij2);
         R vij = half * (vij1 + vij2);
         const auto DD = Mh::s_dd(P, q);
@@ -598,8 +606,8 @@ __device__ inline void store_fixed(const Dev& P, int i, double adx, double ady) 
 // Per-cell part of one RK stage.  EC_INT_ADVAVE is the internal-step call of ADVAVE
 // followed by ADX2D -= ADVUA (internal_step.F:387-392).
 // -------------------------------------------------------------------------------------
-template <typename R, bool LIM>
-__global__ void __launch_bounds__(128, sizeof(R) == 4 ? 8 : (LIM ? 1 : 5)) k_ext_cell(const Dev P, int iext, int K, int parts) {
+template <typename R, Edges EDGES>
+__global__ void __launch_bounds__(128, sizeof(R) == 4 ? 8 : (EDGES == kSeen ? 5 : 1)) k_ext_cell(const Dev P, int iext, int K, int parts) {
   pdl_enter();
   int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
   if (i > P.N) return;
@@ -625,7 +633,7 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 8 : (LIM ? 1 : 5)) k_ext
   }
   double xf, yf, px, py;
   if (parts & (EC_ADVAVE | EC_INT_ADVAVE)) {
-    advave_cell<R, LIM>(P, i, weti, parts & EC_WET, xf, yf, px, py);
+    advave_cell<R, EDGES>(P, i, weti, parts & EC_WET, xf, yf, px, py);
     if (P.isbce[i] == 2) {
       if (P.gcy) {  // advave_edge_gcy.F
         xf = xf + fob * P.ua[i] * P.iucp[i];
@@ -1371,9 +1379,11 @@ __device__ __forceinline__ bool grid_barrier(const Dev& P, unsigned target) {
   if (threadIdx.x == 0) {
     asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(P.bar) : "memory");
     unsigned seen = 0;
-    for (int it = 0; it < P.bar_polls && seen < target; ++it)
+    int it = 0;
+    do {
       asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(P.bar) : "memory");
-    if (seen < target || (seen & kBarStopped)) {
+    } while (seen < target && ++it < P.bar_polls);
+    if (seen < target || (seen & kBarStopped) || P.bar_polls == 0) {
       ok = 0;
       asm volatile("red.relaxed.gpu.global.or.b32 [%0], %1;" ::"l"(P.bar), "r"(kBarStopped) : "memory");
       *P.bar_err = 1;
@@ -1582,9 +1592,10 @@ __global__ void k_ext_prep(const Dev P) {
 // QDIS = QDIS*RAMP (bcond_gcn.F:645-648).
 __global__ void k_begin_step(const Dev P, int advance) {
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
+  const unsigned stopped = *P.bar & kBarStopped;  // a wait ran out: see grid_barrier
   int slot = P.ctl[0] + advance;
   P.ctl[0] = slot;
-  *P.bar = *P.bar & kBarStopped;
+  *P.bar = stopped;
   double ramp = P.sched[(size_t)slot * P.sl.len];
   for (int j = 1; j <= P.numqbc; ++j) P.qdis[j] = P.qdis0[j] * ramp;
 }
@@ -1679,7 +1690,7 @@ void launch_wet_cells(const Dev& P, cudaStream_t s, int pdl) {
 void launch_ext_cell(const Dev& P, cudaStream_t s, int iext, int K, int parts, int pdl) {
   FVG_F32_FORWARD(launch_ext_cell(P, s, iext, K, parts, pdl));
   void (*k)(const Dev, int, int, int);
-  k = per_edge(P) ? k_ext_cell<RF, true> : k_ext_cell<RF, false>;
+  k = P.limiter ? k_ext_cell<RF, kLimitedEdges> : per_edge(P) ? k_ext_cell<RF, kListed> : k_ext_cell<RF, kSeen>;
   const int b = col_threads(P, P.N, 128);
   launch_maybe_pdl(pdl, k, dim3(nblk(P.N, b)), dim3(b), s, P, iext, K, parts);
 }

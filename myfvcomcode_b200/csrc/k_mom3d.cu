@@ -255,7 +255,7 @@ __global__ void __launch_bounds__(256) k_alfa3(const Dev P) {
 
 // An edge by its own list entry (per_edge).  q: the edge's slot in the cell slot table (offsets
 // and DLTXC/DLTYC of the edge).
-template <typename R>
+template <typename R, bool LIM>
 __device__ inline EdgeFlux<R> edge_flux3(const Dev& P, size_t q, int ia, int ib, int k, R dij, bool exflux_form) {
   typedef Mesh<R> Mh;
   const R half = (R)0.5, one = (R)1.0;
@@ -274,10 +274,17 @@ __device__ inline EdgeFlux<R> edge_flux3(const Dev& P, size_t q, int ia, int ib,
   ga = load_g3<R>(P, ia, k);
   gb = load_g3<R>(P, ib, k);
   const size_t qa = C3(P, ia, k), qb = C3(P, ib, k);
-  edge_faces<R>(P.limiter, (R)U[ia], (R)U[ib], ga.ux, ga.uy, xija, yija, gb.ux, gb.uy, xijb, yijb, Mh::alfa3(P, 0), qa,
-                qb, uij1, uij2);
-  edge_faces<R>(P.limiter, (R)V[ia], (R)V[ib], ga.vx, ga.vy, xija, yija, gb.vx, gb.vy, xijb, yijb, Mh::alfa3(P, 1), qa,
-                qb, vij1, vij2);
+  if constexpr (LIM) {
+    lim_faces<R>(P.limiter, (R)U[ia], (R)U[ib], ga.ux * xija + ga.uy * yija, gb.ux * xijb + gb.uy * yijb,
+                 Mh::alfa3(P, 0)[qa], Mh::alfa3(P, 0)[qb], uij1, uij2);
+    lim_faces<R>(P.limiter, (R)V[ia], (R)V[ib], ga.vx * xija + ga.vy * yija, gb.vx * xijb + gb.vy * yijb,
+                 Mh::alfa3(P, 1)[qa], Mh::alfa3(P, 1)[qb], vij1, vij2);
+  } else {
+    uij1 = (R)U[ia] + ga.ux * xija + ga.uy * yija;
+    uij2 = (R)U[ib] + gb.ux * xijb + gb.uy * yijb;
+    vij1 = (R)V[ia] + ga.vx * xija + ga.vy * yija;
+    vij2 = (R)V[ib] + gb.vx * xijb + gb.vy * yijb;
+  }
   R uij = half * (uij1 + uij2);
   R vij = half * (vij1 + vij2);
   R viscof1 = arta * sqrt(ga.ux * ga.ux + ga.vy * ga.vy + half * ((ga.uy + ga.vx) * (ga.uy + ga.vx)));
@@ -345,7 +352,7 @@ __device__ inline void advection3d_tail(const Dev& P, int i, int k, R xr, R yr) 
 // ADVECTION_EDGE_GCN (advection_edge_gcn.F:397-708): per cell and layer, the cell's three
 // edges in ascending edge number.
 // -------------------------------------------------------------------------------------
-template <typename R>
+template <typename R, bool LIM>
 __global__ void __launch_bounds__(256) k_advection3d(const Dev P) {
   int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
   if (i > P.N) return;
@@ -363,7 +370,7 @@ __global__ void __launch_bounds__(256) k_advection3d(const Dev P) {
     if (!(P.iswetct[ia] * P.iswetc[ia] == 1 || P.iswetct[ib] * P.iswetc[ib] == 1)) continue;
     const int j1 = ci.w, j2 = P.ce_j2[q];
     R dij = (R)(0.5 * (P.dt[j1] * P.dz(j1, k) + P.dt[j2] * P.dz(j2, k)));
-    EdgeFlux<R> f = edge_flux3<R>(P, q, ia, ib, k, dij, false);
+    EdgeFlux<R> f = edge_flux3<R, LIM>(P, q, ia, ib, k, dij, false);
     R isb = (R)isbc;
     R tp = (R)((double)(float)(1 - isbc) * P.epor[i]);
     // viscous part: GCN (fxx + 3 fxx ISBC) EPOR; GCY (advection_edge_gcy.F) fxx TPA
@@ -807,7 +814,7 @@ __device__ inline void adv_uv_tail(const Dev& P, int i, int k, R xr, R yr, R vmr
 // internal barotropic pressure gradient from EGF, vertical advection, baroclinic
 // pressure gradient, Coriolis, river momentum and the explicit update to UF/VF.
 // -------------------------------------------------------------------------------------
-template <typename R>
+template <typename R, bool LIM>
 __global__ void __launch_bounds__(256) k_adv_uv(const Dev P) {
   int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
   if (i > P.N) return;
@@ -829,7 +836,7 @@ __global__ void __launch_bounds__(256) k_adv_uv(const Dev P) {
     double elij = 0.5 * (P.egf[j1] + P.egf[j2]);
     R dij = (R)(0.5 * (P.dt[j1] * P.dz(j1, k) + P.dt[j2] * P.dz(j2, k)));
     if (P.iswetct[ia] * P.iswetc[ia] == 1 || P.iswetct[ib] * P.iswetc[ib] == 1) {
-      EdgeFlux<R> f = edge_flux3<R>(P, q, ia, ib, k, dij, true);
+      EdgeFlux<R> f = edge_flux3<R, LIM>(P, q, ia, ib, k, dij, true);
       vmr = vmr + f.viscof;
       R isb = (R)isbc;
       R tp = (R)((double)(float)(1 - isbc) * P.epor[i]);
@@ -1443,7 +1450,9 @@ static void launch_mom3d(const Dev& P, cudaStream_t s) {
   Dev Q = col_shape(P, P.N, P.KBM1);
   if (per_edge(P)) {
     if (P.limiter) launch_alfa3(P, s);
-    (UV ? k_adv_uv<RF> : k_advection3d<RF>)<<<col_grid(Q, P.N, P.KBM1), Q.col_bc, 0, s>>>(Q);
+    auto k = P.limiter ? (UV ? k_adv_uv<RF, true> : k_advection3d<RF, true>)
+                       : (UV ? k_adv_uv<RF, false> : k_advection3d<RF, false>);
+    k<<<col_grid(Q, P.N, P.KBM1), Q.col_bc, 0, s>>>(Q);
     return;
   }
   if (Q.col_bc > 128) Q.col_bc = 128;  // the kernel's largest block

@@ -1188,20 +1188,19 @@ __global__ void __launch_bounds__(128) k_vdif_ts(const Dev P, int parts) {
 // OBC_TS_TYPE and the neighbour clamp, or keep T1/S1 on inflow.
 // -------------------------------------------------------------------------------------
 // One block per layer, its threads over the rivers; a node of several rivers is the last one's
-// (riv_own).
+// (riv_ts).
 __global__ void k_bcond_ts_riv(const Dev P) {
   const int k = blockIdx.x + 1;
   for (int r = threadIdx.x + 1; r <= P.numqbc; r += blockDim.x) {
-    int n1 = P.river_location == 0 ? P.inodeq[r] : P.n_icellq[r];
-    int n2 = P.river_location == 0 ? 0 : P.n_icellq[(size_t)(P.numqbc + 1) + r];
-    const int own = P.riv_own[r];
-    if (own & 1) {
-      P.tf1[N3(P, n1, k)] = P.tdis[r];
-      P.sf1[N3(P, n1, k)] = P.sdis[r];
+    const int2 n = P.riv_ts[r];
+    const double t = P.tdis[r], s = P.sdis[r];
+    if (n.x > 0) {
+      P.tf1[N3(P, n.x, k)] = t;
+      P.sf1[N3(P, n.x, k)] = s;
     }
-    if (own & 2) {
-      P.tf1[N3(P, n2, k)] = P.tdis[r];
-      P.sf1[N3(P, n2, k)] = P.sdis[r];
+    if (n.y > 0) {
+      P.tf1[N3(P, n.y, k)] = t;
+      P.sf1[N3(P, n.y, k)] = s;
     }
   }
 }
