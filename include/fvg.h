@@ -336,8 +336,8 @@ int fvg_closure_status(fvg_handle* h, int32_t* columns_on_network, int32_t* wait
                    as one resident cooperative kernel (with "compact" in use or possible);
                    0 launches every stage.  FP64 results do
                    not depend on it; fvg_get_tuning reports whether it is in use;
-   "ext_loop_polls" = most polls of a grid barrier of that kernel (default 4194304, about
-                   two seconds; 0: no wait at all); a barrier that takes more ends the
+   "ext_loop_polls" = most polls of a grid barrier of that kernel (default 4194304, a
+                   few seconds; 0: no wait at all); a barrier that takes more ends the
                    call with FVG_ERR_TIMEOUT (see fvg_run);
    "branches"     = 1 (default): up to 20 million cell-layers the independent parts of a step
                    (BAROPG beside ADVECTION; momentum, turbulence and tracers after VERTVL)

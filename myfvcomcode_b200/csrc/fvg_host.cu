@@ -29,7 +29,7 @@ namespace {
 constexpr long kBranchCells = 20000000;
 constexpr size_t kBranchShare = 16;
 
-// Most polls of a grid barrier of the resident external loop (about two seconds).  A phase
+// Most polls of a grid barrier of the resident external loop (a few seconds).  A phase
 // takes microseconds; what the wait has to outlast is a block that starts late behind the
 // kernels of other models on the card.
 constexpr int kLoopPolls = 1 << 22;

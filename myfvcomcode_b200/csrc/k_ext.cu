@@ -1341,7 +1341,8 @@ __global__ void __launch_bounds__(256, 5) k_stage_node(const Dev P, int st) {
 // Resident blocks per SM of the stage cell kernel, external mode of a step: FP64 four blocks of
 // 128 registers 2,524 us against five of 96 (spilling 100 bytes) 2,905 (200k nodes; 50k 1,024
 // against 1,122); FP32 six 923, seven 966, eight 996, five 1,005 (50k; 200k 2,302, 2,267,
-// 2,447, 2,200).
+// 2,447, 2,200).  One count serves every size: six lose 5 % of the external mode to five at
+// 200k, five lose 9 % to six at 50k, whose cells fill one round of six and not of five.
 template <typename R>
 constexpr int kStageBlocks = sizeof(R) == 4 ? 6 : 4;
 // WALK: one wave of blocks whose threads walk the cells.

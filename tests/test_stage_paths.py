@@ -1,7 +1,8 @@
 """Paths of the external loop that its other tests do not take: the launched stage kernels with
 and without evict-first loads and walking threads, the FP32-flux form in each block shape of the
-resident loop and with ghost cells, and lists longer than a thread of the loop keeps (three
-rivers at a node or a cell, three open-boundary entries of a cell)."""
+resident loop and with ghost cells, and lists longer than a thread of the loop keeps (four
+rivers at a node or a cell, three open-boundary entries of a cell), and meshes that the packed
+records do not fit."""
 import numpy as np
 import pytest
 
@@ -139,3 +140,28 @@ def test_long_lists(what):
     assert not bad, bad
     for m in models:
         m.close()
+
+
+@pytest.mark.parametrize("metric", ["DLTXC", "XIJC", "DLTYE", "EPOR"])
+def test_metrics_of_their_own_take_the_general_stages(metric):
+    # a mesh whose edge metrics are not those of its coordinates, or whose masks are not 0 or 1
+    from myfvcomcode_b200 import cases
+    from myfvcomcode_b200.engine import Fvcom
+    from tests.test_parity_gpu import routine_failures
+    case = cases.estuary_channel(nx=24, ny=6, kb=6, lx=4800.0, ly=1200.0, IRAMP=10)
+    a = case["grid"][metric]
+    a[50] = 0.5 if metric == "EPOR" else a[50] + 1e-3
+    m = Fvcom(case)
+    assert m.get_tuning("ext_loop") == 0
+    m.set_precision("fp32flux")
+    assert m.get_tuning("compact") == 0
+    m.close()
+    failures = routine_failures(case, 2)
+    assert not failures, failures
+    from oracle.oracle import Oracle
+    x, y = Fvcom(case), Oracle(case)
+    x.run(5)
+    y.run(5)
+    bad = parity.compare(x, y, ["el", "ua", "va", "u", "v", "t1", "s1"], rtol=1e-9)
+    assert not bad, bad
+    x.close()
