@@ -328,8 +328,9 @@ __global__ void __launch_bounds__(256) k_mlp_adam(float* par, float* m, float* v
 // FP32 forward pass (the reference of the tensor-core kernel).  A block of 128 threads takes
 // tiles of 128 samples; the layers are products from shared memory, eight samples by eight
 // units per thread, so that four loads serve 64 multiply-adds.  One thread per sample read
-// every weight from L1 for each multiply-add: 698 us for 1,000,003 samples; the arithmetic
-// (4,800 multiply-adds and 128 tanh per sample) bounds it now.
+// every weight from L1 for each multiply-add: 698 us for 1,000,003 samples against 367.  Shared
+// memory bounds it now (82 % of its wavefronts, more than half of them bank conflicts of the
+// stores of h and the loads of W; the FMA pipe at 48 %).
 // -------------------------------------------------------------------------------------
 constexpr int FR = 128;      // samples per tile, threads per block
 constexpr int FD = FR + 4;   // stride of the unit-major activations
