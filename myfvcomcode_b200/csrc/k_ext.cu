@@ -397,9 +397,10 @@ __device__ inline bool wet_other(const Dev& P, bool judge, int i, int s, int o, 
   return P.iswetce[o] * P.iswetc[o] == 1;
 }
 
-// ADVAVE_EDGE_GCN for one cell (advave_edge_gcn.F:115-1003), over the cell's slot table.  EDGES:
-// the edges as the cell sees them, or each by its own list entry (per_edge), plain or limited.  The edge fluxes are evaluated in R; the surface-slope pressure
-// gradient PSTX/PSTY stays FP64.
+// ADVAVE_EDGE_GCN for one cell (advave_edge_gcn.F:115-1003), over the cell's slot table.
+// EDGES: the edges as the cell sees them, or each by its own list entry (per_edge), plain or
+// limited.  The edge fluxes are evaluated in R; the surface-slope pressure gradient PSTX/PSTY
+// stays FP64.
 enum Edges { kSeen, kListed, kLimitedEdges };
 template <typename R, Edges EDGES>
 __device__ inline void advave_cell(const Dev& P, int i, int weti, bool judge, double& xfo, double& yfo, double& px,

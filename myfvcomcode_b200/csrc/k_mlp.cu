@@ -31,18 +31,19 @@ constexpr int OW1 = 0, OB1 = OW1 + MH * MI, OW2 = OB1 + MH, OB2 = OW2 + MH * MH,
 // GELU in its tanh form, 0.5 z (1 + tanh(u)), u = c (z + 0.044715 z^3), c = sqrt(2/pi), as
 // z * s with s = 0.5 (1 + tanh(u)) = 1 / (1 + exp(-2u)), which does not cancel for negative z
 // and costs half of tanhf's instructions (the function took nearly half of the forward pass);
-// and its derivative s + 2 z s (1 - s) u', where 1 - s is exp(-2u) s for s near 1, which does
-// not cancel (1 - s lost up to 2e-6 of the derivative for z of 4 to 6).  A batch's gradient
-// against 64 bits, 24 seeds each, over tanhf's form: 1 sample 0.93, 33 0.94, 1,000 0.82 of its
-// error (1.08, 1.07 and 0.88 with 1 - s); the forward pass 0.97.
+// and its derivative s + 2 z s (1 - s) u'.  1 - s is taken as exp(-2u) s, which does not cancel
+// (1 - s lost up to 2e-6 of the derivative for z of 4 to 6); the exponential is held finite, so
+// that its product with s = 0 is a number.  A batch's gradient against 64 bits, 24 seeds each,
+// over tanhf's form: 1 sample 0.93, 33 0.94, 1,000 0.82 of its error (1.08, 1.07 and 0.88 with
+// 1 - s); the forward pass 0.97.
 constexpr float kGc = 0.79788456080286536f, kGa = 0.044715f;
 __device__ __forceinline__ float gelu_e(float z, float z2) {
   return __expf(z * fmaf(-2.0f * kGc * kGa, z2, -2.0f * kGc));
 }
 __device__ __forceinline__ float gelu(float z) { return z * __fdividef(1.0f, 1.0f + gelu_e(z, z * z)); }
 __device__ __forceinline__ float gelu2(float z, float& d) {
-  const float z2 = z * z, e = gelu_e(z, z2), s = __fdividef(1.0f, 1.0f + e), w = s < 0.5f ? 1.0f - s : e * s;
-  d = fmaf(2.0f * z * s * w, kGc * fmaf(3.0f * kGa, z2, 1.0f), s);
+  const float z2 = z * z, e = fminf(gelu_e(z, z2), 3.4e38f), s = __fdividef(1.0f, 1.0f + e);
+  d = fmaf(2.0f * z * s * (e * s), kGc * fmaf(3.0f * kGa, z2, 1.0f), s);
   return z * s;
 }
 
